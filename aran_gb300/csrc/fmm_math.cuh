@@ -101,8 +101,36 @@ __host__ __device__ constexpr int m2l_lane_stride(int p) {
 __host__ __device__ constexpr int m2l_lane_vpre(int p, int m) {
   return m2l_lane_vtail(p) - m2l_lane_vtail(p - m);
 }
-// orders with a lane-parallel M2L kernel
+// orders with lane-parallel M2M / L2L kernels
 __host__ __device__ constexpr bool m2l_lane_order(int p) { return p == 4 || p == 8 || p == 12; }
+
+// Stream layout of the lane-parallel M2L kernel with the translation along z
+// in a scaled frame.  With A(l, m) = 4^l / sqrt((l-m)! (l+m)!) the vertical
+// factors are
+//   V(j, m, n) = (-1)^{j+m} (beta_j A(j, m)) (A(n, m) / beta_n) H(j + n) s^{j+n} r^{-(j+n+1)},
+//   H(k) = k! / 4^k, s = +-1 the side of the offset,
+// so with the A, beta, sign and radial factors folded into the rotation
+// blocks the translation's factors H depend on j + n alone and are constants
+// of the code.  Each degree's block is scaled on both sides by A, which keeps
+// it symmetric; the kernel divides its sources and its sums by A.  (4^l keeps
+// A and H within 1e-8 .. 1e16 up to order 16.)  One block per offset:
+//  * cos(m phi), m = 0..p, padded to a multiple of four, then sin(m phi) alike;
+//  * the forward lower triangles, degree l times A A s^l r^-l / beta_l, in
+//    groups of four like above;
+//  * the backward lower triangles, column m of degree l times
+//    (-1)^{l+m} A A beta_l s^l r^-(l+1), in the same order.
+__host__ __device__ constexpr int m2l_hk_cp(int p) { return (p + 4) & ~3; }
+__host__ __device__ constexpr int m2l_hk_f(int p) { return 2 * m2l_hk_cp(p); }
+__host__ __device__ constexpr int m2l_hk_b(int p) {
+  return m2l_hk_f(p) + 8 * ((m2l_lane_nf(p) + 3) / 4);
+}
+__host__ __device__ constexpr int m2l_hk_stride(int p) {
+  return m2l_hk_b(p) + 8 * ((m2l_lane_nb(p) + 3) / 4);
+}
+// orders with a lane-parallel M2L kernel
+__host__ __device__ constexpr bool m2l_hk_order(int p) {
+  return p >= 4 && p <= 16 && (p & 1) == 0;
+}
 
 FMM_HD int sq_off(int l) { return (l * (l + 1) * (2 * l + 1)) / 6; }  // sum_{i<l} (i+1)^2
 FMM_HD int sq_size(int L) { return sq_off(L); }

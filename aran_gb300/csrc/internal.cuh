@@ -144,7 +144,7 @@ struct OpTables {
   DBuf<T> vl;       // tri(p+1)*(p+1) (L2L vertical, 2^-l folded)
   DBuf<T> gz, gm;   // gradient coefficients
   DBuf<T> dir_m2l, dir_m2m, dir_l2l;
-  DBuf<T> dir_lanes; // lane-parallel M2L stream tables (FP32, m2l_lane_order)
+  DBuf<T> dir_lanes; // lane-parallel M2L stream tables (FP32, m2l_hk_order)
   DBuf<float> oct_lanes[2];   // lane-parallel M2M / L2L octant-0 stream tables (FP32)
   DBuf<uint8_t> lm; // (l,m) of coefficient index, 2*tri(p+1)
 };
@@ -223,6 +223,8 @@ struct AranGpuSolver3d {
   aran::DBuf<float> tc_tab;
   aran::DBuf<int8_t> tc_dvec;
   int tc_p = -1;
+  // sums of the parts of a split lane-parallel M2L pass
+  aran::DBuf<float> m2l_part;
   aran::DBuf<int> sys_off;
   aran::DBuf<double> sys_box;
   std::vector<int> h_sys_off;
@@ -256,6 +258,10 @@ void kkylin_pass(AranGpuSolver3d *s, int stage);
 void launch_m2l(AranGpuSolver3d *s, bool fp64, int first, int count, cudaStream_t st);
 bool launch_m2l_lanes(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,
                       const cplx<float> *mult, cplx<float> *loc, cudaStream_t st);
+bool launch_m2l_lanes_b(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,
+                        const cplx<float> *mult, cplx<float> *loc, cudaStream_t st);
+bool launch_m2l_lanes_c(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,
+                        const cplx<float> *mult, cplx<float> *loc, cudaStream_t st);
 // m2m_lanes.cu: lane-parallel FP32 M2M (parents of depths dhi down to dlo)
 // and L2L (children of depths dlo up to dhi, from depth 3) at the orders
 // m2l_lane_order accepts; false leaves the pass to passes.cu's kernels

@@ -799,7 +799,7 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   const int nm = tri(p), nl = tri(p + 1);
   const bool field = s->cfg.field != 0;
   const bool kk = s->cfg.flavour == ARAN_FLAVOUR_KKYLIN;
-  multb.reserve((size_t)t.nnodes * nm * 2);
+  multb.reserve((size_t)t.nnodes * nm * 2 + 2);   // the M2L copies whole 16-byte units
   locb.reserve((size_t)t.nnodes * nl * 2);
   cplx<T> *mult = reinterpret_cast<cplx<T> *>(multb.ptr);
   cplx<T> *loc = reinterpret_cast<cplx<T> *>(locb.ptr);

@@ -124,55 +124,55 @@ __global__ void k_m2l_vertical(int p, int ndir, int stride, int rp_off, int vv_o
   tb[vv_off + m2l_vrow_off(p, n) + k] = vt[tri(l, m) * p + n] * tb[rp_off + l + n + 1];
 }
 
-// lane-parallel M2L stream tables (layout: m2l_lane_* in fmm_math.cuh),
-// gathered from the FP32 offset tables: same factors, consumption order
-__global__ void k_m2l_lane_tables(int p, int ndir, const float *__restrict__ src, DirLayout D,
+// A(l, m) = 4^l / sqrt((l-m)! (l+m)!), the frame of the lane-parallel M2L
+__device__ double hk_scale(int l, int m) {
+  double f = 1.;
+  for (int k = 2; k <= l - m; ++k) f *= k;
+  for (int k = 2; k <= l + m; ++k) f *= k;
+  return ldexp(1., 2 * l) / sqrt(f);
+}
+
+// lane-parallel M2L stream tables (layout: m2l_hk_* in fmm_math.cuh) from
+// the offset tables: same factors, scaled frame, consumption order
+template <typename T>
+__global__ void k_m2l_lane_tables(int p, int ndir, double ex, double ey, double ez,
+                                  const T *__restrict__ src, DirLayout D,
                                   float *__restrict__ dst) {
-  const int stride = m2l_lane_stride(p);
+  const int stride = m2l_hk_stride(p);
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)ndir * stride) return;
   const int d = (int)(i / stride), e = (int)(i % stride);
-  const float *s = src + (size_t)d * D.stride;
-  const int F = m2l_lane_f(p), V = m2l_lane_v(p), B = m2l_lane_b(p);
+  const T *s = src + (size_t)d * D.stride;
+  const int CP = m2l_hk_cp(p), F = m2l_hk_f(p), B = m2l_hk_b(p);
+  // length of the offset and the side it points to
+  const double dx = (d % 7 - 3) * ex, dy = ((d / 7) % 7 - 3) * ey, dz = (d / 49 - 3) * ez;
+  const double r = sqrt(dx * dx + dy * dy + dz * dz);
+  if (!(r > 0.)) {
+    dst[i] = 0.f;
+    return;
+  }
+  const double sr = (dz < 0. ? -1. : 1.) / r;
   // q-th float of a grouped rotation stream: term 4 (q / 8) + q % 4, part
-  // (q / 4) % 2; term t = tet(l) + m'(m'+1)/2 + m is row m', column m of
-  // degree l
+  // (q / 4) % 2
   auto rot = [&](int q, int nterm, int nc, int base, bool back) -> float {
     const int t = 4 * (q >> 3) + (q & 3), part = (q >> 2) & 1;
     if (t >= nterm) return 0.f;
     int l = 0;
     while (m2l_lane_tet(l + 1) <= t) ++l;
-    int r = t - m2l_lane_tet(l), mp = 0;
-    while (tri(mp + 1) <= r) ++mp;
-    const int m = r - tri(mp);
-    const double f = back ? (((l + m) & 1) ? -beta_l(l) : beta_l(l)) : 1. / beta_l(l);
+    int rr = t - m2l_lane_tet(l), mp = 0;
+    while (tri(mp + 1) <= rr) ++mp;
+    const int m = rr - tri(mp);
+    double f = hk_scale(l, m) * hk_scale(l, mp);
+    for (int k = 0; k < l; ++k) f *= sr;
+    f *= back ? (((l + m) & 1) ? -beta_l(l) : beta_l(l)) / r : 1. / beta_l(l);
     return (float)(f * s[base + 2 * (m2l_plane_off(nc, m) + tri(l, mp) - tri(m)) + part]);
   };
   float v = 0.f;
   if (e < F) {
-    if (e < 2 * (p + 1)) v = s[D.ph + e];
-  } else if (e < V) {
-    v = rot(e - F, m2l_lane_nf(p), tri(p), D.ef, false);
+    const int m = e < CP ? e : e - CP;
+    if (m <= p) v = (float)s[D.ph + 2 * m + (e < CP ? 0 : 1)];
   } else if (e < B) {
-    const int t = e - V;
-    if (t < m2l_lane_nv(p)) {
-      int m = 0;
-      while (m2l_lane_vpre(p, m + 1) <= t) ++m;
-      const int r = t - m2l_lane_vpre(p, m), k = p - m;
-      int j, n;
-      if (r < tri(k)) {          // lower triangle: row j, column n <= j
-        int jj = 0;
-        while (tri(jj + 1) <= r) ++jj;
-        j = m + jj;
-        n = m + (r - tri(jj));
-      } else {                   // row j = p
-        j = p;
-        n = m + (r - tri(k));
-      }
-      const int slot = m * (p + 1) - m * (m - 1) / 2 + (j - m);   // m-major slot of (j, m)
-      const double sg = ((j + m) & 1) ? -1. : 1.;
-      v = (float)(sg * beta_l(n) / beta_l(j) * s[D.vv + m2l_vrow_off(p, n) + slot]);
-    }
+    v = rot(e - F, m2l_lane_nf(p), tri(p), D.ef, false);
   } else {
     v = rot(e - B, m2l_lane_nb(p), tri(p + 1), D.ei, true);
   }
@@ -300,12 +300,11 @@ void build_tables_t(AranGpuSolver3d *s, OpTables<T> &tb, cudaStream_t st) {
       k_m2l_vertical<T><<<ceil_div(ne, 256), 256, 0, st>>>(p, ndir, L.stride, L.rp, L.vv,
                                                             tb.vt.ptr, dst.ptr);
       ACHECK(cudaGetLastError());
-      if (sizeof(T) == 4 && m2l_lane_order(p)) {
-        const int64_t nl = (int64_t)ndir * m2l_lane_stride(p);
+      if (sizeof(T) == 4 && m2l_hk_order(p)) {
+        const int64_t nl = (int64_t)ndir * m2l_hk_stride(p);
         tb.dir_lanes.reserve(nl);
-        k_m2l_lane_tables<<<ceil_div(nl, 256), 256, 0, st>>>(
-            p, ndir, reinterpret_cast<const float *>(dst.ptr), L,
-            reinterpret_cast<float *>(tb.dir_lanes.ptr));
+        k_m2l_lane_tables<T><<<ceil_div(nl, 256), 256, 0, st>>>(
+            p, ndir, ex, ey, ez, dst.ptr, L, reinterpret_cast<float *>(tb.dir_lanes.ptr));
         ACHECK(cudaGetLastError());
       }
     }

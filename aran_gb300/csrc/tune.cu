@@ -234,7 +234,11 @@ int aran_gpu_autotune3d(const AranGpuConfig3d *cfg, int64_t n, const double *xyz
       continue;
     }
     if (m2l_lane_order(cfg->order)) cands.push_back({m, ARAN_M2L_LANES, 0, 0});
-    cands.push_back({m, ARAN_M2L_SIBLING, 0, 0});
+    // the library's own choice; at the other lane-parallel orders that is
+    // their lane kernel
+    const int own = m2l_hk_order(cfg->order) && !m2l_lane_order(cfg->order) ? ARAN_M2L_AUTO
+                                                                            : ARAN_M2L_SIBLING;
+    cands.push_back({m, own, 0, 0});
     int nst = 0, g = 0;
     const int nc = m2l_sibling_configs(cfg->order, &nst, &g, 0);
     for (int k = 0; k < nc; ++k) {

@@ -130,6 +130,9 @@ def m2l_kernel_name(precision: str, p: int, choice: str) -> str:
     """The M2L kernel a solve runs: choice is ARAN_M2L_KERNEL ("lanes",
     "sibling", "tc" or empty); a kernel that does not serve the order or the
     precision hands over to the next in tc, lanes, sibling."""
+    if precision == "mixed" and p in (6, 10, 14, 16) and choice != "sibling":
+        return (f"k_m2l_sibling_lanes<{p}> (rotate M2L, FP32 lane pairs, all levels, one launch "
+                "or one and its parts' sum)")
     if precision != "mixed" or p not in (4, 8, 12) or choice == "sibling":
         return "k_m2l_sibling (rotate M2L, all levels, one launch)"
     if choice == "tc" and p in (8, 12):
