@@ -7,13 +7,11 @@
 // sources directly (both sides of a pair are evaluated by their own targets
 // instead of the symmetric update).
 //
-// Work decomposition: one block per target leaf; threads-per-target (tpt)
-// grows as the leaf shrinks (n <= 8: 16, <= 16: 8, <= 32: 4, <= 64: 2,
-// else 1), and a target's tpt threads take its near *leaves* round-robin so
-// the per-leaf set-up is amortised over the leaf's points.  Near ranges of
-// more than kBigRange points (a coarse leaf next to a deep subtree, common in
-// clustered sets) are cut into leaf-aligned chunks processed by extra blocks
-// that accumulate atomically.
+// Work decomposition: mixed precision takes a warp per target leaf
+// (k_p2p_warp), FP64 a block (k_p2p64).  Near ranges of more than kBigRange
+// points (a coarse leaf next to a deep subtree, common in clustered sets) are
+// cut into leaf-aligned chunks processed by extra blocks that accumulate
+// atomically.
 //
 // Mixed precision: positions are FP32 relative to their leaf centre, the
 // centre difference comes from FP32 hi+lo centre pairs, per-source-leaf FP32
@@ -95,43 +93,32 @@ __global__ void k_big_items(const int *__restrict__ heavy, int nleaves,
     items[coff + i] = make_int4(L, boundary(i), boundary(i + 1), 0);
 }
 
-template <typename T, bool FIELD, bool MIXED, bool BIG>
-__global__ void __launch_bounds__(128, 10) k_p2p(
-    const int4 *__restrict__ items, const int *__restrict__ near_off,
-    const int *__restrict__ near_rng, const int2 *__restrict__ be, const float4 *__restrict__ chi,
+// one chunk of a heavy near range of a mixed solve: threads-per-target (tpt)
+// grows as the leaf shrinks (n <= 8: 16, <= 16: 8, <= 32: 4, <= 64: 2, else
+// 1), and a target's tpt threads take the chunk's leaves round-robin (tiny
+// target leaves) or split every source leaf's points
+template <bool FIELD>
+__global__ void __launch_bounds__(128, 10) k_p2p_chunk(
+    const int4 *__restrict__ items, const int2 *__restrict__ be, const float4 *__restrict__ chi,
     const float4 *__restrict__ clo, const double *__restrict__ sx, const double *__restrict__ sy,
-    const double *__restrict__ sz, const double *__restrict__ sq,
-    const real4<float> *__restrict__ rel32, double *__restrict__ acc_pot,
-    double *__restrict__ acc_fld) {
-  int L, ia = 0, ib = 0;
-  if (BIG) {
-    int4 it = items[blockIdx.x];
-    L = it.x;
-    ia = it.y;
-    ib = it.z;
-  } else {
-    L = blockIdx.x;
-  }
+    const double *__restrict__ sz, const real4<float> *__restrict__ rel32,
+    double *__restrict__ acc_pot, double *__restrict__ acc_fld) {
+  const int4 it = items[blockIdx.x];
+  const int L = it.x, ia = it.y, ib = it.z;
   const int2 tbe = be[L];
   const int b = tbe.x, nt = tbe.y - tbe.x;
   const int tpt = nt <= 8 ? 16 : (nt <= 16 ? 8 : (nt <= 32 ? 4 : (nt <= 64 ? 2 : 1)));
   const int gsz = blockDim.x / tpt;
   const int sub = threadIdx.x % tpt;
   const bool leaf_strided = nt <= 8;
-  const int r0 = near_off[L], r1 = near_off[L + 1];
-  float4 tch = make_float4(0.f, 0.f, 0.f, 0.f), tcl = tch;
-  if (MIXED) {
-    tch = chi[L];
-    tcl = clo[L];
-  }
+  const float4 tch = chi[L], tcl = clo[L];
   for (int tb = 0; tb < nt; tb += gsz) {
     const int ti = tb + threadIdx.x / tpt;
     const bool active = ti < nt;
     if (!__any_sync(kFull, active)) continue;   // a warp with no target of this pass
     const int t = b + (active ? ti : 0);
-    double pot = 0, fx = 0, fy = 0, fz = 0;
-    // mixed: per-source-leaf FP32 sums are added with Kahan compensation in
-    // FP32 (FP64 adds per leaf would occupy the FP64 pipe, 1/64 of FP32)
+    // per-source-leaf FP32 sums are added with Kahan compensation in FP32
+    // (FP64 adds per leaf would occupy the FP64 pipe, 1/64 of FP32)
     float ks0 = 0.f, ks1 = 0.f, ks2 = 0.f, ks3 = 0.f;
     float kc0 = 0.f, kc1 = 0.f, kc2 = 0.f, kc3 = 0.f;
     auto kahan = [](float &sum, float &comp, float v) {
@@ -141,124 +128,186 @@ __global__ void __launch_bounds__(128, 10) k_p2p(
       sum = t2;
     };
     const double tx64 = sx[t], ty64 = sy[t], tz64 = sz[t];
-    float tx = 0.f, ty = 0.f, tz = 0.f;
-    if (MIXED) {
-      real4<float> r = rel32[t];
-      tx = r.x; ty = r.y; tz = r.z;
-    }
-    int kleaf = 0;
-    // tiny target leaves: a target's threads take whole source leaves in turn;
-    // otherwise they split every source leaf's points (keeps the warp converged)
+    const real4<float> r = rel32[t];
     auto do_leaf = [&](int lf, int j0, int js) {
       const int2 sbe = be[lf];
-      if (MIXED) {
-        const float4 sh = chi[lf], sl = clo[lf];
-        // target position relative to the source leaf centre
-        const float ox = tx - ((sh.x - tch.x) + (sl.x - tcl.x));
-        const float oy = ty - ((sh.y - tch.y) + (sl.y - tcl.y));
-        const float oz = tz - ((sh.z - tch.z) + (sl.z - tcl.z));
-        const float thr2 = tch.w;
-        float p0 = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;
+      const float4 sh = chi[lf], sl = clo[lf];
+      // target position relative to the source leaf centre
+      const float ox = r.x - ((sh.x - tch.x) + (sl.x - tcl.x));
+      const float oy = r.y - ((sh.y - tch.y) + (sl.y - tcl.y));
+      const float oz = r.z - ((sh.z - tch.z) + (sl.z - tcl.z));
+      const float thr2 = tch.w;
+      float p0 = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;
 #pragma unroll 4
-        for (int j = sbe.x + j0; j < sbe.y; j += js) {
-          const real4<float> sj = rel32[j];
-          float dx = ox - sj.x, dy = oy - sj.y, dz = oz - sj.z;
-          float r2 = dx * dx + dy * dy + dz * dz;
-          if (__builtin_expect(r2 < thr2, 0)) {
-            if (j == t) {
-              r2 = 0.f;
-            } else {
-              // close pair: difference from the FP64 positions
-              dx = (float)(tx64 - sx[j]);
-              dy = (float)(ty64 - sy[j]);
-              dz = (float)(tz64 - sz[j]);
-              r2 = dx * dx + dy * dy + dz * dz;
-            }
-          }
-          const bool ok = FIELD ? (r2 > 1e-10f) : (r2 > 0.f);
-          const float inv = ok ? rsqrt_ftz(r2) : 0.f;
-          const float qi = sj.q * inv;
-          p0 += qi;
-          if (FIELD) {
-            const float q3 = qi * inv * inv;
-            f0 -= q3 * dx;
-            f1 -= q3 * dy;
-            f2 -= q3 * dz;
+      for (int j = sbe.x + j0; j < sbe.y; j += js) {
+        const real4<float> sj = rel32[j];
+        float dx = ox - sj.x, dy = oy - sj.y, dz = oz - sj.z;
+        float r2 = dx * dx + dy * dy + dz * dz;
+        if (__builtin_expect(r2 < thr2, 0)) {
+          if (j == t) {
+            r2 = 0.f;
+          } else {
+            // close pair: difference from the FP64 positions
+            dx = (float)(tx64 - sx[j]);
+            dy = (float)(ty64 - sy[j]);
+            dz = (float)(tz64 - sz[j]);
+            r2 = dx * dx + dy * dy + dz * dz;
           }
         }
-        kahan(ks0, kc0, p0);
+        const bool ok = FIELD ? (r2 > 1e-10f) : (r2 > 0.f);
+        const float inv = ok ? rsqrt_ftz(r2) : 0.f;
+        const float qi = sj.q * inv;
+        p0 += qi;
         if (FIELD) {
-          kahan(ks1, kc1, f0);
-          kahan(ks2, kc2, f1);
-          kahan(ks3, kc3, f2);
+          const float q3 = qi * inv * inv;
+          f0 -= q3 * dx;
+          f1 -= q3 * dy;
+          f2 -= q3 * dz;
         }
-      } else {
-        for (int j = sbe.x + j0; j < sbe.y; j += js) {
-          const double dx = tx64 - sx[j], dy = ty64 - sy[j], dz = tz64 - sz[j];
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          // the point itself and coincident points: r2 == 0, skipped
-          const bool ok = FIELD ? (r2 > 1e-10) : (r2 > 0.);
-          const double inv = ok ? rsqrt(r2) : 0.;
-          const double qi = sq[j] * inv;
-          pot += qi;
-          if (FIELD) {
-            const double q3 = qi * inv * inv;
-            fx -= q3 * dx;
-            fy -= q3 * dy;
-            fz -= q3 * dz;
-          }
-        }
+      }
+      kahan(ks0, kc0, p0);
+      if (FIELD) {
+        kahan(ks1, kc1, f0);
+        kahan(ks2, kc2, f1);
+        kahan(ks3, kc3, f2);
       }
     };
-    if (BIG) {
-      if (leaf_strided)
-        for (int lf = ia + sub; lf < ib; lf += tpt) do_leaf(lf, 0, 1);
-      else
-        for (int lf = ia; lf < ib; ++lf) do_leaf(lf, sub, tpt);
-    } else {
-      for (int rr = r0; rr < r1; ++rr) {
-        const int la = near_rng[2 * rr], lb = near_rng[2 * rr + 1];
-        if (lb <= la) continue;
-        if (rng_count(be, la, lb) > kBigRange) continue;  // chunked by the BIG pass
-        if (leaf_strided) {
-          for (int lf = la; lf < lb; ++lf, ++kleaf)
-            if (kleaf % tpt == sub) do_leaf(lf, 0, 1);
-        } else {
-          for (int lf = la; lf < lb; ++lf) do_leaf(lf, sub, tpt);
+    if (leaf_strided)
+      for (int lf = ia + sub; lf < ib; lf += tpt) do_leaf(lf, 0, 1);
+    else
+      for (int lf = ia; lf < ib; ++lf) do_leaf(lf, sub, tpt);
+    double v[4] = {(double)ks0 - (double)kc0, (double)ks1 - (double)kc1,
+                   (double)ks2 - (double)kc2, (double)ks3 - (double)kc3};
+    for (int o = 1; o < tpt; o <<= 1)
+#pragma unroll
+      for (int c = 0; c < (FIELD ? 4 : 1); ++c) v[c] += __shfl_xor_sync(kFull, v[c], o);
+    if (active && sub == 0) {
+      atomicAdd(&acc_pot[t], v[0]);
+      if (FIELD)
+        for (int c = 0; c < 3; ++c) atomicAdd(&acc_fld[3 * (size_t)t + c], v[1 + c]);
+    }
+  }
+}
+
+// 1/sqrt(x) in FP64 from the hardware approximation's upper word y0 (20
+// significant bits, so y0^2 is exact) by one third-order Householder step,
+// y0 + y0 e (1/2 + 3/8 e) with e = 1 - x y0^2 rounded once: five FP64
+// operations, within an ulp of the correctly rounded value.  Outside the
+// normal range's middle the library function takes over.
+__device__ __forceinline__ double rsqrt_h3(double x) {
+  double a;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(a) : "d"(x));
+  const double y0 = __hiloint2double(__double2hiint(a), 0);
+  const double e = fma(-x, y0 * y0, 1.0);
+  return fma(y0, e * fma(e, 0.375, 0.5), y0);
+}
+
+// FP64 near field, a block of 128 threads per target leaf (BIG: per chunk of
+// a heavy range).  The FP64 pipe takes half a lane per cycle and scheduler,
+// so its instructions times idle lanes are the whole cost and index
+// arithmetic is free: a leaf of n targets gets floor(128 / n) threads per
+// target, which stride over the concatenation of the leaf's near ranges (the
+// sorted particles of a range lie side by side), so all lanes but a few are
+// busy to the last source; the field takes 18 FP64 operations a pair.
+// Measured on GB300, 200k Plummer particles (leaf 64, 5.9e8 directed pairs):
+// 16.3 ms and 8.0 ms for the chunks, the FP64 pipe active 88 % of the SMs'
+// active cycles; the whole FP64 solve of order 12 went from 69.5 to 54.8 ms
+// against 16, 8, 4, .. threads per target by powers of two (56 % of the
+// lanes at 18 points a leaf) and the library's reciprocal square root.
+template <bool FIELD, bool BIG>
+__global__ void __launch_bounds__(128, 8) k_p2p64(
+    const int4 *__restrict__ items, const int *__restrict__ near_off,
+    const int *__restrict__ near_rng, const int2 *__restrict__ be,
+    const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
+    const double *__restrict__ sq, double *__restrict__ acc_pot, double *__restrict__ acc_fld) {
+  constexpr int NV = FIELD ? 4 : 1;
+  __shared__ double red[NV][128];
+  int L = blockIdx.x, ia = 0, ib = 0;
+  if (BIG) {
+    const int4 it = items[blockIdx.x];
+    L = it.x;
+    ia = it.y;
+    ib = it.z;
+  }
+  const int2 tbe = be[L];
+  const int nt = tbe.y - tbe.x;
+  const int r0 = BIG ? 0 : near_off[L], r1 = BIG ? 1 : near_off[L + 1];
+  const long long guard = __double_as_longlong(FIELD ? 1e-10 : 0.);
+  for (int tb = 0; tb < nt; tb += 128) {
+    const int rem = min(nt - tb, 128);
+    const int s = 128 / rem;                  // threads per target
+    const int ti = threadIdx.x / s, sub = threadIdx.x - ti * s;
+    const bool active = ti < rem;
+    const int t = tbe.x + tb + (active ? ti : 0);
+    double v[NV];
+#pragma unroll
+    for (int c = 0; c < NV; ++c) v[c] = 0.;
+    if (active) {
+      const double tx = sx[t], ty = sy[t], tz = sz[t];
+      // source j of the concatenated ranges; je the end of its range
+      int rr = r0 - 1, je = 0, j = sub;
+      auto advance = [&]() -> bool {   // j counts past je: into the next ranges
+        while (j >= je) {
+          if (++rr >= r1) return false;
+          int la, lb;
+          if (BIG) {
+            la = ia;
+            lb = ib;
+          } else {
+            la = near_rng[2 * rr];
+            lb = near_rng[2 * rr + 1];
+          }
+          if (lb <= la) continue;
+          const int b0 = be[la].x, e0 = be[lb - 1].y;
+          if (!BIG && e0 - b0 > kBigRange) continue;   // chunked by the BIG pass
+          j += b0 - je;
+          je = e0;
         }
+        return true;
+      };
+      while (advance()) {
+        const double dx = tx - sx[j], dy = ty - sy[j], dz = tz - sz[j];
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        // the point itself and coincident points: r2 == 0, skipped (r2 >= 0:
+        // its bits order like its value)
+        const long long bits = __double_as_longlong(r2);
+        if (bits > guard) {
+          const unsigned ex = (unsigned)(bits >> 52);
+          double inv = rsqrt_h3(r2);
+          if (ex - 23u > 2000u) inv = rsqrt(r2);
+          const double qi = sq[j] * inv;
+          v[0] += qi;
+          if (FIELD) {
+            const double q3 = qi * (inv * inv);
+            v[NV > 1 ? 1 : 0] -= q3 * dx;
+            v[NV > 1 ? 2 : 0] -= q3 * dy;
+            v[NV > 1 ? 3 : 0] -= q3 * dz;
+          }
+        }
+        j += s;
       }
     }
-    if (MIXED) {
-      pot = (double)ks0 - (double)kc0;
-      fx = (double)ks1 - (double)kc1;
-      fy = (double)ks2 - (double)kc2;
-      fz = (double)ks3 - (double)kc3;
-    }
-    for (int o = 1; o < tpt; o <<= 1) {
-      pot += __shfl_xor_sync(kFull, pot, o);
-      if (FIELD) {
-        fx += __shfl_xor_sync(kFull, fx, o);
-        fy += __shfl_xor_sync(kFull, fy, o);
-        fz += __shfl_xor_sync(kFull, fz, o);
-      }
+    // the s sums of a target, halving
+#pragma unroll
+    for (int c = 0; c < NV; ++c) red[c][threadIdx.x] = v[c];
+    __syncthreads();
+    int o = 1;
+    while (2 * o < s) o *= 2;
+    for (; o > 0 && s > 1; o >>= 1) {
+      if (active && sub < o && sub + o < s)
+#pragma unroll
+        for (int c = 0; c < NV; ++c) red[c][threadIdx.x] += red[c][threadIdx.x + o];
+      __syncthreads();
     }
     if (active && sub == 0) {
-      if (BIG) {
-        atomicAdd(&acc_pot[t], pot);
-        if (FIELD) {
-          atomicAdd(&acc_fld[3 * (size_t)t], fx);
-          atomicAdd(&acc_fld[3 * (size_t)t + 1], fy);
-          atomicAdd(&acc_fld[3 * (size_t)t + 2], fz);
-        }
-      } else {
-        acc_pot[t] = pot;
-        if (FIELD) {
-          acc_fld[3 * (size_t)t] = fx;
-          acc_fld[3 * (size_t)t + 1] = fy;
-          acc_fld[3 * (size_t)t + 2] = fz;
-        }
+#pragma unroll
+      for (int c = 0; c < NV; ++c) {
+        double *dst = c == 0 ? &acc_pot[t] : &acc_fld[3 * (size_t)t + (c - 1)];
+        if (BIG) atomicAdd(dst, red[c][threadIdx.x]);
+        else *dst = red[c][threadIdx.x];
       }
     }
+    __syncthreads();
   }
 }
 
@@ -413,31 +462,30 @@ __global__ void __launch_bounds__(128, 8) k_p2p_warp(
   else body(std::integral_constant<int, 1>{});
 }
 
-template <bool FIELD, bool MIXED, bool BIG>
-void launch_one(AranGpuSolver3d *s, int grid, cudaStream_t st) {
+template <bool FIELD>
+void launch_mixed(AranGpuSolver3d *s, cudaStream_t st) {
   DevTree &t = s->tree;
-  using T = typename std::conditional<MIXED, float, double>::type;
-  k_p2p<T, FIELD, MIXED, BIG><<<grid, 128, 0, st>>>(
-      t.big_items.ptr, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr,
-      t.leaf_clo.ptr, s->sx.ptr, s->sy.ptr, s->sz.ptr, s->sq.ptr, s->rel32.ptr, s->acc_pot.ptr,
-      s->acc_fld.ptr);
+  k_p2p_warp<FIELD><<<ceil_div(t.nleaves, 4), 128, 0, st>>>(
+      t.nleaves, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr,
+      s->sx.ptr, s->sy.ptr, s->sz.ptr, s->rel32.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
+  if (!t.n_big) return;
+  k_p2p_chunk<FIELD><<<t.n_big, 128, 0, st>>>(
+      t.big_items.ptr, t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr, s->sx.ptr, s->sy.ptr,
+      s->sz.ptr, s->rel32.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
   ACHECK(cudaGetLastError());
   s->launches++;
 }
 
-template <bool FIELD, bool MIXED>
-void launch_pair(AranGpuSolver3d *s, cudaStream_t st) {
+template <bool FIELD, bool BIG>
+void launch_fp64(AranGpuSolver3d *s, int grid, cudaStream_t st) {
   DevTree &t = s->tree;
-  if constexpr (MIXED) {
-    k_p2p_warp<FIELD><<<ceil_div(t.nleaves, 4), 128, 0, st>>>(
-        t.nleaves, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr,
-        s->sx.ptr, s->sy.ptr, s->sz.ptr, s->rel32.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
-    ACHECK(cudaGetLastError());
-    s->launches++;
-  } else {
-    launch_one<FIELD, MIXED, false>(s, s->tree.nleaves, st);
-  }
-  if (s->tree.n_big) launch_one<FIELD, MIXED, true>(s, s->tree.n_big, st);
+  k_p2p64<FIELD, BIG><<<grid, 128, 0, st>>>(
+      t.big_items.ptr, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, s->sx.ptr, s->sy.ptr,
+      s->sz.ptr, s->sq.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
 }
 
 }  // namespace
@@ -479,11 +527,17 @@ void launch_p2p(AranGpuSolver3d *s, cudaStream_t st) {
   const bool mixed = s->cfg.precision == ARAN_PRECISION_MIXED;
   const bool field = s->cfg.field != 0;
   if (mixed) {
-    if (field) launch_pair<true, true>(s, st);
-    else launch_pair<false, true>(s, st);
+    if (field) launch_mixed<true>(s, st);
+    else launch_mixed<false>(s, st);
   } else {
-    if (field) launch_pair<true, false>(s, st);
-    else launch_pair<false, false>(s, st);
+    const int nb = s->tree.n_big;
+    if (field) {
+      launch_fp64<true, false>(s, s->tree.nleaves, st);
+      if (nb) launch_fp64<true, true>(s, nb, st);
+    } else {
+      launch_fp64<false, false>(s, s->tree.nleaves, st);
+      if (nb) launch_fp64<false, true>(s, nb, st);
+    }
   }
 }
 
