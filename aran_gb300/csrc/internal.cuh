@@ -223,8 +223,9 @@ struct AranGpuSolver3d {
   aran::DBuf<float> tc_tab;
   aran::DBuf<int8_t> tc_dvec;
   int tc_p = -1;
-  // sums of the parts of a split lane-parallel M2L pass
+  // sums of the parts of a split M2L pass
   aran::DBuf<float> m2l_part;
+  aran::DBuf<double> m2l_part64;
   aran::DBuf<int> sys_off;
   aran::DBuf<double> sys_box;
   std::vector<int> h_sys_off;
@@ -253,6 +254,21 @@ void run_passes(AranGpuSolver3d *s);
 // kkylin.cu: stage 0 = M2M, 1 = M2L, 2 = L2L
 void build_kkylin_tables(AranGpuSolver3d *s);
 void kkylin_pass(AranGpuSolver3d *s, int stage);
+// parts of the offset list per group of parents of an M2L pass: the least
+// number of waves of CTAs times the work of a part (1 / K of the offsets and
+// the set-up, about 1/40 of a whole list)
+inline int split_parts(int groups, int resident) {
+  int best = 1;
+  double cost = 1e30;
+  for (int k : {1, 2, 3, 4, 6, 8, 12, 16}) {
+    const double c = (double)(((int64_t)groups * k + resident - 1) / resident) * (1. / k + 0.025);
+    if (c < 0.97 * cost) {
+      cost = c;
+      best = k;
+    }
+  }
+  return best;
+}
 // m2l.cu: M2L into the children of parents[first, first + count), in FP64
 // (mult64/loc64) or FP32 (mult32/loc32)
 void launch_m2l(AranGpuSolver3d *s, bool fp64, int first, int count, cudaStream_t st);

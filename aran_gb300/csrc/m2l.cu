@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
                   const T *__restrict__ dirs, M2LOffsets D,
                   const uint8_t *__restrict__ lm_g, double scale_e,
                   const cplx<T> *__restrict__ mult, cplx<T> *__restrict__ loc,
-                  int *__restrict__ err, int polls) {
+                  int *__restrict__ err, int polls, int nsplit, cplx<T> *__restrict__ parts) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int nm = tri(p), nl = tri(p + 1);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -162,7 +162,10 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
     s_nact = tot;
   }
   __syncthreads();
-  const int nact = s_nact;
+  // this CTA's part of the offset list
+  const int first = s_nact * (int)blockIdx.y / nsplit;
+  const int nact = s_nact * ((int)blockIdx.y + 1) / nsplit - first;
+  active += first;
   const uint32_t tbytes = (uint32_t)(D.stride * sizeof(T));
 
   if (w == kSibWarps) {
@@ -353,17 +356,41 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
     if (NST > 0 && lane == 0) mbar_arrive(&empty[b]);
   }
   cp_async_wait_all();   // source copies still in flight after an early stop
-  if (nact > 0) {
+  if (nact > 0 || nsplit > 1) {
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       if (!tvalid[g]) continue;
       const T ih = (T)(ldexp(1.0, depth[tg[g]]) / scale_e);
+      // a part's sums go to the workspace [part][parent][child][coefficient]
+      cplx<T> *out = nsplit == 1
+                         ? loc + (size_t)tg[g] * nl
+                         : parts + (((size_t)blockIdx.y * nparents + blockIdx.x * G + g) *
+                                        kSibWarps + w) * nl;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         int c = lane + 32 * r;
-        if (c < nl) loc[(size_t)tg[g] * nl + c] = cmake<T>(acc[g][r].re * ih, acc[g][r].im * ih);
+        if (c < nl) out[c] = cmake<T>(acc[g][r].re * ih, acc[g][r].im * ih);
       }
     }
+  }
+}
+
+// the parts of a split pass added in order, one warp per child
+template <typename T>
+__global__ void __launch_bounds__(32 * kSibWarps)
+    k_m2l_parts_sum(int nparents, int nsplit, const int *__restrict__ parents,
+                    const int *__restrict__ child, const int *__restrict__ begin,
+                    const int *__restrict__ end, int nl, const cplx<T> *__restrict__ parts,
+                    cplx<T> *__restrict__ loc) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int t = child[parents[blockIdx.x]] + w;
+  if (end[t] <= begin[t]) return;
+  const size_t step = (size_t)nparents * kSibWarps * nl;
+  const cplx<T> *p = parts + ((size_t)blockIdx.x * kSibWarps + w) * nl;
+  for (int c = lane; c < nl; c += 32) {
+    cplx<T> v = cmake<T>(0, 0);
+    for (int k = 0; k < nsplit; ++k) v = cadd(v, p[k * step + c]);
+    loc[(size_t)t * nl + c] = v;
   }
 }
 
@@ -409,12 +436,34 @@ bool try_launch(AranGpuSolver3d *s, OpTables<T> &tb, const M2LOffsets &D, const 
   size_t sm = m2l_smem<T, NST, G>(p, D.stride);
   if ((int)sm > dev_smem) return false;
   smem_opt_in(k_m2l_sibling<T, NST, R, G>, sm);
-  k_m2l_sibling<T, NST, R, G><<<ceil_div(count, G), 32 * (kSibWarps + 1), sm, st>>>(
+  // few parents: their offset lists are split over CTAs.  An FP64 CTA keeps
+  // its SM's FP64 pipe busy alone (half a lane a cycle per scheduler), FP32
+  // ones share an SM.  The FP64 root levels of a mixed order-16 solve, 72
+  // parents, took 12.6 ms unsplit on 36 SMs and take 3.0 ms
+  const int groups = ceil_div(count, G);
+  int nsm = 0;
+  ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
+  const int nsplit = split_parts(groups, sizeof(T) == 8 ? nsm : 2 * nsm);
+  DBuf<T> &pb = sizeof(T) == 8 ? reinterpret_cast<DBuf<T> &>(s->m2l_part64)
+                               : reinterpret_cast<DBuf<T> &>(s->m2l_part);
+  cplx<T> *parts = nullptr;
+  if (nsplit > 1) {
+    pb.reserve((size_t)nsplit * count * kSibWarps * tri(p + 1) * 2);
+    parts = reinterpret_cast<cplx<T> *>(pb.ptr);
+  }
+  k_m2l_sibling<T, NST, R, G><<<dim3(groups, nsplit), 32 * (kSibWarps + 1), sm, st>>>(
       count, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr, t.ncol.ptr,
       t.ijk.ptr, t.depth.ptr, p, tb.dir_m2l.ptr, D, tb.lm.ptr, s->scale_e, mult, loc,
-      s->err_dev.ptr, consumer_wait_polls());
+      s->err_dev.ptr, consumer_wait_polls(), nsplit, parts);
   ACHECK(cudaGetLastError());
   s->launches++;
+  if (nsplit > 1) {
+    k_m2l_parts_sum<T><<<count, 32 * kSibWarps, 0, st>>>(count, nsplit, parents, t.child.ptr,
+                                                         t.begin.ptr, t.end.ptr, tri(p + 1), parts,
+                                                         loc);
+    ACHECK(cudaGetLastError());
+    s->launches++;
+  }
   return true;
 }
 
@@ -461,10 +510,19 @@ void launch_t(AranGpuSolver3d *s, OpTables<T> &tb, const int *parents, int count
 #undef ARAN_TRY
     if (ok) return;
   }
+  // FP64: one parent per CTA.  A column without a source at an offset costs
+  // FP64 operations, which are all that counts there, and sharing a table
+  // read between columns saves nothing (200k Plummer particles at order 12,
+  // the whole solve: 48.8 ms, 54.8 with two parents)
+  if (sizeof(T) == 8 && nl <= 96 &&
+      try_launch<T, 3, 3, 1>(s, tb, D, parents, count, mult, loc, st, dev_smem))
+    return;
+  if (sizeof(T) == 8 && nl > 96 && nl <= 160 &&
+      try_launch<T, 1, 5, 1>(s, tb, D, parents, count, mult, loc, st, dev_smem))
+    return;
   // (two table slots keep a p <= 12 FP32 CTA under a third of the shared
   // memory, so three CTAs share an SM)
   if (nl <= 96) {
-    if (sizeof(T) == 8 && try_launch<T, 3, 3, 2>(s, tb, D, parents, count, mult, loc, st, dev_smem)) return;
     if (try_launch<T, 2, 3, 2>(s, tb, D, parents, count, mult, loc, st, dev_smem)) return;
     if (try_launch<T, 1, 3, 2>(s, tb, D, parents, count, mult, loc, st, dev_smem)) return;
     if (try_launch<T, 1, 3, 1>(s, tb, D, parents, count, mult, loc, st, dev_smem)) return;

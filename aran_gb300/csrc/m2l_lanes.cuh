@@ -724,22 +724,6 @@ __global__ void __launch_bounds__(256) k_m2l_lanes_sum(LaneArgs a) {
   }
 }
 
-// parts of the offset list per group of parents: the least number of
-// waves of CTAs times the work of a part (1 / K of the offsets and the set-up,
-// about 1/40 of a whole list)
-inline int lane_split(int groups, int resident) {
-  int best = 1;
-  double cost = 1e30;
-  for (int k : {1, 2, 3, 4, 6, 8, 12, 16}) {
-    const double c = (double)(((int64_t)groups * k + resident - 1) / resident) * (1. / k + 0.025);
-    if (c < 0.97 * cost) {
-      cost = c;
-      best = k;
-    }
-  }
-  return best;
-}
-
 template <int P>
 bool launch_p(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,
               const cplx<float> *mult, cplx<float> *loc, cudaStream_t st) {
@@ -771,7 +755,7 @@ bool launch_p(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int c
   a.err = s->err_dev.ptr;
   a.polls = consumer_wait_polls();
   const int groups = ceil_div(count, D::PAR);
-  a.nsplit = lane_split(groups, nsm * D::CTAS);
+  a.nsplit = split_parts(groups, nsm * D::CTAS);
   a.part = nullptr;
   if (a.nsplit > 1) {
     s->m2l_part.reserve((size_t)a.nsplit * groups * D::W * D::NL * 32);
