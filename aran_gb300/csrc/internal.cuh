@@ -192,6 +192,7 @@ struct AranGpuSolver3d {
   aran::DBuf<double> sx, sy, sz, sq;     // sorted FP64 positions/charges
   aran::DBuf<aran::real4<double>> rel64;
   aran::DBuf<aran::real4<float>> rel32;
+  aran::DBuf<float4> abs_hi, abs_lo;     // FP32 hi + lo positions (hi.w = charge), mixed
   aran::DBuf<double> acc_pot, acc_fld;   // sorted accumulators (FP64)
   aran::DBuf<double> io_xyz, io_q, io_pot, io_fld;  // staging for host calls
   aran::DBuf<double> mult64, loc64;
@@ -223,7 +224,7 @@ struct AranGpuSolver3d {
   aran::DBuf<float> tc_tab;
   aran::DBuf<int8_t> tc_dvec;
   int tc_p = -1;
-  // sums of the parts of a split M2L pass
+  // sums of the segments (lane-parallel FP32) or parts (FP64) of an M2L pass
   aran::DBuf<float> m2l_part;
   aran::DBuf<double> m2l_part64;
   aran::DBuf<int> sys_off;
@@ -254,7 +255,7 @@ void run_passes(AranGpuSolver3d *s);
 // kkylin.cu: stage 0 = M2M, 1 = M2L, 2 = L2L
 void build_kkylin_tables(AranGpuSolver3d *s);
 void kkylin_pass(AranGpuSolver3d *s, int stage);
-// parts of the offset list per group of parents of an M2L pass: the least
+// parts of the offset lists of a small FP64 M2L pass: the least
 // number of waves of CTAs times the work of a part (1 / K of the offsets and
 // the set-up, about 1/40 of a whole list)
 inline int split_parts(int groups, int resident) {

@@ -436,20 +436,19 @@ bool try_launch(AranGpuSolver3d *s, OpTables<T> &tb, const M2LOffsets &D, const 
   size_t sm = m2l_smem<T, NST, G>(p, D.stride);
   if ((int)sm > dev_smem) return false;
   smem_opt_in(k_m2l_sibling<T, NST, R, G>, sm);
-  // few parents: their offset lists are split over CTAs.  An FP64 CTA keeps
-  // its SM's FP64 pipe busy alone (half a lane a cycle per scheduler), FP32
-  // ones share an SM.  The FP64 root levels of a mixed order-16 solve, 72
+  // few parents: their offset lists are split over CTAs (FP64 only: the sums
+  // of a split list round differently, which FP32 results would show).  An
+  // FP64 CTA keeps its SM's FP64 pipe busy alone (half a lane a cycle per
+  // scheduler).  The FP64 root levels of a mixed order-16 solve, 72
   // parents, took 12.6 ms unsplit on 36 SMs and take 3.0 ms
   const int groups = ceil_div(count, G);
   int nsm = 0;
   ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
-  const int nsplit = split_parts(groups, sizeof(T) == 8 ? nsm : 2 * nsm);
-  DBuf<T> &pb = sizeof(T) == 8 ? reinterpret_cast<DBuf<T> &>(s->m2l_part64)
-                               : reinterpret_cast<DBuf<T> &>(s->m2l_part);
+  const int nsplit = sizeof(T) == 8 ? split_parts(groups, nsm) : 1;
   cplx<T> *parts = nullptr;
   if (nsplit > 1) {
-    pb.reserve((size_t)nsplit * count * kSibWarps * tri(p + 1) * 2);
-    parts = reinterpret_cast<cplx<T> *>(pb.ptr);
+    s->m2l_part64.reserve((size_t)nsplit * count * kSibWarps * tri(p + 1) * 2);
+    parts = reinterpret_cast<cplx<T> *>(s->m2l_part64.ptr);
   }
   k_m2l_sibling<T, NST, R, G><<<dim3(groups, nsplit), 32 * (kSibWarps + 1), sm, st>>>(
       count, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr, t.ncol.ptr,

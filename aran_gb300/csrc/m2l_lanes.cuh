@@ -40,12 +40,13 @@
 // order 12 the FMA pipes are active 54 % of the cycles, 63 % of the issue
 // slots are used, shared memory moves data in 49 %).  Measured on GB300, M2L
 // of a 4 M-particle Plummer set (leaf 64, 38.9 M translations): order 12
-// 11.2 ms (14.3 with the vertical factors in the table stream, the sums in
-// shared memory and 8 warps a CTA; 11.6 with 8 warps; 11.7 with neighbouring
-// degrees packed through the rotations too, the packing's moves costing what
-// the products saved), order 8 4.8 ms (6.5), order 16 23.5 ms, order 10
-// 7.7 ms and order 6 3.2 ms (about 118, 42 and 20 with the kernel of m2l.cu,
-// whose lanes run over one translation's coefficients).
+// 11.6 ms (14.3 with the vertical factors in the table stream, the sums in
+// shared memory and 8 warps a CTA; with 8 warps and the rest as now 0.4 more;
+// with neighbouring degrees packed through the rotations too 0.5 more, the
+// packing's moves costing what the products saved), order 8 5.0 ms (6.5),
+// order 16 25.8 ms, order 10 7.9 ms and order 6 3.2 ms (about 118, 42 and 20
+// with the kernel of m2l.cu, whose lanes run over one translation's
+// coefficients).
 //
 // The offset tables stream through a three-slot ring of TMA bulk copies;
 // the next offset's source multipoles are brought into shared memory by one
@@ -53,17 +54,19 @@
 // wait is bounded; a wait that gives up sets the error word and the CTA
 // stops.
 //
-// A pass with few parents would leave most SMs idle (one CTA takes its
-// parents through up to 189 offsets in turn), so a CTA may take one of
-// `nsplit` parts of its offset list; the parts' sums go to a workspace and
-// k_m2l_lanes_sum adds them in order (10k uniform particles, order 8, leaf
-// 20: 0.11 ms, 0.55 in one part).
+// A target's sum is the sum of 8 or 16 segments of the offset list, each summed
+// on its own: a pass with few parents, which would leave most SMs idle (one
+// CTA takes its parents through up to 189 offsets in turn), gives the
+// segments to several CTAs, which leave their sums in a workspace for
+// k_m2l_lanes_sum to add (10k uniform particles, order 8, leaf 20: 0.11 ms,
+// 0.55 in one part); a pass with many parents adds them up as it goes.  So
+// the result does not depend on how many CTAs share a target's offsets: a
+// system solved alone, in a forest or beside others gets the same bits.
 #pragma once
-
-#include <type_traits>
 
 #include "internal.cuh"
 #include "async.cuh"
+#include "f32x2.cuh"
 #include "tcgen05.cuh"
 
 namespace aran {
@@ -77,6 +80,9 @@ constexpr unsigned kFull = 0xffffffffu;
 __host__ __device__ constexpr int lane_pair(int l) {
   return ((l + 1) / 2) * ((l + 1) / 2 + 1) - ((l & 1) ? (l + 1) / 2 : 0);
 }
+
+// column of (l, m) among a target's sums
+__host__ __device__ constexpr int lane_col(int l, int m) { return 2 * lane_pair(l) + m; }
 
 template <int P>
 struct LaneDims {
@@ -100,6 +106,11 @@ struct LaneDims {
   static constexpr int CTAS = P <= 4 ? 3 : 1;
   static constexpr bool TM = P >= 8;                // sums in tensor memory
   static constexpr int NCH = (2 * NP + 15) / 16;    // 16-column pieces of a warp's sums
+  // segments of the 189 offsets: more of them spread a small pass over more
+  // CTAs, each costs a large one a pass of its sums through the L2 (0.1 ms of
+  // 11.3 at order 12, 0.15 ms of 27.3 at order 16, 4 M particles)
+  static constexpr int SEGS = P <= 12 ? 16 : 8;
+  static constexpr int COLS = 16 * NCH;             // columns of a warp in the workspace
   // columns of a CTA: W / 4 warps share each quarter of the rows
   static constexpr int TCOLS = NCH * 16 * (W / 4) <= 256 ? 256 : 512;
   static_assert(NCH * 16 * (W / 4) <= 512, "sums exceed the tensor memory");
@@ -118,35 +129,6 @@ constexpr size_t lanes_smem() {
 
 __device__ __forceinline__ float sel4(const float4 &v, int k) {
   return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
-}
-
-// f(0) .. f(N - 1) with the index a compile-time constant
-template <int N, int I = 0, typename F>
-__device__ __forceinline__ void static_for(F &&f) {
-  if constexpr (I < N) {
-    f(std::integral_constant<int, I>{});
-    static_for<N, I + 1>(f);
-  }
-}
-
-// packed FP32 pairs
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
 }
 
 // 16 columns of this warp's tensor-memory rows, read and written without
@@ -224,10 +206,28 @@ struct LaneArgs {
   double scale_e;
   const cplx<float> *mult;
   cplx<float> *loc;
-  float *part;      // nsplit > 1: [part][group][warp][coefficient][lane]
+  float *part;      // sums [segment][group][warp][column / 4][lane][column % 4]; one CTA
+                    // per group (nsplit = 1): the running sum in segment 0's place
   int *err;
   int polls;
 };
+
+// four sums of a lane to the workspace: stored, or added to what it holds
+__device__ __forceinline__ void part_put(float4 *dst, bool add, float x, float y, float z,
+                                         float w) {
+  if (add)
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(x),
+                 "f"(y), "f"(z), "f"(w)
+                 : "memory");
+  else
+    *dst = make_float4(x, y, z, w);
+}
+// the reductions' sum: denormals are flushed
+__device__ __forceinline__ float add_ftz(float a, float b) {
+  float r;
+  asm("add.rn.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 
 template <int P>
 __device__ __forceinline__ void m2l_lanes_body(const LaneArgs &a) {
@@ -260,7 +260,6 @@ __device__ __forceinline__ void m2l_lanes_body(const LaneArgs &a) {
   uint16_t *active = reinterpret_cast<uint16_t *>(smem_raw + off);
   off += 192 * sizeof(uint16_t);
   uint16_t *dcode = reinterpret_cast<uint16_t *>(smem_raw + off);   // 189 of them
-  __shared__ int s_nact;
   __shared__ uint32_t s_tmem;
 
   for (int i = threadIdx.x; i < PAR * 216; i += blockDim.x) grid[i] = -1;
@@ -360,15 +359,22 @@ __device__ __forceinline__ void m2l_lanes_body(const LaneArgs &a) {
       active[pos] = (uint16_t)di;
     }
   }
-  if (threadIdx.x == 0) {
-    int tot = 0;
-    for (int k = 0; k < 6; ++k) tot += __popc(mask[k]);
-    s_nact = tot;
-  }
   __syncthreads();
-  // this CTA's part of the offset list
-  const int a0 = s_nact * (int)blockIdx.y / a.nsplit;
-  const int nact = s_nact * ((int)blockIdx.y + 1) / a.nsplit - a0;
+  // this CTA's segments of the offset list; offset di belongs to segment
+  // di D::SEGS / 189
+  const int seg0 = D::SEGS * (int)blockIdx.y / a.nsplit;
+  const int seg1 = D::SEGS * ((int)blockIdx.y + 1) / a.nsplit;
+  auto active_below = [&](int seg) -> int {
+    const int d = (189 * seg + D::SEGS - 1) / D::SEGS;   // offsets below it
+    int n = 0;
+    for (int k = 0; k < 6; ++k) {
+      const int left = d - 32 * k;
+      if (left > 0) n += __popc(mask[k] & (left >= 32 ? kFull : (1u << left) - 1u));
+    }
+    return n;
+  };
+  const int a0 = active_below(seg0);
+  const int nact = active_below(seg1) - a0;
   active += a0;
 
   // the ring: thread 0 fills the first slots; afterwards warp 0 refills
@@ -422,21 +428,33 @@ __device__ __forceinline__ void m2l_lanes_body(const LaneArgs &a) {
   find_next(0);
   prefetch();
 
+  // the segments' sums: stored (split pass) or added to the running sum
+  const bool whole = a.nsplit == 1;
+  const size_t seg_step = (size_t)gridDim.x * W * D::COLS * 8;
+  float4 *my_part = reinterpret_cast<float4 *>(a.part) +
+                    ((size_t)blockIdx.x * W + w) * D::COLS * 8 + lane;
+  bool started = false;    // the running sum holds a segment
   int it = 0;
-  for (; it < nact; ++it) {
+  bool stop = false;
+  for (int seg = seg0; seg < seg1 && !stop; ++seg) {
+  bool any_src = false;    // this warp met a source in the segment
+  for (; it < nact && active[it] * D::SEGS / 189 == seg; ++it) {
     const int b = it % kLaneNst;
     const bool ok =
         __all_sync(kFull, mbar_wait_or_flag(&full[b], (it / kLaneNst) & 1, a.err, a.polls));
     if (!ok) {
       if (lane == 0) atomicOr(a.err, kErrTimeout);
+      stop = true;
       break;
     }
     if (it == next_i) {
       const float *tb = tab + (size_t)b * STRIDE;
       if (!__all_sync(kFull, mbar_wait(&sbar[w], sph))) {
         if (lane == 0) atomicOr(a.err, kErrTimeout);
+        stop = true;
         break;
       }
+      any_src = true;
       sph ^= 1u;
       pending = false;
       __syncwarp();
@@ -632,51 +650,66 @@ __device__ __forceinline__ void m2l_lanes_body(const LaneArgs &a) {
     }
     __syncwarp();
   }
+  // the segment's sum to the workspace, four columns at a time, and back to
+  // zero; added with reductions, which the L2 carries out while the next
+  // segment runs (loading, adding and storing the running sum here took 15 %
+  // longer at order 16)
+  if (stop || (whole && !any_src)) continue;
+  float4 *dst = whole ? my_part : my_part + seg * seg_step;
+  const bool add = whole && started;
+  started = true;
+  if constexpr (TM) {
+    uint32_t zero[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) zero[i] = 0u;
+    tm_wait_st();
+#pragma unroll 1
+    for (int ch = 0; ch < NCH; ++ch) {
+      uint32_t r[16];
+      tm_ld16(tm + 16 * ch, r);
+      tm_wait_ld(r);
+      tm_st16(tm + 16 * ch, zero);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        part_put(dst + 32 * (4 * ch + i), add, __uint_as_float(r[4 * i]),
+                 __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                 __uint_as_float(r[4 * i + 3]));
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < NP; q += 2) {
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      unpack2(racc[q], v[0], v[1]);
+      racc[q] = 0ull;
+      if (q + 1 < NP) {
+        unpack2(racc[q + 1 < NP ? q + 1 : 0], v[2], v[3]);
+        racc[q + 1 < NP ? q + 1 : 0] = 0ull;
+      }
+      part_put(dst + 16 * q, add, v[0], v[1], v[2], v[3]);
+    }
+  }
+  }
   // copies still in flight after an early exit land before the CTA leaves
   if (pending) mbar_wait(&sbar[w], sph);
   if (threadIdx.x == 0)
     for (int i = it; i < issued; ++i) mbar_wait(&full[i % kLaneNst], (i / kLaneNst) & 1);
   __syncwarp();
-  // the sums: to the workspace as they are (parts), else back from the
-  // mirror frame and the scaled frame into the target's local
-  const bool whole = a.nsplit == 1;
-  const float ih =
-      whole && tgt >= 0 ? (float)((double)(1ull << a.depth[tgt]) / a.scale_e) : 0.f;   // 2^depth / scale
-  float *lo_ = reinterpret_cast<float *>(a.loc) + (size_t)(tgt >= 0 ? tgt : 0) * NL * 2 + h;
-  float *po = whole ? nullptr
-                    : a.part + (((size_t)blockIdx.y * gridDim.x + blockIdx.x) * W + w) *
-                                   NL * 32 + lane;
-  const bool wr = whole ? (nact > 0 && tgt >= 0) : true;
-  if (TM) tm_wait_st();
-  uint32_t r[16];
-#pragma unroll
-  for (int l = 0; l <= P; ++l)
-#pragma unroll
-    for (int k = 0; k <= l / 2; ++k) {
-      const int q = lane_pair(l) + k;
-      float v[2];
-      if (TM) {
-        if ((q & 7) == 0) {
-          tm_ld16(tm + 16 * (q >> 3), r);
-          tm_wait_ld(r);
-        }
-        v[0] = __uint_as_float(r[2 * (q & 7)]);
-        v[1] = __uint_as_float(r[2 * (q & 7) + 1]);
-      } else {
-        unpack2(racc[TM ? 0 : q], v[0], v[1]);
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int m = 2 * k + e;
-        if (m > l) continue;
-        const int c = l * (l + 1) / 2 + m;
+  // back from the mirror frame and the scaled frame into the target's local
+  if (whole && started && tgt >= 0) {
+    const float ih = (float)((double)(1ull << a.depth[tgt]) / a.scale_e);   // 2^depth / scale
+    float *lo = reinterpret_cast<float *>(a.loc) + (size_t)tgt * NL * 2 + h;
+    int c = 0;
+    for (int l = 0; l <= P; ++l)
+#pragma unroll 4
+      for (int m = 0; m <= l; ++m, ++c) {
         const bool neg = ((bz & (l + m)) ^ (bx & m) ^ (h & (bx ^ by))) & 1;
-        if (wr) {
-          if (whole) lo_[2 * c] = v[e] * K.inva[c] * (neg ? -ih : ih);
-          else po[32 * c] = v[e];
-        }
+        const int col = lane_col(l, m);
+        const float v = __ldcg(reinterpret_cast<const float *>(my_part + 32 * (col >> 2)) +
+                               (col & 3));
+        lo[2 * c] = v * K.inva[c] * (neg ? -ih : ih);
       }
-    }
+  }
+  if (TM) tm_wait_st();
   if (TM) {
     tc_fence_before();
     __syncthreads();
@@ -696,8 +729,8 @@ __global__ void __launch_bounds__(32 * LaneDims<P>::W, LaneDims<P>::CTAS)
   m2l_lanes_body<P>(a);
 }
 
-// the parts of a split pass added in order: block (group, warp), one thread
-// per lane and every eighth coefficient
+// the segments of a split pass added in order: block (group, warp), one
+// thread per lane and every eighth coefficient
 template <int P>
 __global__ void __launch_bounds__(256) k_m2l_lanes_sum(LaneArgs a) {
   constexpr int NL = LaneDims<P>::NL;
@@ -710,18 +743,38 @@ __global__ void __launch_bounds__(256) k_m2l_lanes_sum(LaneArgs a) {
   if (a.end[t] <= a.begin[t]) return;
   const int bx = cw & 1, by = (cw >> 1) & 1, bz = (cw >> 2) & 1;
   const float ih = (float)((double)(1ull << a.depth[t]) / a.scale_e);
-  const size_t step = (size_t)gridDim.x * W * NL * 32;
+  constexpr int COLS = LaneDims<P>::COLS;
+  const size_t step = (size_t)gridDim.x * W * COLS * 32;
   for (int c = threadIdx.x >> 5; c < NL; c += 8) {
-    const float *p = a.part + ((size_t)blockIdx.x * W + w) * NL * 32 + 32 * c + lane;
-    float v = 0.f;
-    for (int k = 0; k < a.nsplit; ++k) v += p[k * step];
     int l = 0;
     while ((l + 1) * (l + 2) / 2 <= c) ++l;
     const int m = c - l * (l + 1) / 2;
+    const int col = lane_col(l, m);
+    const float *p = a.part + ((size_t)blockIdx.x * W + w) * COLS * 32 +
+                     (32 * (col >> 2) + lane) * 4 + (col & 3);
+    float v = p[0];
+#pragma unroll
+    for (int k = 1; k < LaneDims<P>::SEGS; ++k) v = add_ftz(v, p[k * step]);
     const bool neg = ((bz & (l + m)) ^ (bx & m) ^ (h & (bx ^ by))) & 1;
     reinterpret_cast<float *>(a.loc)[((size_t)t * NL + c) * 2 + h] =
         v * kLaneConst<P>.inva[c] * (neg ? -ih : ih);
   }
+}
+
+// CTAs that share a group's segments: the least number of waves of CTAs
+// times the work of each (1 / K of the segments and the set-up, about 1/40 of
+// a whole list); none where the workspace of all segments would be large
+inline int lane_split(int groups, int resident, int segs) {
+  int best = 1;
+  double cost = 1e30;
+  for (int k = 1; k <= (groups <= 2 * resident ? segs : 1); k *= 2) {
+    const double c = (double)(((int64_t)groups * k + resident - 1) / resident) * (1. / k + 0.025);
+    if (c < 0.97 * cost) {
+      cost = c;
+      best = k;
+    }
+  }
+  return best;
 }
 
 template <int P>
@@ -755,12 +808,9 @@ bool launch_p(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int c
   a.err = s->err_dev.ptr;
   a.polls = consumer_wait_polls();
   const int groups = ceil_div(count, D::PAR);
-  a.nsplit = split_parts(groups, nsm * D::CTAS);
-  a.part = nullptr;
-  if (a.nsplit > 1) {
-    s->m2l_part.reserve((size_t)a.nsplit * groups * D::W * D::NL * 32);
-    a.part = s->m2l_part.ptr;
-  }
+  a.nsplit = lane_split(groups, nsm * D::CTAS, D::SEGS);
+  s->m2l_part.reserve((size_t)(a.nsplit > 1 ? D::SEGS : 1) * groups * D::W * D::COLS * 32);
+  a.part = s->m2l_part.ptr;
   kern<<<dim3(groups, a.nsplit), 32 * D::W, sm, st>>>(a);
   ACHECK(cudaGetLastError());
   s->launches++;
