@@ -7,8 +7,8 @@
 // sources directly (both sides of a pair are evaluated by their own targets
 // instead of the symmetric update).
 //
-// Work decomposition: mixed precision takes a warp per target leaf
-// (k_p2p_warp), FP64 a block (k_p2p64).  Near ranges of more than kBigRange
+// Work decomposition: a block per target leaf (k_p2p_tile in mixed precision,
+// k_p2p64 in FP64).  Near ranges of more than kBigRange
 // points (a coarse leaf next to a deep subtree, common in clustered sets) are
 // cut into leaf-aligned chunks processed by extra blocks that accumulate
 // atomically.
@@ -20,9 +20,8 @@
 // the FP64 positions.
 #include <cub/cub.cuh>
 
-#include <type_traits>
-
 #include "internal.cuh"
+#include "f32x2.cuh"
 
 namespace aran {
 
@@ -91,102 +90,6 @@ __global__ void k_big_items(const int *__restrict__ heavy, int nleaves,
   };
   for (int i = threadIdx.x; i < nch; i += blockDim.x)
     items[coff + i] = make_int4(L, boundary(i), boundary(i + 1), 0);
-}
-
-// one chunk of a heavy near range of a mixed solve: threads-per-target (tpt)
-// grows as the leaf shrinks (n <= 8: 16, <= 16: 8, <= 32: 4, <= 64: 2, else
-// 1), and a target's tpt threads take the chunk's leaves round-robin (tiny
-// target leaves) or split every source leaf's points
-template <bool FIELD>
-__global__ void __launch_bounds__(128, 10) k_p2p_chunk(
-    const int4 *__restrict__ items, const int2 *__restrict__ be, const float4 *__restrict__ chi,
-    const float4 *__restrict__ clo, const double *__restrict__ sx, const double *__restrict__ sy,
-    const double *__restrict__ sz, const real4<float> *__restrict__ rel32,
-    double *__restrict__ acc_pot, double *__restrict__ acc_fld) {
-  const int4 it = items[blockIdx.x];
-  const int L = it.x, ia = it.y, ib = it.z;
-  const int2 tbe = be[L];
-  const int b = tbe.x, nt = tbe.y - tbe.x;
-  const int tpt = nt <= 8 ? 16 : (nt <= 16 ? 8 : (nt <= 32 ? 4 : (nt <= 64 ? 2 : 1)));
-  const int gsz = blockDim.x / tpt;
-  const int sub = threadIdx.x % tpt;
-  const bool leaf_strided = nt <= 8;
-  const float4 tch = chi[L], tcl = clo[L];
-  for (int tb = 0; tb < nt; tb += gsz) {
-    const int ti = tb + threadIdx.x / tpt;
-    const bool active = ti < nt;
-    if (!__any_sync(kFull, active)) continue;   // a warp with no target of this pass
-    const int t = b + (active ? ti : 0);
-    // per-source-leaf FP32 sums are added with Kahan compensation in FP32
-    // (FP64 adds per leaf would occupy the FP64 pipe, 1/64 of FP32)
-    float ks0 = 0.f, ks1 = 0.f, ks2 = 0.f, ks3 = 0.f;
-    float kc0 = 0.f, kc1 = 0.f, kc2 = 0.f, kc3 = 0.f;
-    auto kahan = [](float &sum, float &comp, float v) {
-      const float y = v - comp;
-      const float t2 = sum + y;
-      comp = (t2 - sum) - y;
-      sum = t2;
-    };
-    const double tx64 = sx[t], ty64 = sy[t], tz64 = sz[t];
-    const real4<float> r = rel32[t];
-    auto do_leaf = [&](int lf, int j0, int js) {
-      const int2 sbe = be[lf];
-      const float4 sh = chi[lf], sl = clo[lf];
-      // target position relative to the source leaf centre
-      const float ox = r.x - ((sh.x - tch.x) + (sl.x - tcl.x));
-      const float oy = r.y - ((sh.y - tch.y) + (sl.y - tcl.y));
-      const float oz = r.z - ((sh.z - tch.z) + (sl.z - tcl.z));
-      const float thr2 = tch.w;
-      float p0 = 0.f, f0 = 0.f, f1 = 0.f, f2 = 0.f;
-#pragma unroll 4
-      for (int j = sbe.x + j0; j < sbe.y; j += js) {
-        const real4<float> sj = rel32[j];
-        float dx = ox - sj.x, dy = oy - sj.y, dz = oz - sj.z;
-        float r2 = dx * dx + dy * dy + dz * dz;
-        if (__builtin_expect(r2 < thr2, 0)) {
-          if (j == t) {
-            r2 = 0.f;
-          } else {
-            // close pair: difference from the FP64 positions
-            dx = (float)(tx64 - sx[j]);
-            dy = (float)(ty64 - sy[j]);
-            dz = (float)(tz64 - sz[j]);
-            r2 = dx * dx + dy * dy + dz * dz;
-          }
-        }
-        const bool ok = FIELD ? (r2 > 1e-10f) : (r2 > 0.f);
-        const float inv = ok ? rsqrt_ftz(r2) : 0.f;
-        const float qi = sj.q * inv;
-        p0 += qi;
-        if (FIELD) {
-          const float q3 = qi * inv * inv;
-          f0 -= q3 * dx;
-          f1 -= q3 * dy;
-          f2 -= q3 * dz;
-        }
-      }
-      kahan(ks0, kc0, p0);
-      if (FIELD) {
-        kahan(ks1, kc1, f0);
-        kahan(ks2, kc2, f1);
-        kahan(ks3, kc3, f2);
-      }
-    };
-    if (leaf_strided)
-      for (int lf = ia + sub; lf < ib; lf += tpt) do_leaf(lf, 0, 1);
-    else
-      for (int lf = ia; lf < ib; ++lf) do_leaf(lf, sub, tpt);
-    double v[4] = {(double)ks0 - (double)kc0, (double)ks1 - (double)kc1,
-                   (double)ks2 - (double)kc2, (double)ks3 - (double)kc3};
-    for (int o = 1; o < tpt; o <<= 1)
-#pragma unroll
-      for (int c = 0; c < (FIELD ? 4 : 1); ++c) v[c] += __shfl_xor_sync(kFull, v[c], o);
-    if (active && sub == 0) {
-      atomicAdd(&acc_pot[t], v[0]);
-      if (FIELD)
-        for (int c = 0; c < 3; ++c) atomicAdd(&acc_fld[3 * (size_t)t + c], v[1 + c]);
-    }
-  }
 }
 
 // 1/sqrt(x) in FP64 from the hardware approximation's upper word y0 (20
@@ -311,171 +214,242 @@ __global__ void __launch_bounds__(128, 8) k_p2p64(
   }
 }
 
-// Mixed near field, one warp per target leaf (four per block).  The warp
-// walks the leaf's near source leaves; for each it stages up to 32 source
-// points in shared memory, shifted to the target leaf's frame by the lane
-// that loads them, and every lane sums them against its own targets from
-// broadcast reads: lanes per target S = 32 / (n rounded up to a power of
-// two) for n <= 16, else 1 (32 targets per pass), so the per-leaf set-up (centres, Kahan adds of the
-// leaf partials) is paid once per lane per source leaf.  The pair loop has no
-// branch: the distance is clamped below at h/8, and a lane whose chunk held a
-// closer pair (or the point itself) takes the stand-ins back and adds those
-// pairs from the FP64 positions afterwards.
+// Mixed near field, a block of T threads per target leaf.  The sources of a
+// leaf are the concatenation of its near ranges (the sorted particles of a
+// range lie side by side): the block stages up to 2 T of them at a time in
+// shared memory, as offsets from the target leaf's centre made from FP32
+// hi + lo positions, and the threads sum them two at a time in packed FP32
+// pairs: a leaf of n targets gets floor(T / n) threads per target, so the
+// lanes are busy whatever n is.  The pair loop has no branch: pairs closer
+// than h/8 (and the point itself) are left out, and a thread whose part held
+// one adds those pairs from the FP64 positions afterwards.  A thread's part
+// of a tile goes into Kahan sums, the parts of a target are added with
+// compensation.
 // Ranges of more than kBigRange points are left to the chunked pass.
-template <bool FIELD>
-__global__ void __launch_bounds__(128, 8) k_p2p_warp(
-    int nleaves, const int *__restrict__ near_off, const int *__restrict__ near_rng,
+// Bound by issue and the FP32 pipes: 13 operations a pair with the field (3
+// subtractions, 3 for r^2, 4 for q/r and q/r^3, 3 sums), 23 instructions for
+// two pairs; about two thirds of the instructions are the pair loop's.
+// Measured on GB300 against a warp per leaf with 1 to 32 lanes per target (in
+// powers of two), sources staged leaf by leaf and pairs taken singly: 300k
+// blobs (leaf 64) 0.45 ms, 1.08 before; 4M Plummer 3.9 ms, 5.2; 10k uniform
+// (leaf 20, potential) 0.02 ms, 0.09; heavy chunks of a 2M Plummer set 0.36
+// ms, 0.94.  T = 64, 96 and 256 took 0.68, 0.70 and 0.66 ms on the blobs
+// where 128 took 0.61; tiles of twice and four times the sources changed
+// nothing; 10 blocks an SM with 48 registers a thread beat 8, 6 and 12.
+constexpr int kP2pRanges = 32;   // near ranges taken together
+constexpr int kTileThreads = 128;
+
+template <bool FIELD, bool BIG, int T>
+__global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
+    const int4 *__restrict__ items, const int *__restrict__ near_off,
+    const int *__restrict__ near_rng,
     const int2 *__restrict__ be, const float4 *__restrict__ chi, const float4 *__restrict__ clo,
     const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
-    const real4<float> *__restrict__ rel32, double *__restrict__ acc_pot,
-    double *__restrict__ acc_fld) {
-  __shared__ float4 sbuf[4][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int L = blockIdx.x * 4 + w;
-  if (L >= nleaves) return;
+    const real4<float> *__restrict__ rel32, const float4 *__restrict__ phi,
+    const float4 *__restrict__ plo, double *__restrict__ acc_pot, double *__restrict__ acc_fld) {
+  constexpr int NV = FIELD ? 4 : 1;
+  // pair p of the tile: (-x0, -x1, -y0, -y1) and (-z0, -z1, q0, q1)
+  __shared__ ulonglong2 tA[T], tB[T];
+  __shared__ int tj[2 * T];                       // their particles
+  __shared__ int rs[kP2pRanges], rp[kP2pRanges];  // ranges: first particle, place
+  __shared__ int s_tot;
+  __shared__ float red[2 * NV][T];
+  int L = blockIdx.x, ia = 0, ib = 0;
+  if (BIG) {
+    const int4 it = items[blockIdx.x];
+    L = it.x;
+    ia = it.y;
+    ib = it.z;
+  }
   const int2 tbe = be[L];
-  const int b = tbe.x, nt = tbe.y - tbe.x;
-  // lanes per target as a compile-time constant: one body per S
-  const int Sd = nt <= 1 ? 32 : (nt <= 2 ? 16 : (nt <= 4 ? 8 : (nt <= 8 ? 4 : (nt <= 16 ? 2 : 1))));
-  auto body = [&](auto sc) {
-  constexpr int S = decltype(sc)::value;
-  const int sub = lane & (S - 1);
+  const int nt = tbe.y - tbe.x;
   const float4 tch = chi[L], tcl = clo[L];
   const float thr2 = FIELD ? fmaxf(tch.w, 1e-10f) : tch.w;
-  const int r0 = near_off[L], r1 = near_off[L + 1];
-  float4 *buf = sbuf[w];
-  const int step = 32 / S;
-  for (int tb = 0; tb < nt; tb += step) {
-    const int ti0 = tb + lane / S;
-    const bool act0 = ti0 < nt;
-    const int t0 = b + (act0 ? ti0 : 0);
-    const real4<float> q0 = rel32[t0];
-    float ks[4] = {}, kc[4] = {};
-    auto kahan = [](float &sum, float &comp, float v) {
-      const float y = v - comp;
-      const float t2 = sum + y;
-      comp = (t2 - sum) - y;
-      sum = t2;
-    };
-    // one target against a staged source, r2 clamped below at thr2 (h/8
-    // squared, at least the field guard 1e-10): close pairs and the point
-    // itself add a bounded stand-in that close_fix takes back
-    auto pair = [&](const real4<float> &q, const float4 &sv, float *p, float &rmin) {
-      const float dx = q.x - sv.x, dy = q.y - sv.y, dz = q.z - sv.z;
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      rmin = fminf(rmin, r2);
-      const float inv = rsqrt_ftz(fmaxf(r2, thr2));
-      const float qi = sv.w * inv;
-      p[0] += qi;
-      if (FIELD) {
-        const float q3 = qi * inv * inv;
-        p[1] -= q3 * dx;
-        p[2] -= q3 * dy;
-        p[3] -= q3 * dz;
-      }
-    };
-    // for a close pair: remove the stand-in (the same FP32 expressions) and
-    // add the pair from the FP64 positions (nothing for the point itself or
-    // inside the field guard)
-    auto close_fix = [&](const real4<float> &q, int t, const float4 &sv, int j, float *p) {
-      const float dx = q.x - sv.x, dy = q.y - sv.y, dz = q.z - sv.z;
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      if (!(r2 < thr2)) return;
-      {
-        const float inv = rsqrt_ftz(fmaxf(r2, thr2));
-        const float qi = sv.w * inv;
-        p[0] -= qi;
-        if (FIELD) {
-          const float q3 = qi * inv * inv;
-          p[1] += q3 * dx;
-          p[2] += q3 * dy;
-          p[3] += q3 * dz;
-        }
-      }
-      if (j == t) return;
-      const float ex = (float)(sx[t] - sx[j]), ey = (float)(sy[t] - sy[j]),
-                  ez = (float)(sz[t] - sz[j]);
-      const float e2 = ex * ex + ey * ey + ez * ez;
-      if (!(FIELD ? (e2 > 1e-10f) : (e2 > 0.f))) return;
-      const float inv = rsqrt_ftz(e2);
-      const float qi = sv.w * inv;
-      p[0] += qi;
-      if (FIELD) {
-        const float q3 = qi * inv * inv;
-        p[1] -= q3 * ex;
-        p[2] -= q3 * ey;
-        p[3] -= q3 * ez;
-      }
-    };
-    for (int rr = r0; rr < r1; ++rr) {
-      const int la = near_rng[2 * rr], lb = near_rng[2 * rr + 1];
-      if (lb <= la) continue;
-      if (rng_count(be, la, lb) > kBigRange) continue;  // chunked by the BIG pass
-      for (int lf = la; lf < lb; ++lf) {
-        const int2 sbe = be[lf];
-        const float4 sh = chi[lf], sl = clo[lf];
-        // source leaf centre relative to the target leaf centre
-        const float cx = (sh.x - tch.x) + (sl.x - tcl.x);
-        const float cy = (sh.y - tch.y) + (sl.y - tcl.y);
-        const float cz = (sh.z - tch.z) + (sl.z - tcl.z);
-        for (int j0 = sbe.x; j0 < sbe.y; j0 += 32) {
-          const int cnt = min(32, sbe.y - j0);
-          __syncwarp();
-          if (lane < cnt) {
-            const real4<float> r = rel32[j0 + lane];
-            buf[lane] = make_float4(cx + r.x, cy + r.y, cz + r.z, r.q);
+  const int r0 = BIG ? 0 : near_off[L], r1 = BIG ? 1 : near_off[L + 1];
+  for (int tb = 0; tb < nt; tb += T) {
+    const int rem = min(nt - tb, T);
+    const int S = T / rem;                        // threads per target
+    // target by target within a part, so that a warp reads few pairs at a time
+    const int sub = threadIdx.x / rem, ti = threadIdx.x - sub * rem;
+    const bool active = sub < S;
+    const int t = tbe.x + tb + ti;
+    const real4<float> q0 = rel32[t];
+    const uint64_t tx2 = pack2(q0.x, q0.x), ty2 = pack2(q0.y, q0.y), tz2 = pack2(q0.z, q0.z);
+    float ks[NV] = {}, kc[NV] = {};
+    for (int rb = r0; rb < r1; rb += kP2pRanges) {
+      // places of the ranges in their concatenation (heavy ones empty)
+      if (threadIdx.x < kP2pRanges) {
+        const int rr = rb + threadIdx.x;
+        int first = 0, len = 0;
+        if (rr < r1) {
+          const int la = BIG ? ia : near_rng[2 * rr], lb = BIG ? ib : near_rng[2 * rr + 1];
+          if (lb > la) {
+            first = be[la].x;
+            len = be[lb - 1].y - first;
+            if (!BIG && len > kBigRange) len = 0;   // chunked by the BIG pass
           }
-          __syncwarp();
-          float p0[4] = {0.f, 0.f, 0.f, 0.f};
-          float rmin = 3.0e38f;
-#pragma unroll 4
-          for (int k = sub; k < cnt; k += S) pair(q0, buf[k], p0, rmin);
-          const bool flag = rmin < thr2;
-          if (__any_sync(kFull, flag) && flag)
-            for (int k = sub; k < cnt; k += S) close_fix(q0, t0, buf[k], j0 + k, p0);
-#pragma unroll
-          for (int c = 0; c < (FIELD ? 4 : 1); ++c) kahan(ks[c], kc[c], p0[c]);
         }
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(kFull, incl, o);
+          if (threadIdx.x >= o) incl += v;
+        }
+        rs[threadIdx.x] = first;
+        rp[threadIdx.x] = incl - len;
+        if (threadIdx.x == kP2pRanges - 1) s_tot = incl;
+      }
+      __syncthreads();
+      const int tot = s_tot;
+      for (int k0 = 0; k0 < tot; k0 += 2 * T) {
+        const int np = min(T, (tot - k0 + 1) / 2);   // pairs of this tile
+        if (threadIdx.x < np) {
+          const int k = k0 + 2 * threadIdx.x;
+          int g = 0;                                 // last range that starts at or before k
+#pragma unroll
+          for (int o = kP2pRanges / 2; o > 0; o >>= 1)
+            if (rp[g + o] <= k) g += o;
+          float x[2], y[2], z[2], q[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (e == 1)
+              while (g < kP2pRanges - 1 && rp[g + 1] <= k + 1) ++g;
+            const bool in = k + e < tot;
+            const int j = in ? rs[g] + (k + e - rp[g]) : -1;
+            tj[2 * threadIdx.x + e] = j;
+            if (in) {
+              const float4 hi = phi[j], lo = plo[j];
+              x[e] = (tch.x - hi.x) + (tcl.x - lo.x);
+              y[e] = (tch.y - hi.y) + (tcl.y - lo.y);
+              z[e] = (tch.z - hi.z) + (tcl.z - lo.z);
+              q[e] = hi.w;
+            } else {                                 // no source: no charge, far away
+              x[e] = 1e18f;
+              y[e] = z[e] = q[e] = 0.f;
+            }
+          }
+          tA[threadIdx.x] = make_ulonglong2(pack2(x[0], x[1]), pack2(y[0], y[1]));
+          tB[threadIdx.x] = make_ulonglong2(pack2(z[0], z[1]), pack2(q[0], q[1]));
+        }
+        __syncthreads();
+        if (active) {
+          uint64_t p2[NV];
+#pragma unroll
+          for (int c = 0; c < NV; ++c) p2[c] = 0ull;
+          unsigned close = 0;   // 1 + pair of the last close pair, above it the one before
+#pragma unroll 2
+          for (int p = sub; p < np; p += S) {
+            const ulonglong2 A = tA[p], B = tB[p];
+            const uint64_t dx = add2(tx2, A.x), dy = add2(ty2, A.y), dz = add2(tz2, B.x);
+            const uint64_t r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+            float ra, rb2;
+            unpack2(r2, ra, rb2);
+            const bool ca = ra < thr2, cb = rb2 < thr2;
+            if (ca || cb) close = (close << 16) + (unsigned)(p + 1);
+            const uint64_t inv = pack2(ca ? 0.f : rsqrt_ftz(ra), cb ? 0.f : rsqrt_ftz(rb2));
+            const uint64_t qi = mul2(B.y, inv);
+            p2[0] = add2(p2[0], qi);
+            if (FIELD) {
+              const uint64_t q3 = mul2(qi, mul2(inv, inv));
+              p2[NV > 1 ? 1 : 0] = fma2(q3, dx, p2[NV > 1 ? 1 : 0]);
+              p2[NV > 1 ? 2 : 0] = fma2(q3, dy, p2[NV > 1 ? 2 : 0]);
+              p2[NV > 1 ? 3 : 0] = fma2(q3, dz, p2[NV > 1 ? 3 : 0]);
+            }
+          }
+          float pv[NV];
+#pragma unroll
+          for (int c = 0; c < NV; ++c) {
+            float lo, hi;
+            unpack2(p2[c], lo, hi);
+            pv[c] = lo + hi;
+          }
+          if (close) {
+            // close pairs, left out above, from the FP64 positions (nothing
+            // for the point itself or inside the field guard).  Mostly the
+            // point itself alone, whose place is known; else the part is
+            // searched
+            const bool one = close < 65536u;
+            for (int p = one ? (int)close - 1 : sub; p < np; p += one ? T : S) {
+              const float4 fa = reinterpret_cast<const float4 *>(tA)[p],
+                           fb = reinterpret_cast<const float4 *>(tB)[p];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const float dx = q0.x + (e ? fa.y : fa.x), dy = q0.y + (e ? fa.w : fa.z),
+                            dz = q0.z + (e ? fb.y : fb.x);
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                if (!(r2 < thr2)) continue;
+                const int j = tj[2 * p + e];
+                if (j < 0) continue;
+                if (j == t) continue;
+                const float sq = e ? fb.w : fb.z;
+                const float ex = (float)(sx[t] - sx[j]), ey = (float)(sy[t] - sy[j]),
+                            ez = (float)(sz[t] - sz[j]);
+                const float e2 = ex * ex + ey * ey + ez * ez;
+                if (!(FIELD ? (e2 > 1e-10f) : (e2 > 0.f))) continue;
+                const float inv = rsqrt_ftz(e2);
+                const float qi = sq * inv;
+                pv[0] += qi;
+                if (FIELD) {
+                  const float q3 = qi * (inv * inv);
+                  pv[NV > 1 ? 1 : 0] += q3 * ex;
+                  pv[NV > 1 ? 2 : 0] += q3 * ey;
+                  pv[NV > 1 ? 3 : 0] += q3 * ez;
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < NV; ++c) {
+            const float y = pv[c] - kc[c];
+            const float s = ks[c] + y;
+            kc[c] = (s - ks[c]) - y;
+            ks[c] = s;
+          }
+        }
+        __syncthreads();
       }
     }
-    double v[4];
+    // a target's parts added by one thread per value, compensated, and
+    // stored (the field is minus the gradient's sum)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) v[c] = (double)ks[c] - (double)kc[c];
-    for (int o = 1; o < S; o <<= 1)
-#pragma unroll
-      for (int c = 0; c < (FIELD ? 4 : 1); ++c) v[c] += __shfl_xor_sync(kFull, v[c], o);
-    if (act0 && sub == 0) {
-      acc_pot[t0] = v[0];
-      if (FIELD) {
-        acc_fld[3 * (size_t)t0] = v[1];
-        acc_fld[3 * (size_t)t0 + 1] = v[2];
-        acc_fld[3 * (size_t)t0 + 2] = v[3];
-      }
+    for (int c = 0; c < NV; ++c) {
+      red[c][threadIdx.x] = ks[c];
+      red[NV + c][threadIdx.x] = kc[c];
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < rem * NV; i += T) {
+      const int tt = i / NV, c = i - tt * NV;
+      float s = red[c][tt], e = -red[NV + c][tt];
+      for (int k = 1; k < S; ++k) {
+        const float v = red[c][tt + k * rem];
+        const float n = s + v, bb = n - s;
+        e += ((s - (n - bb)) + (v - bb)) - red[NV + c][tt + k * rem];
+        s = n;
+      }
+      const double v = (double)s + (double)e;
+      const int64_t o = tbe.x + tb + tt;
+      double *dst = c == 0 ? acc_pot + o : acc_fld + 3 * o + (c - 1);
+      const double w = c == 0 ? v : -v;
+      if (BIG) atomicAdd(dst, w);
+      else *dst = w;
+    }
+    __syncthreads();
   }
-  };
-  if (Sd == 32) body(std::integral_constant<int, 32>{});
-  else if (Sd == 16) body(std::integral_constant<int, 16>{});
-  else if (Sd == 8) body(std::integral_constant<int, 8>{});
-  else if (Sd == 4) body(std::integral_constant<int, 4>{});
-  else if (Sd == 2) body(std::integral_constant<int, 2>{});
-  else body(std::integral_constant<int, 1>{});
 }
 
 template <bool FIELD>
 void launch_mixed(AranGpuSolver3d *s, cudaStream_t st) {
   DevTree &t = s->tree;
-  k_p2p_warp<FIELD><<<ceil_div(t.nleaves, 4), 128, 0, st>>>(
-      t.nleaves, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr,
-      s->sx.ptr, s->sy.ptr, s->sz.ptr, s->rel32.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
-  ACHECK(cudaGetLastError());
-  s->launches++;
-  if (!t.n_big) return;
-  k_p2p_chunk<FIELD><<<t.n_big, 128, 0, st>>>(
-      t.big_items.ptr, t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr, s->sx.ptr, s->sy.ptr,
-      s->sz.ptr, s->rel32.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
-  ACHECK(cudaGetLastError());
-  s->launches++;
+  auto run = [&](auto kern, int grid) {
+    kern<<<grid, kTileThreads, 0, st>>>(
+        t.big_items.ptr, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr,
+        t.leaf_clo.ptr, s->sx.ptr, s->sy.ptr, s->sz.ptr, s->rel32.ptr, s->abs_hi.ptr,
+        s->abs_lo.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
+    ACHECK(cudaGetLastError());
+    s->launches++;
+  };
+  run(k_p2p_tile<FIELD, false, kTileThreads>, t.nleaves);
+  if (t.n_big) run(k_p2p_tile<FIELD, true, kTileThreads>, t.n_big);
 }
 
 template <bool FIELD, bool BIG>

@@ -4,7 +4,7 @@
 //   clear_func :399-410   -> one memset of all expansions
 //   up_func :412-450      -> k_p2m (leaves) + k_m2m_rotate (level by level)
 //   far_func :333-354     -> k_m2l_sibling (m2l.cu)
-//   near_func :254-324    -> k_p2p_warp, k_p2p64 (p2p.cu)
+//   near_func :254-324    -> k_p2p_tile, k_p2p64 (p2p.cu)
 //   down_func :452-490    -> k_l2l_rotate (level by level) + k_l2p
 // The operators are the "point and shoot" rotation flavour of
 // aran/aransphericalseriesd-rotate.c (rotate to the z axis, translate along

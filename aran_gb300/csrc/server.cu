@@ -96,7 +96,8 @@ int64_t footprint_bytes(const AranGpuConfig3d *c, int64_t n) {
   b += n * (4 * 8 + 2 * 8 + 8);    // sorted positions/charges, keys (2x), perm/idx
   b += n * (4 * real + 4 * 8);     // relative coordinates, accumulators
   b += nodes * (8 + 12 + 1 + 16 + 24 + 27 * 4 + 4 * 4 + 8);       // node arrays
-  b += nodes * (int64_t)(tri(p) + tri(p + 1)) * 2 * real;          // expansions
+  b += nodes * (int64_t)(tri(p) + 2 * tri(p + 1)) * 2 * real;      // expansions, M2L sums
+  b += n * (8 * real);                                             // hi + lo positions
   b += nodes * (189 * 6 + 8) + nodes * 60 * 8;                     // far/near lists
   return b + (64ll << 20);
 }

@@ -446,21 +446,30 @@ __global__ void k_parent_scatter(int nn, const int *__restrict__ flags, const in
   if (flags[i]) parents[pos[i]] = i;
 }
 
-// relative (leaf-centred) particle coordinates for the kernels
+// relative (leaf-centred) particle coordinates for the kernels; in FP32 also
+// the positions as hi + lo pairs
 template <typename T>
 __global__ void k_relative(int64_t n, const int *__restrict__ incl, const int *__restrict__ leaf_node,
                            const double *__restrict__ center, const double *__restrict__ sx,
                            const double *__restrict__ sy, const double *__restrict__ sz,
-                           const double *__restrict__ sq, real4<T> *__restrict__ rel) {
+                           const double *__restrict__ sq, real4<T> *__restrict__ rel,
+                           float4 *__restrict__ hi, float4 *__restrict__ lo) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int node = leaf_node[incl[i] - 1];
+  const double x = sx[i], y = sy[i], z = sz[i];
   real4<T> r;
-  r.x = (T)(sx[i] - center[3 * node]);
-  r.y = (T)(sy[i] - center[3 * node + 1]);
-  r.z = (T)(sz[i] - center[3 * node + 2]);
+  r.x = (T)(x - center[3 * node]);
+  r.y = (T)(y - center[3 * node + 1]);
+  r.z = (T)(z - center[3 * node + 2]);
   r.q = (T)sq[i];
   rel[i] = r;
+  if (sizeof(T) == 4) {
+    const float hx = (float)x, hy = (float)y, hz = (float)z;
+    hi[i] = make_float4(hx, hy, hz, (float)r.q);
+    lo[i] = make_float4((float)(x - (double)hx), (float)(y - (double)hy),
+                        (float)(z - (double)hz), 0.f);
+  }
 }
 
 template <typename T>
@@ -749,14 +758,17 @@ void build_lists(AranGpuSolver3d *s) {
   // relative coordinates
   if (s->cfg.precision == ARAN_PRECISION_MIXED) {
     s->rel32.reserve(n);
+    s->abs_hi.reserve(n);
+    s->abs_lo.reserve(n);
     k_relative<float><<<ceil_div(n, TB), TB, 0, st>>>(n, incl, t.leaf_node.ptr, t.center.ptr,
                                                        s->sx.ptr, s->sy.ptr, s->sz.ptr, s->sq.ptr,
-                                                       s->rel32.ptr);
+                                                       s->rel32.ptr, s->abs_hi.ptr,
+                                                       s->abs_lo.ptr);
   } else {
     s->rel64.reserve(n);
     k_relative<double><<<ceil_div(n, TB), TB, 0, st>>>(n, incl, t.leaf_node.ptr, t.center.ptr,
                                                         s->sx.ptr, s->sy.ptr, s->sz.ptr, s->sq.ptr,
-                                                        s->rel64.ptr);
+                                                        s->rel64.ptr, nullptr, nullptr);
   }
   s->launches++;
   // near ranges (and semifar nodes) per leaf
