@@ -149,23 +149,6 @@ struct OpTables {
   DBuf<uint8_t> lm; // (l,m) of coefficient index, 2*tri(p+1)
 };
 
-// tables of the kkylin flavour (kkylin.cu): alpha/beta and, per direction
-// (343 M2L offsets, 8 M2M and 8 L2L octants), r, cos/sin theta, cos/sin phi
-// and the harmonics of the direction
-template <typename T>
-struct KkTables {
-  int p = -1;
-  DBuf<T> alpha, ialpha, beta, dirs[3];   // ialpha = 1 / alpha
-  int stride[3] = {0, 0, 0};
-  void release() {
-    alpha.release();
-    ialpha.release();
-    beta.release();
-    for (auto &d : dirs) d.release();
-    p = -1;
-  }
-};
-
 struct Stage {
   enum { TOTAL, SORT, TREE, LISTS, P2M, M2M, M2L, L2L, L2P, P2P, H2D, D2H, SEMI_P2L, SEMI_M2P,
          NSTAGE };
@@ -182,8 +165,6 @@ struct AranGpuSolver3d {
   double scale_e = 1.;   // 2^E >= root extent
   aran::OpTables<double> t64;
   aran::OpTables<float> t32;
-  aran::KkTables<double> kk64;
-  aran::KkTables<float> kk32;
   aran::DevTree tree;
   // particles (sorted)
   aran::DBuf<uint64_t> keys_in, keys_out;
@@ -252,9 +233,6 @@ void build_tables_fp64(AranGpuSolver3d *s);   // FP64 tables beside a mixed solv
 int dir_offset(int p, int kind, int what);
 // passes.cu
 void run_passes(AranGpuSolver3d *s);
-// kkylin.cu: stage 0 = M2M, 1 = M2L, 2 = L2L
-void build_kkylin_tables(AranGpuSolver3d *s);
-void kkylin_pass(AranGpuSolver3d *s, int stage);
 // parts of the offset lists of a small FP64 M2L pass: the least
 // number of waves of CTAs times the work of a part (1 / K of the offsets and
 // the set-up, about 1/40 of a whole list)

@@ -798,7 +798,6 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   const int p = s->cfg.order;
   const int nm = tri(p), nl = tri(p + 1);
   const bool field = s->cfg.field != 0;
-  const bool kk = s->cfg.flavour == ARAN_FLAVOUR_KKYLIN;
   multb.reserve((size_t)t.nnodes * nm * 2 + 2);   // the M2L copies whole 16-byte units
   locb.reserve((size_t)t.nnodes * nl * 2);
   cplx<T> *mult = reinterpret_cast<cplx<T> *>(multb.ptr);
@@ -807,8 +806,9 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   s->acc_fld.reserve(3 * t.n);
   // FP64 root levels of the mixed rotation path: nodes of depth <= R keep
   // FP64 expansions (the first n_root nodes, level-major order); M2M into
-  // them, M2L at them and L2L between them run in FP64
-  const int R = (sizeof(T) == 4 && !kk && s->root64_depth >= 0)
+  // them, M2L at them and L2L between them run in FP64 (the kkylin flavour
+  // runs without them)
+  const int R = (sizeof(T) == 4 && s->cfg.flavour != ARAN_FLAVOUR_KKYLIN && s->root64_depth >= 0)
                     ? (s->root64_depth < t.nlevels - 1 ? s->root64_depth : t.nlevels - 1)
                     : -1;
   const int n_root = R >= 0 ? t.level_off[R + 1] : 0;
@@ -858,8 +858,7 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2M + 1], st));
   // M2M, deepest level first
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2M], st));
-  if (kk) kkylin_pass(s, 0);
-  else if (R < 0) m2m_levels<T>(s, tb, mult, t.nlevels - 2, 0, st);
+  if (R < 0) m2m_levels<T>(s, tb, mult, t.nlevels - 2, 0, st);
   else {
     // FP32 up to the children of depth-R parents, widened, then FP64; the
     // FP64 multipoles of depths <= R go back to FP32 for the semifar M2P
@@ -871,8 +870,7 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2M + 1], st));
   // M2L over every node of depth >= 2
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2L], st));
-  if (kk) kkylin_pass(s, 1);
-  else if (R < 0) launch_m2l(s, sizeof(T) == 8, 0, t.n_parents, st);
+  if (R < 0) launch_m2l(s, sizeof(T) == 8, 0, t.n_parents, st);
   else {
     launch_m2l(s, true, 0, n_root_parents, st);
     launch_m2l(s, false, n_root_parents, t.n_parents - n_root_parents, st);
@@ -883,8 +881,7 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2L + 1], st));
   // L2L
   ACHECK(cudaEventRecord(s->ev[2 * Stage::L2L], st));
-  if (kk) kkylin_pass(s, 2);
-  else if (R < 0) l2l_levels<T>(s, tb, loc, 3, t.nlevels - 1, st);
+  if (R < 0) l2l_levels<T>(s, tb, loc, 3, t.nlevels - 1, st);
   else {
     // the FP32 locals of depths <= R hold only semifar P2L terms: added to
     // the FP64 ones, carried down in FP64, narrowed back for the deeper levels

@@ -722,12 +722,11 @@ void build_lists(AranGpuSolver3d *s) {
   }
   DBuf<int> &cntbuf = s->scan_tmp;
   cntbuf.reserve((size_t)nn + 1 + (size_t)n + 1);
-  // M2L pairs: the lists only feed the kkylin M2L (the rotation kernels
-  // find their sources from the colleague grids); otherwise counts and
-  // lists are made when asked for (count_far_lists, build_far_lists)
+  // M2L pairs: the kernels find their sources from the colleague grids;
+  // counts and lists are made when asked for (count_far_lists,
+  // build_far_lists)
   t.far_counted = false;
   t.far_built = false;
-  if (s->cfg.flavour == ARAN_FLAVOUR_KKYLIN) build_far_lists(s);
 
   // leaves in Morton order
   DBuf<int> &lflags = s->idx_in;  // reuse (n ints)
