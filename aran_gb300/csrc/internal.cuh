@@ -168,7 +168,7 @@ struct AranGpuSolver3d {
   aran::DevTree tree;
   // particles (sorted)
   aran::DBuf<uint64_t> keys_in, keys_out;
-  aran::DBuf<int> idx_in, perm;
+  aran::DBuf<int> idx_in, perm, sort_tmp;
   aran::DBuf<uint8_t> cub_tmp;
   aran::DBuf<double> sx, sy, sz, sq;     // sorted FP64 positions/charges
   aran::DBuf<aran::real4<double>> rel64;

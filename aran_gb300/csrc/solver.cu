@@ -202,7 +202,7 @@ void aran_gpu_solver3d_destroy(AranGpuSolver3d *s) {
     tb->oct_lanes[0].release(); tb->oct_lanes[1].release();
   }
   s->keys_in.release(); s->keys_out.release(); s->idx_in.release(); s->perm.release();
-  s->cub_tmp.release(); s->sx.release(); s->sy.release(); s->sz.release(); s->sq.release();
+  s->cub_tmp.release(); s->sort_tmp.release(); s->sx.release(); s->sy.release(); s->sz.release(); s->sq.release();
   s->rel64.release(); s->rel32.release(); s->abs_hi.release(); s->abs_lo.release(); s->acc_pot.release(); s->acc_fld.release();
   s->io_xyz.release(); s->io_q.release(); s->io_pot.release(); s->io_fld.release();
   s->mult64.release(); s->loc64.release(); s->mult32.release(); s->loc32.release();

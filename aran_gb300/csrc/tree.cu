@@ -23,6 +23,8 @@
 // level's kernels then run over the nodes of all systems at once.
 #include <cub/cub.cuh>
 
+#include <utility>
+
 #include "internal.cuh"
 
 namespace aran {
@@ -446,6 +448,31 @@ __global__ void k_parent_scatter(int nn, const int *__restrict__ flags, const in
   if (flags[i]) parents[pos[i]] = i;
 }
 
+// system (a sort key) and place of every sorted particle
+__global__ void k_sort_systems(int64_t n, int nsys, const int *__restrict__ off,
+                               const int *__restrict__ perm, int *__restrict__ sys,
+                               int *__restrict__ pos) {
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int o = perm[i];
+  int lo = 0, hi = nsys;                 // last system with off <= o
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (off[mid] <= o) lo = mid; else hi = mid;
+  }
+  sys[i] = lo;
+  pos[i] = (int)i;
+}
+
+__global__ void k_sort_gather(int64_t n, const int *__restrict__ pos,
+                              const uint64_t *__restrict__ keys, const int *__restrict__ perm,
+                              uint64_t *__restrict__ keys_o, int *__restrict__ perm_o) {
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  keys_o[i] = keys[pos[i]];
+  perm_o[i] = perm[pos[i]];
+}
+
 // relative (leaf-centred) particle coordinates for the kernels; in FP32 also
 // the positions as hi + lo pairs
 template <typename T>
@@ -516,6 +543,35 @@ void grow_nodes(DevTree &t, size_t need, size_t keep, cudaStream_t st) {
   t.center.grow_keep(3 * need, 3 * keep, st);
 }
 
+// A forest's particles, sorted by key over all systems, into their systems: a
+// stable sort by system of the sorted places (one pass per 8 bits of the
+// system number), which leaves each system's keys and input order as a sort
+// of its own would.  (A segmented sort gives a system one block: 48 systems of
+// 1 k to 100 k particles 1.46 ms, this 0.35.)
+void sort_systems(AranGpuSolver3d *s, int64_t n, int nsys, cudaStream_t st) {
+  const int TB = 256;
+  DBuf<int> &tmp = s->sort_tmp;
+  tmp.reserve(4 * (size_t)n);
+  int *sys_in = tmp.ptr, *sys_out = sys_in + n, *pos_in = sys_out + n, *pos_out = pos_in + n;
+  k_sort_systems<<<ceil_div(n, TB), TB, 0, st>>>(n, nsys, s->sys_off.ptr, s->perm.ptr, sys_in,
+                                                  pos_in);
+  ACHECK(cudaGetLastError());
+  int bits = 1;
+  while ((1 << bits) < nsys) ++bits;
+  size_t bytes = 0;
+  ACHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, sys_in, sys_out, pos_in, pos_out, (int)n,
+                                         0, bits, st));
+  s->cub_tmp.reserve(bytes);
+  ACHECK(cub::DeviceRadixSort::SortPairs(s->cub_tmp.ptr, bytes, sys_in, sys_out, pos_in, pos_out,
+                                         (int)n, 0, bits, st));
+  k_sort_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, pos_out, s->keys_out.ptr, s->perm.ptr,
+                                                 s->keys_in.ptr, s->idx_in.ptr);
+  ACHECK(cudaGetLastError());
+  std::swap(s->keys_in, s->keys_out);
+  std::swap(s->idx_in, s->perm);
+  s->launches += 5;
+}
+
 // the nodes of one level about to be split are shown to the host leaf
 // predicate; those it keeps as leaves lose their flag
 void apply_leaf_predicate(AranGpuSolver3d *s, int off, int cnt, int d, int *d_flags,
@@ -575,25 +631,14 @@ void build_tree(AranGpuSolver3d *s, int64_t n, const double *d_xyz, const double
   k_keys<<<ceil_div(n, TB), TB, 0, st>>>(n, d_xyz, d_q, nsys, s->sys_off.ptr, s->sys_box.ptr,
                                           s->keys_in.ptr, s->idx_in.ptr, s->err_dev.ptr);
   s->launches++;
-  // the systems are contiguous in the input: each is sorted in place
   size_t bytes = 0;
-  if (nsys == 1) {
-    ACHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, s->keys_in.ptr, s->keys_out.ptr,
-                                           s->idx_in.ptr, s->perm.ptr, (int)n, 0, 3 * kKeyBits, st));
-    s->cub_tmp.reserve(bytes);
-    ACHECK(cub::DeviceRadixSort::SortPairs(s->cub_tmp.ptr, bytes, s->keys_in.ptr, s->keys_out.ptr,
-                                           s->idx_in.ptr, s->perm.ptr, (int)n, 0, 3 * kKeyBits, st));
-  } else {
-    const int *ob = s->sys_off.ptr, *oe = s->sys_off.ptr + 1;
-    ACHECK(cub::DeviceSegmentedRadixSort::SortPairs(nullptr, bytes, s->keys_in.ptr, s->keys_out.ptr,
-                                                    s->idx_in.ptr, s->perm.ptr, (int)n, nsys,
-                                                    ob, oe, 0, 3 * kKeyBits, st));
-    s->cub_tmp.reserve(bytes);
-    ACHECK(cub::DeviceSegmentedRadixSort::SortPairs(s->cub_tmp.ptr, bytes, s->keys_in.ptr,
-                                                    s->keys_out.ptr, s->idx_in.ptr, s->perm.ptr,
-                                                    (int)n, nsys, ob, oe, 0, 3 * kKeyBits, st));
-  }
+  ACHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, s->keys_in.ptr, s->keys_out.ptr,
+                                         s->idx_in.ptr, s->perm.ptr, (int)n, 0, 3 * kKeyBits, st));
+  s->cub_tmp.reserve(bytes);
+  ACHECK(cub::DeviceRadixSort::SortPairs(s->cub_tmp.ptr, bytes, s->keys_in.ptr, s->keys_out.ptr,
+                                         s->idx_in.ptr, s->perm.ptr, (int)n, 0, 3 * kKeyBits, st));
   s->launches += 4;
+  if (nsys > 1) sort_systems(s, n, nsys, st);
   s->sx.reserve(n);
   s->sy.reserve(n);
   s->sz.reserve(n);
