@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(128, 8) k_p2p64(
 // where 128 took 0.61; tiles of twice and four times the sources changed
 // nothing; 10 blocks an SM with 48 registers a thread beat 8, 6 and 12.
 constexpr int kP2pRanges = 32;   // near ranges taken together
-constexpr int kTileThreads = 128;
 
 template <bool FIELD, bool BIG, int T>
 __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
@@ -440,16 +439,23 @@ __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
 template <bool FIELD>
 void launch_mixed(AranGpuSolver3d *s, cudaStream_t st) {
   DevTree &t = s->tree;
+  // 64 threads per leaf at leaf capacities up to 24, 128 above (1M Plummer,
+  // 400k uniform, 300k blobs: 0.77, 0.18, 0.27 ms at capacity 20 with 64, 0.92,
+  // 0.20, 0.31 with 128; 2.08, 0.17, 0.63 and 1.27, 0.19, 0.57 at 64).  (The
+  // capacity and not the mean occupancy: a system's bits do not depend on
+  // its company in a forest.)
+  const bool small = s->cfg.maxbox <= 24;
+  const int T = small ? 64 : 128;
   auto run = [&](auto kern, int grid) {
-    kern<<<grid, kTileThreads, 0, st>>>(
+    kern<<<grid, T, 0, st>>>(
         t.big_items.ptr, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr,
         t.leaf_clo.ptr, s->sx.ptr, s->sy.ptr, s->sz.ptr, s->rel32.ptr, s->abs_hi.ptr,
         s->abs_lo.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
     ACHECK(cudaGetLastError());
     s->launches++;
   };
-  run(k_p2p_tile<FIELD, false, kTileThreads>, t.nleaves);
-  if (t.n_big) run(k_p2p_tile<FIELD, true, kTileThreads>, t.n_big);
+  run(small ? k_p2p_tile<FIELD, false, 64> : k_p2p_tile<FIELD, false, 128>, t.nleaves);
+  if (t.n_big) run(small ? k_p2p_tile<FIELD, true, 64> : k_p2p_tile<FIELD, true, 128>, t.n_big);
 }
 
 template <bool FIELD, bool BIG>
