@@ -29,6 +29,7 @@
 #include <cstring>
 
 #include "internal.cuh"
+#include "f32x2.cuh"
 
 namespace aran {
 namespace {
@@ -55,17 +56,6 @@ __device__ __forceinline__ zd zinv(zd a) {
   double w = 1.0 / r2;
   return cmake(a.re * w, -a.im * w);
 }
-// a^e by binary exponentiation
-__device__ __forceinline__ zd zpow(zd a, int e) {
-  zd r = cmake(1.0, 0.0);
-  while (e) {
-    if (e & 1) r = zmul(r, a);
-    a = zmul(a, a);
-    e >>= 1;
-  }
-  return r;
-}
-
 __device__ __forceinline__ double shfl_sum(double v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -101,13 +91,19 @@ __global__ void k2_keys(int64_t n, int nsys, const int64_t *__restrict__ offs,
 
 __global__ void k2_gather(int64_t n, const int *__restrict__ perm, const double *__restrict__ xy,
                           const double *__restrict__ q, double *__restrict__ sx,
-                          double *__restrict__ sy, double *__restrict__ sq) {
+                          double *__restrict__ sy, double *__restrict__ sq,
+                          float4 *__restrict__ hl) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
-  sx[i] = xy[2 * (int64_t)o];
-  sy[i] = xy[2 * (int64_t)o + 1];
+  const double x = xy[2 * (int64_t)o], y = xy[2 * (int64_t)o + 1];
+  sx[i] = x;
+  sy[i] = y;
   sq[i] = q[o];
+  if (hl) {              // FP32 hi + lo positions of the mixed near field
+    const float hx = (float)x, hy = (float)y;
+    hl[i] = make_float4(hx, hy, (float)(x - (double)hx), (float)(y - (double)hy));
+  }
 }
 
 // ---------------------------------------------------------------- quadtree
@@ -381,8 +377,15 @@ __global__ void k2_m2m(int cnt, int off, int p, const int *__restrict__ child,
 }
 
 // M2L: warp per target node, lanes per local term i:
-// L_i += (-1/z)^i sum_{j=1}^{p-1} C(i+j-1, j-1) a_{-j} z^{-j}, z = zt - zs
-// (aran_laurent_seriesd_to_taylor, aranlaurentseriesd.c:409-452).
+// L_i += (-1)^i w^i sum_{j=1}^{p-1} C(i+j-1, j-1) a_{-j} w^j, w = 1 / (zt - zs)
+// (aran_laurent_seriesd_to_taylor, aranlaurentseriesd.c:409-452).  The FP64
+// pipe is the whole cost (half a lane a cycle per scheduler), so the lanes
+// take a source each for w, a scan of products makes its powers (five
+// complex products) and the terms a_{-j} w^j are shared through shared
+// memory: two operations per (i, j) where Horner's rule in every lane took
+// six, about 70 a source where it took 175.  60k particles, order 20, leaf
+// 32 (137k translations) on GB300: 0.53 ms, 1.52 before.
+template <int S>
 __global__ void __launch_bounds__(128) k2_m2l(int nn, int p, const int *__restrict__ far_off,
                                               const int *__restrict__ far_src,
                                               const double *__restrict__ center,
@@ -392,7 +395,7 @@ __global__ void __launch_bounds__(128) k2_m2l(int nn, int p, const int *__restri
   const int P1 = p + 1;
   const int SP = p | 1;                  // odd row stride: conflict-free lanes
   double *tab = smem;                    // tab[i * SP + j] = C(i+j-1, j-1)
-  zd *src = reinterpret_cast<zd *>(smem + P1 * SP);
+  zd *src = reinterpret_cast<zd *>(smem + ((P1 * SP + 1) & ~1));
   for (int x = threadIdx.x; x < P1 * SP; x += blockDim.x) {
     int i = x / SP, j = x % SP;
     tab[x] = (j >= 1 && j < p) ? binom[(i + j - 1) * nb + (j - 1)] : 0.0;
@@ -401,33 +404,65 @@ __global__ void __launch_bounds__(128) k2_m2l(int nn, int p, const int *__restri
   int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int t = blockIdx.x * (blockDim.x >> 5) + wl;
   if (t >= nn) return;
-  int f0 = far_off[t], f1 = far_off[t + 1];
+  const int f0 = far_off[t], f1 = far_off[t + 1];
   if (f0 == f1) return;
-  zd *ms = src + wl * P1;
-  double tx = center[2 * t], ty = center[2 * t + 1];
-  zd acc[3];
-  for (int s = 0; s < 3; ++s) acc[s] = cmake(0.0, 0.0);
-  for (int f = f0; f < f1; ++f) {
-    int sn = far_src[f];
-    __syncwarp();
-    for (int k = lane; k <= p; k += 32) ms[k] = mult[(int64_t)sn * P1 + k];
-    __syncwarp();
-    zd inv = zinv(cmake(tx - center[2 * sn], ty - center[2 * sn + 1]));
-    zd ninv = cmake(-inv.re, -inv.im);
-    for (int s = 0; s < 3; ++s) {
-      int i = lane + 32 * s;
-      if (i > p) break;
-      const double *row = tab + i * SP;
-      zd sum = cmake(0.0, 0.0);
-      for (int j = p - 1; j >= 1; --j) sum = zmul(cadd(sum, zscale(ms[j], row[j])), inv);
-      acc[s] = cadd(acc[s], zmul(sum, zpow(ninv, i)));
+  zd *ms = src + wl * 32 * S;
+  const double tx = center[2 * t], ty = center[2 * t + 1];
+  zd acc[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) acc[s] = cmake(0.0, 0.0);
+  for (int g = f0; g < f1; g += 32) {
+    const int cnt = min(32, f1 - g);
+    // lane k: w of source g + k
+    int sn = far_src[g + min(lane, cnt - 1)];
+    const zd w = zinv(cmake(tx - center[2 * sn], ty - center[2 * sn + 1]));
+    for (int k = 0; k < cnt; ++k) {
+      const int sk = __shfl_sync(0xffffffffu, sn, k);
+      zd a[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        const int j = lane + 32 * s;
+        a[s] = j >= 1 && j < p ? mult[(int64_t)sk * P1 + j] : cmake(0.0, 0.0);
+      }
+      zd v = cmake(__shfl_sync(0xffffffffu, w.re, k), __shfl_sync(0xffffffffu, w.im, k));
+      // lane l: w^(l+1)
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const zd u = cmake(__shfl_up_sync(0xffffffffu, v.re, o),
+                           __shfl_up_sync(0xffffffffu, v.im, o));
+        if (lane >= o) v = zmul(v, u);
+      }
+      zd wp[S];
+      wp[0] = cmake(__shfl_up_sync(0xffffffffu, v.re, 1), __shfl_up_sync(0xffffffffu, v.im, 1));
+      if (lane == 0) wp[0] = cmake(1.0, 0.0);
+      const zd w32 = cmake(__shfl_sync(0xffffffffu, v.re, 31), __shfl_sync(0xffffffffu, v.im, 31));
+#pragma unroll
+      for (int s = 1; s < S; ++s) wp[s] = zmul(wp[s - 1], w32);
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < S; ++s) ms[lane + 32 * s] = zmul(a[s], wp[s]);
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        const int i = lane + 32 * s;
+        if (i > p) break;
+        const double *row = tab + i * SP;
+        zd sum = cmake(0.0, 0.0);
+        for (int j = 1; j < p; ++j) {
+          sum.re = fma(row[j], ms[j].re, sum.re);
+          sum.im = fma(row[j], ms[j].im, sum.im);
+        }
+        acc[s] = cmake(fma(-sum.im, wp[s].im, fma(sum.re, wp[s].re, acc[s].re)),
+                       fma(sum.im, wp[s].re, fma(sum.re, wp[s].im, acc[s].im)));
+      }
     }
   }
-  for (int s = 0; s < 3; ++s) {
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
     int i = lane + 32 * s;
     if (i <= p) {
       zd *o = loc + (int64_t)t * P1 + i;
-      *o = cadd(*o, acc[s]);
+      *o = cadd(*o, (i & 1) ? cmake(-acc[s].re, -acc[s].im) : acc[s]);
     }
   }
 }
@@ -460,34 +495,82 @@ __global__ void k2_l2l(int cnt, int off, int p, const int *__restrict__ parent,
   }
 }
 
-// P2P: warp per leaf, lanes over targets; every source of the near ranges
+// 1 / x in FP64 from the upper word y0 of the hardware approximation (20
+// significant bits) by one third-order Newton (Householder) step, y0 + y0 (e
+// + e^2) with e = 1 - x y0 rounded once: three FP64 operations, within an ulp
+// of the correctly rounded value
+__device__ __forceinline__ double rcp_h3(double x) {
+  double a;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(a) : "d"(x));
+  const double y0 = __hiloint2double(__double2hiint(a), 0);
+  const double e = fma(-x, y0, 1.0);
+  return fma(y0, fma(e, e, e), y0);
+}
+
+// P2P: a block of 128 threads per leaf, every source of the near ranges
 // (tests/dummypot.c:62-76, both directions covered by the symmetric lists).
-__global__ void k2_p2p(int nleaves, const int *__restrict__ leaf_be, const int *__restrict__ near_off,
-                       const int2 *__restrict__ near_rng, const double *__restrict__ sx,
-                       const double *__restrict__ sy, const double *__restrict__ sq,
-                       zd *__restrict__ near_acc) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= nleaves) return;
-  int b = leaf_be[warp], e = leaf_be[warp + 1];
-  int r0 = near_off[warp], r1 = near_off[warp + 1];
-  for (int base = b; base < e; base += 32) {
-    int i = base + lane;
-    bool on = i < e;
-    double xi = on ? sx[i] : 0.0, yi = on ? sy[i] : 0.0;
+// As in the 3D FP64 near field the FP64 pipe times idle lanes is the cost: a
+// leaf of n targets gets floor(128 / n) threads per target, striding over
+// the concatenation of its near ranges; 10 FP64 operations a pair (a warp
+// per leaf with its targets in the lanes kept 46 % of them busy at 15 points
+// a leaf, and the correctly rounded reciprocal took half the operations).
+__global__ void __launch_bounds__(128) k2_p2p(int nleaves, const int *__restrict__ leaf_be,
+                                              const int *__restrict__ near_off,
+                                              const int2 *__restrict__ near_rng,
+                                              const double *__restrict__ sx,
+                                              const double *__restrict__ sy,
+                                              const double *__restrict__ sq,
+                                              zd *__restrict__ near_acc) {
+  __shared__ zd red[128];
+  const int L = blockIdx.x;
+  const int b = leaf_be[L], nt = leaf_be[L + 1] - b;
+  const int r0 = near_off[L], r1 = near_off[L + 1];
+  for (int tb = 0; tb < nt; tb += 128) {
+    const int rem = min(nt - tb, 128);
+    const int s = 128 / rem;                  // threads per target
+    const int ti = threadIdx.x / s, sub = threadIdx.x - ti * s;
+    const bool active = ti < rem;
+    const int t = b + tb + (active ? ti : 0);
     double re = 0.0, im = 0.0;
-    for (int r = r0; r < r1; ++r) {
-      int2 rg = near_rng[r];
-      int j0 = leaf_be[rg.x], j1 = leaf_be[rg.y];
-      for (int j = j0; j < j1; ++j) {
-        double dx = xi - sx[j], dy = yi - sy[j];
-        double r2 = dx * dx + dy * dy;
-        if (!on || j == i) continue;
-        double w = sq[j] * __drcp_rn(r2);
-        re += dx * w;
-        im -= dy * w;
+    if (active) {
+      const double xi = sx[t], yi = sy[t];
+      int rr = r0 - 1, je = 0, j = sub;
+      for (;;) {
+        bool more = true;
+        while (j >= je) {                      // j counts past je: into the next ranges
+          if (++rr >= r1) {
+            more = false;
+            break;
+          }
+          const int2 rg = near_rng[rr];
+          j += leaf_be[rg.x] - je;
+          je = leaf_be[rg.y];
+        }
+        if (!more) break;
+        const double dx = xi - sx[j], dy = yi - sy[j];
+        const double r2 = dx * dx + dy * dy;
+        if (j != t) {
+          const unsigned ex = ((unsigned)__double2hiint(r2) >> 20) & 2047u;
+          double inv = rcp_h3(r2);
+          if (ex - 23u > 2000u) inv = __drcp_rn(r2);
+          const double w = sq[j] * inv;
+          re = fma(dx, w, re);
+          im = fma(-dy, w, im);
+        }
+        j += s;
       }
     }
-    if (on) near_acc[i] = cmake(re, im);
+    red[threadIdx.x] = cmake(re, im);
+    __syncthreads();
+    int o = 1;
+    while (2 * o < s) o *= 2;
+    for (; o > 0 && s > 1; o >>= 1) {
+      if (active && sub < o && sub + o < s)
+        red[threadIdx.x] = cadd(red[threadIdx.x], red[threadIdx.x + o]);
+      __syncthreads();
+    }
+    if (active && sub == 0) near_acc[t] = red[threadIdx.x];
+    __syncthreads();
   }
 }
 
@@ -628,11 +711,16 @@ __global__ void k2f_m2m(int cnt, int off, int p, const int *__restrict__ child,
   }
 }
 
-// M2L, warp per target node, lane i <-> local term i.  Per source, lane j
-// makes w^j (binary powers) and s_j = ma_j w^j; then
-// la_i += (1/h) (-1)^i w^i sum_j C(i+j-1, j-1) s_j, with the s_j of the
-// source read from shared memory (double-buffered, so one __syncwarp per
-// source) and the next source's coefficients loaded while this one runs.
+// M2L, warp per target node, lane i <-> local term i, for orders up to PM.
+// Lane k makes w of source k; per source a scan of products makes its powers
+// (lane j: w^j) and s_j = ma_j w^j, shared through shared memory
+// (double-buffered, so one __syncwarp per source); then
+// la_i += (1/h) (-1)^i w^i sum_j C(i+j-1, j-1) s_j with the row of binomials
+// in registers and the two parts of s_j in one packed product.  The next
+// source's coefficients are loaded while this one runs.  128 systems of order
+// 20, 3.4 M translations, on GB300: 0.55 ms; 1.45 with the binomials read from
+// shared memory, binary powers in every lane and w made per source.
+template <int PM>
 __global__ void __launch_bounds__(128) k2f_m2l(int nn, int p, const int *__restrict__ far_off,
                                                const int *__restrict__ far_src,
                                                const int *__restrict__ sysn,
@@ -641,62 +729,65 @@ __global__ void __launch_bounds__(128) k2f_m2l(int nn, int p, const int *__restr
                                                const double *__restrict__ center,
                                                const float *__restrict__ binom, int nb,
                                                const zf *__restrict__ mult, zf *__restrict__ loc) {
-  extern __shared__ float smemf[];
+  constexpr int PE = (PM + 1) & ~1;
+  __shared__ __align__(16) uint64_t sbuf[4][2][32];
   const int P1 = p + 1;
-  const int SP = p | 1;
-  float *tab = smemf;                    // tab[i * SP + j] = C(i+j-1, j-1)
-  zf *sbuf = reinterpret_cast<zf *>(smemf + ((P1 * SP + 1) & ~1));
-  for (int x = threadIdx.x; x < P1 * SP; x += blockDim.x) {
-    int i = x / SP, j = x % SP;
-    tab[x] = (j >= 1 && j < p) ? binom[(i + j - 1) * nb + (j - 1)] : 0.f;
-  }
-  __syncthreads();
-  int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int t = blockIdx.x * (blockDim.x >> 5) + wl;
+  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x * 4 + wl;
   if (t >= nn) return;
-  int f0 = far_off[t], f1 = far_off[t + 1];
+  const int f0 = far_off[t], f1 = far_off[t + 1];
   if (f0 == f1) return;
-  zf *sw = sbuf + wl * 2 * 32;           // two buffers of 32 per warp
+  // row i = lane of the binomials C(i+j-1, j-1), j = 1 .. p-1, each twice
+  uint64_t row[PE];
+#pragma unroll
+  for (int j = 0; j < PE; ++j) {
+    const float c = j >= 1 && j < p && lane <= p ? binom[(lane + j - 1) * nb + (j - 1)] : 0.f;
+    row[j] = pack2(c, c);
+  }
   const double tx = center[2 * t], ty = center[2 * t + 1];
   const double h = node_size2(sysbox, sysn[t], depth[t]), ih = 1.0 / h;
-  const float *row = tab + (lane <= p ? lane : 0) * SP;
   zf acc = cmake(0.f, 0.f);
   const bool mine = lane >= 1 && lane < p;   // lanes holding a source term
-  int sn = far_src[f0];
-  zf ma = mine ? mult[(int64_t)sn * P1 + lane] : cmake(0.f, 0.f);
-  for (int f = f0; f < f1; ++f) {
+  for (int g = f0; g < f1; g += 32) {
+    const int cnt = min(32, f1 - g);
+    const int sn = far_src[g + min(lane, cnt - 1)];
     // w = h / (zt - zs): the centre offset in node sizes (small integers,
     // exact in FP32) from FP64, its inverse in FP32
     const float ux = (float)((tx - center[2 * sn]) * ih), uy = (float)((ty - center[2 * sn + 1]) * ih);
     const float iu2 = 1.f / (ux * ux + uy * uy);
     const zf w = cmake(ux * iu2, -uy * iu2);
-    // prefetch the next source's term
-    zf nma = cmake(0.f, 0.f);
-    int nsn = sn;
-    if (f + 1 < f1) {
-      nsn = far_src[f + 1];
-      if (mine) nma = mult[(int64_t)nsn * P1 + lane];
-    }
-    // w^lane by binary powers
-    zf wp = cmake(1.f, 0.f), b = w;
-    for (int e = lane; e; e >>= 1) {
-      if (e & 1) wp = zfmul(wp, b);
-      b = zfmul(b, b);
-    }
-    zf *buf = sw + 32 * (f & 1);
-    buf[lane] = zfmul(ma, wp);
-    __syncwarp();
-    if (lane <= p) {
-      zf sum = cmake(0.f, 0.f);
-      for (int j = 1; j < p; ++j) {
-        const zf sj = buf[j];
-        sum.re = fmaf(row[j], sj.re, sum.re);
-        sum.im = fmaf(row[j], sj.im, sum.im);
+    int sk = __shfl_sync(0xffffffffu, sn, 0);
+    zf ma = mine ? mult[(int64_t)sk * P1 + lane] : cmake(0.f, 0.f);
+    for (int k = 0; k < cnt; ++k) {
+      zf nma = cmake(0.f, 0.f);
+      sk = __shfl_sync(0xffffffffu, sn, k + 1 < cnt ? k + 1 : k);
+      if (k + 1 < cnt && mine) nma = mult[(int64_t)sk * P1 + lane];
+      // lane l: w^l
+      zf v = cmake(__shfl_sync(0xffffffffu, w.re, k), __shfl_sync(0xffffffffu, w.im, k));
+      if (lane == 0) v = cmake(1.f, 0.f);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const zf u = cmake(__shfl_up_sync(0xffffffffu, v.re, o),
+                           __shfl_up_sync(0xffffffffu, v.im, o));
+        if (lane > o) v = zfmul(v, u);
       }
-      acc = cadd(acc, zfmul(sum, wp));
+      uint64_t *buf = sbuf[wl][k & 1];
+      const zf sj = zfmul(ma, v);
+      buf[lane] = pack2(sj.re, sj.im);
+      __syncwarp();
+      uint64_t sum2 = 0ull, sum3 = 0ull;
+#pragma unroll
+      for (int j = 0; j < PE; j += 2) {
+        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2 *>(buf + j);
+        sum2 = fma2(row[j], b2.x, sum2);
+        sum3 = fma2(row[j + 1], b2.y, sum3);
+      }
+      zf sum;
+      unpack2(add2(sum2, sum3), sum.re, sum.im);
+      acc = cadd(acc, zfmul(sum, v));
+      ma = nma;
     }
-    sn = nsn;
-    ma = nma;
+    __syncwarp();
   }
   // (-1)^i of every term, applied once
   const float ihf = (float)(1.0 / h);
@@ -739,70 +830,183 @@ __global__ void k2f_l2l(int cnt, int off, int p, const int *__restrict__ parent,
   }
 }
 
-// near field, warp per target leaf: each near range is staged 32 sources at
-// a time in shared memory as FP32 positions relative to the target leaf's
-// centre (the FP64 difference rounded once), and lanes sum their targets
-// against them in FP32; a pair closer than h/8 (h the target leaf's size),
-// where that rounding would show, is recomputed from the FP64 positions.
-// FP32 partial sums per range, FP64 sums per target.
-__global__ void __launch_bounds__(128) k2f_p2p(int nleaves, const int *__restrict__ leaf_be,
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// near field, a block of T threads per target leaf, as the 3D one
+// (k_p2p_tile): the concatenated near ranges are staged in tiles of 2 T
+// sources as offsets from the leaf's centre (FP32 hi + lo positions), and
+// floor(T / n) threads per target sum two sources per packed instruction.
+// A pair closer than h/8 (h the target leaf's size), where the offset's
+// rounding would show, is left out of the loop and added from the FP64
+// positions.  A thread's parts of the tiles go into Kahan sums, the parts of
+// a target are added with compensation.  Bound by the reciprocal unit (a
+// quarter of a warp per cycle), 8 cycles a pair and scheduler, on large
+// leaves, by the blocks' set-up on small ones.
+constexpr int k2Ranges = 32;     // near ranges taken together
+template <int T>                 // threads, and pairs of a tile
+__global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleaves, const int *__restrict__ leaf_be,
                         const int *__restrict__ near_off, const int2 *__restrict__ near_rng,
                         const int *__restrict__ leaf_node, const int *__restrict__ sysn,
                         const uint8_t *__restrict__ depth, const double *__restrict__ sysbox,
                         const double *__restrict__ center, const double *__restrict__ sx,
                         const double *__restrict__ sy, const double *__restrict__ sq,
-                        zd *__restrict__ near_acc) {
-  __shared__ float4 stg[4][32];
-  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * 4 + wl;
-  if (warp >= nleaves) return;
-  const int b = leaf_be[warp], e = leaf_be[warp + 1];
-  const int r0 = near_off[warp], r1 = near_off[warp + 1];
-  const int node = leaf_node[warp];
+                        const float4 *__restrict__ hl, zd *__restrict__ near_acc) {
+  // pair p of the tile: (-x0, -x1, -y0, -y1) and (q0, q1)
+  __shared__ ulonglong2 tA[T];
+  __shared__ uint64_t tQ[T];
+  __shared__ int tj[2 * T];                     // their particles
+  __shared__ int rs[k2Ranges], rp[k2Ranges];    // ranges: first particle, place
+  __shared__ int s_tot;
+  __shared__ float red[4][T];
+  const int L = blockIdx.x;
+  const int b = leaf_be[L], nt = leaf_be[L + 1] - b;
+  const int r0 = near_off[L], r1 = near_off[L + 1];
+  const int node = leaf_node[L];
   const double cx = center[2 * node], cy = center[2 * node + 1];
+  const float chx = (float)cx, chy = (float)cy;
+  const float clx = (float)(cx - (double)chx), cly = (float)(cy - (double)chy);
   const double hh = node_size2(sysbox, sysn[node], depth[node]);
   const float thr2 = (float)(hh * hh / 64.0);
-  float4 *buf = stg[wl];
-  for (int base = b; base < e; base += 32) {
-    const int i = base + lane;
-    const bool on = i < e;
-    const double xi = on ? sx[i] : cx, yi = on ? sy[i] : cy;
-    const float xr = (float)(xi - cx), yr = (float)(yi - cy);
-    double re = 0.0, im = 0.0;
-    for (int r = r0; r < r1; ++r) {
-      const int2 rg = near_rng[r];
-      const int j0 = leaf_be[rg.x], j1 = leaf_be[rg.y];
-      float fr = 0.f, fi = 0.f;
-      for (int c0 = j0; c0 < j1; c0 += 32) {
-        const int cnt = min(32, j1 - c0);
-        __syncwarp();
-        if (lane < cnt) {
-          const int j = c0 + lane;
-          buf[lane] = make_float4((float)(sx[j] - cx), (float)(sy[j] - cy), (float)sq[j],
-                                  __int_as_float(j));
+  for (int tb = 0; tb < nt; tb += T) {
+    const int rem = min(nt - tb, T);
+    const int S = T / rem;                      // threads per target
+    const int sub = threadIdx.x / rem, ti = threadIdx.x - sub * rem;
+    const bool active = sub < S;
+    const int t = b + tb + ti;
+    const float4 th = hl[t];
+    const float tx = (th.x - chx) + (th.z - clx), ty = (th.y - chy) + (th.w - cly);
+    const uint64_t tx2 = pack2(tx, tx), ty2 = pack2(ty, ty);
+    float ks[2] = {}, kc[2] = {};
+    for (int rb = r0; rb < r1; rb += k2Ranges) {
+      if (threadIdx.x < k2Ranges) {
+        const int rr = rb + threadIdx.x;
+        int first = 0, len = 0;
+        if (rr < r1) {
+          const int2 rg = near_rng[rr];
+          first = leaf_be[rg.x];
+          len = leaf_be[rg.y] - first;
         }
-        __syncwarp();
-        for (int k = 0; k < cnt; ++k) {
-          const float4 sv = buf[k];
-          float dx = xr - sv.x, dy = yr - sv.y;
-          float r2 = dx * dx + dy * dy;
-          if (r2 < thr2) {
-            const int j = __float_as_int(sv.w);
-            if (j == i || !on) continue;
-            dx = (float)(xi - sx[j]);
-            dy = (float)(yi - sy[j]);
-            r2 = dx * dx + dy * dy;
-            if (!(r2 > 0.f)) continue;
-          }
-          const float wgt = sv.z * __frcp_rn(r2);
-          fr = fmaf(dx, wgt, fr);
-          fi = fmaf(-dy, wgt, fi);
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (threadIdx.x >= o) incl += v;
         }
+        rs[threadIdx.x] = first;
+        rp[threadIdx.x] = incl - len;
+        if (threadIdx.x == k2Ranges - 1) s_tot = incl;
       }
-      re += fr;
-      im += fi;
+      __syncthreads();
+      const int tot = s_tot;
+      for (int k0 = 0; k0 < tot; k0 += 2 * T) {
+        const int np = min(T, (tot - k0 + 1) / 2);
+        if (threadIdx.x < np) {
+          const int k = k0 + 2 * threadIdx.x;
+          int g = 0;                            // last range that starts at or before k
+#pragma unroll
+          for (int o = k2Ranges / 2; o > 0; o >>= 1)
+            if (rp[g + o] <= k) g += o;
+          float x[2], y[2], q[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (e == 1)
+              while (g < k2Ranges - 1 && rp[g + 1] <= k + 1) ++g;
+            const bool in = k + e < tot;
+            const int j = in ? rs[g] + (k + e - rp[g]) : -1;
+            tj[2 * threadIdx.x + e] = j;
+            x[e] = 1e18f;                       // no source: no charge, far away
+            y[e] = q[e] = 0.f;
+            if (in) {
+              const float4 v = hl[j];
+              x[e] = (chx - v.x) + (clx - v.z);
+              y[e] = (chy - v.y) + (cly - v.w);
+              q[e] = (float)sq[j];
+            }
+          }
+          tA[threadIdx.x] = make_ulonglong2(pack2(x[0], x[1]), pack2(y[0], y[1]));
+          tQ[threadIdx.x] = pack2(q[0], q[1]);
+        }
+        __syncthreads();
+        if (active) {
+          uint64_t p2r = 0ull, p2i = 0ull;
+          unsigned close = 0;   // 1 + pair of the last close pair, above it the one before
+#pragma unroll 2
+          for (int p = sub; p < np; p += S) {
+            const ulonglong2 A = tA[p];
+            const uint64_t q2 = tQ[p];
+            const uint64_t dx = add2(tx2, A.x), dy = add2(ty2, A.y);
+            const uint64_t r2 = fma2(dy, dy, mul2(dx, dx));
+            float ra, rb2;
+            unpack2(r2, ra, rb2);
+            const bool ca = ra < thr2, cb = rb2 < thr2;
+            if (ca || cb) close = (close << 16) + (unsigned)(p + 1);
+            const uint64_t w = mul2(q2, pack2(ca ? 0.f : rcp_ftz(ra), cb ? 0.f : rcp_ftz(rb2)));
+            p2r = fma2(dx, w, p2r);
+            p2i = fma2(dy, w, p2i);
+          }
+          float lo, hi, pr, pi;
+          unpack2(p2r, lo, hi);
+          pr = lo + hi;
+          unpack2(p2i, lo, hi);
+          pi = lo + hi;
+          if (close) {
+            const bool one = close < 65536u;
+            for (int p = one ? (int)close - 1 : sub; p < np; p += one ? T : S) {
+              const float4 fa = reinterpret_cast<const float4 *>(tA)[p];
+              const float2 fq = reinterpret_cast<const float2 *>(tQ)[p];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                float dx = tx + (e ? fa.y : fa.x), dy = ty + (e ? fa.w : fa.z);
+                float r2 = fmaf(dy, dy, dx * dx);
+                if (!(r2 < thr2)) continue;
+                const int j = tj[2 * p + e];
+                if (j < 0 || j == t) continue;
+                dx = (float)(sx[t] - sx[j]);
+                dy = (float)(sy[t] - sy[j]);
+                r2 = dx * dx + dy * dy;
+                if (!(r2 > 0.f)) continue;
+                const float w = (e ? fq.y : fq.x) * __frcp_rn(r2);
+                pr = fmaf(dx, w, pr);
+                pi = fmaf(dy, w, pi);
+              }
+            }
+          }
+          const float v[2] = {pr, pi};
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const float y = v[c] - kc[c];
+            const float n = ks[c] + y;
+            kc[c] = (n - ks[c]) - y;
+            ks[c] = n;
+          }
+        }
+        __syncthreads();
+      }
     }
-    if (on) near_acc[i] = cmake(re, im);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      red[c][threadIdx.x] = ks[c];
+      red[2 + c][threadIdx.x] = kc[c];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * rem; i += T) {
+      const int tt = i >> 1, c = i & 1;
+      float s = red[c][tt], e = -red[2 + c][tt];
+      for (int k = 1; k < S; ++k) {
+        const float v = red[c][tt + k * rem];
+        const float n = s + v, bb = n - s;
+        e += ((s - (n - bb)) + (v - bb)) - red[2 + c][tt + k * rem];
+        s = n;
+      }
+      const double v = (double)s + (double)e;
+      double *o = reinterpret_cast<double *>(near_acc + b + tb + tt);
+      o[c] = c ? -v : v;       // sum of q (dx - i dy) / r^2
+    }
+    __syncthreads();
   }
 }
 
@@ -879,6 +1083,7 @@ struct AranGpuSolver2d {
   aran::DBuf<int> err2;   // input checks of the key pass
   aran::DBuf<uint8_t> cub_tmp;
   aran::DBuf<double> sx, sy, sq, io_xy, io_q, io_acc;
+  aran::DBuf<float4> hl;   // FP32 hi + lo positions (mixed near field)
   // forest
   aran::DBuf<int> nsys_, ij, begin, end, child, parent, col, ncol, far_off, far_src;
   aran::DBuf<int> lf_begin, lf_end, leaf_node, leaf_be, near_off;
@@ -1018,7 +1223,10 @@ void build_forest(AranGpuSolver2d *s, int nsys, const double *dxy, const double 
   s->sx.reserve(n);
   s->sy.reserve(n);
   s->sq.reserve(n);
-  k2_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, s->perm.ptr, dxy, dq, s->sx.ptr, s->sy.ptr, s->sq.ptr);
+  const bool mixed = s->cfg.precision == ARAN_PRECISION_MIXED;
+  if (mixed) s->hl.reserve(n);
+  k2_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, s->perm.ptr, dxy, dq, s->sx.ptr, s->sy.ptr, s->sq.ptr,
+                                             mixed ? s->hl.ptr : nullptr);
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::SORT + 1], st));
 
@@ -1136,10 +1344,17 @@ void run_passes2_mixed(AranGpuSolver2d *s, double *dacc) {
   ACHECK(cudaEventRecord(s->ev_lists, st));
   ACHECK(cudaStreamWaitEvent(s1, s->ev_lists, 0));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2P], s1));
-  k2f_p2p<<<ceil_div(nl, 4), 128, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr,
-                                            s->leaf_node.ptr, s->nsys_.ptr, s->depth.ptr,
-                                            s->sysbox.ptr, s->center.ptr, s->sx.ptr, s->sy.ptr,
-                                            s->sq.ptr, s->near_acc.ptr);
+  // a warp per leaf up to leaf capacity 64: 64 systems of 1k to 60k particles
+  // took 0.25 / 0.26 / 0.39 ms at capacities 20 / 32 / 64 with 32 threads, 0.55
+  // / 0.41 / 0.40 with 128; 0.50 and 0.51 at 96.  (The capacity and not the mean
+  // occupancy of the batch: a system's bits do not depend on its company.)
+  const int T = s->cfg.maxbox <= 64 ? 32 : 128;
+  auto p2p = T == 32 ? k2f_p2p<32> : k2f_p2p<128>;
+  p2p<<<nl, T, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr,
+                                 s->leaf_node.ptr, s->nsys_.ptr, s->depth.ptr, s->sysbox.ptr,
+                                 s->center.ptr, s->sx.ptr, s->sy.ptr, s->sq.ptr, s->hl.ptr,
+                                 s->near_acc.ptr);
+  ACHECK(cudaGetLastError());
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2P + 1], s1));
   ACHECK(cudaEventRecord(s->ev_p2p, s1));
@@ -1163,10 +1378,12 @@ void run_passes2_mixed(AranGpuSolver2d *s, double *dacc) {
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2M + 1], st));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2L], st));
   {
-    size_t smem = (size_t)(((P1 * (p | 1)) + 1) & ~1) * sizeof(float) + 4 * 2 * 32 * sizeof(zf);
-    k2f_m2l<<<ceil_div(nn, 4), 128, smem, st>>>(nn, p, s->far_off.ptr, s->far_src.ptr, s->nsys_.ptr,
-                                                 s->depth.ptr, s->sysbox.ptr, s->center.ptr,
-                                                 s->binom32.ptr, s->nb, s->mult32.ptr, s->loc32.ptr);
+    // the instance whose row of binomials is the shortest that holds the order
+    auto kern = p <= 12 ? k2f_m2l<12> : (p <= 20 ? k2f_m2l<20> : k2f_m2l<31>);
+    kern<<<ceil_div(nn, 4), 128, 0, st>>>(nn, p, s->far_off.ptr, s->far_src.ptr, s->nsys_.ptr,
+                                          s->depth.ptr, s->sysbox.ptr, s->center.ptr,
+                                          s->binom32.ptr, s->nb, s->mult32.ptr, s->loc32.ptr);
+    ACHECK(cudaGetLastError());
     s->launches++;
   }
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2L + 1], st));
@@ -1204,9 +1421,9 @@ void run_passes2(AranGpuSolver2d *s, double *dacc) {
   ACHECK(cudaEventRecord(s->ev_lists, st));
   ACHECK(cudaStreamWaitEvent(s1, s->ev_lists, 0));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2P], s1));
-  k2_p2p<<<ceil_div((int64_t)nl * 32, 128), 128, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr,
-                                                          s->near_rng.ptr, s->sx.ptr, s->sy.ptr,
-                                                          s->sq.ptr, s->near_acc.ptr);
+  k2_p2p<<<nl, 128, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr, s->sx.ptr,
+                             s->sy.ptr, s->sq.ptr, s->near_acc.ptr);
+  ACHECK(cudaGetLastError());
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2P + 1], s1));
   ACHECK(cudaEventRecord(s->ev_p2p, s1));
@@ -1229,9 +1446,13 @@ void run_passes2(AranGpuSolver2d *s, double *dacc) {
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2M + 1], st));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2L], st));
   {
-    size_t smem = (size_t)P1 * (p | 1) * sizeof(double) + 4 * (size_t)P1 * sizeof(zd);
-    k2_m2l<<<ceil_div(nn, 4), 128, smem, st>>>(nn, p, s->far_off.ptr, s->far_src.ptr, s->center.ptr,
-                                                s->binom.ptr, s->nb, s->mult.ptr, s->loc.ptr);
+    const int S = (P1 + 31) / 32;        // terms per lane
+    const size_t smem = (size_t)((P1 * (p | 1) + 1) & ~1) * sizeof(double) + 4 * 32 * S * sizeof(zd);
+    auto kern = S == 1 ? k2_m2l<1> : (S == 2 ? k2_m2l<2> : k2_m2l<3>);
+    smem_opt_in(kern, smem);
+    kern<<<ceil_div(nn, 4), 128, smem, st>>>(nn, p, s->far_off.ptr, s->far_src.ptr, s->center.ptr,
+                                             s->binom.ptr, s->nb, s->mult.ptr, s->loc.ptr);
+    ACHECK(cudaGetLastError());
     s->launches++;
   }
   ACHECK(cudaEventRecord(s->ev[2 * Stage::M2L + 1], st));
@@ -1343,6 +1564,7 @@ void aran_gpu_solver2d_destroy(AranGpuSolver2d *s) {
   s->sx.release();
   s->sy.release();
   s->sq.release();
+  s->hl.release();
   s->io_xy.release();
   s->io_q.release();
   s->io_acc.release();
