@@ -259,16 +259,28 @@ bool launch_m2l_lanes_c(AranGpuSolver3d *s, OpTables<float> &tb, const int *pare
                         const cplx<float> *mult, cplx<float> *loc, cudaStream_t st);
 // m2m_lanes.cu: lane-parallel FP32 M2M (parents of depths dhi down to dlo)
 // and L2L (children of depths dlo up to dhi, from depth 3) at the orders
-// m2l_lane_order accepts; false leaves the pass to passes.cu's kernels
+// m2l_hk_order accepts; false leaves the pass to passes.cu's kernels
 void build_oct_lane_tables(OpTables<float> &tb, cudaStream_t st);
 bool launch_m2m_lanes(AranGpuSolver3d *s, OpTables<float> &tb, cplx<float> *mult, int dhi,
                       int dlo, cudaStream_t st);
 bool launch_l2l_lanes(AranGpuSolver3d *s, OpTables<float> &tb, cplx<float> *loc, int dlo,
                       int dhi, cudaStream_t st);
+void launch_oct_lanes_b(AranGpuSolver3d *s, bool down, const float *tab, cplx<float> *ser, int d0,
+                        int d1, cudaStream_t st);
+void launch_oct_lanes_c(AranGpuSolver3d *s, bool down, const float *tab, cplx<float> *ser, int d0,
+                        int d1, cudaStream_t st);
 // m2l_tc.cu: the FP32 M2L on the tensor cores (orders 8 and 12); false
 // leaves it to the other kernels
 bool launch_m2l_tc(AranGpuSolver3d *s, const int *parents, int count, const float *mult,
                    float *loc, cudaStream_t st);
+// leaf_ops.cu: FP32 P2M into mult32 and L2P from loc32 at the orders with a
+// compile-time instance; false leaves them to passes.cu
+bool launch_leaf_p2m(AranGpuSolver3d *s, cudaStream_t st);
+bool launch_leaf_p2m_b(AranGpuSolver3d *s, cudaStream_t st);
+bool launch_leaf_p2m_c(AranGpuSolver3d *s, cudaStream_t st);
+bool launch_leaf_l2p(AranGpuSolver3d *s, cudaStream_t st);
+bool launch_leaf_l2p_b(AranGpuSolver3d *s, cudaStream_t st);
+bool launch_leaf_l2p_c(AranGpuSolver3d *s, cudaStream_t st);
 // p2p.cu
 constexpr int kBigRange = 2048;   // near ranges above this many particles are chunked
 void build_p2p_work(AranGpuSolver3d *s);
