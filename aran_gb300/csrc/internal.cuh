@@ -116,7 +116,7 @@ struct DevTree {
   DBuf<int> m2l_targets;              // nodes with non-empty far lists
   int n_m2l_targets = 0;
   DBuf<int2> leaf_be;                 // particle [begin, end) per leaf ordinal
-  DBuf<float4> leaf_chi, leaf_clo;    // FP32 leaf centre split hi + lo; chi.w = close-pair r^2
+  DBuf<float4> leaf_chi, leaf_clo;    // FP32 leaf centre in the box, hi + lo; chi.w = close-pair r^2
   DBuf<int4> big_items;               // (leaf, lf_a, lf_b, 0): chunks of heavy near ranges
   DBuf<int> big_rng;                  // [0] chunk total, [1] range count, then heavy range indices
   DBuf<int> semi_off;                 // CSR over leaves of semifar nodes (threshold > 0)
@@ -173,7 +173,7 @@ struct AranGpuSolver3d {
   aran::DBuf<double> sx, sy, sz, sq;     // sorted FP64 positions/charges
   aran::DBuf<aran::real4<double>> rel64;
   aran::DBuf<aran::real4<float>> rel32;
-  aran::DBuf<float4> abs_hi, abs_lo;     // FP32 hi + lo positions (hi.w = charge), mixed
+  aran::DBuf<float4> abs_hi, abs_lo;     // FP32 hi + lo positions in the box (hi.w = charge), mixed
   aran::DBuf<double> acc_pot, acc_fld;   // sorted accumulators (FP64)
   aran::DBuf<double> io_xyz, io_q, io_pot, io_fld;  // staging for host calls
   aran::DBuf<double> mult64, loc64;

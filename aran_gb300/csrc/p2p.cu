@@ -41,13 +41,16 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
 __global__ void k_leaf_info(int nleaves, const int *__restrict__ leaf_node,
                             const int *__restrict__ begin, const int *__restrict__ end,
                             const uint8_t *__restrict__ depth, const double *__restrict__ center,
+                            const int *__restrict__ sys, const double *__restrict__ sys_box,
                             double ex, double ey, double ez, int2 *__restrict__ be,
                             float4 *__restrict__ chi, float4 *__restrict__ clo) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= nleaves) return;
   int node = leaf_node[L];
   be[L] = make_int2(begin[node], end[node]);
-  double cx = center[3 * node], cy = center[3 * node + 1], cz = center[3 * node + 2];
+  const double *b = sys_box + 9 * sys[node];   // from the box's corner, as the positions
+  double cx = center[3 * node] - b[0], cy = center[3 * node + 1] - b[1],
+         cz = center[3 * node + 2] - b[2];
   float hx = (float)cx, hy = (float)cy, hz = (float)cz;
   double h = fmin(ex, fmin(ey, ez)) / ldexp(1.0, depth[node]);
   float thr = (float)(h * 0.125);
@@ -481,7 +484,8 @@ void build_p2p_work(AranGpuSolver3d *s) {
   double ex = s->cfg.ub[0] - s->cfg.lb[0], ey = s->cfg.ub[1] - s->cfg.lb[1],
          ez = s->cfg.ub[2] - s->cfg.lb[2];
   k_leaf_info<<<ceil_div(nl, TB), TB, 0, st>>>(nl, t.leaf_node.ptr, t.begin.ptr, t.end.ptr,
-                                               t.depth.ptr, t.center.ptr, ex, ey, ez,
+                                               t.depth.ptr, t.center.ptr, t.sys.ptr,
+                                               s->sys_box.ptr, ex, ey, ez,
                                                t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr);
   ACHECK(cudaGetLastError());
   s->launches++;

@@ -479,7 +479,8 @@ template <typename T>
 __global__ void k_relative(int64_t n, const int *__restrict__ incl, const int *__restrict__ leaf_node,
                            const double *__restrict__ center, const double *__restrict__ sx,
                            const double *__restrict__ sy, const double *__restrict__ sz,
-                           const double *__restrict__ sq, real4<T> *__restrict__ rel,
+                           const double *__restrict__ sq, const int *__restrict__ sys,
+                           const double *__restrict__ sys_box, real4<T> *__restrict__ rel,
                            float4 *__restrict__ hi, float4 *__restrict__ lo) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -492,10 +493,14 @@ __global__ void k_relative(int64_t n, const int *__restrict__ incl, const int *_
   r.q = (T)sq[i];
   rel[i] = r;
   if (sizeof(T) == 4) {
-    const float hx = (float)x, hy = (float)y, hz = (float)z;
+    // FP32 hi + lo position from the box's corner: 48 bits of the box's extent,
+    // wherever the box lies
+    const double *b = sys_box + 9 * sys[node];
+    const double bx = x - b[0], by = y - b[1], bz = z - b[2];
+    const float hx = (float)bx, hy = (float)by, hz = (float)bz;
     hi[i] = make_float4(hx, hy, hz, (float)r.q);
-    lo[i] = make_float4((float)(x - (double)hx), (float)(y - (double)hy),
-                        (float)(z - (double)hz), 0.f);
+    lo[i] = make_float4((float)(bx - (double)hx), (float)(by - (double)hy),
+                        (float)(bz - (double)hz), 0.f);
   }
 }
 
@@ -806,13 +811,14 @@ void build_lists(AranGpuSolver3d *s) {
     s->abs_lo.reserve(n);
     k_relative<float><<<ceil_div(n, TB), TB, 0, st>>>(n, incl, t.leaf_node.ptr, t.center.ptr,
                                                        s->sx.ptr, s->sy.ptr, s->sz.ptr, s->sq.ptr,
-                                                       s->rel32.ptr, s->abs_hi.ptr,
-                                                       s->abs_lo.ptr);
+                                                       t.sys.ptr, s->sys_box.ptr, s->rel32.ptr,
+                                                       s->abs_hi.ptr, s->abs_lo.ptr);
   } else {
     s->rel64.reserve(n);
     k_relative<double><<<ceil_div(n, TB), TB, 0, st>>>(n, incl, t.leaf_node.ptr, t.center.ptr,
                                                         s->sx.ptr, s->sy.ptr, s->sz.ptr, s->sq.ptr,
-                                                        s->rel64.ptr, nullptr, nullptr);
+                                                        t.sys.ptr, s->sys_box.ptr, s->rel64.ptr,
+                                                        nullptr, nullptr);
   }
   s->launches++;
   // near ranges (and semifar nodes) per leaf

@@ -48,3 +48,17 @@ def test_many_near_ranges(aran, oracle):
         p64, f64 = s.solve(x, q)
     assert np.linalg.norm(pot - p64) < 1e-6 * np.linalg.norm(p64)
     assert np.linalg.norm(fld - f64) < 1e-6 * np.linalg.norm(f64)
+
+
+def test_box_far_from_the_origin(aran):
+    """Positions exact in FP64 in either box: only the box's extent counts, so
+    results differ by the order of FP64 additions at most."""
+    x, q = W.uniform(5000, 3)
+    x = np.round(x * 2.0**30) / 2.0**30
+    h = np.array([2.0**20, -(2.0**21), 3.0])
+    out = []
+    for lb in (np.zeros(3), h):
+        with aran.Solver3d(tuple(lb), tuple(lb + 1.0), maxbox=40, order=8, precision="mixed") as s:
+            out.append(s.solve(x + lb, q))
+    for a, b in zip(*out):
+        assert np.linalg.norm(a - b) <= 1e-10 * np.linalg.norm(b)
