@@ -265,6 +265,12 @@ bool launch_m2m_lanes(AranGpuSolver3d *s, OpTables<float> &tb, cplx<float> *mult
                       int dlo, cudaStream_t st);
 bool launch_l2l_lanes(AranGpuSolver3d *s, OpTables<float> &tb, cplx<float> *loc, int dlo,
                       int dhi, cudaStream_t st);
+// oct_wide.cu: M2M into / L2L from the cnt nodes list[..] (or off onwards): FP32
+// with an octant-0 stream table (the bits of the lane-parallel kernels), FP64
+void launch_oct_wide(AranGpuSolver3d *s, bool down, const float *stream, cplx<float> *ser,
+                     int cnt, int off, const int *list, cudaStream_t st);
+void launch_oct_wide64(AranGpuSolver3d *s, bool down, cplx<double> *ser, int cnt, int off,
+                       const int *list, cudaStream_t st);
 void launch_oct_lanes_b(AranGpuSolver3d *s, bool down, const float *tab, cplx<float> *ser, int d0,
                         int d1, cudaStream_t st);
 void launch_oct_lanes_c(AranGpuSolver3d *s, bool down, const float *tab, cplx<float> *ser, int d0,

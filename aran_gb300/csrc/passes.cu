@@ -2,10 +2,13 @@
 //
 // LibAran runs them as callbacks from tree traversals (aran/aransolver3d.c):
 //   clear_func :399-410   -> one memset of all expansions
-//   up_func :412-450      -> k_p2m (leaves) + k_m2m_rotate (level by level)
+//   up_func :412-450      -> k_p2m (leaves) + M2M level by level: k_oct_wide
+//                            (oct_wide.cu), k_oct_lanes (m2m_lanes.cuh), and
+//                            k_m2m_rotate for the FP32 orders those do not serve
 //   far_func :333-354     -> k_m2l_sibling (m2l.cu)
 //   near_func :254-324    -> k_p2p_tile, k_p2p64 (p2p.cu)
-//   down_func :452-490    -> k_l2l_rotate (level by level) + k_l2p
+//   down_func :452-490    -> L2L level by level (the same two files,
+//                            k_l2l_rotate) + k_l2p
 // The operators are the "point and shoot" rotation flavour of
 // aran/aransphericalseriesd-rotate.c (rotate to the z axis, translate along
 // z, rotate back), with even/odd real rotation blocks and the z-phases
@@ -435,25 +438,42 @@ DirOffsets offsets(int p, int kind) {
   return d;
 }
 
+// place in the parents list of the first internal node of each depth >= 1
+std::vector<int> parents_first(const DevTree &t) {
+  std::vector<int> first(t.nlevels + 1, 0);
+  for (int d = 1; d < t.nlevels; ++d)
+    first[d + 1] = first[d] + (d < (int)t.level_internal.size() ? t.level_internal[d] : 0);
+  return first;
+}
+
 // M2M into the parents of depths dhi down to dlo (deepest first)
 template <typename T>
 void m2m_levels(AranGpuSolver3d *s, OpTables<T> &tb, cplx<T> *mult, int dhi, int dlo,
                 cudaStream_t st) {
   DevTree &t = s->tree;
   const int p = s->cfg.order;
-  const int nm = tri(p), nl = tri(p + 1);
-  if constexpr (sizeof(T) == 4)
+  if constexpr (sizeof(T) == 8) {
+    // level by level, the internal nodes of depth >= 1 from the parents list
+    const std::vector<int> first = parents_first(t);
+    for (int d = dhi; d >= dlo; --d) {
+      if (d < 0 || d > t.nlevels - 2 || t.level_internal[d] == 0) continue;
+      if (d == 0) launch_oct_wide64(s, false, mult, t.level_off[1], 0, nullptr, st);
+      else launch_oct_wide64(s, false, mult, t.level_internal[d], 0, t.parents.ptr + first[d], st);
+    }
+  } else {
     if (launch_m2m_lanes(s, tb, mult, dhi, dlo, st)) return;
-  DirOffsets D = offsets<T>(p, 1);
-  size_t sm = ((2 * nl + 15) & ~15) + (size_t)8 * 3 * nm * sizeof(cplx<T>) + 64;
-  smem_opt_in(k_m2m_rotate<T>, sm);
-  for (int d = dhi; d >= dlo; --d) {
-    if (d < 0 || d > t.nlevels - 2 || t.level_internal[d] == 0) continue;
-    int off = t.level_off[d], cnt = t.level_off[d + 1] - off;
-    k_m2m_rotate<T><<<cnt, 256, sm, st>>>(cnt, off, t.child.ptr, t.begin.ptr, t.end.ptr, p,
-                                          tb.dir_m2m.ptr, D, tb.vm.ptr, tb.lm.ptr, mult);
-    ACHECK(cudaGetLastError());
-    s->launches++;
+    const int nm = tri(p), nl = tri(p + 1);
+    DirOffsets D = offsets<T>(p, 1);
+    size_t sm = ((2 * nl + 15) & ~15) + (size_t)8 * 3 * nm * sizeof(cplx<T>) + 64;
+    smem_opt_in(k_m2m_rotate<T>, sm);
+    for (int d = dhi; d >= dlo; --d) {
+      if (d < 0 || d > t.nlevels - 2 || t.level_internal[d] == 0) continue;
+      int off = t.level_off[d], cnt = t.level_off[d + 1] - off;
+      k_m2m_rotate<T><<<cnt, 256, sm, st>>>(cnt, off, t.child.ptr, t.begin.ptr, t.end.ptr, p,
+                                            tb.dir_m2m.ptr, D, tb.vm.ptr, tb.lm.ptr, mult);
+      ACHECK(cudaGetLastError());
+      s->launches++;
+    }
   }
 }
 
@@ -464,20 +484,26 @@ void l2l_levels(AranGpuSolver3d *s, OpTables<T> &tb, cplx<T> *loc, int dlo, int 
                 cudaStream_t st) {
   DevTree &t = s->tree;
   const int p = s->cfg.order;
-  const int nl = tri(p + 1);
-  if constexpr (sizeof(T) == 4)
+  if constexpr (sizeof(T) == 8) {
+    const std::vector<int> first = parents_first(t);
+    for (int d = (dlo < 3 ? 3 : dlo) - 1; d < dhi && d < t.nlevels - 1; ++d)
+      if (t.level_internal[d] > 0)
+        launch_oct_wide64(s, true, loc, t.level_internal[d], 0, t.parents.ptr + first[d], st);
+  } else {
     if (launch_l2l_lanes(s, tb, loc, dlo, dhi, st)) return;
-  DirOffsets D = offsets<T>(p, 2);
-  const int WPB = 4;
-  size_t sm = ((2 * nl + 15) & ~15) + (size_t)WPB * 2 * nl * sizeof(cplx<T>) + 64;
-  smem_opt_in(k_l2l_rotate<T>, sm);
-  for (int d = dlo < 3 ? 3 : dlo; d <= dhi && d < t.nlevels; ++d) {
-    int off = t.level_off[d], cnt = t.level_off[d + 1] - off;
-    k_l2l_rotate<T><<<ceil_div(cnt, WPB), WPB * 32, sm, st>>>(
-        cnt, off, t.parent.ptr, t.child.ptr, t.begin.ptr, t.end.ptr, p, tb.dir_l2l.ptr, D,
-        tb.vl.ptr, tb.lm.ptr, loc);
-    ACHECK(cudaGetLastError());
-    s->launches++;
+    const int nl = tri(p + 1);
+    DirOffsets D = offsets<T>(p, 2);
+    const int WPB = 4;
+    size_t sm = ((2 * nl + 15) & ~15) + (size_t)WPB * 2 * nl * sizeof(cplx<T>) + 64;
+    smem_opt_in(k_l2l_rotate<T>, sm);
+    for (int d = dlo < 3 ? 3 : dlo; d <= dhi && d < t.nlevels; ++d) {
+      int off = t.level_off[d], cnt = t.level_off[d + 1] - off;
+      k_l2l_rotate<T><<<ceil_div(cnt, WPB), WPB * 32, sm, st>>>(
+          cnt, off, t.parent.ptr, t.child.ptr, t.begin.ptr, t.end.ptr, p, tb.dir_l2l.ptr, D,
+          tb.vl.ptr, tb.lm.ptr, loc);
+      ACHECK(cudaGetLastError());
+      s->launches++;
+    }
   }
 }
 
