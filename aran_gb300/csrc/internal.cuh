@@ -131,6 +131,26 @@ struct DevTree {
   int64_t n_near_rng = 0;
 };
 
+// task lists and stream tables of the FP64 M2L (m2l_fp64.cu)
+struct M2lFp64Sched {
+  int rounds[3], first[3];   // rounds of a stage, its first round
+  int off[3], stride;        // table: first entry of a stage, entries of a unit
+};
+struct M2lFp64Tables {
+  int nunits = 0;
+  M2lFp64Sched sched = {};
+  DBuf<double> tabs;
+  DBuf<uint64_t> task;
+  DBuf<int> trip;
+  DBuf<unsigned> units;
+  void release() {
+    tabs.release();
+    task.release();
+    trip.release();
+    units.release();
+  }
+};
+
 // Per-order operator tables (device).  Direction tables: 343 M2L offsets,
 // 8 M2M octants, 8 L2L octants.
 template <typename T>
@@ -147,6 +167,7 @@ struct OpTables {
   DBuf<T> dir_lanes; // lane-parallel M2L stream tables (FP32, m2l_hk_order)
   DBuf<float> oct_lanes[2];   // lane-parallel M2M / L2L octant-0 stream tables (FP32)
   DBuf<uint8_t> lm; // (l,m) of coefficient index, 2*tri(p+1)
+  M2lFp64Tables m2l64;   // FP64 only
 };
 
 struct Stage {
@@ -233,24 +254,12 @@ void build_tables_fp64(AranGpuSolver3d *s);   // FP64 tables beside a mixed solv
 int dir_offset(int p, int kind, int what);
 // passes.cu
 void run_passes(AranGpuSolver3d *s);
-// parts of the offset lists of a small FP64 M2L pass: the least
-// number of waves of CTAs times the work of a part (1 / K of the offsets and
-// the set-up, about 1/40 of a whole list)
-inline int split_parts(int groups, int resident) {
-  int best = 1;
-  double cost = 1e30;
-  for (int k : {1, 2, 3, 4, 6, 8, 12, 16}) {
-    const double c = (double)(((int64_t)groups * k + resident - 1) / resident) * (1. / k + 0.025);
-    if (c < 0.97 * cost) {
-      cost = c;
-      best = k;
-    }
-  }
-  return best;
-}
 // m2l.cu: M2L into the children of parents[first, first + count), in FP64
 // (mult64/loc64) or FP32 (mult32/loc32)
 void launch_m2l(AranGpuSolver3d *s, bool fp64, int first, int count, cudaStream_t st);
+// m2l_fp64.cu
+void build_m2l_fp64_tables(OpTables<double> &tb, cudaStream_t st);
+void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStream_t st);
 bool launch_m2l_lanes(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,
                       const cplx<float> *mult, cplx<float> *loc, cudaStream_t st);
 bool launch_m2l_lanes_b(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,

@@ -1,4 +1,6 @@
-// m2l.cu -- multipole-to-local translations (far_func of
+// m2l.cu -- FP32 multipole-to-local translations of the orders that
+// m2l_lanes.cuh does not serve, the choice between the M2L kernels (FP64:
+// m2l_fp64.cu) and the sibling kernel (far_func of
 // aran/aransolver3d.c:333-354) with the "point and shoot" operator of
 // aran_spherical_seriesd_to_local_rotate (aran/aransphericalseriesd-rotate.c:
 // 165-207): rotate the source multipole so the translation runs along z,
@@ -32,13 +34,6 @@ namespace {
 __constant__ uint16_t c_dir_codes[316];
 __constant__ int8_t c_dir_vec[316 * 3];
 
-// asynchronous copy of one complex coefficient (8 bytes FP32, 16 bytes FP64)
-template <typename T>
-__device__ __forceinline__ void cp_async_cplx(cplx<T> *dst, const cplx<T> *src) {
-  if (sizeof(cplx<T>) == 8) cp_async8(dst, src);
-  else cp_async16(dst, src);
-}
-
 struct M2LOffsets {
   int ef, ei, ph, rp, vv, stride;  // in T units; ef/ei: (E, O) pairs in source-order planes
 };
@@ -47,7 +42,7 @@ constexpr int kSibWarps = 8;   // consumers: one per child of the parent
 constexpr int kMaxRounds = ((kMaxOrder + 1) * (kMaxOrder + 2) / 2 + 31) / 32;
 
 template <typename T, int NST, int R, int G>
-__global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
+__global__ void __launch_bounds__(32 * (kSibWarps + 1), 3)
     k_m2l_sibling(int nparents, const int *__restrict__ parents, const int *__restrict__ child,
                   const int *__restrict__ begin, const int *__restrict__ end,
                   const int *__restrict__ col, const int *__restrict__ ncol,
@@ -55,7 +50,7 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
                   const T *__restrict__ dirs, M2LOffsets D,
                   const uint8_t *__restrict__ lm_g, double scale_e,
                   const cplx<T> *__restrict__ mult, cplx<T> *__restrict__ loc,
-                  int *__restrict__ err, int polls, int nsplit, cplx<T> *__restrict__ parts) {
+                  int *__restrict__ err, int polls) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int nm = tri(p), nl = tri(p + 1);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -162,10 +157,7 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
     s_nact = tot;
   }
   __syncthreads();
-  // this CTA's part of the offset list
-  const int first = s_nact * (int)blockIdx.y / nsplit;
-  const int nact = s_nact * ((int)blockIdx.y + 1) / nsplit - first;
-  active += first;
+  const int nact = s_nact;
   const uint32_t tbytes = (uint32_t)(D.stride * sizeof(T));
 
   if (w == kSibWarps) {
@@ -224,7 +216,7 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
         if (c >= nm) continue;
         cplx<T> *dst = cbuf + g * (nm + nl) + nl + c;
         if (next_i < nact && next_s[g] >= 0)
-          cp_async_cplx(dst, mult + (size_t)next_s[g] * nm + c);
+          cp_async8(dst, mult + (size_t)next_s[g] * nm + c);
         else
           *dst = cmake<T>(0, 0);
       }
@@ -356,41 +348,17 @@ __global__ void __launch_bounds__(32 * (kSibWarps + 1), sizeof(T) == 4 ? 3 : 2)
     if (NST > 0 && lane == 0) mbar_arrive(&empty[b]);
   }
   cp_async_wait_all();   // source copies still in flight after an early stop
-  if (nact > 0 || nsplit > 1) {
+  if (nact > 0) {
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       if (!tvalid[g]) continue;
       const T ih = (T)(ldexp(1.0, depth[tg[g]]) / scale_e);
-      // a part's sums go to the workspace [part][parent][child][coefficient]
-      cplx<T> *out = nsplit == 1
-                         ? loc + (size_t)tg[g] * nl
-                         : parts + (((size_t)blockIdx.y * nparents + blockIdx.x * G + g) *
-                                        kSibWarps + w) * nl;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         int c = lane + 32 * r;
-        if (c < nl) out[c] = cmake<T>(acc[g][r].re * ih, acc[g][r].im * ih);
+        if (c < nl) loc[(size_t)tg[g] * nl + c] = cmake<T>(acc[g][r].re * ih, acc[g][r].im * ih);
       }
     }
-  }
-}
-
-// the parts of a split pass added in order, one warp per child
-template <typename T>
-__global__ void __launch_bounds__(32 * kSibWarps)
-    k_m2l_parts_sum(int nparents, int nsplit, const int *__restrict__ parents,
-                    const int *__restrict__ child, const int *__restrict__ begin,
-                    const int *__restrict__ end, int nl, const cplx<T> *__restrict__ parts,
-                    cplx<T> *__restrict__ loc) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int t = child[parents[blockIdx.x]] + w;
-  if (end[t] <= begin[t]) return;
-  const size_t step = (size_t)nparents * kSibWarps * nl;
-  const cplx<T> *p = parts + ((size_t)blockIdx.x * kSibWarps + w) * nl;
-  for (int c = lane; c < nl; c += 32) {
-    cplx<T> v = cmake<T>(0, 0);
-    for (int k = 0; k < nsplit; ++k) v = cadd(v, p[k * step + c]);
-    loc[(size_t)t * nl + c] = v;
   }
 }
 
@@ -436,33 +404,12 @@ bool try_launch(AranGpuSolver3d *s, OpTables<T> &tb, const M2LOffsets &D, const 
   size_t sm = m2l_smem<T, NST, G>(p, D.stride);
   if ((int)sm > dev_smem) return false;
   smem_opt_in(k_m2l_sibling<T, NST, R, G>, sm);
-  // few parents: their offset lists are split over CTAs (FP64 only: the sums
-  // of a split list round differently, which FP32 results would show).  An
-  // FP64 CTA keeps its SM's FP64 pipe busy alone (half a lane a cycle per
-  // scheduler).  The FP64 root levels of a mixed order-16 solve, 72
-  // parents, took 12.6 ms unsplit on 36 SMs and take 3.0 ms
-  const int groups = ceil_div(count, G);
-  int nsm = 0;
-  ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
-  const int nsplit = sizeof(T) == 8 ? split_parts(groups, nsm) : 1;
-  cplx<T> *parts = nullptr;
-  if (nsplit > 1) {
-    s->m2l_part64.reserve((size_t)nsplit * count * kSibWarps * tri(p + 1) * 2);
-    parts = reinterpret_cast<cplx<T> *>(s->m2l_part64.ptr);
-  }
-  k_m2l_sibling<T, NST, R, G><<<dim3(groups, nsplit), 32 * (kSibWarps + 1), sm, st>>>(
+  k_m2l_sibling<T, NST, R, G><<<ceil_div(count, G), 32 * (kSibWarps + 1), sm, st>>>(
       count, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr, t.ncol.ptr,
       t.ijk.ptr, t.depth.ptr, p, tb.dir_m2l.ptr, D, tb.lm.ptr, s->scale_e, mult, loc,
-      s->err_dev.ptr, consumer_wait_polls(), nsplit, parts);
+      s->err_dev.ptr, consumer_wait_polls());
   ACHECK(cudaGetLastError());
   s->launches++;
-  if (nsplit > 1) {
-    k_m2l_parts_sum<T><<<count, 32 * kSibWarps, 0, st>>>(count, nsplit, parents, t.child.ptr,
-                                                         t.begin.ptr, t.end.ptr, tri(p + 1), parts,
-                                                         loc);
-    ACHECK(cudaGetLastError());
-    s->launches++;
-  }
   return true;
 }
 
@@ -471,13 +418,11 @@ void launch_t(AranGpuSolver3d *s, OpTables<T> &tb, const int *parents, int count
               const cplx<T> *mult, cplx<T> *loc, cudaStream_t st) {
   if (count <= 0) return;
   const int kern = m2l_kernel_choice(s);
-  if constexpr (sizeof(T) == 4) {
-    if (kern == ARAN_M2L_TENSOR &&
-        launch_m2l_tc(s, parents, count, reinterpret_cast<const float *>(mult),
-                      reinterpret_cast<float *>(loc), st))
-      return;
-    if (kern != ARAN_M2L_SIBLING && launch_m2l_lanes(s, tb, parents, count, mult, loc, st)) return;
-  }
+  if (kern == ARAN_M2L_TENSOR &&
+      launch_m2l_tc(s, parents, count, reinterpret_cast<const float *>(mult),
+                    reinterpret_cast<float *>(loc), st))
+    return;
+  if (kern != ARAN_M2L_SIBLING && launch_m2l_lanes(s, tb, parents, count, mult, loc, st)) return;
   upload_codes(s->device);
   const int p = s->cfg.order;
   M2LOffsets D;
@@ -492,8 +437,8 @@ void launch_t(AranGpuSolver3d *s, OpTables<T> &tb, const int *parents, int count
   // R = rounds of 32 lanes over the tri(p+1) local coefficients; G parents
   // per CTA (each warp takes child w of every one of them)
   const int nl = tri(p + 1);
-  // a sibling configuration set on the solver (FP32 part), when it serves nl
-  if (sizeof(T) == 4 && s->m2l_nst > 0 && s->m2l_g > 0) {
+  // a sibling configuration set on the solver, when it serves nl
+  if (s->m2l_nst > 0 && s->m2l_g > 0) {
     const int nst = s->m2l_nst, g = s->m2l_g;
     bool ok = false;
 #define ARAN_TRY(NST_, R_, G_)                                                               \
@@ -509,17 +454,7 @@ void launch_t(AranGpuSolver3d *s, OpTables<T> &tb, const int *parents, int count
 #undef ARAN_TRY
     if (ok) return;
   }
-  // FP64: one parent per CTA.  A column without a source at an offset costs
-  // FP64 operations, which are all that counts there, and sharing a table
-  // read between columns saves nothing (200k Plummer particles at order 12,
-  // the whole solve: 48.8 ms, 54.8 with two parents)
-  if (sizeof(T) == 8 && nl <= 96 &&
-      try_launch<T, 3, 3, 1>(s, tb, D, parents, count, mult, loc, st, dev_smem))
-    return;
-  if (sizeof(T) == 8 && nl > 96 && nl <= 160 &&
-      try_launch<T, 1, 5, 1>(s, tb, D, parents, count, mult, loc, st, dev_smem))
-    return;
-  // (two table slots keep a p <= 12 FP32 CTA under a third of the shared
+  // (two table slots keep a p <= 12 CTA under a third of the shared
   // memory, so three CTAs share an SM)
   if (nl <= 96) {
     if (try_launch<T, 2, 3, 2>(s, tb, D, parents, count, mult, loc, st, dev_smem)) return;
@@ -570,9 +505,7 @@ void launch_m2l(AranGpuSolver3d *s, bool fp64, int first, int count, cudaStream_
                     reinterpret_cast<const cplx<float> *>(s->mult32.ptr),
                     reinterpret_cast<cplx<float> *>(s->loc32.ptr), st);
   else
-    launch_t<double>(s, s->t64, parents, count,
-                     reinterpret_cast<const cplx<double> *>(s->mult64.ptr),
-                     reinterpret_cast<cplx<double> *>(s->loc64.ptr), st);
+    launch_m2l_fp64(s, parents, count, st);
 }
 
 }  // namespace aran

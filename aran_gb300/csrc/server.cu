@@ -99,6 +99,7 @@ int64_t footprint_bytes(const AranGpuConfig3d *c, int64_t n) {
   b += nodes * (int64_t)(tri(p) + 2 * tri(p + 1)) * 2 * real;      // expansions, M2L sums
   b += n * (8 * real);                                             // hi + lo positions
   b += nodes * (189 * 6 + 8) + nodes * 60 * 8;                     // far/near lists
+  b += 140ll * 2 * (p + 2) * (p + 2) * (p + 2) * 8;                // FP64 M2L stream tables
   return b + (64ll << 20);
 }
 

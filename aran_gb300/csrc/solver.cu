@@ -192,7 +192,7 @@ void aran_gpu_solver3d_destroy(AranGpuSolver3d *s) {
     tb->rec.release(); tb->p2mf.release(); tb->vt.release(); tb->vm.release(); tb->vl.release();
     tb->gz.release(); tb->gm.release(); tb->dir_m2l.release(); tb->dir_m2m.release();
     tb->dir_l2l.release(); tb->dir_lanes.release(); tb->lm.release();
-    tb->oct_lanes[0].release(); tb->oct_lanes[1].release();
+    tb->oct_lanes[0].release(); tb->oct_lanes[1].release(); tb->m2l64.release();
   }
   {
     auto *tb = &s->t32;

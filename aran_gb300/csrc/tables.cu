@@ -313,6 +313,8 @@ void build_tables_t(AranGpuSolver3d *s, OpTables<T> &tb, cudaStream_t st) {
   if constexpr (sizeof(T) == 4) {
     build_oct_lane_tables(tb, st);
     ACHECK(cudaStreamSynchronize(st));
+  } else {
+    build_m2l_fp64_tables(tb, st);
   }
   scratch.release();
 }
