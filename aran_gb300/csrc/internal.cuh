@@ -125,6 +125,7 @@ struct DevTree {
   DBuf<int> parents;                  // internal nodes of depth >= 1 (their children take M2L)
   int n_parents = 0;
   int n_big = 0;
+  int n_heavy = 0;                    // heavy near ranges (the chunked P2P pass)
   int64_t n_far = 0;
   bool far_counted = false;           // far_off and n_far made (count_far_lists)
   bool far_built = false;             // far_src/far_dir written (build_far_lists)

@@ -489,18 +489,9 @@ void build_p2p_work(AranGpuSolver3d *s) {
                                                t.leaf_be.ptr, t.leaf_chi.ptr, t.leaf_clo.ptr);
   ACHECK(cudaGetLastError());
   s->launches++;
-  // chunk total and heavy-range count, as k_near listed them
-  int *hb = s->h_small + 8;   // pinned
-  hb[0] = hb[1] = 0;
-  if (t.n_near_rng > 0) {
-    ACHECK(cudaMemcpyAsync(hb, t.big_rng.ptr, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    ACHECK(cudaStreamSynchronize(st));
-  }
-  const int nbig = hb[0], nheavy = hb[1];
-  t.n_big = nbig;
-  if (nbig) {
-    t.big_items.reserve(nbig);
-    k_big_items<<<nheavy, 64, 0, st>>>(t.big_rng.ptr + 2, nl, t.near_off.ptr, t.near_rng.ptr,
+  if (t.n_big) {
+    t.big_items.reserve(t.n_big);
+    k_big_items<<<t.n_heavy, 64, 0, st>>>(t.big_rng.ptr + 2, nl, t.near_off.ptr, t.near_rng.ptr,
                                        t.leaf_be.ptr, t.big_items.ptr);
     ACHECK(cudaGetLastError());
     s->launches++;

@@ -164,7 +164,7 @@ int aran_gpu_solver3d_create(const AranGpuConfig3d *cfg, AranGpuSolver3d **out) 
       build_tables_fp64(s);
     }
     s->err_dev.reserve(4);
-    ACHECK(cudaHostAlloc(&s->h_small, 16 * sizeof(int), cudaHostAllocDefault));
+    ACHECK(cudaHostAlloc(&s->h_small, 64 * sizeof(int), cudaHostAllocDefault));
     ACHECK(cudaMemset(s->err_dev.ptr, 0, sizeof(int)));
   } catch (const CudaError &ce) {
     int r = from_cuda(ce);

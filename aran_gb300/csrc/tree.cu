@@ -5,9 +5,9 @@
 // (vsg_prtree3d_near_far_traversal_full, aran/aransolver3d.c:1189-1190) by a
 // Morton-sorted, level-synchronous build:
 //   1. 63-bit keys from the 21-bit quantised coordinates, radix sort;
-//   2. level by level, a node with more than maxbox points (and depth below
-//      the limit) gets its 8 octants, whose point ranges are found by binary
-//      search in the sorted keys;
+//   2. a node with more than maxbox points (and depth below the limit) gets its
+//      8 octants; the internal nodes of all levels are read off the sorted keys
+//      at once (a leaf predicate is asked level by level);
 //   3. colleagues (adjacent same-depth non-empty nodes, <= 27) level by level;
 //   4. far lists: non-empty children of the parent's internal colleagues that
 //      are not adjacent (the M2L sources of aran/aransolver3d.c:333-354);
@@ -23,7 +23,9 @@
 // level's kernels then run over the nodes of all systems at once.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <utility>
+#include <vector>
 
 #include "internal.cuh"
 
@@ -95,12 +97,202 @@ __global__ void k_roots(NodeArrays na, int nsys, const int *__restrict__ sys_off
   na.depth[r] = 0;
   na.begin[r] = sys_off[r];
   na.end[r] = sys_off[r + 1];
-  na.child[r] = -1;
+  na.child[r] = -1;                      // until k_make_nodes or k_make_children
   na.parent[r] = -1;
   na.sys[r] = r;
   na.center[3 * r] = node_center_axis(b[0], b[3], 0, 0);
   na.center[3 * r + 1] = node_center_axis(b[1], b[4], 0, 0);
   na.center[3 * r + 2] = node_center_axis(b[2], b[5], 0, 0);
+}
+
+// ---------------------------------------------------------------------------
+// Subdivision of all levels at once.  A node of depth d holds the particles
+// that share the first d digits of their keys (within a system).  One starts at
+// sorted place i if d exceeds the digits that places i - 1 and i share, and has
+// more than maxbox points if places i and i + maxbox share d: the internal nodes
+// that start at i are those of the depths lo .. hi.  Counted per depth and block
+// of places and scanned depth by depth, their numbers are their ranks in level
+// order, the children of the node of rank r in its level lie at eight times r
+// in the next, and one readback (the counts) is all that the host waits for;
+// level by level each took one, with a flag pass, a scan and a binary search
+// of its own: 40 us a level.  Bound by latency: 10k uniform particles (4 levels)
+// 0.056 ms, 0.165 before; 4M Plummer particles (11 levels) 0.115 ms, 0.524.
+// ---------------------------------------------------------------------------
+constexpr int kPlaceBlock = 256, kPlaceItems = 4, kPlaces = kPlaceBlock * kPlaceItems;
+constexpr int kPlaceSlots = kPlaces / 32;   // warp-wide runs of places in a block
+static_assert(kPlaceSlots == 32, "a warp scans a block's slots");
+
+__device__ __forceinline__ int shared_digits(uint64_t a, uint64_t b) {
+  return a == b ? kKeyBits : (__clzll((long long)(a ^ b)) - 1) / 3;
+}
+
+__device__ __forceinline__ int system_of(int64_t i, int nsys, const int *__restrict__ sys_off) {
+  int lo = 0, hi = nsys;                 // last system with sys_off <= i
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (sys_off[mid] <= i) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// depths lo .. hi of the internal nodes that start at place i
+__device__ __forceinline__ void internal_depths(int64_t i, int64_t n, int nsys,
+                                                const int *__restrict__ sys_off,
+                                                const uint64_t *__restrict__ keys, int maxbox,
+                                                int maxd, int &lo, int &hi) {
+  lo = kKeyBits + 1;
+  hi = -1;
+  if (i >= n) return;
+  const int sy = system_of(i, nsys, sys_off);
+  if (i + maxbox >= sys_off[sy + 1]) return;
+  const uint64_t k = keys[i];
+  lo = i == sys_off[sy] ? 0 : shared_digits(keys[i - 1], k) + 1;
+  hi = min(shared_digits(k, keys[i + maxbox]), maxd - 1);
+  if (lo > hi) {
+    lo = kKeyBits + 1;
+    hi = -1;
+  }
+}
+
+// counts[d][block]: internal nodes of depth d that start in the block's places
+__global__ void __launch_bounds__(kPlaceBlock)
+    k_count_internal(int64_t n, int nsys, const int *__restrict__ sys_off,
+                     const uint64_t *__restrict__ keys, int maxbox, int maxd,
+                     int *__restrict__ counts) {
+  __shared__ int cnt[kKeyBits][kPlaceSlots + 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int c = 0; c < kPlaceItems; ++c) {
+    int lo, hi, v = 0;
+    internal_depths((int64_t)blockIdx.x * kPlaces + c * kPlaceBlock + threadIdx.x, n, nsys, sys_off,
+                    keys, maxbox, maxd, lo, hi);
+    const int d0 = __reduce_min_sync(0xffffffffu, lo), d1 = __reduce_max_sync(0xffffffffu, hi);
+    for (int d = d0; d <= d1; ++d) {
+      const unsigned m = __ballot_sync(0xffffffffu, lo <= d && d <= hi);
+      if (lane == d) v = __popc(m);
+    }
+    if (lane < kKeyBits) cnt[lane][c * (kPlaceBlock / 32) + w] = v;
+  }
+  __syncthreads();
+  for (int d = w; d < kKeyBits; d += kPlaceBlock / 32) {
+    const int t = __reduce_add_sync(0xffffffffu, cnt[d][lane]);
+    if (lane == 0) counts[(int64_t)d * gridDim.x + blockIdx.x] = t;
+  }
+}
+
+// place and parent's rank of every internal node, by rank in level order
+__global__ void __launch_bounds__(kPlaceBlock)
+    k_list_internal(int64_t n, int nsys, const int *__restrict__ sys_off,
+                    const uint64_t *__restrict__ keys, int maxbox, int maxd,
+                    const int *__restrict__ first, int *__restrict__ start,
+                    int *__restrict__ prank) {
+  __shared__ int pre[kKeyBits][kPlaceSlots + 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int lo[kPlaceItems], hi[kPlaceItems];
+#pragma unroll
+  for (int c = 0; c < kPlaceItems; ++c) {
+    int v = 0;
+    internal_depths((int64_t)blockIdx.x * kPlaces + c * kPlaceBlock + threadIdx.x, n, nsys, sys_off,
+                    keys, maxbox, maxd, lo[c], hi[c]);
+    const int d0 = __reduce_min_sync(0xffffffffu, lo[c]), d1 = __reduce_max_sync(0xffffffffu, hi[c]);
+    for (int d = d0; d <= d1; ++d) {
+      const unsigned m = __ballot_sync(0xffffffffu, lo[c] <= d && d <= hi[c]);
+      if (lane == d) v = __popc(m);
+    }
+    if (lane < kKeyBits) pre[lane][c * (kPlaceBlock / 32) + w] = v;
+  }
+  __syncthreads();
+  // ranks before each run of places
+  for (int d = w; d < kKeyBits; d += kPlaceBlock / 32) {
+    const int mine = pre[d][lane];
+    int v = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    pre[d][lane] = first[(int64_t)d * gridDim.x + blockIdx.x] + v - mine;
+  }
+  __syncthreads();
+  const unsigned before = (1u << lane) - 1;
+#pragma unroll
+  for (int c = 0; c < kPlaceItems; ++c) {
+    const int slot = c * (kPlaceBlock / 32) + w;
+    const int64_t i = (int64_t)blockIdx.x * kPlaces + c * kPlaceBlock + threadIdx.x;
+    const int d0 = __reduce_min_sync(0xffffffffu, lo[c]), d1 = __reduce_max_sync(0xffffffffu, hi[c]);
+    unsigned up = 0;                     // the depth above's starts in this run
+    for (int d = d0; d <= d1; ++d) {
+      const unsigned m = __ballot_sync(0xffffffffu, lo[c] <= d && d <= hi[c]);
+      if (lo[c] <= d && d <= hi[c]) {
+        const int rk = pre[d][slot] + __popc(m & before);
+        start[rk] = (int)i;
+        if (d > 0) prank[rk] = pre[d - 1][slot] + __popc(up & (before | 1u << lane)) - 1;
+      }
+      up = m;
+    }
+  }
+}
+
+// first rank and first node of each depth (by value to the kernel)
+struct LevelStarts {
+  int rank[kKeyBits + 1], node[kKeyBits + 2];
+};
+
+// every third bit of a key from bit 0
+__device__ __forceinline__ int every_third(uint64_t v) {
+  v &= 0x1249249249249249ull;
+  v = (v ^ (v >> 2)) & 0x10c30c30c30c30c3ull;
+  v = (v ^ (v >> 4)) & 0x100f00f00f00f00full;
+  v = (v ^ (v >> 8)) & 0x001f0000ff0000ffull;
+  v = (v ^ (v >> 16)) & 0x001f00000000ffffull;
+  v = (v ^ (v >> 32)) & 0x00000000001fffffull;
+  return (int)v;
+}
+
+// eight threads per internal node, thread c making child c: its points end at
+// the first key beyond its digits, and begin where child c-1's end
+__global__ void k_make_nodes(int total, LevelStarts ls, const int *__restrict__ start,
+                             const int *__restrict__ prank, int nsys,
+                             const int *__restrict__ sys_off, const uint64_t *__restrict__ keys,
+                             int maxbox, int maxd, NodeArrays na,
+                             const double *__restrict__ sys_box, int *__restrict__ parents) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(g & 7);
+  const bool live = (g >> 3) < total;
+  const int rk = live ? (int)(g >> 3) : 0;
+  int d = 0;
+  while (d < kKeyBits - 1 && rk >= ls.rank[d + 1]) ++d;
+  const int i = start[rk], sy = system_of(i, nsys, sys_off);
+  const int shift = 3 * (kKeyBits - d - 1);
+  const uint64_t up = keys[i] >> (shift + 3), pk = (up << 3) | (uint64_t)c;
+  int lo = i, hi = sys_off[sy + 1];
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if ((keys[mid] >> shift) <= pk) lo = mid + 1; else hi = mid;
+  }
+  // the eight threads of a node are eight consecutive lanes
+  const int prev = __shfl_up_sync(0xffffffffu, lo, 1, 8);
+  if (!live) return;
+  const int node = d == 0 ? sy : ls.node[d] + 8 * (prank[rk] - ls.rank[d - 1]) + (int)(up & 7);
+  const int base = ls.node[d + 1] + 8 * (rk - ls.rank[d]);
+  if (c == 0) {
+    na.child[node] = base;
+    if (d > 0) parents[rk - ls.rank[1]] = node;
+  }
+  const int cn = base + c, b = c == 0 ? i : prev;
+  const double *bx = sys_box + 9 * sy;
+  const int ci = every_third(pk), cj = every_third(pk >> 1), ck = every_third(pk >> 2);
+  na.key[cn] = pk;
+  na.ijk[3 * cn] = ci;
+  na.ijk[3 * cn + 1] = cj;
+  na.ijk[3 * cn + 2] = ck;
+  na.depth[cn] = (uint8_t)(d + 1);
+  na.begin[cn] = b;
+  na.end[cn] = lo;
+  if (!(lo - b > maxbox && d + 1 < maxd)) na.child[cn] = -1;   // else its own threads set it
+  na.parent[cn] = node;
+  na.sys[cn] = sy;
+  na.center[3 * cn] = node_center_axis(bx[0], bx[3], d + 1, ci);
+  na.center[3 * cn + 1] = node_center_axis(bx[1], bx[4], d + 1, cj);
+  na.center[3 * cn + 2] = node_center_axis(bx[2], bx[5], d + 1, ck);
 }
 
 __global__ void k_flag_internal(int cnt, int off, const int *__restrict__ begin,
@@ -343,15 +535,99 @@ __device__ __forceinline__ bool adjacent_ml(const int *ijk, const uint8_t *depth
   return true;
 }
 
-// Near ranges (and semifar nodes) of leaf ordinal L; mode 0 counts, mode 1
-// writes.  With a semifar threshold T > 0 an internal colleague's subtree is
-// walked: descendants touching the leaf are walked further (near when they
+// totals that the host reads after the counting pass
+struct NearTotals {
+  int chunks, heavy;
+};
+
+// chunks of a range of c points in the chunked P2P pass, 0 if it is not heavy
+__device__ __forceinline__ int heavy_chunks(int c) {
+  return c > kBigRange ? (c + kBigRange - 1) / kBigRange : 0;
+}
+
+// Near ranges of leaf ordinal L, a warp per leaf: its colleagues (lane j takes
+// colleague j), then the leaf colleagues of each ancestor.  WRITE false counts:
+// ranges per leaf (zero for the ordinals from the last leaf up to nbound) and the
+// heavy ranges' chunks; true writes.  A range is every leaf under a node;
+// ranges above kBigRange points are listed for the chunked P2P pass: big[0] =
+// chunk total, big[1] = heavy ranges, then per heavy range its index and the
+// offset of its first chunk.  Bound by the chain of loads up the tree.  All lists
+// of 150k Plummer particles 0.177 ms; 0.290 with a thread per leaf and three
+// more readbacks; of 10k uniform particles 0.108 ms, 0.181.
+template <bool WRITE>
+__global__ void k_near_warp(int nbound, const int *__restrict__ nleaves_p,
+                            const int *__restrict__ leaf_node, const int *__restrict__ begin,
+                            const int *__restrict__ end, const int *__restrict__ child,
+                            const int *__restrict__ parent, const int *__restrict__ col,
+                            const int *__restrict__ ncol, const int *__restrict__ lf_begin,
+                            const int *__restrict__ lf_end, int *__restrict__ near_cnt,
+                            NearTotals *__restrict__ tot, const int *__restrict__ near_off,
+                            int *__restrict__ near_rng, int *__restrict__ big) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int L = (int)(g >> 5), lane = (int)(g & 31);
+  if (L >= nbound) return;
+  if (L >= *nleaves_p) {
+    if (!WRITE && lane == 0) near_cnt[L] = 0;
+    return;
+  }
+  int a = leaf_node[L];
+  int k = WRITE ? near_off[L] : 0;
+  int chunks = 0, heavy = 0;
+  bool own = true;
+  do {
+    const int up = parent[a], nc = ncol[a];
+    bool take = false;
+    int q = 0, b = 0, e = 0;
+    if (lane < nc) {
+      q = col[27 * a + lane];
+      b = begin[q];
+      e = end[q];
+      take = own || (child[q] < 0 && e != b);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (take) {
+      const int nch = heavy_chunks(e - b);
+      if (WRITE) {
+        const int at = k + __popc(m & ((1u << lane) - 1));
+        near_rng[2 * at] = lf_begin[q];
+        near_rng[2 * at + 1] = lf_end[q];
+        if (nch) {
+          const int coff = atomicAdd(&big[0], nch);
+          const int h = atomicAdd(&big[1], 1);
+          big[2 + 2 * h] = at;
+          big[3 + 2 * h] = coff;
+        }
+      } else if (nch) {
+        chunks += nch;
+        ++heavy;
+      }
+    }
+    k += __popc(m);
+    a = up;
+    own = false;
+  } while (a >= 0);
+  if (!WRITE) {
+    chunks = __reduce_add_sync(0xffffffffu, chunks);
+    heavy = __reduce_add_sync(0xffffffffu, heavy);
+    if (lane == 0) {
+      near_cnt[L] = k;
+      if (heavy) {
+        atomicAdd(&tot->chunks, chunks);
+        atomicAdd(&tot->heavy, heavy);
+      }
+    }
+  }
+}
+
+// Near ranges and semifar nodes of leaf ordinal L with a semifar threshold T > 0;
+// mode 0 counts, mode 1 writes.  An internal colleague's subtree is walked: descendants touching the leaf are walked further (near when they
 // are leaves), a descendant that does not touch it is a semifar node of the
 // leaf when it holds more than T points and a near range otherwise; a
 // coarser leaf colleague of an ancestor is near unless the shallowest node
 // between that ancestor and L that does not touch it holds more than T
 // points (it then reaches L through its own semifar P2L/M2P).
-__global__ void k_near(int nleaves, const int *__restrict__ leaf_node, const int *__restrict__ begin,
+__global__ void k_near(int nbound, const int *__restrict__ nleaves_p,
+                       const int *__restrict__ leaf_node, const int *__restrict__ begin,
                        const int *__restrict__ end, const int *__restrict__ child,
                        const int *__restrict__ parent, const int *__restrict__ col,
                        const int *__restrict__ ncol, const int *__restrict__ lf_begin,
@@ -360,25 +636,28 @@ __global__ void k_near(int nleaves, const int *__restrict__ leaf_node, const int
                        const int *__restrict__ near_off, int *__restrict__ near_rng,
                        int *__restrict__ semi_cnt, const int *__restrict__ semi_off,
                        int *__restrict__ semi_node, int *__restrict__ semi_leaf,
-                       int *__restrict__ big, int mode) {
+                       NearTotals *__restrict__ tot, int *__restrict__ big, int mode) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
-  if (L >= nleaves) return;
+  if (L >= nbound) return;
+  if (L >= *nleaves_p) {
+    if (!mode) near_cnt[L] = semi_cnt[L] = 0;
+    return;
+  }
   int node = leaf_node[L];
   int k = 0, ks = 0;
   int w = mode ? near_off[L] : 0;
-  int ws = (mode && T > 0) ? semi_off[L] : 0;
-  // a range is every leaf under node q, so it holds end[q] - begin[q]
-  // points; ranges above kBigRange are listed for the chunked P2P pass:
-  // big[0] = chunk total, big[1] = heavy ranges, then per heavy range its
-  // index and the offset of its first chunk
+  int ws = mode ? semi_off[L] : 0;
   auto emit = [&](int q) {
+    const int nch = heavy_chunks(end[q] - begin[q]);
     if (mode) {
       near_rng[2 * (w + k)] = lf_begin[q];
       near_rng[2 * (w + k) + 1] = lf_end[q];
-      const int c = end[q] - begin[q];
-      if (c > kBigRange) {
-        const int coff = atomicAdd(&big[0], (c + kBigRange - 1) / kBigRange);
-        const int h = atomicAdd(&big[1], 1);
+    }
+    if (nch) {
+      int *sum = mode ? big : &tot->chunks;   // chunks, then heavy ranges
+      const int coff = atomicAdd(&sum[0], nch);
+      const int h = atomicAdd(&sum[1], 1);
+      if (mode) {
         big[2 + 2 * h] = w + k;
         big[3 + 2 * h] = coff;
       }
@@ -388,7 +667,7 @@ __global__ void k_near(int nleaves, const int *__restrict__ leaf_node, const int
   int nc = ncol[node];
   for (int j = 0; j < nc; ++j) {
     int q = col[27 * node + j];
-    if (T <= 0 || child[q] < 0) {
+    if (child[q] < 0) {
       emit(q);
       continue;
     }
@@ -419,18 +698,16 @@ __global__ void k_near(int nleaves, const int *__restrict__ leaf_node, const int
     for (int j = 0; j < na; ++j) {
       int q = col[27 * a + j];
       if (child[q] >= 0 || end[q] == begin[q]) continue;
-      if (T > 0) {
-        int x = -1;
-        for (int y = node; y != a; y = parent[y])
-          if (!adjacent_ml(ijk, depth, q, y)) x = y;
-        if (x >= 0 && end[x] - begin[x] > T) continue;
-      }
+      int x = -1;
+      for (int y = node; y != a; y = parent[y])
+        if (!adjacent_ml(ijk, depth, q, y)) x = y;
+      if (x >= 0 && end[x] - begin[x] > T) continue;
       emit(q);
     }
   }
   if (!mode) {
     near_cnt[L] = k;
-    if (T > 0) semi_cnt[L] = ks;
+    semi_cnt[L] = ks;
   }
 }
 
@@ -619,13 +896,152 @@ void apply_leaf_predicate(AranGpuSolver3d *s, int off, int cnt, int d, int *d_fl
   ACHECK(cudaStreamSynchronize(st));
 }
 
+int depth_limit(const AranGpuConfig3d &c) {
+  return c.max_depth > 0 && c.max_depth < kKeyBits ? c.max_depth : kKeyBits;
+}
+
+size_t node_estimate(const AranGpuSolver3d *s, int64_t n) {
+  return (size_t)s->nsys + (size_t)(8 * (n / (s->cfg.maxbox + 1) + 1) * 2 + 64);
+}
+
+// the error word, read with the first counts
+void check_points(const AranGpuSolver3d *s, int err) {
+  if (err & kErrNonFinite) throw InputError{"a particle coordinate or charge is NaN or infinite"};
+  if ((err & kErrOutside) && s->cfg.precision == ARAN_PRECISION_MIXED)
+    throw InputError{"a particle lies outside the solver's box (mixed precision needs every point "
+                     "inside [lbound, ubound])"};
+}
+
+// the octree of the sorted keys, and its internal nodes of depth >= 1 in node
+// order (one M2L block each: their children)
+void subdivide(AranGpuSolver3d *s, int64_t n, cudaStream_t st) {
+  const AranGpuConfig3d &c = s->cfg;
+  DevTree &t = s->tree;
+  const int TB = 256, nsys = s->nsys, maxd = depth_limit(c);
+  const int nb = (int)((n + kPlaces - 1) / kPlaces);
+  const int nc = kKeyBits * nb;
+  DBuf<int> &tmp = s->scan_tmp;
+  tmp.reserve(2 * (size_t)nc + 2);
+  int *first = tmp.ptr + nc + 1;
+  k_count_internal<<<nb, kPlaceBlock, 0, st>>>(n, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox,
+                                               maxd, tmp.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
+  ACHECK(cudaMemsetAsync(tmp.ptr + nc, 0, sizeof(int), st));
+  exclusive_scan(s, tmp.ptr, first, nc + 1, st);
+  // first rank of each depth and their total, with the error word
+  int *hb = s->h_small + 16;
+  ACHECK(cudaMemcpy2DAsync(hb, sizeof(int), first, nb * sizeof(int), sizeof(int), kKeyBits + 1,
+                           cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaMemcpyAsync(s->h_small + 2, s->err_dev.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaStreamSynchronize(st));
+  check_points(s, s->h_small[2]);
+  LevelStarts ls = {};
+  t.level_off.assign(1, 0);
+  t.level_internal.clear();
+  int off = 0, cnt = nsys, d = 0;
+  for (; cnt > 0; ++d) {
+    ls.node[d] = off;
+    off += cnt;
+    t.level_off.push_back(off);
+    const int ninternal = d < kKeyBits ? hb[d + 1] - hb[d] : 0;
+    t.level_internal.push_back(ninternal);
+    cnt = 8 * ninternal;
+  }
+  for (int k = 0; k <= kKeyBits; ++k) ls.rank[k] = hb[k];
+  for (int k = d; k < kKeyBits + 2; ++k) ls.node[k] = off;
+  t.nnodes = off;
+  t.nlevels = d;
+  const int total = hb[kKeyBits];
+  t.n_parents = total - t.level_internal[0];
+  t.parents.reserve(t.n_parents + 1);
+  grow_nodes(t, std::max((size_t)off, node_estimate(s, n)), 0, st);
+  NodeArrays na = arrays(t);
+  k_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(na, nsys, s->sys_off.ptr, s->sys_box.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
+  if (total == 0) return;
+  DBuf<int> &list = s->sort_tmp;
+  list.reserve(2 * (size_t)total);
+  k_list_internal<<<nb, kPlaceBlock, 0, st>>>(n, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox,
+                                              maxd, first, list.ptr, list.ptr + total);
+  ACHECK(cudaGetLastError());
+  k_make_nodes<<<ceil_div(8 * (int64_t)total, TB), TB, 0, st>>>(
+      total, ls, list.ptr, list.ptr + total, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox, maxd,
+      na, s->sys_box.ptr, t.parents.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches += 2;
+}
+
+// the same level by level, each level's internal nodes shown to the leaf
+// predicate before they are split
+void subdivide_levels(AranGpuSolver3d *s, int64_t n, cudaStream_t st) {
+  const AranGpuConfig3d &c = s->cfg;
+  DevTree &t = s->tree;
+  const int TB = 256, nsys = s->nsys, maxd = depth_limit(c);
+  grow_nodes(t, node_estimate(s, n), 0, st);
+  t.level_off.assign(1, 0);
+  t.level_internal.clear();
+  NodeArrays na = arrays(t);
+  k_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(na, nsys, s->sys_off.ptr, s->sys_box.ptr);
+  s->launches++;
+  int off = 0, cnt = nsys;
+  DBuf<int> &flags = s->scan_tmp;
+  int d = 0;
+  int *hostbuf = s->h_small;   // pinned: the level's readbacks go together
+  hostbuf[2] = 0;
+  while (cnt > 0) {
+    t.level_off.push_back(off + cnt);
+    flags.reserve(2 * (size_t)cnt + 2);
+    int *pos = flags.ptr + cnt;
+    k_flag_internal<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, t.begin.ptr, t.end.ptr, c.maxbox,
+                                                       d, maxd, flags.ptr);
+    s->launches++;
+    apply_leaf_predicate(s, off, cnt, d, flags.ptr, st);
+    exclusive_scan(s, flags.ptr, pos, cnt, st);
+    ACHECK(cudaMemcpyAsync(&hostbuf[0], pos + cnt - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ACHECK(cudaMemcpyAsync(&hostbuf[1], flags.ptr + cnt - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (d == 0) ACHECK(cudaMemcpyAsync(&hostbuf[2], s->err_dev.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ACHECK(cudaStreamSynchronize(st));
+    check_points(s, hostbuf[2]);
+    int ninternal = hostbuf[0] + hostbuf[1];
+    t.level_internal.push_back(ninternal);
+    int child_off = off + cnt;
+    size_t need = (size_t)child_off + 8 * (size_t)ninternal;
+    if (need > t.key.cap) {
+      grow_nodes(t, need, child_off, st);
+      na = arrays(t);
+    }
+    k_make_children<<<ceil_div(8 * (int64_t)cnt, TB), TB, 0, st>>>(cnt, off, child_off, flags.ptr, pos,
+                                                       s->keys_out.ptr, d, na, s->sys_box.ptr);
+    s->launches++;
+    off = child_off;
+    cnt = 8 * ninternal;
+    ++d;
+  }
+  t.nnodes = off;
+  t.nlevels = d;
+  const int nn = t.nnodes;
+  DBuf<int> &fl = s->scan_tmp;
+  fl.reserve(2 * (size_t)nn + 2);
+  k_parent_flags<<<ceil_div(nn, TB), TB, 0, st>>>(nn, t.child.ptr, t.depth.ptr, fl.ptr);
+  s->launches++;
+  ACHECK(cudaMemsetAsync(fl.ptr + nn, 0, sizeof(int), st));
+  exclusive_scan(s, fl.ptr, fl.ptr + nn + 1, nn + 1, st);
+  ACHECK(cudaMemcpyAsync(s->h_small + 6, fl.ptr + nn + 1 + nn, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaStreamSynchronize(st));
+  const int np = s->h_small[6];
+  t.n_parents = np;
+  t.parents.reserve(np + 1);
+  k_parent_scatter<<<ceil_div(nn, TB), TB, 0, st>>>(nn, fl.ptr, fl.ptr + nn + 1, t.parents.ptr);
+  s->launches++;
+}
+
 }  // namespace
 
 void build_tree(AranGpuSolver3d *s, int64_t n, const double *d_xyz, const double *d_q) {
   cudaStream_t st = s->s0;
-  const AranGpuConfig3d &c = s->cfg;
-  DevTree &t = s->tree;
-  t.n = n;
+  s->tree.n = n;
   const int TB = 256;
   const int nsys = s->nsys;
 
@@ -653,55 +1069,8 @@ void build_tree(AranGpuSolver3d *s, int64_t n, const double *d_xyz, const double
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::SORT + 1], st));
 
-  // level-synchronous subdivision
-  int maxd = c.max_depth > 0 ? c.max_depth : kKeyBits;
-  if (maxd > kKeyBits) maxd = kKeyBits;
-  size_t est = (size_t)nsys + (size_t)(8 * (n / (c.maxbox + 1) + 1) * 2 + 64);
-  grow_nodes(t, est, 0, st);
-  t.level_off.assign(1, 0);
-  t.level_internal.clear();
-  NodeArrays na = arrays(t);
-  k_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(na, nsys, s->sys_off.ptr, s->sys_box.ptr);
-  s->launches++;
-  int off = 0, cnt = nsys;
-  DBuf<int> &flags = s->scan_tmp;
-  int d = 0;
-  int *hostbuf = s->h_small;   // pinned: the level's readbacks go together
-  hostbuf[2] = 0;
-  while (cnt > 0) {
-    t.level_off.push_back(off + cnt);
-    flags.reserve(2 * (size_t)cnt + 2);
-    int *pos = flags.ptr + cnt;
-    k_flag_internal<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, t.begin.ptr, t.end.ptr, c.maxbox,
-                                                       d, maxd, flags.ptr);
-    s->launches++;
-    if (s->leaf_pred) apply_leaf_predicate(s, off, cnt, d, flags.ptr, st);
-    exclusive_scan(s, flags.ptr, pos, cnt, st);
-    ACHECK(cudaMemcpyAsync(&hostbuf[0], pos + cnt - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ACHECK(cudaMemcpyAsync(&hostbuf[1], flags.ptr + cnt - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    if (d == 0) ACHECK(cudaMemcpyAsync(&hostbuf[2], s->err_dev.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ACHECK(cudaStreamSynchronize(st));
-    if (hostbuf[2] & kErrNonFinite) throw InputError{"a particle coordinate or charge is NaN or infinite"};
-    if ((hostbuf[2] & kErrOutside) && c.precision == ARAN_PRECISION_MIXED)
-      throw InputError{"a particle lies outside the solver's box (mixed precision needs every point "
-                       "inside [lbound, ubound])"};
-    int ninternal = hostbuf[0] + hostbuf[1];
-    t.level_internal.push_back(ninternal);
-    int child_off = off + cnt;
-    size_t need = (size_t)child_off + 8 * (size_t)ninternal;
-    if (need > t.key.cap) {
-      grow_nodes(t, need, child_off, st);
-      na = arrays(t);
-    }
-    k_make_children<<<ceil_div(8 * (int64_t)cnt, TB), TB, 0, st>>>(cnt, off, child_off, flags.ptr, pos,
-                                                       s->keys_out.ptr, d, na, s->sys_box.ptr);
-    s->launches++;
-    off = child_off;
-    cnt = 8 * ninternal;
-    ++d;
-  }
-  t.nnodes = off;
-  t.nlevels = d;
+  if (s->leaf_pred) subdivide_levels(s, n, st);
+  else subdivide(s, n, st);
   ACHECK(cudaEventRecord(s->ev[2 * Stage::TREE + 1], st));
 }
 
@@ -786,13 +1155,13 @@ void build_lists(AranGpuSolver3d *s) {
                                                        lflags.ptr);
   s->launches++;
   inclusive_scan(s, lflags.ptr, incl, n, st);
-  ACHECK(cudaMemcpyAsync(s->h_small + 3, incl + n - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-  ACHECK(cudaStreamSynchronize(st));
-  const int nleaves = s->h_small[3];
-  t.nleaves = nleaves;
+  // the number of leaves stays on the device until the near ranges are counted;
+  // nlb bounds it
+  const int *nleaves_p = incl + n - 1;
+  const int nlb = (int)std::min<int64_t>(n, nn);
   t.lf_begin.reserve(nn);
   t.lf_end.reserve(nn);
-  t.leaf_node.reserve(nleaves + 1);
+  t.leaf_node.reserve(nlb + 1);
   k_leaf_ranges<<<ceil_div(nn, TB), TB, 0, st>>>(nn, t.begin.ptr, t.end.ptr, t.child.ptr, incl,
                                                   t.lf_begin.ptr, t.lf_end.ptr, t.leaf_node.ptr);
   s->launches++;
@@ -823,30 +1192,46 @@ void build_lists(AranGpuSolver3d *s) {
   s->launches++;
   // near ranges (and semifar nodes) per leaf
   const int T = s->cfg.semifar_threshold;
-  t.near_off.reserve(nleaves + 1);
-  int *semi_cnt = nullptr;
+  t.near_off.reserve(nlb + 1);
+  if (T > 0) t.semi_off.reserve(nlb + 1);
+  cntbuf.reserve(2 * ((size_t)nlb + 1) + 2);
+  int *semi_cnt = cntbuf.ptr + nlb + 1;
+  NearTotals *tot = reinterpret_cast<NearTotals *>(semi_cnt + nlb + 1);
+  ACHECK(cudaMemsetAsync(cntbuf.ptr + nlb, 0, sizeof(int), st));
+  ACHECK(cudaMemsetAsync(semi_cnt + nlb, 0, sizeof(int) + sizeof(NearTotals), st));
+  auto near = [&](bool write) {
+    if (T > 0) {
+      k_near<<<ceil_div(nlb, TB), TB, 0, st>>>(
+          nlb, nleaves_p, t.leaf_node.ptr, t.begin.ptr, t.end.ptr, t.child.ptr, t.parent.ptr,
+          t.col.ptr, t.ncol.ptr, t.lf_begin.ptr, t.lf_end.ptr, t.ijk.ptr, t.depth.ptr, T,
+          cntbuf.ptr, t.near_off.ptr, t.near_rng.ptr, semi_cnt, t.semi_off.ptr, t.semi_node.ptr,
+          t.semi_leaf.ptr, tot, t.big_rng.ptr, write);
+    } else {
+      auto kern = write ? k_near_warp<true> : k_near_warp<false>;
+      kern<<<ceil_div(32 * (int64_t)nlb, TB), TB, 0, st>>>(
+          nlb, nleaves_p, t.leaf_node.ptr, t.begin.ptr, t.end.ptr, t.child.ptr, t.parent.ptr,
+          t.col.ptr, t.ncol.ptr, t.lf_begin.ptr, t.lf_end.ptr, cntbuf.ptr, tot, t.near_off.ptr,
+          t.near_rng.ptr, t.big_rng.ptr);
+    }
+    ACHECK(cudaGetLastError());
+    s->launches++;
+  };
+  near(false);
+  exclusive_scan(s, cntbuf.ptr, t.near_off.ptr, nlb + 1, st);
+  int *hb = s->h_small;
+  hb[5] = 0;
+  ACHECK(cudaMemcpyAsync(hb + 3, nleaves_p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaMemcpyAsync(hb + 4, t.near_off.ptr + nlb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaMemcpyAsync(hb + 8, tot, sizeof(NearTotals), cudaMemcpyDeviceToHost, st));
   if (T > 0) {
-    t.semi_off.reserve(nleaves + 1);
-    cntbuf.reserve(2 * ((size_t)nleaves + 1) + (size_t)n + 1);
-    semi_cnt = cntbuf.ptr + nleaves + 1;
-  }
-  k_near<<<ceil_div(nleaves, TB), TB, 0, st>>>(nleaves, t.leaf_node.ptr, t.begin.ptr, t.end.ptr,
-                                                t.child.ptr, t.parent.ptr, t.col.ptr, t.ncol.ptr,
-                                                t.lf_begin.ptr, t.lf_end.ptr, t.ijk.ptr, t.depth.ptr,
-                                                T, cntbuf.ptr, nullptr, nullptr, semi_cnt, nullptr,
-                                                nullptr, nullptr, nullptr, 0);
-  s->launches++;
-  ACHECK(cudaMemsetAsync(cntbuf.ptr + nleaves, 0, sizeof(int), st));
-  exclusive_scan(s, cntbuf.ptr, t.near_off.ptr, nleaves + 1, st);
-  s->h_small[5] = 0;
-  ACHECK(cudaMemcpyAsync(s->h_small + 4, t.near_off.ptr + nleaves, sizeof(int), cudaMemcpyDeviceToHost, st));
-  if (T > 0) {
-    ACHECK(cudaMemsetAsync(semi_cnt + nleaves, 0, sizeof(int), st));
-    exclusive_scan(s, semi_cnt, t.semi_off.ptr, nleaves + 1, st);
-    ACHECK(cudaMemcpyAsync(s->h_small + 5, t.semi_off.ptr + nleaves, sizeof(int), cudaMemcpyDeviceToHost, st));
+    exclusive_scan(s, semi_cnt, t.semi_off.ptr, nlb + 1, st);
+    ACHECK(cudaMemcpyAsync(hb + 5, t.semi_off.ptr + nlb, sizeof(int), cudaMemcpyDeviceToHost, st));
   }
   ACHECK(cudaStreamSynchronize(st));
-  const int nrng = s->h_small[4], nsemi = s->h_small[5];
+  t.nleaves = hb[3];
+  const int nrng = hb[4], nsemi = hb[5];
+  t.n_big = hb[8];
+  t.n_heavy = hb[9];
   t.n_near_rng = nrng;
   t.n_semi = nsemi;
   t.near_rng.reserve(2 * (size_t)nrng + 2);
@@ -854,32 +1239,10 @@ void build_lists(AranGpuSolver3d *s) {
     t.semi_node.reserve(nsemi + 1);
     t.semi_leaf.reserve(nsemi + 1);
   }
-  // heavy-range list (k_near's write pass fills it): at most one entry per range
-  t.big_rng.reserve(2 * (size_t)nrng + 2);
+  // heavy-range list (the write pass fills it)
+  t.big_rng.reserve(2 * (size_t)t.n_heavy + 2);
   ACHECK(cudaMemsetAsync(t.big_rng.ptr, 0, 2 * sizeof(int), st));
-  k_near<<<ceil_div(nleaves, TB), TB, 0, st>>>(nleaves, t.leaf_node.ptr, t.begin.ptr, t.end.ptr,
-                                                t.child.ptr, t.parent.ptr, t.col.ptr, t.ncol.ptr,
-                                                t.lf_begin.ptr, t.lf_end.ptr, t.ijk.ptr, t.depth.ptr,
-                                                T, nullptr, t.near_off.ptr, t.near_rng.ptr, nullptr,
-                                                t.semi_off.ptr, t.semi_node.ptr, t.semi_leaf.ptr,
-                                                t.big_rng.ptr, 1);
-  s->launches++;
-  // internal nodes of depth >= 1: one M2L block each (their children)
-  {
-    DBuf<int> &fl = s->scan_tmp;
-    fl.reserve(2 * (size_t)nn + 2);
-    k_parent_flags<<<ceil_div(nn, TB), TB, 0, st>>>(nn, t.child.ptr, t.depth.ptr, fl.ptr);
-    s->launches++;
-    ACHECK(cudaMemsetAsync(fl.ptr + nn, 0, sizeof(int), st));
-    exclusive_scan(s, fl.ptr, fl.ptr + nn + 1, nn + 1, st);
-    ACHECK(cudaMemcpyAsync(s->h_small + 6, fl.ptr + nn + 1 + nn, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ACHECK(cudaStreamSynchronize(st));
-    const int np = s->h_small[6];
-    t.n_parents = np;
-    t.parents.reserve(np + 1);
-    k_parent_scatter<<<ceil_div(nn, TB), TB, 0, st>>>(nn, fl.ptr, fl.ptr + nn + 1, t.parents.ptr);
-    s->launches++;
-  }
+  near(true);
   build_p2p_work(s);
   ACHECK(cudaEventRecord(s->ev[2 * Stage::LISTS + 1], st));
 }
