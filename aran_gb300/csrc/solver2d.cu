@@ -90,7 +90,8 @@ __global__ void k2_keys(int64_t n, int nsys, const int64_t *__restrict__ offs,
 }
 
 __global__ void k2_gather(int64_t n, const int *__restrict__ perm, const double *__restrict__ xy,
-                          const double *__restrict__ q, double *__restrict__ sx,
+                          const double *__restrict__ q, const uint64_t *__restrict__ keys,
+                          const double *__restrict__ sysbox, double *__restrict__ sx,
                           double *__restrict__ sy, double *__restrict__ sq,
                           float4 *__restrict__ hl) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -100,9 +101,12 @@ __global__ void k2_gather(int64_t n, const int *__restrict__ perm, const double 
   sx[i] = x;
   sy[i] = y;
   sq[i] = q[o];
-  if (hl) {              // FP32 hi + lo positions of the mixed near field
-    const float hx = (float)x, hy = (float)y;
-    hl[i] = make_float4(hx, hy, (float)(x - (double)hx), (float)(y - (double)hy));
+  if (hl) {              // FP32 hi + lo positions of the mixed near field, from the
+                         // corner of the system's box
+    const double *b = sysbox + 6 * (keys[i] >> kSysShift);
+    const double bx = x - b[0], by = y - b[1];
+    const float hx = (float)bx, hy = (float)by;
+    hl[i] = make_float4(hx, hy, (float)(bx - (double)hx), (float)(by - (double)hy));
   }
 }
 
@@ -866,7 +870,8 @@ __global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleave
   const int b = leaf_be[L], nt = leaf_be[L + 1] - b;
   const int r0 = near_off[L], r1 = near_off[L + 1];
   const int node = leaf_node[L];
-  const double cx = center[2 * node], cy = center[2 * node + 1];
+  const double *box = sysbox + 6 * sysn[node];
+  const double cx = center[2 * node] - box[0], cy = center[2 * node + 1] - box[1];
   const float chx = (float)cx, chy = (float)cy;
   const float clx = (float)(cx - (double)chx), cly = (float)(cy - (double)chy);
   const double hh = node_size2(sysbox, sysn[node], depth[node]);
@@ -1083,7 +1088,7 @@ struct AranGpuSolver2d {
   aran::DBuf<int> err2;   // input checks of the key pass
   aran::DBuf<uint8_t> cub_tmp;
   aran::DBuf<double> sx, sy, sq, io_xy, io_q, io_acc;
-  aran::DBuf<float4> hl;   // FP32 hi + lo positions (mixed near field)
+  aran::DBuf<float4> hl;   // FP32 hi + lo positions in the box (mixed near field)
   // forest
   aran::DBuf<int> nsys_, ij, begin, end, child, parent, col, ncol, far_off, far_src;
   aran::DBuf<int> lf_begin, lf_end, leaf_node, leaf_be, near_off;
@@ -1225,7 +1230,8 @@ void build_forest(AranGpuSolver2d *s, int nsys, const double *dxy, const double 
   s->sq.reserve(n);
   const bool mixed = s->cfg.precision == ARAN_PRECISION_MIXED;
   if (mixed) s->hl.reserve(n);
-  k2_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, s->perm.ptr, dxy, dq, s->sx.ptr, s->sy.ptr, s->sq.ptr,
+  k2_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, s->perm.ptr, dxy, dq, s->keys_out.ptr,
+                                             s->sysbox.ptr, s->sx.ptr, s->sy.ptr, s->sq.ptr,
                                              mixed ? s->hl.ptr : nullptr);
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::SORT + 1], st));

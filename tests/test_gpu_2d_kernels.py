@@ -46,3 +46,17 @@ def test_orders(aran, oracle, precision, orders):
             acc = s.solve(x, q)
         ref, _ = oracle.solve2d(x, q, [0, len(q)], [[-1.0, -1.0, 1.0, 1.0]], 12, p)
         assert rel_l2(acc, ref) < (1e-12 if precision == "fp64" else 3e-6), p
+
+
+def test_box_far_from_the_origin(aran):
+    """Positions exact in FP64 in either box: only the box's extent counts, so
+    mixed results differ by the order of additions at most."""
+    rng = np.random.default_rng(8)
+    x = np.round(rng.uniform(-1, 1, (4000, 2)) * 2.0**30) / 2.0**30
+    q = rng.uniform(-1, 1, len(x))
+    out = []
+    for h in (np.zeros(2), np.array([2.0**20, -(2.0**21)])):
+        box = np.concatenate([h - 1.0, h + 1.0])[None, :]
+        with aran.Solver2d(maxbox=32, order=20, precision="mixed") as s:
+            out.append(s.solve(x + h, q, boxes=box))
+    assert rel_l2(out[1], out[0]) <= 1e-10
