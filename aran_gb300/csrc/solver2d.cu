@@ -30,6 +30,7 @@
 
 #include "internal.cuh"
 #include "f32x2.cuh"
+#include "subdivide.cuh"
 
 namespace aran {
 namespace {
@@ -131,6 +132,89 @@ __global__ void k2_roots(int nsys, const int64_t *__restrict__ offs, const doubl
   na.parent[s] = -1;
   na.center[2 * s] = node_center_axis(b[0], b[2], 0, 0);
   na.center[2 * s + 1] = node_center_axis(b[1], b[3], 0, 0);
+}
+
+// sorted keys (system id above the digits) for subdivide.cuh
+struct Keys2 {
+  int64_t n;
+  const uint64_t *keys;
+  int maxbox, maxd;
+
+  // digits that two keys share, -1 in different systems
+  static __device__ __forceinline__ int shared(uint64_t a, uint64_t b) {
+    const uint64_t v = a ^ b;
+    if (v == 0) return kKeyBits;
+    if (v >> kSysShift) return -1;
+    return (__clzll((long long)v) - (64 - kSysShift)) / 2;
+  }
+  // depths lo .. hi of the internal nodes that start at place i
+  __device__ __forceinline__ void internal_depths(int64_t i, int &lo, int &hi) const {
+    lo = kKeyBits + 1;
+    hi = -1;
+    if (i + maxbox >= n) return;
+    const uint64_t k = keys[i];
+    lo = i == 0 ? 0 : shared(keys[i - 1], k) + 1;
+    hi = min(shared(k, keys[i + maxbox]), maxd - 1);
+    if (lo > hi) {
+      lo = kKeyBits + 1;
+      hi = -1;
+    }
+  }
+};
+
+// every second bit of a key from bit 0
+__device__ __forceinline__ int every_second(uint64_t v) {
+  v &= 0x5555555555555555ull;
+  v = (v | (v >> 1)) & 0x3333333333333333ull;
+  v = (v | (v >> 2)) & 0x0f0f0f0f0f0f0f0full;
+  v = (v | (v >> 4)) & 0x00ff00ff00ff00ffull;
+  v = (v | (v >> 8)) & 0x0000ffff0000ffffull;
+  v = (v | (v >> 16)) & 0x00000000ffffffffull;
+  return (int)v;
+}
+
+// four threads per internal node, thread c making child c: its points end at
+// the first key beyond its digits, and begin where child c-1's end
+__global__ void k2_make_nodes(int total, LevelStarts ls, const int *__restrict__ start,
+                              const int *__restrict__ prank, Keys2 ks, Nodes2 na,
+                              const double *__restrict__ sysbox) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(g & 3);
+  const bool live = (g >> 2) < total;
+  const int rk = live ? (int)(g >> 2) : 0;
+  int d = 0;
+  while (d < kKeyBits - 1 && rk >= ls.rank[d + 1]) ++d;
+  const int i = start[rk];
+  const uint64_t k = ks.keys[i];
+  const int sy = (int)(k >> kSysShift);
+  const int shift = 2 * (kKeyBits - d - 1);
+  const uint64_t up = k >> (shift + 2), pk = (up << 2) | (uint64_t)c;   // with the system id
+  int lo = i;
+  int64_t hi = ks.n;
+  while (lo < hi) {
+    const int mid = (int)((lo + hi) >> 1);
+    if ((ks.keys[mid] >> shift) <= pk) lo = mid + 1; else hi = mid;
+  }
+  // the four threads of a node are four consecutive lanes
+  const int prev = __shfl_up_sync(0xffffffffu, lo, 1, 4);
+  if (!live) return;
+  const int node = d == 0 ? sy : ls.node[d] + 4 * (prank[rk] - ls.rank[d - 1]) + (int)(up & 3);
+  const int base = ls.node[d + 1] + 4 * (rk - ls.rank[d]);
+  if (c == 0) na.child[node] = base;
+  const int cn = base + c, b = c == 0 ? i : prev;
+  const double *bx = sysbox + 6 * sy;
+  const uint64_t cell = pk & ((1ull << 2 * (d + 1)) - 1);
+  const int ci = every_second(cell), cj = every_second(cell >> 1);
+  na.sys[cn] = sy;
+  na.ij[2 * cn] = ci;
+  na.ij[2 * cn + 1] = cj;
+  na.depth[cn] = (uint8_t)(d + 1);
+  na.begin[cn] = b;
+  na.end[cn] = lo;
+  if (!(lo - b > ks.maxbox && d + 1 < ks.maxd)) na.child[cn] = -1;   // else its own threads set it
+  na.parent[cn] = node;
+  na.center[2 * cn] = node_center_axis(bx[0], bx[2], d + 1, ci);
+  na.center[2 * cn + 1] = node_center_axis(bx[1], bx[3], d + 1, cj);
 }
 
 __global__ void k2_flag(int cnt, int off, const int *__restrict__ begin, const int *__restrict__ end,
@@ -246,13 +330,14 @@ __global__ void k2_leaf_starts(int nn, const int *__restrict__ begin, const int 
   if (child[i] < 0 && end[i] > begin[i]) flags[begin[i]] = 1;
 }
 
-__global__ void k2_leaf_ranges(int nn, const int *__restrict__ begin, const int *__restrict__ end,
+__global__ void k2_leaf_ranges(int nn, int n, const int *__restrict__ begin, const int *__restrict__ end,
                                const int *__restrict__ child, const int *__restrict__ incl,
                                int *__restrict__ lf_begin, int *__restrict__ lf_end,
                                int *__restrict__ leaf_node, int *__restrict__ leaf_be) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nn) return;
   int b = begin[i], e = end[i];
+  if (i == 0) leaf_be[incl[n - 1]] = n;          // closes the last leaf
   if (e > b) {
     lf_begin[i] = incl[b] - 1;
     lf_end[i] = incl[e - 1];
@@ -265,15 +350,21 @@ __global__ void k2_leaf_ranges(int nn, const int *__restrict__ begin, const int 
   }
 }
 
-// near leaf-ordinal ranges of leaf L; mode 0 counts, mode 1 writes
-__global__ void k2_near(int nleaves, const int *__restrict__ leaf_node, const int *__restrict__ begin,
+// near leaf-ordinal ranges of leaf L; mode 0 counts (zero for the ordinals from
+// the last leaf up to nbound), mode 1 writes
+__global__ void k2_near(int nbound, const int *__restrict__ nleaves_p,
+                        const int *__restrict__ leaf_node, const int *__restrict__ begin,
                         const int *__restrict__ end, const int *__restrict__ child,
                         const int *__restrict__ parent, const int *__restrict__ col,
                         const int *__restrict__ ncol, const int *__restrict__ lf_begin,
                         const int *__restrict__ lf_end, int *__restrict__ near_cnt,
                         const int *__restrict__ near_off, int2 *__restrict__ near_rng, int mode) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
-  if (L >= nleaves) return;
+  if (L >= nbound) return;
+  if (L >= *nleaves_p) {
+    if (!mode) near_cnt[L] = 0;
+    return;
+  }
   int node = leaf_node[L];
   int k = 0;
   int w = mode ? near_off[L] : 0;
@@ -1086,6 +1177,8 @@ struct AranGpuSolver2d {
   aran::DBuf<uint64_t> keys_in, keys_out;
   aran::DBuf<int> idx_in, perm, incl, flags;
   aran::DBuf<int> err2;   // input checks of the key pass
+  aran::DBuf<int> internal;   // places and parents of the internal nodes
+  int *h_small = nullptr;     // pinned host words for the readbacks
   aran::DBuf<uint8_t> cub_tmp;
   aran::DBuf<double> sx, sy, sq, io_xy, io_q, io_acc;
   aran::DBuf<float4> hl;   // FP32 hi + lo positions in the box (mixed near field)
@@ -1194,6 +1287,89 @@ void leaf_predicate2(AranGpuSolver2d *s, int off, int cnt, int d, cudaStream_t s
   ACHECK(cudaStreamSynchronize(st));
 }
 
+// the input checks of the key pass
+void check_points2(const AranGpuSolver2d *s, int e) {
+  if (e & kErrNonFinite) throw InputError{"a particle coordinate or charge is NaN or infinite"};
+  if ((e & kErrOutside) && s->cfg.precision == ARAN_PRECISION_MIXED)
+    throw InputError{"a particle lies outside its system's box (mixed precision needs every "
+                     "point inside it)"};
+}
+
+size_t node_estimate2(const AranGpuSolver2d *s, int nsys) {
+  return (size_t)nsys + 4 * (s->n / (s->cfg.maxbox + 1) + 1) * 2 + 64;
+}
+
+// the quadtrees of the sorted keys, all levels at once (subdivide.cuh): 128
+// systems of 1k to 60k particles 0.073 ms, 0.39 level by level; one of 60k 0.057
+// ms, 0.36
+void subdivide2(AranGpuSolver2d *s, int nsys, cudaStream_t st) {
+  const int TB = 256;
+  const int64_t n = s->n;
+  const int maxd = s->cfg.max_depth > 0 ? s->cfg.max_depth : kKeyBits;
+  const int nb = place_blocks(n), nc = kKeyBits * nb;
+  s->flags.reserve(2 * (size_t)nc + 2);
+  int *first = s->flags.ptr + nc + 1, *hb = s->h_small + 16;
+  const Keys2 keys = {n, s->keys_out.ptr, s->cfg.maxbox, maxd};
+  count_internal(keys, nb, s->flags.ptr, first, hb,
+                 [&](const int *in, int *out, int k) { ex_scan(s, in, out, k, st); }, st);
+  s->launches++;
+  ACHECK(cudaMemcpyAsync(s->h_small, s->err2.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaStreamSynchronize(st));
+  check_points2(s, s->h_small[0]);
+  const LevelStarts ls = level_starts(hb, nsys, 4, s->level_off, nullptr);
+  s->nlevels = (int)s->level_off.size() - 1;
+  s->nnodes = s->level_off.back();
+  const int total = hb[kKeyBits];
+  grow(s, std::max((size_t)s->nnodes, node_estimate2(s, nsys)), 0, st);
+  k2_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(nsys, s->offs.ptr, s->sysbox.ptr, nodes(s));
+  ACHECK(cudaGetLastError());
+  s->launches++;
+  if (total == 0) return;
+  s->internal.reserve(2 * (size_t)total);
+  int *list = s->internal.ptr;
+  k_list_internal<<<nb, kPlaceBlock, 0, st>>>(keys, first, list, list + total);
+  ACHECK(cudaGetLastError());
+  k2_make_nodes<<<ceil_div(4 * (int64_t)total, TB), TB, 0, st>>>(total, ls, list, list + total, keys,
+                                                                 nodes(s), s->sysbox.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches += 2;
+}
+
+// the same level by level, each level's internal nodes shown to the leaf
+// predicate before they are split
+void subdivide_levels2(AranGpuSolver2d *s, int nsys, cudaStream_t st) {
+  const int TB = 256, maxd = s->cfg.max_depth > 0 ? s->cfg.max_depth : kKeyBits;
+  check_points2(s, read_int(s->err2.ptr, st));
+  grow(s, node_estimate2(s, nsys), 0, st);
+  k2_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(nsys, s->offs.ptr, s->sysbox.ptr, nodes(s));
+  s->launches++;
+  s->level_off.assign(1, 0);
+  int off = 0, cnt = nsys, d = 0;
+  while (cnt > 0) {
+    s->level_off.push_back(off + cnt);
+    s->flags.reserve(2 * (size_t)cnt + 2);
+    int *pos = s->flags.ptr + cnt + 1;
+    k2_flag<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, s->begin.ptr, s->end.ptr, s->cfg.maxbox, d,
+                                               maxd, s->flags.ptr);
+    s->launches++;
+    leaf_predicate2(s, off, cnt, d, st);
+    ACHECK(cudaMemsetAsync(s->flags.ptr + cnt, 0, sizeof(int), st));
+    ex_scan(s, s->flags.ptr, pos, cnt + 1, st);
+    int ninternal = read_int(pos + cnt, st);
+    int child_off = off + cnt;
+    size_t need = (size_t)child_off + 4 * (size_t)ninternal;
+    if (need > s->begin.cap) grow(s, need, child_off, st);
+    k2_children<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, child_off, s->flags.ptr, pos,
+                                                   s->keys_out.ptr, d, nodes(s), s->sysbox.ptr);
+    s->launches++;
+    off = child_off;
+    cnt = 4 * ninternal;
+    ++d;
+  }
+  s->nnodes = off;
+  s->nlevels = d;
+}
+
 void build_forest(AranGpuSolver2d *s, int nsys, const double *dxy, const double *dq) {
   cudaStream_t st = s->s0;
   const int TB = 256;
@@ -1207,13 +1383,6 @@ void build_forest(AranGpuSolver2d *s, int nsys, const double *dxy, const double 
   k2_keys<<<ceil_div(n, TB), TB, 0, st>>>(n, nsys, s->offs.ptr, s->sysbox.ptr, dxy, dq,
                                            s->keys_in.ptr, s->idx_in.ptr, s->err2.ptr);
   s->launches++;
-  {
-    const int e = read_int(s->err2.ptr, st);
-    if (e & kErrNonFinite) throw InputError{"a particle coordinate or charge is NaN or infinite"};
-    if ((e & kErrOutside) && s->cfg.precision == ARAN_PRECISION_MIXED)
-      throw InputError{"a particle lies outside its system's box (mixed precision needs every "
-                       "point inside it)"};
-  }
   int sysbits = 1;
   while ((1ll << sysbits) < nsys) ++sysbits;
   size_t bytes = 0;
@@ -1236,35 +1405,8 @@ void build_forest(AranGpuSolver2d *s, int nsys, const double *dxy, const double 
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::SORT + 1], st));
 
-  int maxd = s->cfg.max_depth > 0 ? s->cfg.max_depth : kKeyBits;
-  grow(s, (size_t)nsys + 4 * (n / (s->cfg.maxbox + 1) + 1) * 2 + 64, 0, st);
-  k2_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(nsys, s->offs.ptr, s->sysbox.ptr, nodes(s));
-  s->launches++;
-  s->level_off.assign(1, 0);
-  int off = 0, cnt = nsys, d = 0;
-  while (cnt > 0) {
-    s->level_off.push_back(off + cnt);
-    s->flags.reserve(2 * (size_t)cnt + 2);
-    int *pos = s->flags.ptr + cnt + 1;
-    k2_flag<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, s->begin.ptr, s->end.ptr, s->cfg.maxbox, d,
-                                               maxd, s->flags.ptr);
-    s->launches++;
-    if (s->leaf_pred) leaf_predicate2(s, off, cnt, d, st);
-    ACHECK(cudaMemsetAsync(s->flags.ptr + cnt, 0, sizeof(int), st));
-    ex_scan(s, s->flags.ptr, pos, cnt + 1, st);
-    int ninternal = read_int(pos + cnt, st);
-    int child_off = off + cnt;
-    size_t need = (size_t)child_off + 4 * (size_t)ninternal;
-    if (need > s->begin.cap) grow(s, need, child_off, st);
-    k2_children<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, child_off, s->flags.ptr, pos,
-                                                   s->keys_out.ptr, d, nodes(s), s->sysbox.ptr);
-    s->launches++;
-    off = child_off;
-    cnt = 4 * ninternal;
-    ++d;
-  }
-  s->nnodes = off;
-  s->nlevels = d;
+  if (s->leaf_pred) subdivide_levels2(s, nsys, st);
+  else subdivide2(s, nsys, st);
   ACHECK(cudaEventRecord(s->ev[2 * Stage::TREE + 1], st));
 }
 
@@ -1289,12 +1431,6 @@ void build_lists2(AranGpuSolver2d *s) {
   s->launches++;
   ACHECK(cudaMemsetAsync(s->flags.ptr + nn, 0, sizeof(int), st));
   ex_scan(s, s->flags.ptr, s->far_off.ptr, nn + 1, st);
-  s->nfar = read_int(s->far_off.ptr + nn, st);
-  s->far_src.reserve(s->nfar + 1);
-  k2_far<<<ceil_div(nn, TB), TB, 0, st>>>(nn, s->begin.ptr, s->end.ptr, s->child.ptr, s->parent.ptr,
-                                           s->ij.ptr, s->col.ptr, s->ncol.ptr, nullptr, s->far_off.ptr,
-                                           s->far_src.ptr, 1);
-  s->launches++;
   // leaves in key order
   s->incl.reserve(n);
   ACHECK(cudaMemsetAsync(s->flags.ptr, 0, n * sizeof(int), st));
@@ -1308,33 +1444,45 @@ void build_lists2(AranGpuSolver2d *s) {
     ACHECK(cub::DeviceScan::InclusiveSum(s->cub_tmp.ptr, bytes, s->flags.ptr, s->incl.ptr, (int)n, st));
     s->launches += 2;
   }
-  s->nleaves = read_int(s->incl.ptr + n - 1, st);
-  const int nl = s->nleaves;
+  // the number of leaves stays on the device until all lists are counted; nlb
+  // bounds it
+  const int *nleaves_p = s->incl.ptr + n - 1;
+  const int nlb = (int)std::min<int64_t>(n, nn);
   s->lf_begin.reserve(nn);
   s->lf_end.reserve(nn);
-  s->leaf_node.reserve(nl + 1);
-  s->leaf_be.reserve(nl + 1);
-  k2_leaf_ranges<<<ceil_div(nn, TB), TB, 0, st>>>(nn, s->begin.ptr, s->end.ptr, s->child.ptr,
+  s->leaf_node.reserve(nlb + 1);
+  s->leaf_be.reserve(nlb + 1);
+  k2_leaf_ranges<<<ceil_div(nn, TB), TB, 0, st>>>(nn, (int)n, s->begin.ptr, s->end.ptr, s->child.ptr,
                                                    s->incl.ptr, s->lf_begin.ptr, s->lf_end.ptr,
                                                    s->leaf_node.ptr, s->leaf_be.ptr);
   s->launches++;
-  int nint = (int)n;
-  ACHECK(cudaMemcpyAsync(s->leaf_be.ptr + nl, &nint, sizeof(int), cudaMemcpyHostToDevice, st));
-  s->near_off.reserve(nl + 1);
-  k2_near<<<ceil_div(nl, TB), TB, 0, st>>>(nl, s->leaf_node.ptr, s->begin.ptr, s->end.ptr,
-                                            s->child.ptr, s->parent.ptr, s->col.ptr, s->ncol.ptr,
-                                            s->lf_begin.ptr, s->lf_end.ptr, s->flags.ptr, nullptr,
-                                            nullptr, 0);
+  s->near_off.reserve(nlb + 1);
+  auto near = [&](int mode) {
+    k2_near<<<ceil_div(nlb, TB), TB, 0, st>>>(
+        nlb, nleaves_p, s->leaf_node.ptr, s->begin.ptr, s->end.ptr, s->child.ptr, s->parent.ptr,
+        s->col.ptr, s->ncol.ptr, s->lf_begin.ptr, s->lf_end.ptr, s->flags.ptr, s->near_off.ptr,
+        s->near_rng.ptr, mode);
+    ACHECK(cudaGetLastError());
+    s->launches++;
+  };
+  near(0);
+  ACHECK(cudaMemsetAsync(s->flags.ptr + nlb, 0, sizeof(int), st));
+  ex_scan(s, s->flags.ptr, s->near_off.ptr, nlb + 1, st);
+  int *hb = s->h_small;
+  ACHECK(cudaMemcpyAsync(hb, s->far_off.ptr + nn, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaMemcpyAsync(hb + 1, nleaves_p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaMemcpyAsync(hb + 2, s->near_off.ptr + nlb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaStreamSynchronize(st));
+  s->nfar = hb[0];
+  s->nleaves = hb[1];
+  s->nrng = hb[2];
+  s->far_src.reserve(s->nfar + 1);
+  k2_far<<<ceil_div(nn, TB), TB, 0, st>>>(nn, s->begin.ptr, s->end.ptr, s->child.ptr, s->parent.ptr,
+                                           s->ij.ptr, s->col.ptr, s->ncol.ptr, nullptr, s->far_off.ptr,
+                                           s->far_src.ptr, 1);
   s->launches++;
-  ACHECK(cudaMemsetAsync(s->flags.ptr + nl, 0, sizeof(int), st));
-  ex_scan(s, s->flags.ptr, s->near_off.ptr, nl + 1, st);
-  s->nrng = read_int(s->near_off.ptr + nl, st);
   s->near_rng.reserve(s->nrng + 1);
-  k2_near<<<ceil_div(nl, TB), TB, 0, st>>>(nl, s->leaf_node.ptr, s->begin.ptr, s->end.ptr,
-                                            s->child.ptr, s->parent.ptr, s->col.ptr, s->ncol.ptr,
-                                            s->lf_begin.ptr, s->lf_end.ptr, nullptr, s->near_off.ptr,
-                                            s->near_rng.ptr, 1);
-  s->launches++;
+  near(1);
   ACHECK(cudaEventRecord(s->ev[2 * Stage::LISTS + 1], st));
 }
 
@@ -1523,6 +1671,7 @@ int aran_gpu_solver2d_create(const AranGpuConfig2d *cfg, AranGpuSolver2d **out) 
     ACHECK(cudaGetDevice(&s->device));
     ACHECK(cudaStreamCreateWithFlags(&s->s0, cudaStreamNonBlocking));
     ACHECK(cudaStreamCreateWithFlags(&s->s1, cudaStreamNonBlocking));
+    ACHECK(cudaHostAlloc(&s->h_small, 64 * sizeof(int), cudaHostAllocDefault));
     for (auto &ev : s->ev) ACHECK(cudaEventCreate(&ev));
     ACHECK(cudaEventCreateWithFlags(&s->ev_lists, cudaEventDisableTiming));
     ACHECK(cudaEventCreateWithFlags(&s->ev_p2p, cudaEventDisableTiming));
@@ -1563,6 +1712,8 @@ void aran_gpu_solver2d_destroy(AranGpuSolver2d *s) {
   s->keys_out.release();
   s->idx_in.release();
   s->err2.release();
+  s->internal.release();
+  if (s->h_small) cudaFreeHost(s->h_small);
   s->perm.release();
   s->incl.release();
   s->flags.release();

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "subdivide.cuh"
 
 namespace aran {
 
@@ -105,23 +106,6 @@ __global__ void k_roots(NodeArrays na, int nsys, const int *__restrict__ sys_off
   na.center[3 * r + 2] = node_center_axis(b[2], b[5], 0, 0);
 }
 
-// ---------------------------------------------------------------------------
-// Subdivision of all levels at once.  A node of depth d holds the particles
-// that share the first d digits of their keys (within a system).  One starts at
-// sorted place i if d exceeds the digits that places i - 1 and i share, and has
-// more than maxbox points if places i and i + maxbox share d: the internal nodes
-// that start at i are those of the depths lo .. hi.  Counted per depth and block
-// of places and scanned depth by depth, their numbers are their ranks in level
-// order, the children of the node of rank r in its level lie at eight times r
-// in the next, and one readback (the counts) is all that the host waits for;
-// level by level each took one, with a flag pass, a scan and a binary search
-// of its own: 40 us a level.  Bound by latency: 10k uniform particles (4 levels)
-// 0.056 ms, 0.165 before; 4M Plummer particles (11 levels) 0.115 ms, 0.524.
-// ---------------------------------------------------------------------------
-constexpr int kPlaceBlock = 256, kPlaceItems = 4, kPlaces = kPlaceBlock * kPlaceItems;
-constexpr int kPlaceSlots = kPlaces / 32;   // warp-wide runs of places in a block
-static_assert(kPlaceSlots == 32, "a warp scans a block's slots");
-
 __device__ __forceinline__ int shared_digits(uint64_t a, uint64_t b) {
   return a == b ? kKeyBits : (__clzll((long long)(a ^ b)) - 1) / 3;
 }
@@ -135,105 +119,29 @@ __device__ __forceinline__ int system_of(int64_t i, int nsys, const int *__restr
   return lo;
 }
 
-// depths lo .. hi of the internal nodes that start at place i
-__device__ __forceinline__ void internal_depths(int64_t i, int64_t n, int nsys,
-                                                const int *__restrict__ sys_off,
-                                                const uint64_t *__restrict__ keys, int maxbox,
-                                                int maxd, int &lo, int &hi) {
-  lo = kKeyBits + 1;
-  hi = -1;
-  if (i >= n) return;
-  const int sy = system_of(i, nsys, sys_off);
-  if (i + maxbox >= sys_off[sy + 1]) return;
-  const uint64_t k = keys[i];
-  lo = i == sys_off[sy] ? 0 : shared_digits(keys[i - 1], k) + 1;
-  hi = min(shared_digits(k, keys[i + maxbox]), maxd - 1);
-  if (lo > hi) {
+// sorted keys for subdivide.cuh
+struct Keys3 {
+  int64_t n;
+  int nsys;
+  const int *sys_off;
+  const uint64_t *keys;
+  int maxbox, maxd;
+
+  // depths lo .. hi of the internal nodes that start at place i
+  __device__ __forceinline__ void internal_depths(int64_t i, int &lo, int &hi) const {
     lo = kKeyBits + 1;
     hi = -1;
-  }
-}
-
-// counts[d][block]: internal nodes of depth d that start in the block's places
-__global__ void __launch_bounds__(kPlaceBlock)
-    k_count_internal(int64_t n, int nsys, const int *__restrict__ sys_off,
-                     const uint64_t *__restrict__ keys, int maxbox, int maxd,
-                     int *__restrict__ counts) {
-  __shared__ int cnt[kKeyBits][kPlaceSlots + 1];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int c = 0; c < kPlaceItems; ++c) {
-    int lo, hi, v = 0;
-    internal_depths((int64_t)blockIdx.x * kPlaces + c * kPlaceBlock + threadIdx.x, n, nsys, sys_off,
-                    keys, maxbox, maxd, lo, hi);
-    const int d0 = __reduce_min_sync(0xffffffffu, lo), d1 = __reduce_max_sync(0xffffffffu, hi);
-    for (int d = d0; d <= d1; ++d) {
-      const unsigned m = __ballot_sync(0xffffffffu, lo <= d && d <= hi);
-      if (lane == d) v = __popc(m);
-    }
-    if (lane < kKeyBits) cnt[lane][c * (kPlaceBlock / 32) + w] = v;
-  }
-  __syncthreads();
-  for (int d = w; d < kKeyBits; d += kPlaceBlock / 32) {
-    const int t = __reduce_add_sync(0xffffffffu, cnt[d][lane]);
-    if (lane == 0) counts[(int64_t)d * gridDim.x + blockIdx.x] = t;
-  }
-}
-
-// place and parent's rank of every internal node, by rank in level order
-__global__ void __launch_bounds__(kPlaceBlock)
-    k_list_internal(int64_t n, int nsys, const int *__restrict__ sys_off,
-                    const uint64_t *__restrict__ keys, int maxbox, int maxd,
-                    const int *__restrict__ first, int *__restrict__ start,
-                    int *__restrict__ prank) {
-  __shared__ int pre[kKeyBits][kPlaceSlots + 1];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int lo[kPlaceItems], hi[kPlaceItems];
-#pragma unroll
-  for (int c = 0; c < kPlaceItems; ++c) {
-    int v = 0;
-    internal_depths((int64_t)blockIdx.x * kPlaces + c * kPlaceBlock + threadIdx.x, n, nsys, sys_off,
-                    keys, maxbox, maxd, lo[c], hi[c]);
-    const int d0 = __reduce_min_sync(0xffffffffu, lo[c]), d1 = __reduce_max_sync(0xffffffffu, hi[c]);
-    for (int d = d0; d <= d1; ++d) {
-      const unsigned m = __ballot_sync(0xffffffffu, lo[c] <= d && d <= hi[c]);
-      if (lane == d) v = __popc(m);
-    }
-    if (lane < kKeyBits) pre[lane][c * (kPlaceBlock / 32) + w] = v;
-  }
-  __syncthreads();
-  // ranks before each run of places
-  for (int d = w; d < kKeyBits; d += kPlaceBlock / 32) {
-    const int mine = pre[d][lane];
-    int v = mine;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += u;
-    }
-    pre[d][lane] = first[(int64_t)d * gridDim.x + blockIdx.x] + v - mine;
-  }
-  __syncthreads();
-  const unsigned before = (1u << lane) - 1;
-#pragma unroll
-  for (int c = 0; c < kPlaceItems; ++c) {
-    const int slot = c * (kPlaceBlock / 32) + w;
-    const int64_t i = (int64_t)blockIdx.x * kPlaces + c * kPlaceBlock + threadIdx.x;
-    const int d0 = __reduce_min_sync(0xffffffffu, lo[c]), d1 = __reduce_max_sync(0xffffffffu, hi[c]);
-    unsigned up = 0;                     // the depth above's starts in this run
-    for (int d = d0; d <= d1; ++d) {
-      const unsigned m = __ballot_sync(0xffffffffu, lo[c] <= d && d <= hi[c]);
-      if (lo[c] <= d && d <= hi[c]) {
-        const int rk = pre[d][slot] + __popc(m & before);
-        start[rk] = (int)i;
-        if (d > 0) prank[rk] = pre[d - 1][slot] + __popc(up & (before | 1u << lane)) - 1;
-      }
-      up = m;
+    if (i >= n) return;
+    const int sy = system_of(i, nsys, sys_off);
+    if (i + maxbox >= sys_off[sy + 1]) return;
+    const uint64_t k = keys[i];
+    lo = i == sys_off[sy] ? 0 : shared_digits(keys[i - 1], k) + 1;
+    hi = min(shared_digits(k, keys[i + maxbox]), maxd - 1);
+    if (lo > hi) {
+      lo = kKeyBits + 1;
+      hi = -1;
     }
   }
-}
-
-// first rank and first node of each depth (by value to the kernel)
-struct LevelStarts {
-  int rank[kKeyBits + 1], node[kKeyBits + 2];
 };
 
 // every third bit of a key from bit 0
@@ -918,44 +826,27 @@ void subdivide(AranGpuSolver3d *s, int64_t n, cudaStream_t st) {
   const AranGpuConfig3d &c = s->cfg;
   DevTree &t = s->tree;
   const int TB = 256, nsys = s->nsys, maxd = depth_limit(c);
-  const int nb = (int)((n + kPlaces - 1) / kPlaces);
-  const int nc = kKeyBits * nb;
+  const int nb = place_blocks(n), nc = kKeyBits * nb;
   DBuf<int> &tmp = s->scan_tmp;
   tmp.reserve(2 * (size_t)nc + 2);
   int *first = tmp.ptr + nc + 1;
-  k_count_internal<<<nb, kPlaceBlock, 0, st>>>(n, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox,
-                                               maxd, tmp.ptr);
-  ACHECK(cudaGetLastError());
-  s->launches++;
-  ACHECK(cudaMemsetAsync(tmp.ptr + nc, 0, sizeof(int), st));
-  exclusive_scan(s, tmp.ptr, first, nc + 1, st);
+  const Keys3 keys = {n, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox, maxd};
   // first rank of each depth and their total, with the error word
   int *hb = s->h_small + 16;
-  ACHECK(cudaMemcpy2DAsync(hb, sizeof(int), first, nb * sizeof(int), sizeof(int), kKeyBits + 1,
-                           cudaMemcpyDeviceToHost, st));
+  count_internal(keys, nb, tmp.ptr, first, hb,
+                 [&](const int *in, int *out, int k) { exclusive_scan(s, in, out, k, st); }, st);
+  s->launches++;
   ACHECK(cudaMemcpyAsync(s->h_small + 2, s->err_dev.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   ACHECK(cudaStreamSynchronize(st));
   check_points(s, s->h_small[2]);
-  LevelStarts ls = {};
-  t.level_off.assign(1, 0);
   t.level_internal.clear();
-  int off = 0, cnt = nsys, d = 0;
-  for (; cnt > 0; ++d) {
-    ls.node[d] = off;
-    off += cnt;
-    t.level_off.push_back(off);
-    const int ninternal = d < kKeyBits ? hb[d + 1] - hb[d] : 0;
-    t.level_internal.push_back(ninternal);
-    cnt = 8 * ninternal;
-  }
-  for (int k = 0; k <= kKeyBits; ++k) ls.rank[k] = hb[k];
-  for (int k = d; k < kKeyBits + 2; ++k) ls.node[k] = off;
-  t.nnodes = off;
-  t.nlevels = d;
+  const LevelStarts ls = level_starts(hb, nsys, 8, t.level_off, &t.level_internal);
+  t.nlevels = (int)t.level_off.size() - 1;
+  t.nnodes = t.level_off.back();
   const int total = hb[kKeyBits];
   t.n_parents = total - t.level_internal[0];
   t.parents.reserve(t.n_parents + 1);
-  grow_nodes(t, std::max((size_t)off, node_estimate(s, n)), 0, st);
+  grow_nodes(t, std::max((size_t)t.nnodes, node_estimate(s, n)), 0, st);
   NodeArrays na = arrays(t);
   k_roots<<<ceil_div(nsys, TB), TB, 0, st>>>(na, nsys, s->sys_off.ptr, s->sys_box.ptr);
   ACHECK(cudaGetLastError());
@@ -963,8 +854,7 @@ void subdivide(AranGpuSolver3d *s, int64_t n, cudaStream_t st) {
   if (total == 0) return;
   DBuf<int> &list = s->sort_tmp;
   list.reserve(2 * (size_t)total);
-  k_list_internal<<<nb, kPlaceBlock, 0, st>>>(n, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox,
-                                              maxd, first, list.ptr, list.ptr + total);
+  k_list_internal<<<nb, kPlaceBlock, 0, st>>>(keys, first, list.ptr, list.ptr + total);
   ACHECK(cudaGetLastError());
   k_make_nodes<<<ceil_div(8 * (int64_t)total, TB), TB, 0, st>>>(
       total, ls, list.ptr, list.ptr + total, nsys, s->sys_off.ptr, s->keys_out.ptr, c.maxbox, maxd,

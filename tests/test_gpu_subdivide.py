@@ -2,6 +2,8 @@
 level (taken when a leaf predicate is set; this one keeps every node): the same
 nodes, ranges and lists, number by number, over leaf capacities, depth limits,
 clustered and coincident points, sizes at the edges of a block of places."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -50,3 +52,29 @@ def test_forest(aran):
     off = np.concatenate([[0], np.cumsum(sizes)])
     both(aran, lambda s: s.solve_forest(x, q, off, np.hstack([lo, lo + 2.0]))[0], maxbox=9,
          precision="fp64")
+
+
+@pytest.mark.parametrize("maxbox,max_depth", [(1, 21), (3, 2), (20, 21), (64, 5), (5000, 21)])
+def test_same_tree_2d(aran, maxbox, max_depth):
+    """Results to rounding and the same lists (their sizes and the counters)."""
+    rng = np.random.default_rng(maxbox)
+    sizes = [1, 1023, 1, 6000, 1024, 40]
+    x = [rng.uniform(-1, 1, (n, 2)) for n in sizes]
+    x[3][:3000] = 0.1 + 1e-4 * rng.normal(size=(3000, 2))
+    x[4][:30] = 0.25                                  # coincident
+    x = np.concatenate(x)
+    q = rng.uniform(-1, 1, len(x))
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    keep = aran.LEAF_PREDICATE(lambda v, _d: 0)
+    out = []
+    for pred in (None, keep):
+        with aran.Solver2d(maxbox=maxbox, max_depth=max_depth, order=6) as s:
+            fn = aran.load().aran_gpu_solver2d_set_leaf_predicate
+            assert fn(s._h, ctypes.cast(pred, ctypes.c_void_p) if pred else None, None) == 0
+            acc = s.solve(x, q, off)
+            out.append((s.tree_info(), s.get_stats(), acc))
+    (ia, sa, a), (ib, sb, b) = out
+    assert ia == ib and sa == sb
+    ok = np.isfinite(b)                               # coincident points divide by zero
+    assert np.array_equal(ok, np.isfinite(a)) and ok.sum() >= len(q) - 30
+    assert np.linalg.norm((a - b)[ok]) <= 1e-13 * np.linalg.norm(b[ok])
