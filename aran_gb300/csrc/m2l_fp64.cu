@@ -156,10 +156,24 @@ __device__ __forceinline__ double flip(double v, bool neg) {
   return __hiloint2double(__double2hiint(v) ^ (neg ? 0x80000000 : 0), __double2loint(v));
 }
 
+// sources of a unit: singly; in pairs, u and w made one after the other from
+// sources read twice; in pairs, both made at once
+enum { kF64Single = 0, kF64PairTwice = 1, kF64Pair = 2 };
+
+// shared memory of a warp's sources, and of a warp, in doubles
+__host__ __device__ inline int m2l_fp64_a(int p, int mode) {
+  const int nm = tri(p), nl = tri(p + 1);
+  return mode == kF64Pair && 4 * nm > 2 * nl ? 4 * nm : 2 * nl;
+}
+__host__ __device__ inline int m2l_fp64_warp(int p, int mode) {
+  const int nm = tri(p), nl = tri(p + 1);
+  return m2l_fp64_a(p, mode) + (mode != kF64Single && 4 * nm > 2 * nl ? 4 * nm : 2 * nl);
+}
+
 // R rounds of 32 lanes over the tri(p+1) local coefficients
 template <int R>
-__global__ void __launch_bounds__(32 * kF64Warps, 2)
-    k_m2l_fp64(int nparents, int nsplit, int nunits, bool pairs, const int *__restrict__ parents,
+__global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
+    k_m2l_fp64(int nparents, int nsplit, int nunits, int mode, const int *__restrict__ parents,
                const int *__restrict__ child, const int *__restrict__ begin,
                const int *__restrict__ end, const int *__restrict__ col,
                const int *__restrict__ ncol, const int *__restrict__ ijk,
@@ -174,10 +188,10 @@ __global__ void __launch_bounds__(32 * kF64Warps, 2)
   __shared__ int grid[216];
   const int nm = tri(p), nl = tri(p + 1);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // per warp: A holds the phased sources (u, then w), later z; B the rotated
-  // ones, later the local: real plane, imaginary plane each
-  const int vec = max((pairs ? 4 : 2) * nm, 2 * nl);
-  double *A = reinterpret_cast<double *>(smem_raw) + (size_t)w * 2 * vec, *B = A + vec;
+  // per warp: A holds the phased sources (u and w, or u, then w), later z; B the
+  // rotated ones (u and w), later the local: real plane, imaginary plane each
+  double *A = reinterpret_cast<double *>(smem_raw) + (size_t)w * m2l_fp64_warp(p, mode);
+  double *B = A + m2l_fp64_a(p, mode);
   for (int i = threadIdx.x; i < 216; i += blockDim.x) grid[i] = -1;
   __syncthreads();
   const int P = parents[blockIdx.x];
@@ -215,35 +229,40 @@ __global__ void __launch_bounds__(32 * kF64Warps, 2)
     int s0 = source_of(a, b, c), s1 = (code & 512u) ? source_of(6 - a, 6 - b, 6 - c) : -1;
     if (s0 < 0 && s1 < 0) continue;
     // the opposite source alone: its terms with (-1)^l, odd degrees negated;
-    // a pair where the pairs' vectors do not fit: one after the other
+    // a pair taken singly: one after the other
     const bool both = s0 >= 0 && s1 >= 0;
-    for (int turn = 0; turn < (both && !pairs ? 2 : 1); ++turn) {
-      const bool two = both && pairs;
+    for (int turn = 0; turn < (both && mode == kF64Single ? 2 : 1); ++turn) {
+      const bool two = both && mode != kF64Single;
       const bool opp = both ? turn == 1 : s0 < 0;
       const int sa = opp ? s1 : s0;
       const double *ph = dir + (size_t)(code >> 16) * dstride + ph_off;
       const double *tab = tabs + (size_t)u * S.stride + lane;
-      // mirror S and z-phase of the sources
-      for (int k = lane; k < nm; k += 32) {
-        const int l = lm[2 * k], m = lm[2 * k + 1];
-        const bool sg = ((bz & (l + m)) ^ (bx & m)) & 1, cj = bx ^ by, odd = l & 1;
-        const double cr = ph[2 * m], ci = ph[2 * m + 1];
-        cplx<double> v = mult[(size_t)sa * nm + k];
-        v.re = flip(v.re, sg ^ (opp && odd));
-        v.im = flip(v.im, sg ^ cj ^ (opp && odd));
-        if (two) {
-          cplx<double> x = mult[(size_t)s1 * nm + k];
-          x.re = flip(x.re, sg ^ odd);
-          x.im = flip(x.im, sg ^ cj ^ odd);
-          const cplx<double> d = cmake(v.re - x.re, v.im - x.im);
-          v = cadd(v, x);
-          A[2 * nm + k] = d.re * cr - d.im * ci;
-          A[3 * nm + k] = d.re * ci + d.im * cr;
+      // mirror S and z-phase of the sources: u = y + (-1)^l y' (or the one
+      // source there is), w = y - (-1)^l y'
+      auto load = [&](bool diff) {
+        for (int k = lane; k < nm; k += 32) {
+          const int l = lm[2 * k], m = lm[2 * k + 1];
+          const bool sg = ((bz & (l + m)) ^ (bx & m)) & 1, cj = bx ^ by, odd = l & 1;
+          const double cr = ph[2 * m], ci = ph[2 * m + 1];
+          cplx<double> v = mult[(size_t)sa * nm + k];
+          v.re = flip(v.re, sg ^ (opp && odd));
+          v.im = flip(v.im, sg ^ cj ^ (opp && odd));
+          if (two) {
+            cplx<double> x = mult[(size_t)s1 * nm + k];
+            x.re = flip(x.re, sg ^ odd);
+            x.im = flip(x.im, sg ^ cj ^ odd);
+            const cplx<double> d = cmake(v.re - x.re, v.im - x.im);
+            v = diff ? d : cadd(v, x);
+            if (mode == kF64Pair) {
+              A[2 * nm + k] = d.re * cr - d.im * ci;
+              A[3 * nm + k] = d.re * ci + d.im * cr;
+            }
+          }
+          A[k] = v.re * cr - v.im * ci;
+          A[nm + k] = v.re * ci + v.im * cr;
         }
-        A[k] = v.re * cr - v.im * ci;
-        A[nm + k] = v.re * ci + v.im * cr;
-      }
-      __syncwarp();
+        __syncwarp();
+      };
       // one stage: every lane its dot product of each round
       auto stage = [&](int st, const double *in, auto &&put) {
         const F64Task *tk = task + 32 * S.first[st] + lane;
@@ -268,8 +287,15 @@ __global__ void __launch_bounds__(32 * kF64Warps, 2)
           if (q.dst != 0xffff) put(q, v);
         }
       };
+      load(false);
       stage(0, A, [&](const F64Task &q, double v) { B[q.dst] = v; });
-      if (two) stage(0, A + 2 * nm, [&](const F64Task &q, double v) { B[2 * nm + q.dst] = v; });
+      if (two) {
+        const bool again = mode == kF64PairTwice;
+        __syncwarp();
+        if (again) load(true);
+        stage(0, again ? A : A + 2 * nm,
+              [&](const F64Task &q, double v) { B[2 * nm + q.dst] = v; });
+      }
       __syncwarp();
       // (no source term has order p: its place in z, the last of either plane)
       if (lane < 2) A[lane * nl + nl - 1] = 0.;
@@ -365,15 +391,23 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   OpTables<double> &tb = s->t64;
   const M2lFp64Tables &f = tb.m2l64;
   const int p = s->cfg.order, nm = tri(p), nl = tri(p + 1);
-  int dev_smem = 0, nsm = 0;
+  int dev_smem = 0, sm_smem = 0, nsm = 0;
   ACHECK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
+  ACHECK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
   ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
-  // pairs at a time where their vectors fit (up to order 29)
-  auto bytes = [&](bool pairs) {
-    return (size_t)kF64Warps * 2 * std::max((pairs ? 4 : 2) * nm, 2 * nl) * sizeof(double);
+  // Pairs at a time unless their vectors halve the CTAs of an SM from two to one:
+  // order 26, 60k uniform particles, M2L 53 ms with single sources in two CTAs, 76
+  // with pairs in one; order 29 (one CTA either way) 149 with pairs, 170 without.
+  // Read twice where that keeps two CTAs (from order 21): order 22, 60k Plummer
+  // particles, 44 ms, 71 read once, 50 singly; 2 to 3 % slower below.
+  auto bytes = [&](int mode) { return (size_t)kF64Warps * m2l_fp64_warp(p, mode) * sizeof(double); };
+  auto fit = [&](int mode) {
+    return bytes(mode) + 1024 > (size_t)dev_smem ? 0 : std::min(2, (int)(sm_smem / (bytes(mode) + 2048)));
   };
-  const bool pairs = bytes(true) + 1024 <= (size_t)dev_smem;
-  const size_t sm = bytes(pairs);
+  int mode = kF64Pair;
+  if (fit(kF64PairTwice) > fit(mode)) mode = kF64PairTwice;
+  if (fit(kF64Single) > fit(mode)) mode = kF64Single;
+  const size_t sm = bytes(mode);
   // about 24 CTAs per SM even out the SMs' last CTAs
   const int nsplit = std::min(16, std::max(1, (24 * nsm + count - 1) / count));
   cplx<double> *mult = reinterpret_cast<cplx<double> *>(s->mult64.ptr);
@@ -386,7 +420,7 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   auto kern = nl <= 96 ? k_m2l_fp64<3> : (nl <= 160 ? k_m2l_fp64<5> : (nl <= 256 ? k_m2l_fp64<8> : k_m2l_fp64<16>));
   smem_opt_in(kern, sm);
   kern<<<dim3(count, nsplit), 32 * kF64Warps, sm, st>>>(
-      count, nsplit, f.nunits, pairs, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
+      count, nsplit, f.nunits, mode, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
       t.ncol.ptr, t.ijk.ptr, t.depth.ptr, p, f.sched, reinterpret_cast<const F64Task *>(f.task.ptr),
       f.trip.ptr, f.units.ptr, f.tabs.ptr, tb.dir_m2l.ptr, dir_offset(p, 0, 6),
       dir_offset(p, 0, 4), tb.lm.ptr, s->scale_e, mult, loc, parts);
