@@ -16,7 +16,7 @@ OBJ = os.path.join(ROOT, "_build", "aran_gpu")
 LIB = os.path.join(HERE, "libaran_gpu.so")
 SOURCES = ["tables.cu", "tree.cu", "passes.cu", "p2p.cu", "m2l.cu", "m2l_fp64.cu", "m2l_lanes.cu",
            "m2l_lanes_b.cu", "m2l_lanes_c.cu", "m2l_tc.cu", "m2m_lanes.cu",
-           "m2m_lanes_b.cu", "m2m_lanes_c.cu", "oct_wide.cu", "leaf_ops.cu", "leaf_ops_b.cu", "leaf_ops_c.cu",
+           "m2m_lanes_b.cu", "m2m_lanes_c.cu", "oct_wide.cu", "leaf_ops.cu", "leaf_ops_b.cu", "leaf_ops_c.cu", "leaf_fp64.cu",
            "noalloc.cu", "server.cu", "solver.cu", "compat.cu", "solver2d.cu", "compat2d.cu",
            "semifar.cu", "series3d.cu", "tune.cu", "profiledb.cpp"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

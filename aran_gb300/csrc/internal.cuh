@@ -275,6 +275,9 @@ bool launch_m2m_lanes(AranGpuSolver3d *s, OpTables<float> &tb, cplx<float> *mult
                       int dlo, cudaStream_t st);
 bool launch_l2l_lanes(AranGpuSolver3d *s, OpTables<float> &tb, cplx<float> *loc, int dlo,
                       int dhi, cudaStream_t st);
+// leaf_fp64.cu
+void launch_p2m64(AranGpuSolver3d *s, cudaStream_t st);
+void launch_l2p64(AranGpuSolver3d *s, cudaStream_t st);
 // oct_wide.cu: M2M into / L2L from the cnt nodes list[..] (or off onwards): FP32
 // with an octant-0 stream table (the bits of the lane-parallel kernels), FP64
 void launch_oct_wide(AranGpuSolver3d *s, bool down, const float *stream, cplx<float> *ser,

@@ -1,0 +1,264 @@
+// leaf_fp64.cu -- P2M and L2P in FP64 (up_func's and down_func's leaf parts:
+// aran/arandevelopment3d.c:169-216 and :285-356).  The FP64 pipe takes half a
+// lane per cycle and scheduler, so its instructions times the lanes they leave
+// idle are the whole cost; shared memory and index arithmetic come free.
+#include "internal.cuh"
+
+namespace aran {
+
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kWarps = 4;
+
+__device__ __forceinline__ double leaf_inv_scale(int depth, double scale_e) {
+  return ldexp(1.0, depth) / scale_e;    // 1/h_d = 2^d / 2^E (exact power of two)
+}
+
+// P2M, a warp per window of 32 sorted particles whatever leaves they lie in (a
+// warp per leaf keeps as many lanes busy as the leaf has points).  A lane makes
+// its particle's q S_l^m in m-major order (six operations a coefficient) into
+// shared memory; every 32 values the lanes turn to the values, a lane one of them,
+// and add it up over each leaf's part of the window (one addition a value and
+// particle; by shuffles over the warp it was five on every lane).  A leaf
+// inside the window is stored, parts of a leaf are added to its zeroed multipole.
+// 200k Plummer particles (18 a leaf), order 12: 0.34 ms, 1.44 with a warp per
+// leaf and shuffles.
+__global__ void __launch_bounds__(32 * kWarps)
+    k_p2m64(int64_t n, int nleaves, const int *__restrict__ win_leaf,
+            const int2 *__restrict__ leaf_be, const int *__restrict__ leaf_node,
+            const uint8_t *__restrict__ depth, const real4<double> *__restrict__ rel, int p,
+            const double *__restrict__ rec_g, const double *__restrict__ p2mf_g, double scale_e,
+            double *__restrict__ mult) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nm = tri(p);
+  double *rec = reinterpret_cast<double *>(smem_raw);   // (c0, c1) by (l, m)
+  double *fac = rec + 2 * nm;                            // by m-major place
+  int *coef = reinterpret_cast<int *>(fac + nm);         // (l, m) of a place
+  double *buf = reinterpret_cast<double *>(coef + ((nm + 1) & ~1));
+  for (int i = threadIdx.x; i < 2 * nm; i += blockDim.x) rec[i] = rec_g[i];
+  for (int i = threadIdx.x; i < nm; i += blockDim.x) {
+    int l, m;
+    mmajor_lm(i, p - 1, l, m);
+    fac[i] = p2mf_g[l];
+    coef[i] = tri(l, m);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t win = blockIdx.x * (int64_t)kWarps + w, b0 = 32 * win;
+  if (b0 >= n) return;
+  buf += w * 32 * 33;
+  const int cnt = n - b0 < 32 ? (int)(n - b0) : 32;
+  // leaves of the window: L0 holds its first particle, the next ones start inside
+  const int L0 = win_leaf[win];
+  unsigned bit = 0;
+  if (lane > 0 && L0 + lane < nleaves) {
+    const int64_t at = leaf_be[L0 + lane].x - b0;
+    if (at < cnt) bit = 1u << at;
+  }
+  const unsigned starts = __reduce_or_sync(kFull, bit);
+  double x = 0, y = 0, z = 0, q = 0;
+  if (lane < cnt) {
+    const int L = L0 + __popc(starts & ((2u << lane) - 1u));
+    const double ih = leaf_inv_scale(depth[leaf_node[L]], scale_e);
+    const real4<double> r = rel[b0 + lane];
+    x = r.x * ih;
+    y = r.y * ih;
+    z = r.z * ih;
+    q = r.q;
+  }
+  const double r2 = x * x + y * y + z * z;
+  int k = 0;                               // value: 2 m-major place + part
+  auto put = [&](double v) {
+    buf[(k & 31) * 33 + lane] = v;
+    ++k;
+    if ((k & 31) && k < 2 * nm) return;
+    // the lanes take the values
+    __syncwarp();
+    const int mine = ((k - 1) & ~31) + lane;
+    if (mine < k) {
+      const double f = (mine & 1) ? -fac[mine >> 1] : fac[mine >> 1];
+      const size_t c = 2 * (size_t)coef[mine >> 1] + (mine & 1);
+      unsigned left = starts;
+      int L = L0, j = 0;
+      while (j < cnt) {
+        const int j1 = left ? __ffs(left) - 1 : cnt;
+        left &= left - 1;
+        double sum = 0;
+#pragma unroll 4
+        for (int jj = j; jj < j1; ++jj) sum += buf[lane * 33 + jj];
+        const int2 be = leaf_be[L];
+        double *out = mult + 2 * (size_t)nm * leaf_node[L] + c;
+        if (be.x >= b0 && be.y <= b0 + 32) *out = f * sum;
+        else atomicAdd(out, f * sum);
+        j = j1;
+        ++L;
+      }
+    }
+    __syncwarp();
+  };
+  double dre = q * rec[0], dim = 0;
+  for (int m = 0; m < p; ++m) {
+    if (m > 0) {
+      const double a = rec[2 * tri(m, m)];
+      const double nre = a * (x * dre - y * dim), nim = a * (x * dim + y * dre);
+      dre = nre;
+      dim = nim;
+    }
+    double s1re = dre, s1im = dim, s2re = 0, s2im = 0;
+    put(dre);
+    put(dim);
+    for (int l = m + 1; l < p; ++l) {
+      const double a = rec[2 * tri(l, m)] * z, b = rec[2 * tri(l, m) + 1] * r2;
+      const double sre = a * s1re - b * s2re, sim = a * s1im - b * s2im;
+      s2re = s1re;
+      s2im = s1im;
+      s1re = sre;
+      s1im = sim;
+      put(sre);
+      put(sim);
+    }
+  }
+}
+
+// L2P, a warp per leaf.  What a particle's solid harmonic S_l^m is multiplied
+// with is made once per leaf: for the potential, the z derivative and the x and
+// y derivatives (whose terms of orders m and -m fold into four real factors), so
+// a particle takes 14 operations per (l, m) with the field, 23 before.  200k
+// Plummer particles (18 a leaf), order 12, field: 0.96 ms, 1.73 before.
+template <bool FIELD>
+__global__ void __launch_bounds__(32 * kWarps)
+    k_l2p64(int nleaves, const int *__restrict__ leaf_node, const int2 *__restrict__ leaf_be,
+            const uint8_t *__restrict__ depth, const real4<double> *__restrict__ rel, int p,
+            const double *__restrict__ rec_g, const double *__restrict__ gz_g,
+            const double *__restrict__ gm_g, double scale_e, const cplx<double> *__restrict__ loc,
+            double *__restrict__ acc_pot, double *__restrict__ acc_fld) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int NF = FIELD ? 4 : 1;        // pairs of factors per (l, m)
+  const int nl = tri(p + 1);
+  double2 *rec = reinterpret_cast<double2 *>(smem_raw);
+  for (int i = threadIdx.x; i < nl; i += blockDim.x)
+    rec[i] = make_double2(rec_g[2 * i], rec_g[2 * i + 1]);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double2 *F = rec + nl + (size_t)w * nl * NF;
+  const int L = blockIdx.x * kWarps + w;
+  if (L >= nleaves) return;
+  const int node = leaf_node[L];
+  const cplx<double> *Lc = loc + (size_t)node * nl;
+  for (int c = lane; c < nl; c += 32) {
+    // degree of the triangular index c: floor((sqrt(8c+1)-1)/2), corrected
+    int l = (int)((sqrtf(8.f * c + 1.f) - 1.f) * 0.5f);
+    while (tri(l + 1) <= c) ++l;
+    while (tri(l) > c) --l;
+    const int m = c - tri(l);
+    const double wm = m == 0 ? 1. : 2.;
+    const cplx<double> v = Lc[c];
+    F[c * NF] = make_double2(wm * v.re, -wm * v.im);
+    if (FIELD && l < p) {
+      const cplx<double> a = Lc[tri(l + 1, m)];
+      const double g = wm * gz_g[c];
+      F[c * NF + 1] = make_double2(a.re * g, -a.im * g);
+      // terms of +m and, with S^{-m} = (-1)^m conj(S^m), of -m
+      const double gp = gm_g[l * l + l + m];
+      const cplx<double> bp = Lc[tri(l + 1, m + 1)];
+      double rr = bp.re * gp, ri = -bp.im * gp, ii = bp.re * gp, ir = bp.im * gp;
+      if (m > 0) {
+        const double sg = (m & 1) ? -1. : 1., gn = gm_g[l * l + l - m];
+        cplx<double> u = Lc[tri(l + 1, m - 1)];
+        // L^{1-m} for m > 1
+        if (m > 1) u = ((m - 1) & 1) ? cmake(-u.re, u.im) : cmake(u.re, -u.im);
+        const double ur = sg * (u.re * gn), ui = sg * (u.im * gn);
+        rr += ur;
+        ri += ui;
+        ii -= ur;
+        ir += ui;
+      }
+      F[c * NF + 2] = make_double2(rr, ri);   // real part from S.re, S.im
+      F[c * NF + 3] = make_double2(ir, ii);   // imaginary part
+    }
+  }
+  __syncwarp();
+  const int2 be = leaf_be[L];
+  const double ih = leaf_inv_scale(depth[node], scale_e);
+  for (int i = be.x + lane; i < be.y; i += 32) {
+    const real4<double> r = rel[i];
+    const double x = r.x * ih, y = r.y * ih, z = r.z * ih;
+    const double r2 = x * x + y * y + z * z;
+    double phi = 0, dz = 0, gre = 0, gim = 0;
+    double dre = rec[0].x, dim = 0;
+    auto add = [&](int c, bool grad, double sre, double sim) {
+      const double2 f = F[c * NF];
+      phi = fma(f.x, sre, fma(f.y, sim, phi));
+      if (FIELD && grad) {
+        const double2 a = F[c * NF + 1], g = F[c * NF + 2], h = F[c * NF + 3];
+        dz = fma(a.x, sre, fma(a.y, sim, dz));
+        gre = fma(g.x, sre, fma(g.y, sim, gre));
+        gim = fma(h.x, sre, fma(h.y, sim, gim));
+      }
+    };
+#pragma unroll 1
+    for (int m = 0; m <= p; ++m) {
+      if (m > 0) {
+        const double a = rec[tri(m, m)].x;
+        const double nre = a * (x * dre - y * dim), nim = a * (x * dim + y * dre);
+        dre = nre;
+        dim = nim;
+      }
+      double s1re = dre, s1im = dim, s2re = 0, s2im = 0;
+      add(tri(m, m), m < p, dre, dim);
+#pragma unroll 4
+      for (int l = m + 1; l <= p; ++l) {
+        const int c = tri(l, m);
+        const double2 cc = rec[c];
+        const double a = cc.x * z, b = cc.y * r2;
+        const double sre = a * s1re - b * s2re, sim = a * s1im - b * s2im;
+        s2re = s1re;
+        s2im = s1im;
+        s1re = sre;
+        s1im = sim;
+        add(c, l < p, sre, sim);
+      }
+    }
+    acc_pot[i] += phi;
+    if (FIELD) {
+      acc_fld[3 * (size_t)i] += gre * ih;
+      acc_fld[3 * (size_t)i + 1] += -gim * ih;
+      acc_fld[3 * (size_t)i + 2] += dz * ih;
+    }
+  }
+}
+
+}  // namespace
+
+void launch_p2m64(AranGpuSolver3d *s, cudaStream_t st) {
+  DevTree &t = s->tree;
+  OpTables<double> &tb = s->t64;
+  const int p = s->cfg.order, nm = tri(p);
+  const size_t sm = (size_t)3 * nm * sizeof(double) + ((nm + 1) & ~1) * sizeof(int) +
+                    (size_t)kWarps * 32 * 33 * sizeof(double);
+  smem_opt_in(k_p2m64, sm);
+  k_p2m64<<<ceil_div((t.n + 31) / 32, kWarps), 32 * kWarps, sm, st>>>(
+      t.n, t.nleaves, t.win_leaf.ptr, t.leaf_be.ptr, t.leaf_node.ptr, t.depth.ptr, s->rel64.ptr, p,
+      tb.rec.ptr, tb.p2mf.ptr, s->scale_e, s->mult64.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
+}
+
+void launch_l2p64(AranGpuSolver3d *s, cudaStream_t st) {
+  DevTree &t = s->tree;
+  OpTables<double> &tb = s->t64;
+  const int p = s->cfg.order, nl = tri(p + 1);
+  const bool field = s->cfg.field != 0;
+  const size_t sm = (size_t)nl * sizeof(double2) * (1 + kWarps * (field ? 4 : 1));
+  auto kern = field ? k_l2p64<true> : k_l2p64<false>;
+  smem_opt_in(kern, sm);
+  kern<<<ceil_div(t.nleaves, kWarps), 32 * kWarps, sm, st>>>(
+      t.nleaves, t.leaf_node.ptr, t.leaf_be.ptr, t.depth.ptr, s->rel64.ptr, p, tb.rec.ptr,
+      tb.gz.ptr, tb.gm.ptr, s->scale_e, reinterpret_cast<const cplx<double> *>(s->loc64.ptr),
+      s->acc_pot.ptr, s->acc_fld.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
+}
+
+}  // namespace aran

@@ -2,20 +2,19 @@
 //
 // LibAran runs them as callbacks from tree traversals (aran/aransolver3d.c):
 //   clear_func :399-410   -> one memset of all expansions
-//   up_func :412-450      -> k_p2m (leaves) + M2M level by level: k_oct_wide
-//                            (oct_wide.cu), k_oct_lanes (m2m_lanes.cuh), and
-//                            k_m2m_rotate for the FP32 orders those do not serve
-//   far_func :333-354     -> k_m2l_sibling (m2l.cu)
+//   up_func :412-450      -> P2M (leaf_ops.cuh, FP64 leaf_fp64.cu) + M2M level by
+//                            level (oct_wide.cu, m2m_lanes.cuh)
+//   far_func :333-354     -> m2l_lanes.cuh, m2l.cu, FP64 m2l_fp64.cu
 //   near_func :254-324    -> k_p2p_tile, k_p2p64 (p2p.cu)
-//   down_func :452-490    -> L2L level by level (the same two files,
-//                            k_l2l_rotate) + k_l2p
+//   down_func :452-490    -> L2L level by level + L2P (the files of M2M and P2M)
+// with k_p2m, k_m2m_rotate, k_l2l_rotate and k_l2p here for the FP32 orders that
+// those do not serve (odd ones and above 16; L2L also order 6).
 // The operators are the "point and shoot" rotation flavour of
 // aran/aransphericalseriesd-rotate.c (rotate to the z axis, translate along
 // z, rotate back), with even/odd real rotation blocks and the z-phases
 // applied separately; expansions are stored scaled per level (see
-// fmm_math.cuh).  Every kernel is templated on the arithmetic type: double
-// for the plain FP64 path, float for the mixed path (whose P2P/L2P results
-// are accumulated in FP64).
+// fmm_math.cuh).  The FP64 path runs in double, the mixed path in float (its
+// P2P/L2P results are accumulated in FP64).
 #include "internal.cuh"
 
 namespace aran {
@@ -576,9 +575,11 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
 
   // P2M
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2M], st));
-  {
+  if constexpr (sizeof(T) == 8) {
+    launch_p2m64(s, st);
+  } else {
     const int WPB = 4;
-    if (!(sizeof(T) == 4 && launch_leaf_p2m(s, st))) {
+    if (!launch_leaf_p2m(s, st)) {
       size_t sm = (2 * nl + p + 2) * sizeof(T) + (size_t)WPB * nm * sizeof(cplx<T>) + 64;
       smem_opt_in(k_p2m<T>, sm);
       k_p2m<T><<<ceil_div(t.nleaves, WPB), WPB * 32, sm, st>>>(
@@ -627,7 +628,9 @@ void run_passes_t(AranGpuSolver3d *s, OpTables<T> &tb, DBuf<T> &multb, DBuf<T> &
   // L2P after the near field has written the accumulators
   ACHECK(cudaStreamWaitEvent(st, s->ev[2 * Stage::P2P + 1], 0));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::L2P], st));
-  if (!(sizeof(T) == 4 && launch_leaf_l2p(s, st))) {
+  if constexpr (sizeof(T) == 8) {
+    launch_l2p64(s, st);
+  } else if (!launch_leaf_l2p(s, st)) {
     constexpr int LPB = 4;   // leaves (warps) per block
     size_t sm = ((2 * nl + 1) & ~1) * sizeof(T) +
                 (size_t)LPB * (nl + nm + p * p) * sizeof(cplx<T>) + 64;
