@@ -666,9 +666,9 @@ def cpu_baseline(x, q, name: str, max_solves: int = 1, budget_s: float = 0.0) ->
 # ----------------------------------------------------------------- GPU arm
 # DRAM bytes of one k_m2l_lanes<12> launch on plummer4m (233,161 nodes,
 # 38,977,626 M2L): ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum
-# on one launch of that workload (-k regex:k_m2l_lanes -s 1 -c 1,
-# --clock-control none): 154,687,232 B read + 128,904,192 B written
-M2L_DRAM_BYTES_PLUMMER4M = 154_687_232 + 128_904_192
+# on one launch of that workload (-k 'regex:k_m2l_lanes$' -s 1 -c 1,
+# --clock-control none): 174.40 MB read + 332.85 MB written
+M2L_DRAM_BYTES_PLUMMER4M = 174_400_000 + 332_850_000
 
 
 def run_gpu(args):
