@@ -26,7 +26,8 @@
 // sums are added in order.  Measured on GB300 against the sibling kernel in FP64:
 // 200k Plummer particles at order 12, the whole solve with the near field beside
 // it on the same pipe, 40.2 ms, 48.4 before (42.0 with two CTAs an SM); eight
-// served requests, two of them in FP64 at order 26, 20.0 ms, 35 before.  60k
+// served requests, two of them in FP64 at order 26, 13.9 ms, 35 before (with the
+// P2M and L2P of leaf_fp64.cu).  60k
 // Plummer particles, this kernel alone: 3.8 ms, the FP64 pipe active 92 % of
 // the cycles.
 #include <algorithm>
@@ -189,14 +190,17 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int grid[216];
   const int nm = tri(p), nl = tri(p + 1);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // a CTA takes all eight children of a parent, or half of them
+  const int lane = threadIdx.x & 31, cw = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int halves = kF64Warps / nw, pb = blockIdx.x / halves;
+  const int w = (blockIdx.x - pb * halves) * nw + cw;
   // per warp: A holds the phased sources (u and w, or u, then w), later z; B the
   // rotated ones (u and w), later the local: real plane, imaginary plane each
-  double *A = reinterpret_cast<double *>(smem_raw) + (size_t)w * m2l_fp64_warp(p, mode);
+  double *A = reinterpret_cast<double *>(smem_raw) + (size_t)cw * m2l_fp64_warp(p, mode);
   double *B = A + m2l_fp64_a(p, mode);
   for (int i = threadIdx.x; i < 216; i += blockDim.x) grid[i] = -1;
   __syncthreads();
-  const int P = parents[blockIdx.x];
+  const int P = parents[pb];
   {
     const int pi = ijk[3 * P], pj = ijk[3 * P + 1], pk = ijk[3 * P + 2];
     const int nc = ncol[P];
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
         __syncwarp();
       };
       // one stage: every lane its dot product of each round
-      auto stage = [&](int st, const double *in, auto &&put) {
+      auto stage = [&](int st, const double *in, int last, auto &&put) {
         const F64Task *tk = task + 32 * S.first[st] + lane;
         const int *tr = trip + S.first[st];
         const double *f = tab + S.off[st];
@@ -277,33 +281,56 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
           const double *x = in + q.src;
           if (st == 1 && two && (q.flag & 1)) x += 2 * nm;      // odd degrees from w
           double v = 0.;
+          if (R > 8) {
+            // few warps (order 22 and above): the loads of four steps ahead of their
+            // products (past a product's end they read on, inside the vector and
+            // the table, and count as zero).  60k Plummer particles, order 26 70 ms,
+            // 72 without, order 29 130, 148; order 12, whose warps hide the loads,
+            // 147 ms, 129 without
+            int at = (int)(x - in);
+            for (int k = 0; k < T; k += 4) {
+              double e4[4], x4[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                e4[i] = __ldg(f + 32 * (k + i));
+                x4[i] = in[min(at, last)];
+                at += step;
+                if (st == 1) ++step;
+              }
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (k + i < T) v = fma(e4[i], k + i < q.cnt ? x4[i] : 0., v);
+            }
+            f += 32 * T;
+          } else {
 #pragma unroll 4
-          for (int k = 0; k < T; ++k, f += 32) {
-            const double e = __ldg(f);
-            if (k < q.cnt) {
-              v = fma(e, *x, v);
-              x += step;
-              if (st == 1) ++step;
+            for (int k = 0; k < T; ++k, f += 32) {
+              const double e = __ldg(f);
+              if (k < q.cnt) {
+                v = fma(e, *x, v);
+                x += step;
+                if (st == 1) ++step;
+              }
             }
           }
           if (q.dst != 0xffff) put(q, v);
         }
       };
       load(false);
-      stage(0, A, [&](const F64Task &q, double v) { B[q.dst] = v; });
+      stage(0, A, 2 * nm - 1, [&](const F64Task &q, double v) { B[q.dst] = v; });
       if (two) {
         const bool again = mode == kF64PairTwice;
         __syncwarp();
         if (again) load(true);
-        stage(0, again ? A : A + 2 * nm,
+        stage(0, again ? A : A + 2 * nm, 2 * nm - 1,
               [&](const F64Task &q, double v) { B[2 * nm + q.dst] = v; });
       }
       __syncwarp();
       // (no source term has order p: its place in z, the last of either plane)
       if (lane < 2) A[lane * nl + nl - 1] = 0.;
-      stage(1, B, [&](const F64Task &q, double v) { A[q.dst] = flip(v, opp && (q.flag & 1)); });
+      stage(1, B, (two ? 4 : 2) * nm - 1, [&](const F64Task &q, double v) { A[q.dst] = flip(v, opp && (q.flag & 1)); });
       __syncwarp();
-      stage(2, A, [&](const F64Task &q, double v) { B[q.dst] = v; });
+      stage(2, A, 2 * nl - 1, [&](const F64Task &q, double v) { B[q.dst] = v; });
       __syncwarp();
       // conjugate z-phase
 #pragma unroll
@@ -323,7 +350,7 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
   const double ih = ldexp(1.0, depth[t]) / scale_e;
   cplx<double> *out = nsplit == 1
                           ? loc + (size_t)t * nl
-                          : parts + (((size_t)blockIdx.y * nparents + blockIdx.x) * kF64Warps + w) * nl;
+                          : parts + (((size_t)blockIdx.y * nparents + pb) * kF64Warps + w) * nl;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = lane + 32 * r;
@@ -363,7 +390,7 @@ void build_m2l_fp64_tables(OpTables<double> &tb, cudaStream_t st) {
   M2lFp64Tables &f = tb.m2l64;
   f.nunits = (int)units.size();
   f.sched = h.d;
-  f.tabs.reserve((size_t)h.d.stride * units.size());
+  f.tabs.reserve((size_t)h.d.stride * units.size() + 4 * 32);   // read on by up to 3 steps
   f.task.reserve(nt);
   f.trip.reserve(nr);
   f.units.reserve(units.size());
@@ -397,19 +424,27 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   ACHECK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
   ACHECK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
   ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
-  // Pairs at a time unless their vectors halve the CTAs of an SM from two to one:
-  // order 26, 60k uniform particles, M2L 53 ms with single sources in two CTAs, 76
-  // with pairs in one; order 29 (one CTA either way) 149 with pairs, 170 without.
-  // Read twice where that keeps two CTAs (from order 21): order 22, 60k Plummer
-  // particles, 44 ms, 71 read once, 50 singly; 2 to 3 % slower below.
-  auto bytes = [&](int mode) { return (size_t)kF64Warps * m2l_fp64_warp(p, mode) * sizeof(double); };
-  auto fit = [&](int mode) {
-    return bytes(mode) + 1024 > (size_t)dev_smem ? 0 : std::min(2, (int)(sm_smem / (bytes(mode) + 2048)));
+  // Pairs, made at once (16 warps an SM or more up to order 20); read twice where
+  // that keeps 16 warps (orders 21 to 23): order 22, 60k Plummer particles, M2L 44
+  // ms, 71 made at once, 50 singly; 2 to 3 % slower below.  Above, read twice by
+  // CTAs of four warps where those make 12 (orders 24 to 27): order 26, 72 ms, 76 singly;
+  // singly where that leaves 16 warps and pairs 8 (order 28); order 29 (8 either
+  // way) 148 ms in pairs, 170 singly.
+  auto bytes = [&](int nw, int mode) { return (size_t)nw * m2l_fp64_warp(p, mode) * sizeof(double); };
+  auto warps = [&](int nw, int mode) {
+    return bytes(nw, mode) + 1024 > (size_t)dev_smem
+               ? 0
+               : std::min(16, nw * (int)(sm_smem / (bytes(nw, mode) + 2048)));
   };
-  int mode = kF64Pair;
-  if (fit(kF64PairTwice) > fit(mode)) mode = kF64PairTwice;
-  if (fit(kF64Single) > fit(mode)) mode = kF64Single;
-  const size_t sm = bytes(mode);
+  int nw = kF64Warps, mode = kF64Pair;
+  if (warps(nw, kF64PairTwice) > warps(nw, mode)) mode = kF64PairTwice;
+  if (warps(nw, mode) < 12 && warps(4, kF64PairTwice) >= 12) {
+    nw = 4;
+    mode = kF64PairTwice;
+  } else if (warps(nw, kF64Single) > warps(nw, mode)) {
+    mode = kF64Single;
+  }
+  const size_t sm = bytes(nw, mode);
   // about 24 CTAs per SM even out the SMs' last CTAs
   const int nsplit = std::min(16, std::max(1, (24 * nsm + count - 1) / count));
   cplx<double> *mult = reinterpret_cast<cplx<double> *>(s->mult64.ptr);
@@ -421,7 +456,7 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   }
   auto kern = nl <= 96 ? k_m2l_fp64<3> : (nl <= 160 ? k_m2l_fp64<5> : (nl <= 256 ? k_m2l_fp64<8> : k_m2l_fp64<16>));
   smem_opt_in(kern, sm);
-  kern<<<dim3(count, nsplit), 32 * kF64Warps, sm, st>>>(
+  kern<<<dim3(count * (kF64Warps / nw), nsplit), 32 * nw, sm, st>>>(
       count, nsplit, f.nunits, mode, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
       t.ncol.ptr, t.ijk.ptr, t.depth.ptr, p, f.sched, reinterpret_cast<const F64Task *>(f.task.ptr),
       f.trip.ptr, f.units.ptr, f.tabs.ptr, tb.dir_m2l.ptr, dir_offset(p, 0, 6),

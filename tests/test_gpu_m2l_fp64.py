@@ -1,6 +1,6 @@
 """The FP64 M2L where its instances and its ways of taking opposite offsets
-change (pairs at once up to order 20, read twice from 21, singly from 24, pairs
-again from 29), with sources at both, one or none of an opposite pair, unsplit
+change (pairs at once up to order 20, read twice from 21, by half CTAs from 24,
+singly at 28, pairs again from 29), with sources at both, one or none of an opposite pair, unsplit
 and split offset lists, against the oracle."""
 import numpy as np
 import pytest
