@@ -270,31 +270,39 @@ __device__ __forceinline__ bool adj2(const int *ij, int a, int b) {
   return dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1;
 }
 
-__global__ void k2_colleagues(int cnt, int off, const int *__restrict__ begin,
-                              const int *__restrict__ end, const int *__restrict__ child,
-                              const int *__restrict__ parent, const int *__restrict__ ij,
+// colleagues of every node in node order, 16 threads per node: thread j < 9 walks
+// down from the root of the node's system to the neighbouring cell j, and the
+// cells found are placed by counting smaller node numbers (as in tree.cu)
+__global__ void k2_colleagues(int nn, const int *__restrict__ begin, const int *__restrict__ end,
+                              const int *__restrict__ child, const int *__restrict__ sys,
+                              const int *__restrict__ ij, const uint8_t *__restrict__ depth,
                               int *__restrict__ col, int *__restrict__ ncol) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt) return;
-  int c = off + i;
-  int k = 0;
-  if (end[c] > begin[c]) {
-    int p = parent[c];
-    if (p < 0) {
-      col[9 * c] = c;
-      k = 1;
-    } else {
-      for (int j = 0; j < ncol[p]; ++j) {
-        int c0 = child[col[9 * p + j]];
-        if (c0 < 0) continue;
-        for (int o = 0; o < 4; ++o) {
-          int s = c0 + o;
-          if (end[s] > begin[s] && adj2(ij, c, s) && k < 9) col[9 * c + k++] = s;
-        }
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int c = (int)(g >> 4), t = (int)(g & 15);
+  int q = -1;
+  if (c < nn && t < 9 && end[c] > begin[c]) {
+    const int d = depth[c];
+    const int i = ij[2 * c] + t % 3 - 1, j = ij[2 * c + 1] + t / 3 - 1;
+    if (((i | j) & ~((1 << d) - 1)) == 0) {     // inside the box
+      q = sys[c];
+      for (int b = d - 1; b >= 0 && q >= 0; --b) {
+        const int c0 = child[q];
+        q = c0 < 0 ? -1 : c0 + (((i >> b) & 1) | ((j >> b) & 1) << 1);
       }
+      if (q >= 0 && end[q] == begin[q]) q = -1;
     }
   }
-  ncol[c] = k;
+  int at = 0, n = 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int o = __shfl_sync(0xffffffffu, q, k, 16);
+    if (o >= 0) {
+      ++n;
+      if (o < q) ++at;
+    }
+  }
+  if (q >= 0) col[9 * c + at] = q;
+  if (c < nn && t == 0) ncol[c] = n;
 }
 
 // far sources of node t; mode 0 counts, mode 1 writes
@@ -1417,12 +1425,11 @@ void build_lists2(AranGpuSolver2d *s) {
   const int64_t n = s->n;
   s->col.reserve(9 * (size_t)nn);
   s->ncol.reserve(nn);
-  for (int d = 0; d < s->nlevels; ++d) {
-    int off = s->level_off[d], cnt = s->level_off[d + 1] - off;
-    k2_colleagues<<<ceil_div(cnt, TB), TB, 0, st>>>(cnt, off, s->begin.ptr, s->end.ptr, s->child.ptr,
-                                                     s->parent.ptr, s->ij.ptr, s->col.ptr, s->ncol.ptr);
-    s->launches++;
-  }
+  k2_colleagues<<<ceil_div(16 * (int64_t)nn, TB), TB, 0, st>>>(nn, s->begin.ptr, s->end.ptr,
+                                                               s->child.ptr, s->nsys_.ptr, s->ij.ptr,
+                                                               s->depth.ptr, s->col.ptr, s->ncol.ptr);
+  ACHECK(cudaGetLastError());
+  s->launches++;
   s->flags.reserve((size_t)std::max<int64_t>(nn, n) + 2);
   s->far_off.reserve(nn + 1);
   k2_far<<<ceil_div(nn, TB), TB, 0, st>>>(nn, s->begin.ptr, s->end.ptr, s->child.ptr, s->parent.ptr,
