@@ -232,10 +232,10 @@ void launch_levels(AranGpuSolver3d *s, const float *tab, cplx<float> *ser, int d
   constexpr size_t sm = DOWN ? 0 : (size_t)kOctWarps * OctDims<P, DOWN>::NC * 32 * sizeof(float);
   // levels of fewer nodes go to oct_wide.cu, same bits.  M2M + L2L of 200k
   // uniform particles (5 levels): order 12 0.056 + 0.043 ms, 0.073 + 0.073 with
-  // this kernel on every level; order 8 0.044 + 0.029 and 0.044 + 0.043; from
-  // 512 (M2M, whose cluster costs 10 us a level) or 2048 nodes the wide kernel is
-  // the slower one on 4M Plummer particles
-  constexpr int kWideNodes = DOWN ? (P <= 8 ? 128 : 512) : (P <= 8 ? 0 : 128);
+  // this kernel on every level; order 8 L2L 0.029 and 0.043, M2M of 10k uniform
+  // particles 0.033 and 0.040; from 512 (M2M) or 2048 nodes the wide kernel is the
+  // slower one on 4M Plummer particles
+  constexpr int kWideNodes = DOWN ? (P <= 8 ? 128 : 512) : 128;
   smem_opt_in(k_oct_lanes<P, DOWN>, sm + sizeof(float) * OctDims<P, DOWN>::STRIDE);
   // M2M: parent depths d0 down to d1; L2L: parent depths d0 up to d1.  The
   // internal nodes of depth >= 1 sit in the parents list in node order, so

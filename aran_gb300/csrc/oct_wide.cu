@@ -9,9 +9,10 @@
 // takes one (parent, octant): thread 2c + h makes part h (real, imaginary) of
 // coefficient c through z-phase, rotation, translation along z, rotation back
 // and conjugate phase, each a sum of at most p + 1 products over shared memory
-// with its factors' loads in flight together.  M2M's eight octants are the
-// CTAs of a cluster, which sum their parts in octant order from each other's
-// shared memory.
+// with its factors' loads in flight together.  M2M's eight octants are
+// threads of one CTA where it holds them (up to order 10: order 8 7.5 us a level,
+// 10 with the lane-parallel kernel or a cluster), else the CTAs of a cluster,
+// which sum their parts in octant order from each other's shared memory.
 //
 // In FP32 every sum runs over the same tables (octant 0's stream table, the
 // octant's mirror applied on the way in and out) with the same operations in
@@ -44,15 +45,18 @@ struct WideTab {
   const void *vert;             // direction: vertical factors (vm or vl)
 };
 
-template <typename T, bool DOWN>
+// ONE: M2M with the eight octants' threads in one CTA (tpo threads each)
+template <typename T, bool DOWN, bool ONE>
 __global__ void k_oct_wide(int off, const int *__restrict__ list, const int *__restrict__ child,
                            const int *__restrict__ begin, const int *__restrict__ end, int p,
-                           WideTab tb, const uint8_t *__restrict__ lm, cplx<T> *__restrict__ ser) {
+                           WideTab tb, int tpo, const uint8_t *__restrict__ lm,
+                           cplx<T> *__restrict__ ser) {
   extern __shared__ unsigned char smem_raw[];
   constexpr bool STREAM = sizeof(T) == 4;
   const int LD = DOWN ? p + 1 : p, NC = tri(LD);
-  T *x = reinterpret_cast<T *>(smem_raw), *y = x + 2 * NC;
-  const int o = blockIdx.x, i = threadIdx.x, c = i >> 1, h = i & 1;
+  const int o = ONE ? threadIdx.x / tpo : blockIdx.x;
+  const int i = ONE ? threadIdx.x - o * tpo : threadIdx.x, c = i >> 1, h = i & 1;
+  T *x = reinterpret_cast<T *>(smem_raw) + (ONE ? 4 * NC * o : 0), *y = x + 2 * NC;
   const int par = list ? list[blockIdx.y] : off + (int)blockIdx.y;
   const int c0 = child[par];
   if (c0 < 0) return;                       // the whole cluster
@@ -78,43 +82,53 @@ __global__ void k_oct_wide(int off, const int *__restrict__ list, const int *__r
     }
     return acc;
   };
-  if (live) {
-    if (mine) {
-      const cplx<T> v = ser[(size_t)(DOWN ? par : ch) * NC + c];
-      const T g = ((bx ^ bz) & m & 1) ? (T)-1 : (T)1;
-      const T cj = (bx ^ by) ? -g : g;
-      const T pa = g * (h ? es : ec), pb = cj * (h ? ec : -es);
-      const T sn = (bz && (l & 1)) ? (T)-1 : (T)1;
-      x[i] = sn * fma(v.re, pa, v.im * pb);
-    }
-    __syncthreads();
-    if (mine) y[i] = rotate(x, false);
-    __syncthreads();
-    T z = 0;
-    if (mine) {
-      // translation along z: order m, output degree l, source degrees n
-      const int n0 = DOWN ? l : m, n1 = DOWN ? LD - 1 : l;
-      const T *vf = nullptr, *rp = t0 + tb.rp;
-      if (STREAM)
-        vf = t0 + tb.vt + w_tet(LD) - w_tet(LD - m) +
-             (DOWN ? tri(LD - m) - tri(LD - l) - l : tri(l - m) - m);
-      else
-        vf = static_cast<const T *>(tb.vert) + (size_t)c * (DOWN ? p + 1 : p);
-#pragma unroll 6
-      for (int n = n0; n <= n1; ++n)
-        z = fma(STREAM ? vf[n] : vf[n] * rp[DOWN ? n - l : l - n], y[2 * tri(n, m) + h], z);
-    }
-    __syncthreads();
-    if (mine) x[i] = z;
-    __syncthreads();
+  const bool work = live && mine;
+  if (work) {
+    const cplx<T> v = ser[(size_t)(DOWN ? par : ch) * NC + c];
+    const T g = ((bx ^ bz) & m & 1) ? (T)-1 : (T)1;
+    const T cj = (bx ^ by) ? -g : g;
+    const T pa = g * (h ? es : ec), pb = cj * (h ? ec : -es);
+    const T sn = (bz && (l & 1)) ? (T)-1 : (T)1;
+    x[i] = sn * fma(v.re, pa, v.im * pb);
   }
-  const T a = live && mine ? rotate(x, true) : (T)0;
+  __syncthreads();
+  if (work) y[i] = rotate(x, false);
+  __syncthreads();
+  T z = 0;
+  if (work) {
+    // translation along z: order m, output degree l, source degrees n
+    const int n0 = DOWN ? l : m, n1 = DOWN ? LD - 1 : l;
+    const T *vf = nullptr, *rp = t0 + tb.rp;
+    if (STREAM)
+      vf = t0 + tb.vt + w_tet(LD) - w_tet(LD - m) +
+           (DOWN ? tri(LD - m) - tri(LD - l) - l : tri(l - m) - m);
+    else
+      vf = static_cast<const T *>(tb.vert) + (size_t)c * (DOWN ? p + 1 : p);
+#pragma unroll 6
+    for (int n = n0; n <= n1; ++n)
+      z = fma(STREAM ? vf[n] : vf[n] * rp[DOWN ? n - l : l - n], y[2 * tri(n, m) + h], z);
+  }
+  __syncthreads();
+  if (work) x[i] = z;
+  __syncthreads();
+  const T a = work ? rotate(x, true) : (T)0;
   // conjugate z-phase, mirror on the way out
   const T b = __shfl_xor_sync(kFull, a, 1);
   T v = fma(a, ec, b * (h ? -es : es));
   if (((bz & (l + m)) ^ (bx & m) ^ (h & (bx ^ by))) & 1) v = -v;
   if (DOWN) {
-    if (live && mine) reinterpret_cast<T *>(ser)[(size_t)ch * 2 * NC + i] += v;
+    if (work) reinterpret_cast<T *>(ser)[(size_t)ch * 2 * NC + i] += v;
+  } else if (ONE) {
+    // the eight octants' parts in order
+    if (mine) y[i] = live ? v : (T)0;
+    __syncthreads();
+    const T *all = reinterpret_cast<const T *>(smem_raw) + 2 * NC;
+    for (int k = threadIdx.x; k < 2 * NC; k += blockDim.x) {
+      T sum = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) sum += all[4 * NC * q + k];
+      reinterpret_cast<T *>(ser)[(size_t)par * 2 * NC + k] = sum;
+    }
   } else {
     // the eight octants' parts in order, each CTA an eighth of the values
     if (mine) y[i] = live ? v : (T)0;
@@ -136,18 +150,21 @@ void launch(AranGpuSolver3d *s, const WideTab &tb, const uint8_t *lm, cplx<T> *s
             int off, const int *list, cudaStream_t st) {
   DevTree &t = s->tree;
   const int p = s->cfg.order, NC = tri(DOWN ? p + 1 : p);
-  const size_t sm = (size_t)4 * NC * sizeof(T);
-  auto kern = k_oct_wide<T, DOWN>;
+  // M2M: one CTA for a parent's octants where its threads hold them (order 10)
+  const int tpo = (2 * NC + 31) & ~31;
+  const bool one = !DOWN && 8 * tpo <= 1024;
+  const size_t sm = (size_t)4 * NC * sizeof(T) * (one ? 8 : 1);
+  auto kern = one ? k_oct_wide<T, DOWN, !DOWN> : k_oct_wide<T, DOWN, false>;
   // grid.y holds 65,535 nodes at most
   for (int b = 0; b < cnt; b += 65535) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(8, cnt - b < 65535 ? cnt - b : 65535);
-    cfg.blockDim = dim3((2 * NC + 31) & ~31);
+    cfg.gridDim = dim3(one ? 1 : 8, cnt - b < 65535 ? cnt - b : 65535);
+    cfg.blockDim = dim3(one ? 8 * tpo : tpo);
     cfg.dynamicSmemBytes = sm;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = DOWN ? 1 : 8;
+    attr[0].val.clusterDim.x = DOWN || one ? 1 : 8;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -155,7 +172,7 @@ void launch(AranGpuSolver3d *s, const WideTab &tb, const uint8_t *lm, cplx<T> *s
     ACHECK(cudaLaunchKernelEx(&cfg, kern, off + (list ? 0 : b),
                               (const int *)(list ? list + b : nullptr),
                               (const int *)t.child.ptr, (const int *)t.begin.ptr,
-                              (const int *)t.end.ptr, p, tb, lm, ser));
+                              (const int *)t.end.ptr, p, tb, tpo, lm, ser));
     s->launches++;
   }
 }
