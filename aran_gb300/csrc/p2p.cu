@@ -303,6 +303,9 @@ __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
       }
       __syncthreads();
       const int tot = s_tot;
+      // no tile and none of its barriers (every range heavy): the next ranges
+      // wait until all threads have read this total
+      if (tot == 0) __syncthreads();
       for (int k0 = 0; k0 < tot; k0 += 2 * T) {
         const int np = min(T, (tot - k0 + 1) / 2);   // pairs of this tile
         if (threadIdx.x < np) {
