@@ -15,15 +15,20 @@ __device__ __forceinline__ double leaf_inv_scale(int depth, double scale_e) {
   return ldexp(1.0, depth) / scale_e;    // 1/h_d = 2^d / 2^E (exact power of two)
 }
 
-// P2M, a warp per window of 32 sorted particles whatever leaves they lie in (a
+// P2M, a warp per run of leaves: those that start in the warp's span of kSpan
+// sorted particles, taken 32 particles at a time whatever leaves they lie in (a
 // warp per leaf keeps as many lanes busy as the leaf has points).  A lane makes
 // its particle's q S_l^m in m-major order (six operations a coefficient) into
 // shared memory; every 32 values the lanes turn to the values, a lane one of them,
-// and add it up over each leaf's part of the window (one addition a value and
-// particle; by shuffles over the warp it was five on every lane).  A leaf
-// inside the window is stored, parts of a leaf are added to its zeroed multipole.
-// 200k Plummer particles (18 a leaf), order 12: 0.34 ms, 1.44 with a warp per
-// leaf and shuffles.
+// and add it up particle by particle (one addition a value and particle; by
+// shuffles over the warp it was five on every lane).  A leaf's sum is that of
+// its segments of 32 particles, each added up from its first particle: what else
+// is solved, and with it the leaf's place in a span, does not change its bits.
+// 200k Plummer particles (18 a leaf), order 12: 0.51 ms, 1.44 with a warp per
+// leaf and shuffles (0.34 with the parts of a leaf added as they come, the whole
+// solve 38.1 ms either way); 10k 0.12 ms, 0.15 and 0.23 with spans of 64 and 128.
+constexpr int kSpan = 32;
+
 __global__ void __launch_bounds__(32 * kWarps)
     k_p2m64(int64_t n, int nleaves, const int *__restrict__ win_leaf,
             const int2 *__restrict__ leaf_be, const int *__restrict__ leaf_node,
@@ -45,79 +50,101 @@ __global__ void __launch_bounds__(32 * kWarps)
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t win = blockIdx.x * (int64_t)kWarps + w, b0 = 32 * win;
-  if (b0 >= n) return;
-  buf += w * 32 * 33;
-  const int cnt = n - b0 < 32 ? (int)(n - b0) : 32;
-  // leaves of the window: L0 holds its first particle, the next ones start inside
-  const int L0 = win_leaf[win];
-  unsigned bit = 0;
-  if (lane > 0 && L0 + lane < nleaves) {
-    const int64_t at = leaf_be[L0 + lane].x - b0;
-    if (at < cnt) bit = 1u << at;
-  }
-  const unsigned starts = __reduce_or_sync(kFull, bit);
-  double x = 0, y = 0, z = 0, q = 0;
-  if (lane < cnt) {
+  buf += w * (32 * 33 + 2 * nm);
+  double *carry = buf + 32 * 33;           // sums of a segment that goes on
+  // first leaf that starts at or behind a place (a multiple of 32)
+  auto leaf_from = [&](int64_t at) -> int {
+    if (at >= n) return nleaves;
+    const int L = win_leaf[at >> 5];
+    return leaf_be[L].x < at ? L + 1 : L;
+  };
+  const int64_t span = blockIdx.x * (int64_t)kWarps + w;
+  int L0 = leaf_from(kSpan * span);        // leaf of the round's first particle
+  const int L1 = leaf_from(kSpan * (span + 1));
+  if (L0 >= L1) return;
+  const int stop = leaf_be[L1 - 1].y;
+  bool goes_on = false;                    // L0 began in a round before
+  for (int base = leaf_be[L0].x; base < stop; base += 32) {
+    const int cnt = min(stop - base, 32);
+    // bit i: particle base + i starts a leaf, a segment (never the first)
+    unsigned bit = 0;
+    if (lane > 0 && L0 + lane < L1) {
+      const int at = leaf_be[L0 + lane].x - base;
+      if (at < cnt) bit = 1u << at;
+    }
+    const unsigned starts = __reduce_or_sync(kFull, bit);
     const int L = L0 + __popc(starts & ((2u << lane) - 1u));
-    const double ih = leaf_inv_scale(depth[leaf_node[L]], scale_e);
-    const real4<double> r = rel[b0 + lane];
-    x = r.x * ih;
-    y = r.y * ih;
-    z = r.z * ih;
-    q = r.q;
-  }
-  const double r2 = x * x + y * y + z * z;
-  int k = 0;                               // value: 2 m-major place + part
-  auto put = [&](double v) {
-    buf[(k & 31) * 33 + lane] = v;
-    ++k;
-    if ((k & 31) && k < 2 * nm) return;
-    // the lanes take the values
-    __syncwarp();
-    const int mine = ((k - 1) & ~31) + lane;
-    if (mine < k) {
-      const double f = (mine & 1) ? -fac[mine >> 1] : fac[mine >> 1];
-      const size_t c = 2 * (size_t)coef[mine >> 1] + (mine & 1);
-      unsigned left = starts;
-      int L = L0, j = 0;
-      while (j < cnt) {
-        const int j1 = left ? __ffs(left) - 1 : cnt;
-        left &= left - 1;
-        double sum = 0;
+    const unsigned cuts =
+        __ballot_sync(kFull, lane > 0 && lane < cnt && ((base + lane - leaf_be[L].x) & 31) == 0);
+    double x = 0, y = 0, z = 0, q = 0;
+    if (lane < cnt) {
+      const double ih = leaf_inv_scale(depth[leaf_node[L]], scale_e);
+      const real4<double> r = rel[base + lane];
+      x = r.x * ih;
+      y = r.y * ih;
+      z = r.z * ih;
+      q = r.q;
+    }
+    const double r2 = x * x + y * y + z * z;
+    int k = 0;                               // value: 2 m-major place + part
+    auto put = [&](double v) {
+      buf[(k & 31) * 33 + lane] = v;
+      ++k;
+      if ((k & 31) && k < 2 * nm) return;
+      // the lanes take the values
+      __syncwarp();
+      const int mine = ((k - 1) & ~31) + lane;
+      if (mine < k) {
+        const double f = (mine & 1) ? -fac[mine >> 1] : fac[mine >> 1];
+        const size_t c = 2 * (size_t)coef[mine >> 1] + (mine & 1);
+        double sum = goes_on ? carry[mine] : 0.;
+        unsigned left = cuts;
+        int l = L0, j = 0;
+        while (j < cnt) {
+          const int j1 = left ? __ffs(left) - 1 : cnt;
+          left &= left - 1;
 #pragma unroll 4
-        for (int jj = j; jj < j1; ++jj) sum += buf[lane * 33 + jj];
-        const int2 be = leaf_be[L];
-        double *out = mult + 2 * (size_t)nm * leaf_node[L] + c;
-        if (be.x >= b0 && be.y <= b0 + 32) *out = f * sum;
-        else atomicAdd(out, f * sum);
-        j = j1;
-        ++L;
+          for (int jj = j; jj < j1; ++jj) sum += buf[lane * 33 + jj];
+          j = j1;
+          const int2 be = leaf_be[l];
+          const bool last = base + j == be.y;
+          if (last || ((base + j - be.x) & 31) == 0) {   // a segment ends
+            double *out = mult + 2 * (size_t)nm * leaf_node[l] + c;
+            if (base + j - be.x > 32) sum = *out + sum;
+            *out = last ? f * sum : sum;
+            sum = 0.;
+            if (last) ++l;
+          }
+        }
+        carry[mine] = sum;
+      }
+      __syncwarp();
+    };
+    double dre = q * rec[0], dim = 0;
+    for (int m = 0; m < p; ++m) {
+      if (m > 0) {
+        const double a = rec[2 * tri(m, m)];
+        const double nre = a * (x * dre - y * dim), nim = a * (x * dim + y * dre);
+        dre = nre;
+        dim = nim;
+      }
+      double s1re = dre, s1im = dim, s2re = 0, s2im = 0;
+      put(dre);
+      put(dim);
+      for (int l = m + 1; l < p; ++l) {
+        const double a = rec[2 * tri(l, m)] * z, b = rec[2 * tri(l, m) + 1] * r2;
+        const double sre = a * s1re - b * s2re, sim = a * s1im - b * s2im;
+        s2re = s1re;
+        s2im = s1im;
+        s1re = sre;
+        s1im = sim;
+        put(sre);
+        put(sim);
       }
     }
-    __syncwarp();
-  };
-  double dre = q * rec[0], dim = 0;
-  for (int m = 0; m < p; ++m) {
-    if (m > 0) {
-      const double a = rec[2 * tri(m, m)];
-      const double nre = a * (x * dre - y * dim), nim = a * (x * dim + y * dre);
-      dre = nre;
-      dim = nim;
-    }
-    double s1re = dre, s1im = dim, s2re = 0, s2im = 0;
-    put(dre);
-    put(dim);
-    for (int l = m + 1; l < p; ++l) {
-      const double a = rec[2 * tri(l, m)] * z, b = rec[2 * tri(l, m) + 1] * r2;
-      const double sre = a * s1re - b * s2re, sim = a * s1im - b * s2im;
-      s2re = s1re;
-      s2im = s1im;
-      s1re = sre;
-      s1im = sim;
-      put(sre);
-      put(sim);
-    }
+    L0 += __popc(starts);
+    goes_on = leaf_be[L0].y != base + cnt;
+    if (!goes_on) ++L0;
   }
 }
 
@@ -236,9 +263,9 @@ void launch_p2m64(AranGpuSolver3d *s, cudaStream_t st) {
   OpTables<double> &tb = s->t64;
   const int p = s->cfg.order, nm = tri(p);
   const size_t sm = (size_t)3 * nm * sizeof(double) + ((nm + 1) & ~1) * sizeof(int) +
-                    (size_t)kWarps * 32 * 33 * sizeof(double);
+                    (size_t)kWarps * (32 * 33 + 2 * nm) * sizeof(double);
   smem_opt_in(k_p2m64, sm);
-  k_p2m64<<<ceil_div((t.n + 31) / 32, kWarps), 32 * kWarps, sm, st>>>(
+  k_p2m64<<<ceil_div((t.n + kSpan - 1) / kSpan, kWarps), 32 * kWarps, sm, st>>>(
       t.n, t.nleaves, t.win_leaf.ptr, t.leaf_be.ptr, t.leaf_node.ptr, t.depth.ptr, s->rel64.ptr, p,
       tb.rec.ptr, tb.p2mf.ptr, s->scale_e, s->mult64.ptr);
   ACHECK(cudaGetLastError());
