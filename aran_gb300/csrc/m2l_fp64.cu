@@ -22,14 +22,16 @@
 //    of a parent) read the same table at about the same time.  Tables are
 //    streamed from L2 in the order the lanes use them: [round][step][lane].
 //
-// A CTA takes one part of a parent's units (offsets or pairs); the parts'
-// sums are added in order.  Measured on GB300 against the sibling kernel in FP64:
-// 200k Plummer particles at order 12, the whole solve with the near field beside
-// it on the same pipe, 40.2 ms, 48.4 before (42.0 with two CTAs an SM); eight
-// served requests, two of them in FP64 at order 26, 13.9 ms, 35 before (with the
-// P2M and L2P of leaf_fp64.cu).  60k
-// Plummer particles, this kernel alone: 3.8 ms, the FP64 pipe active 92 % of
-// the cycles.
+// A target's sum is the sum of kF64Segs segments of the units (offsets or pairs):
+// a CTA takes one segment of a parent and leaves its sum in a workspace, the
+// segments are added in order.  So a system's bits do not depend on what else is
+// solved, as they did when passes with few parents alone were split.
+// Measured on GB300 against the sibling kernel in FP64: 200k Plummer particles
+// at order 12, the whole solve with the near field beside it on the same pipe,
+// 40.2 ms, 48.4 before (42.0 with two CTAs an SM); eight served requests, two of
+// them in FP64 at order 26, 13.9 ms, 35 before (with the P2M and L2P of
+// leaf_fp64.cu).  60k Plummer particles, this kernel alone: 3.8 ms, the FP64 pipe
+// active 92 % of the cycles.
 #include <algorithm>
 #include <vector>
 
@@ -40,6 +42,13 @@ namespace aran {
 namespace {
 
 constexpr int kF64Warps = 8;
+constexpr int kF64Segs = 16;
+constexpr size_t kF64PartBytes = 1u << 30;   // workspace of the segments' sums
+
+// first unit of a segment
+__device__ __forceinline__ int seg_unit(int seg, int nunits) {
+  return (seg * nunits + kF64Segs - 1) / kF64Segs;
+}
 
 // one dot product of a stage: first source and destination in the planes of
 // the stage's vectors, length, first step between sources (it grows by one per
@@ -176,7 +185,7 @@ __host__ __device__ inline int m2l_fp64_warp(int p, int mode) {
 // R rounds of 32 lanes over the tri(p+1) local coefficients
 template <int R>
 __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
-    k_m2l_fp64(int nparents, int nsplit, int nunits, int mode, const int *__restrict__ parents,
+    k_m2l_fp64(int nparents, int nunits, int mode, const int *__restrict__ parents,
                const int *__restrict__ child, const int *__restrict__ begin,
                const int *__restrict__ end, const int *__restrict__ col,
                const int *__restrict__ ncol, const int *__restrict__ ijk,
@@ -185,8 +194,7 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
                const unsigned *__restrict__ units, const double *__restrict__ tabs,
                const double *__restrict__ dir, int dstride, int ph_off,
                const uint8_t *__restrict__ lm, double scale_e,
-               const cplx<double> *__restrict__ mult, cplx<double> *__restrict__ loc,
-               cplx<double> *__restrict__ parts) {
+               const cplx<double> *__restrict__ mult, cplx<double> *__restrict__ parts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int grid[216];
   const int nm = tri(p), nl = tri(p + 1);
@@ -228,8 +236,8 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
   cplx<double> acc[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) acc[r] = cmake(0., 0.);
-  const int u0 = nunits * (int)blockIdx.y / nsplit, u1 = nunits * ((int)blockIdx.y + 1) / nsplit;
-  for (int u = u0; u < u1; ++u) {
+  const int seg = blockIdx.y, u1 = seg_unit(seg + 1, nunits);
+  for (int u = seg_unit(seg, nunits); u < u1; ++u) {
     const unsigned code = units[u];
     const int a = code & 7, b = (code >> 3) & 7, c = (code >> 6) & 7;
     int s0 = source_of(a, b, c), s1 = (code & 512u) ? source_of(6 - a, 6 - b, 6 - c) : -1;
@@ -348,9 +356,7 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
     }
   }
   const double ih = ldexp(1.0, depth[t]) / scale_e;
-  cplx<double> *out = nsplit == 1
-                          ? loc + (size_t)t * nl
-                          : parts + (((size_t)blockIdx.y * nparents + pb) * kF64Warps + w) * nl;
+  cplx<double> *out = parts + (((size_t)seg * nparents + pb) * kF64Warps + w) * nl;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = lane + 32 * r;
@@ -362,9 +368,9 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
   }
 }
 
-// the parts of a split pass added in order, one warp per child
+// the segments added in order, one warp per child
 __global__ void __launch_bounds__(32 * kF64Warps)
-    k_m2l_parts_sum(int nparents, int nsplit, const int *__restrict__ parents,
+    k_m2l_parts_sum(int nparents, const int *__restrict__ parents,
                     const int *__restrict__ child, const int *__restrict__ begin,
                     const int *__restrict__ end, int nl, const cplx<double> *__restrict__ parts,
                     cplx<double> *__restrict__ loc) {
@@ -375,7 +381,7 @@ __global__ void __launch_bounds__(32 * kF64Warps)
   const cplx<double> *p = parts + ((size_t)blockIdx.x * kF64Warps + w) * nl;
   for (int c = lane; c < nl; c += 32) {
     cplx<double> v = cmake(0., 0.);
-    for (int k = 0; k < nsplit; ++k) v = cadd(v, p[k * step + c]);
+    for (int k = 0; k < kF64Segs; ++k) v = cadd(v, p[k * step + c]);
     loc[(size_t)t * nl + c] = v;
   }
 }
@@ -420,10 +426,9 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   OpTables<double> &tb = s->t64;
   const M2lFp64Tables &f = tb.m2l64;
   const int p = s->cfg.order, nm = tri(p), nl = tri(p + 1);
-  int dev_smem = 0, sm_smem = 0, nsm = 0;
+  int dev_smem = 0, sm_smem = 0;
   ACHECK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
   ACHECK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
-  ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
   // Pairs, made at once (16 warps an SM or more up to order 20); read twice where
   // that keeps 16 warps (orders 21 to 23): order 22, 60k Plummer particles, M2L 44
   // ms, 71 made at once, 50 singly; 2 to 3 % slower below.  Above, read twice by
@@ -445,29 +450,33 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
     mode = kF64Single;
   }
   const size_t sm = bytes(nw, mode);
-  // about 24 CTAs per SM even out the SMs' last CTAs
-  const int nsplit = std::min(16, std::max(1, (24 * nsm + count - 1) / count));
-  cplx<double> *mult = reinterpret_cast<cplx<double> *>(s->mult64.ptr);
+  // As many parents at a time as the workspace holds.  (One CTA for all segments of a
+  // parent, adding them up as it goes, takes as long or longer: 1,574 parents of
+  // order 12, 200k Plummer particles, 16.3 ms against 14.3; 8,155 parents 77.9
+  // against 77.0.)
+  const size_t per = (size_t)kF64Segs * kF64Warps * nl;     // sums of a parent
+  const int most = (int)(kF64PartBytes / (per * sizeof(cplx<double>)));
+  const int step = ceil_div(count, ceil_div(count, most));
+  s->m2l_part64.reserve(2 * per * step);
+  const cplx<double> *mult = reinterpret_cast<cplx<double> *>(s->mult64.ptr);
   cplx<double> *loc = reinterpret_cast<cplx<double> *>(s->loc64.ptr);
-  cplx<double> *parts = nullptr;
-  if (nsplit > 1) {
-    s->m2l_part64.reserve((size_t)nsplit * count * kF64Warps * nl * 2);
-    parts = reinterpret_cast<cplx<double> *>(s->m2l_part64.ptr);
-  }
-  auto kern = nl <= 96 ? k_m2l_fp64<3> : (nl <= 160 ? k_m2l_fp64<5> : (nl <= 256 ? k_m2l_fp64<8> : k_m2l_fp64<16>));
+  cplx<double> *parts = reinterpret_cast<cplx<double> *>(s->m2l_part64.ptr);
+  auto kern = nl <= 96 ? k_m2l_fp64<3>
+                       : (nl <= 160 ? k_m2l_fp64<5> : (nl <= 256 ? k_m2l_fp64<8> : k_m2l_fp64<16>));
   smem_opt_in(kern, sm);
-  kern<<<dim3(count * (kF64Warps / nw), nsplit), 32 * nw, sm, st>>>(
-      count, nsplit, f.nunits, mode, parents, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
-      t.ncol.ptr, t.ijk.ptr, t.depth.ptr, p, f.sched, reinterpret_cast<const F64Task *>(f.task.ptr),
-      f.trip.ptr, f.units.ptr, f.tabs.ptr, tb.dir_m2l.ptr, dir_offset(p, 0, 6),
-      dir_offset(p, 0, 4), tb.lm.ptr, s->scale_e, mult, loc, parts);
-  ACHECK(cudaGetLastError());
-  s->launches++;
-  if (nsplit > 1) {
-    k_m2l_parts_sum<<<count, 32 * kF64Warps, 0, st>>>(count, nsplit, parents, t.child.ptr,
-                                                      t.begin.ptr, t.end.ptr, nl, parts, loc);
+  for (int first = 0; first < count; first += step) {
+    const int cnt = std::min(step, count - first);
+    kern<<<dim3(cnt * (kF64Warps / nw), kF64Segs), 32 * nw, sm, st>>>(
+        cnt, f.nunits, mode, parents + first, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
+        t.ncol.ptr, t.ijk.ptr, t.depth.ptr, p, f.sched,
+        reinterpret_cast<const F64Task *>(f.task.ptr), f.trip.ptr, f.units.ptr, f.tabs.ptr,
+        tb.dir_m2l.ptr, dir_offset(p, 0, 6), dir_offset(p, 0, 4), tb.lm.ptr, s->scale_e, mult,
+        parts);
     ACHECK(cudaGetLastError());
-    s->launches++;
+    k_m2l_parts_sum<<<cnt, 32 * kF64Warps, 0, st>>>(cnt, parents + first, t.child.ptr, t.begin.ptr,
+                                                    t.end.ptr, nl, parts, loc);
+    ACHECK(cudaGetLastError());
+    s->launches += 2;
   }
 }
 
