@@ -40,4 +40,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return r;
 }
 
+// Kahan's sum
+__device__ __forceinline__ void kahan(float &sum, float &comp, float v) {
+  const float y = v - comp;
+  const float t = sum + y;
+  comp = (t - sum) - y;
+  sum = t;
+}
+
 }  // namespace aran

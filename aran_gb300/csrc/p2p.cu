@@ -246,14 +246,6 @@ __global__ void __launch_bounds__(128, 8) k_p2p64(
 // nothing; 10 blocks an SM with 48 registers a thread beat 8, 6 and 12.
 constexpr int kP2pRanges = 32;   // near ranges taken together
 
-// Kahan's sum
-__device__ __forceinline__ void kahan(float &sum, float &comp, float v) {
-  const float y = v - comp;
-  const float t = sum + y;
-  comp = (t - sum) - y;
-  sum = t;
-}
-
 template <bool FIELD, bool BIG, int T>
 __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
     const int4 *__restrict__ items, const int *__restrict__ near_off,

@@ -701,8 +701,9 @@ __global__ void k2_l2p(int64_t n, int p, const int *__restrict__ incl, const int
 // FP32 expansions scaled by the node size h (the larger side of the
 // system's box / 2^depth): multipole ma_k = a_{-k} / h^{k-1}, local
 // la_k = b_k h^k, so every operator works on O(1) numbers whatever the
-// depth; centres, node sizes and the near-field differences stay FP64 and
-// every particle's sum is FP64.  The operators are those of the FP64 kernels
+// depth; centres and node sizes stay FP64, near-field differences are FP32 hi +
+// lo (close ones FP64) with compensated FP32 sums, and every particle's near and far
+// parts are added in FP64.  The operators are those of the FP64 kernels
 // above with z/h in place of z (rho = h_child / h_parent = 1/2):
 //   M2M  mb_i = sum_{j<i} C(i-1, j-1) rho^{j-1} ma_j u^{i-j} + rho^{i-1} ma_i,
 //        u = (z_child - z_parent) / h_parent;
@@ -945,10 +946,13 @@ __device__ __forceinline__ float rcp_ftz(float x) {
 // floor(T / n) threads per target sum two sources per packed instruction.
 // A pair closer than h/8 (h the target leaf's size), where the offset's
 // rounding would show, is left out of the loop and added from the FP64
-// positions.  A thread's parts of the tiles go into Kahan sums, the parts of
-// a target are added with compensation.  Bound by the reciprocal unit (a
-// quarter of a warp per cycle), 8 cycles a pair and scheduler, on large
-// leaves, by the blocks' set-up on small ones.
+// positions.  Runs of up to RUN pairs go into Kahan sums, the parts of a target
+// are added with compensation: rms error of one-sign sums on leaves of 16, 70 and
+// 120 points 1.9e-8, 1.7e-8, 1.5e-8 (one run a tile 2.0e-8, 4.4e-8, 3.9e-8, and the
+// kernel 2 to 4 % faster); a warp per leaf, with plain FP32 sums over whole ranges,
+// FP64 sums of those and correctly rounded reciprocals, 2.3e-8, 3.6e-8, 4.5e-8.
+// Bound by the reciprocal unit (a quarter of a warp per cycle), 8 cycles a pair and
+// scheduler, on large leaves, by the blocks' set-up on small ones.
 constexpr int k2Ranges = 32;     // near ranges taken together
 template <int T>                 // threads, and pairs of a tile
 __global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleaves, const int *__restrict__ leaf_be,
@@ -958,6 +962,7 @@ __global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleave
                         const double *__restrict__ center, const double *__restrict__ sx,
                         const double *__restrict__ sy, const double *__restrict__ sq,
                         const float4 *__restrict__ hl, zd *__restrict__ near_acc) {
+  constexpr int RUN = 32;                       // pairs summed plainly
   // pair p of the tile: (-x0, -x1, -y0, -y1) and (q0, q1)
   __shared__ ulonglong2 tA[T];
   __shared__ uint64_t tQ[T];
@@ -1036,27 +1041,30 @@ __global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleave
         }
         __syncthreads();
         if (active) {
-          uint64_t p2r = 0ull, p2i = 0ull;
           unsigned close = 0;   // 1 + pair of the last close pair, above it the one before
+          for (int p0 = sub; p0 < np; p0 += RUN * S) {
+            const int p1 = min(np, p0 + RUN * S);
+            uint64_t p2r = 0ull, p2i = 0ull;
 #pragma unroll 2
-          for (int p = sub; p < np; p += S) {
-            const ulonglong2 A = tA[p];
-            const uint64_t q2 = tQ[p];
-            const uint64_t dx = add2(tx2, A.x), dy = add2(ty2, A.y);
-            const uint64_t r2 = fma2(dy, dy, mul2(dx, dx));
-            float ra, rb2;
-            unpack2(r2, ra, rb2);
-            const bool ca = ra < thr2, cb = rb2 < thr2;
-            if (ca || cb) close = (close << 16) + (unsigned)(p + 1);
-            const uint64_t w = mul2(q2, pack2(ca ? 0.f : rcp_ftz(ra), cb ? 0.f : rcp_ftz(rb2)));
-            p2r = fma2(dx, w, p2r);
-            p2i = fma2(dy, w, p2i);
+            for (int p = p0; p < p1; p += S) {
+              const ulonglong2 A = tA[p];
+              const uint64_t q2 = tQ[p];
+              const uint64_t dx = add2(tx2, A.x), dy = add2(ty2, A.y);
+              const uint64_t r2 = fma2(dy, dy, mul2(dx, dx));
+              float ra, rb2;
+              unpack2(r2, ra, rb2);
+              const bool ca = ra < thr2, cb = rb2 < thr2;
+              if (ca || cb) close = (close << 16) + (unsigned)(p + 1);
+              const uint64_t w = mul2(q2, pack2(ca ? 0.f : rcp_ftz(ra), cb ? 0.f : rcp_ftz(rb2)));
+              p2r = fma2(dx, w, p2r);
+              p2i = fma2(dy, w, p2i);
+            }
+            float lo, hi;
+            unpack2(p2r, lo, hi);
+            kahan(ks[0], kc[0], lo + hi);
+            unpack2(p2i, lo, hi);
+            kahan(ks[1], kc[1], lo + hi);
           }
-          float lo, hi, pr, pi;
-          unpack2(p2r, lo, hi);
-          pr = lo + hi;
-          unpack2(p2i, lo, hi);
-          pi = lo + hi;
           if (close) {
             const bool one = close < 65536u;
             for (int p = one ? (int)close - 1 : sub; p < np; p += one ? T : S) {
@@ -1074,18 +1082,10 @@ __global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleave
                 r2 = dx * dx + dy * dy;
                 if (!(r2 > 0.f)) continue;
                 const float w = (e ? fq.y : fq.x) * __frcp_rn(r2);
-                pr = fmaf(dx, w, pr);
-                pi = fmaf(dy, w, pi);
+                kahan(ks[0], kc[0], dx * w);
+                kahan(ks[1], kc[1], dy * w);
               }
             }
-          }
-          const float v[2] = {pr, pi};
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const float y = v[c] - kc[c];
-            const float n = ks[c] + y;
-            kc[c] = (n - ks[c]) - y;
-            ks[c] = n;
           }
         }
         __syncthreads();
