@@ -113,7 +113,8 @@ __host__ __device__ constexpr bool m2l_lane_order(int p) { return p == 4 || p ==
 // blocks the translation's factors H depend on j + n alone and are constants
 // of the code.  Each degree's block is scaled on both sides by A, which keeps
 // it symmetric; the kernel divides its sources and its sums by A.  (4^l keeps
-// A and H within 1e-8 .. 1e16 up to order 16.)  One block per offset:
+// A and H within 1e-8 .. 1e16 up to order 16.)  beta stands for beta_l / beta_0,
+// which makes degree 0's factors one and 1/r.  One block per offset:
 //  * cos(m phi), m = 0..p, padded to a multiple of four, then sin(m phi) alike;
 //  * the forward lower triangles, degree l times A A s^l r^-l / beta_l, in
 //    groups of four like above;
