@@ -192,7 +192,7 @@ struct AranGpuSolver3d {
   aran::DBuf<uint64_t> keys_in, keys_out;
   aran::DBuf<int> idx_in, perm, sort_tmp;
   aran::DBuf<uint8_t> cub_tmp;
-  aran::DBuf<double> sx, sy, sz, sq;     // sorted FP64 positions/charges
+  aran::DBuf<double> sx, sy, sz, sq;     // sorted FP64 positions/charges (mixed: scaled)
   aran::DBuf<aran::real4<double>> rel64;
   aran::DBuf<aran::real4<float>> rel32;
   aran::DBuf<float4> abs_hi, abs_lo;     // FP32 hi + lo positions in the box (hi.w = charge), mixed
@@ -202,7 +202,9 @@ struct AranGpuSolver3d {
   aran::DBuf<float> mult32, loc32;
   aran::DBuf<int> scan_tmp;
   aran::DBuf<unsigned long long> stats_dev;
-  aran::DBuf<int> err_dev;               // device error word (bounded waits)
+  // device error word (bounded waits), then per system the exponent field of its
+  // largest charge (mixed precision)
+  aran::DBuf<int> err_dev;
   int *h_small = nullptr;                // pinned host words for the solve's small readbacks
   int64_t stats[11] = {};
   double ms[16] = {};
@@ -312,6 +314,35 @@ void launch_semifar_m2p(AranGpuSolver3d *s, cudaStream_t st);
 void copy_expansions(AranGpuSolver3d *s, double *mult, double *local);
 
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
+
+// the charges' exponent fields, none in FP64
+inline int *charge_fields(AranGpuSolver3d *s) {
+  return s->cfg.precision == ARAN_PRECISION_MIXED ? s->err_dev.ptr + 1 : nullptr;
+}
+
+#ifdef __CUDACC__
+// the last system that starts at or before place i (of the particles, sorted or not)
+__device__ __forceinline__ int system_of(int64_t i, int nsys, const int *__restrict__ sys_off) {
+  int lo = 0, hi = nsys;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (sys_off[mid] <= i) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// Mixed solves take a power of two out of each system's charges, whose largest
+// then lies in [1, 2), and put it back into the results: the FP32 expansions, which
+// spread over up to 1e16 at high orders, neither overflow nor vanish whatever unit
+// the charges are in, and no bit changes otherwise.  `field`: exponent field of
+// the largest charge, 0 (no charge): nothing is taken out.
+__device__ __forceinline__ double charge_unit(int field) {
+  return field ? ldexp(1.0, field - 1023) : 1.0;
+}
+__device__ __forceinline__ double charge_per_unit(int field) {
+  return field ? ldexp(1.0, 1023 - field) : 1.0;
+}
+#endif
 
 // solver2d.cu: a 2D solve, or only its forest (tree_only, acc unused); and a
 // host copy of the last forest (node arrays, permutation, per-node Laurent

@@ -381,17 +381,19 @@ __global__ void k_l2p(int nleaves, const int *__restrict__ leaf_node, const int 
   }
 }
 
-__global__ void k_scatter(int64_t n, const int *__restrict__ perm, const double *__restrict__ acc_pot,
-                          const double *__restrict__ acc_fld, double *__restrict__ pot,
-                          double *__restrict__ fld) {
+__global__ void k_scatter(int64_t n, const int *__restrict__ perm, int nsys,
+                          const int *__restrict__ sys_off, const int *__restrict__ qmax,
+                          const double *__restrict__ acc_pot, const double *__restrict__ acc_fld,
+                          double *__restrict__ pot, double *__restrict__ fld) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
-  if (pot) pot[o] = acc_pot[i];
+  const double u = qmax ? charge_unit(qmax[system_of(i, nsys, sys_off)]) : 1.0;
+  if (pot) pot[o] = u * acc_pot[i];
   if (fld) {
-    fld[3 * (int64_t)o] = acc_fld[3 * i];
-    fld[3 * (int64_t)o + 1] = acc_fld[3 * i + 1];
-    fld[3 * (int64_t)o + 2] = acc_fld[3 * i + 2];
+    fld[3 * (int64_t)o] = u * acc_fld[3 * i];
+    fld[3 * (int64_t)o + 1] = u * acc_fld[3 * i + 1];
+    fld[3 * (int64_t)o + 2] = u * acc_fld[3 * i + 2];
   }
 }
 
@@ -659,9 +661,9 @@ void run_passes(AranGpuSolver3d *s) {
 
 void scatter_outputs(AranGpuSolver3d *s, double *pot, double *fld) {
   const int TB = 256;
-  k_scatter<<<ceil_div(s->tree.n, TB), TB, 0, s->s0>>>(s->tree.n, s->perm.ptr, s->acc_pot.ptr,
-                                                        s->cfg.field ? s->acc_fld.ptr : nullptr,
-                                                        pot, s->cfg.field ? fld : nullptr);
+  k_scatter<<<ceil_div(s->tree.n, TB), TB, 0, s->s0>>>(
+      s->tree.n, s->perm.ptr, s->nsys, s->sys_off.ptr, charge_fields(s), s->acc_pot.ptr,
+      s->cfg.field ? s->acc_fld.ptr : nullptr, pot, s->cfg.field ? fld : nullptr);
   ACHECK(cudaGetLastError());
   s->launches++;
 }
@@ -696,15 +698,16 @@ void compute_stats(AranGpuSolver3d *s) {
 
 namespace {
 template <typename T>
-__global__ void k_unscale(int nn, int p, const uint8_t *__restrict__ depth, double scale_e,
+__global__ void k_unscale(int nn, int p, const uint8_t *__restrict__ depth,
+                          const int *__restrict__ sys, const int *__restrict__ qmax, double scale_e,
                           const cplx<T> *__restrict__ mult, const cplx<T> *__restrict__ loc,
                           double *__restrict__ om, double *__restrict__ ol) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nn) return;
   int nm = tri(p), nl = tri(p + 1);
-  double h = scale_e / ldexp(1.0, depth[i]);
+  const double h = scale_e / ldexp(1.0, depth[i]), u = qmax ? charge_unit(qmax[sys[i]]) : 1.0;
   for (int l = 0; l <= p; ++l) {
-    double hm = pow(h, l), hl = 1.0 / hm;
+    const double hp = pow(h, l), hm = u * hp, hl = u / hp;
     for (int m = 0; m <= l; ++m) {
       if (l < p && om) {
         cplx<T> v = mult[(size_t)i * nm + tri(l, m)];
@@ -730,12 +733,12 @@ void copy_expansions(AranGpuSolver3d *s, double *mult, double *local) {
   ol.reserve(t.nnodes * nl * 2);
   if (s->cfg.precision == ARAN_PRECISION_MIXED)
     k_unscale<float><<<ceil_div(t.nnodes, 128), 128, 0, s->s0>>>(
-        t.nnodes, p, t.depth.ptr, s->scale_e, reinterpret_cast<cplx<float> *>(s->mult32.ptr),
-        reinterpret_cast<cplx<float> *>(s->loc32.ptr), om.ptr, ol.ptr);
+        t.nnodes, p, t.depth.ptr, t.sys.ptr, charge_fields(s), s->scale_e,
+        reinterpret_cast<cplx<float> *>(s->mult32.ptr), reinterpret_cast<cplx<float> *>(s->loc32.ptr), om.ptr, ol.ptr);
   else
     k_unscale<double><<<ceil_div(t.nnodes, 128), 128, 0, s->s0>>>(
-        t.nnodes, p, t.depth.ptr, s->scale_e, reinterpret_cast<cplx<double> *>(s->mult64.ptr),
-        reinterpret_cast<cplx<double> *>(s->loc64.ptr), om.ptr, ol.ptr);
+        t.nnodes, p, t.depth.ptr, t.sys.ptr, charge_fields(s), s->scale_e,
+        reinterpret_cast<cplx<double> *>(s->mult64.ptr), reinterpret_cast<cplx<double> *>(s->loc64.ptr), om.ptr, ol.ptr);
   ACHECK(cudaGetLastError());
   if (mult) ACHECK(cudaMemcpyAsync(mult, om.ptr, t.nnodes * nm * 2 * sizeof(double), cudaMemcpyDeviceToHost, s->s0));
   if (local) ACHECK(cudaMemcpyAsync(local, ol.ptr, t.nnodes * nl * 2 * sizeof(double), cudaMemcpyDeviceToHost, s->s0));

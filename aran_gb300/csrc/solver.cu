@@ -42,6 +42,7 @@ void smem_raise(const void *kernel, size_t bytes) {
 // solver's box); skipped when they equal the last solve's
 void set_systems(AranGpuSolver3d *s, int nsys, const int64_t *offs, const double *boxes,
                  int64_t n) {
+  s->err_dev.reserve(1 + (size_t)nsys);
   std::vector<int> off(nsys + 1);
   std::vector<double> box(9 * (size_t)nsys);
   for (int k = 0; k <= nsys; ++k) off[k] = offs ? (int)offs[k] : (k ? (int)n : 0);
@@ -67,13 +68,13 @@ void set_systems(AranGpuSolver3d *s, int nsys, const int64_t *offs, const double
 void build_tree_only(AranGpuSolver3d *s, int64_t n, const double *xyz, const double *q) {
   ACHECK(cudaSetDevice(s->device));
   cudaStream_t st = s->s0;
-  ACHECK(cudaMemsetAsync(s->err_dev.ptr, 0, sizeof(int), st));
+  set_systems(s, 1, nullptr, nullptr, n);
+  ACHECK(cudaMemsetAsync(s->err_dev.ptr, 0, 2 * sizeof(int), st));
   s->io_xyz.reserve(3 * n);
   s->io_q.reserve(n);
   ACHECK(cudaMemcpyAsync(s->io_xyz.ptr, xyz, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
   ACHECK(cudaMemcpyAsync(s->io_q.ptr, q, n * sizeof(double), cudaMemcpyHostToDevice, st));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::SORT], st));
-  set_systems(s, 1, nullptr, nullptr, n);
   build_tree(s, n, s->io_xyz.ptr, s->io_q.ptr);
   ACHECK(cudaStreamSynchronize(st));
   s->have_tree = false;   // no lists: counters and list queries need a solve
@@ -263,7 +264,7 @@ int solve_impl(AranGpuSolver3d *s, int nsys, const int64_t *offs, const double *
     const double *dx = xyz, *dq = q;
     double *dpot = pot, *dfld = field;
     ACHECK(cudaEventRecord(s->ev[2 * Stage::TOTAL], st));
-    ACHECK(cudaMemsetAsync(s->err_dev.ptr, 0, sizeof(int), st));
+    ACHECK(cudaMemsetAsync(s->err_dev.ptr, 0, (1 + (size_t)s->nsys) * sizeof(int), st));
     ACHECK(cudaEventRecord(s->ev[2 * Stage::H2D], st));
     if (mem == ARAN_MEM_HOST) {
       s->io_xyz.reserve(3 * n);

@@ -37,18 +37,35 @@ namespace {
 // Morton keys of the particles, each in its system's box (sys_box: lb[3],
 // ub[3], scale[3] per system; particles of system k are sys_off[k] ..
 // sys_off[k+1]-1); a non-finite coordinate or charge sets kErrNonFinite in
-// the error word (the solve then stops before any output)
+// the error word (the solve then stops before any output).  qmax (mixed precision): see
+// charge_unit
 __global__ void k_keys(int64_t n, const double *__restrict__ xyz, const double *__restrict__ q,
                        int nsys, const int *__restrict__ sys_off,
                        const double *__restrict__ sys_box, uint64_t *__restrict__ keys,
-                       int *__restrict__ idx, int *__restrict__ err) {
+                       int *__restrict__ idx, int *__restrict__ err, int *__restrict__ qmax) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int lo = 0, hi = nsys;   // the last system k with sys_off[k] <= i, in [lo, hi)
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (sys_off[mid] <= i) lo = mid; else hi = mid;
+  if (qmax) {
+    // the largest exponent field of each system's charges: by block where the
+    // block's particles are of one system
+    __shared__ int s_sys, s_max;
+    const int sy = i < n ? system_of(i, nsys, sys_off) : 0;
+    if (threadIdx.x == 0) {
+      s_max = 0;
+      s_sys = sys_off[sy + 1] >= min(n, i + blockDim.x) ? sy : -1;
+    }
+    __syncthreads();
+    const int e = i < n ? (__double2hiint(q[i]) >> 20) & 2047 : 0;
+    if (s_sys < 0) {
+      if (i < n) atomicMax(qmax + sy, e);
+    } else {
+      const int w = __reduce_max_sync(0xffffffffu, e);
+      if ((threadIdx.x & 31) == 0) atomicMax(&s_max, w);
+      __syncthreads();
+      if (threadIdx.x == 0) atomicMax(qmax + s_sys, s_max);
+    }
   }
+  if (i >= n) return;
+  const int lo = system_of(i, nsys, sys_off);
   const double *b = sys_box + 9 * lo;
   const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
   if (!(isfinite(x) && isfinite(y) && isfinite(z) && isfinite(q[i]))) atomicOr(err, kErrNonFinite);
@@ -66,16 +83,17 @@ __global__ void k_keys(int64_t n, const double *__restrict__ xyz, const double *
 }
 
 __global__ void k_gather(int64_t n, const int *__restrict__ perm, const double *__restrict__ xyz,
-                         const double *__restrict__ q, double *__restrict__ sx,
-                         double *__restrict__ sy, double *__restrict__ sz,
-                         double *__restrict__ sq) {
+                         const double *__restrict__ q, int nsys,
+                         const int *__restrict__ sys_off, const int *__restrict__ qmax,
+                         double *__restrict__ sx, double *__restrict__ sy,
+                         double *__restrict__ sz, double *__restrict__ sq) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = perm[i];
   sx[i] = xyz[3 * (int64_t)o];
   sy[i] = xyz[3 * (int64_t)o + 1];
   sz[i] = xyz[3 * (int64_t)o + 2];
-  sq[i] = q[o];
+  sq[i] = qmax ? q[o] * charge_per_unit(qmax[system_of(i, nsys, sys_off)]) : q[o];
 }
 
 struct NodeArrays {
@@ -108,15 +126,6 @@ __global__ void k_roots(NodeArrays na, int nsys, const int *__restrict__ sys_off
 
 __device__ __forceinline__ int shared_digits(uint64_t a, uint64_t b) {
   return a == b ? kKeyBits : (__clzll((long long)(a ^ b)) - 1) / 3;
-}
-
-__device__ __forceinline__ int system_of(int64_t i, int nsys, const int *__restrict__ sys_off) {
-  int lo = 0, hi = nsys;                 // last system with sys_off <= i
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (sys_off[mid] <= i) lo = mid; else hi = mid;
-  }
-  return lo;
 }
 
 // sorted keys for subdivide.cuh
@@ -896,8 +905,9 @@ void build_tree(AranGpuSolver3d *s, int64_t n, const double *d_xyz, const double
   s->keys_out.reserve(n);
   s->idx_in.reserve(n);
   s->perm.reserve(n);
+  int *qmax = charge_fields(s);
   k_keys<<<ceil_div(n, TB), TB, 0, st>>>(n, d_xyz, d_q, nsys, s->sys_off.ptr, s->sys_box.ptr,
-                                          s->keys_in.ptr, s->idx_in.ptr, s->err_dev.ptr);
+                                          s->keys_in.ptr, s->idx_in.ptr, s->err_dev.ptr, qmax);
   s->launches++;
   size_t bytes = 0;
   ACHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, s->keys_in.ptr, s->keys_out.ptr,
@@ -911,8 +921,8 @@ void build_tree(AranGpuSolver3d *s, int64_t n, const double *d_xyz, const double
   s->sy.reserve(n);
   s->sz.reserve(n);
   s->sq.reserve(n);
-  k_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, s->perm.ptr, d_xyz, d_q, s->sx.ptr, s->sy.ptr,
-                                            s->sz.ptr, s->sq.ptr);
+  k_gather<<<ceil_div(n, TB), TB, 0, st>>>(n, s->perm.ptr, d_xyz, d_q, nsys, s->sys_off.ptr, qmax,
+                                            s->sx.ptr, s->sy.ptr, s->sz.ptr, s->sq.ptr);
   s->launches++;
   ACHECK(cudaEventRecord(s->ev[2 * Stage::SORT + 1], st));
 
