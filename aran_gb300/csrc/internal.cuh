@@ -261,6 +261,7 @@ void run_passes(AranGpuSolver3d *s);
 // (mult64/loc64) or FP32 (mult32/loc32)
 void launch_m2l(AranGpuSolver3d *s, bool fp64, int first, int count, cudaStream_t st);
 // m2l_fp64.cu
+constexpr int64_t kM2lFp64PartBytes = 512ll << 20;   // workspace of the segments' sums
 void build_m2l_fp64_tables(OpTables<double> &tb, cudaStream_t st);
 void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStream_t st);
 bool launch_m2l_lanes(AranGpuSolver3d *s, OpTables<float> &tb, const int *parents, int count,

@@ -43,7 +43,6 @@ namespace {
 
 constexpr int kF64Warps = 8;
 constexpr int kF64Segs = 16;
-constexpr size_t kF64PartBytes = 1u << 30;   // workspace of the segments' sums
 
 // first unit of a segment
 __device__ __forceinline__ int seg_unit(int seg, int nunits) {
@@ -455,7 +454,7 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   // order 12, 200k Plummer particles, 16.3 ms against 14.3; 8,155 parents 77.9
   // against 77.0.)
   const size_t per = (size_t)kF64Segs * kF64Warps * nl;     // sums of a parent
-  const int most = (int)(kF64PartBytes / (per * sizeof(cplx<double>)));
+  const int most = (int)(kM2lFp64PartBytes / (int64_t)(per * sizeof(cplx<double>)));
   const int step = ceil_div(count, ceil_div(count, most));
   s->m2l_part64.reserve(2 * per * step);
   const cplx<double> *mult = reinterpret_cast<cplx<double> *>(s->mult64.ptr);

@@ -86,21 +86,48 @@ double plan_for_tolerance(double tol, AranGpuConfig3d *cfg) {
   return table_error(kErrFp64, kPlanMaxOrder);
 }
 
+// operator tables of one precision (tables.cu, m2l_fp64.cu)
+int64_t table_bytes(int p, int64_t real) {
+  int64_t b = real * (343ll * dir_offset(p, 0, 6) + 8ll * dir_offset(p, 1, 6) +
+                      8ll * dir_offset(p, 2, 6) + 4ll * (p + 1) * tri(p + 1));
+  if (real == 8) b += 140ll * 2 * (p + 2) * (p + 2) * (p + 2) * 8;
+  else if (m2l_hk_order(p)) b += 343ll * m2l_hk_stride(p) * 4;
+  return b;
+}
+
+// sums of the M2L's segments: 16 for every FP64 parent, up to m2l_fp64.cu's limit;
+// in FP32 (m2l_lanes.cuh) 16 or 8 for passes of up to two waves of CTAs, else one
+int64_t m2l_sum_bytes(int p, int64_t real, int64_t parents) {
+  if (real == 8) {
+    const int64_t b = parents * 16 * 8 * tri(p + 1) * 16;
+    return b < kM2lFp64PartBytes ? b : kM2lFp64PartBytes;
+  }
+  if (!m2l_hk_order(p)) return 0;
+  const int64_t per = 64ll * (2 * (p / 2 + 1) * (p / 2 + 1) + 15);      // columns of a parent
+  const int64_t most = 2 * 152 * (p <= 4 ? 48 : (p <= 8 ? 32 : (p <= 12 ? 24 : 16)));
+  const int64_t split = per * (parents < most ? parents : most) * (p <= 12 ? 16 : 8);
+  return split > per * parents ? split : per * parents;
+}
+
 int64_t footprint_bytes(const AranGpuConfig3d *c, int64_t n) {
   const int p = c->order;
-  const int64_t real = c->precision == ARAN_PRECISION_MIXED ? 4 : 8;
+  const bool mixed = c->precision == ARAN_PRECISION_MIXED;
+  const int64_t real = mixed ? 4 : 8;
   const int64_t nodes = 16 + (8 * n) / (c->maxbox > 1 ? c->maxbox : 2) + n / 8;
   int64_t b = 0;
   b += n * (3 * 8 + 8);            // staged inputs
   b += n * (4 * 8);                // outputs (pot + field) staged
   b += n * (4 * 8 + 2 * 8 + 8);    // sorted positions/charges, keys (2x), perm/idx
   b += n * (4 * real + 4 * 8);     // relative coordinates, accumulators
+  if (mixed) b += n * 32;          // hi + lo positions
   b += nodes * (8 + 12 + 1 + 16 + 24 + 27 * 4 + 4 * 4 + 8);       // node arrays
-  b += nodes * (int64_t)(tri(p) + 2 * tri(p + 1)) * 2 * real;      // expansions, M2L sums
-  b += n * (8 * real);                                             // hi + lo positions
+  b += nodes * (int64_t)(tri(p) + tri(p + 1)) * 2 * real;          // expansions
   b += nodes * (189 * 6 + 8) + nodes * 60 * 8;                     // far/near lists
-  b += 140ll * 2 * (p + 2) * (p + 2) * (p + 2) * 8;                // FP64 M2L stream tables
-  return b + (64ll << 20);
+  // (trees have half as many nodes or fewer, eight to a parent)
+  int64_t fixed = table_bytes(p, real) + m2l_sum_bytes(p, real, 16 + nodes / 16);
+  if (mixed && p >= 16 && c->flavour != ARAN_FLAVOUR_KKYLIN)       // FP64 root levels
+    fixed += table_bytes(p, 8) + m2l_sum_bytes(p, 8, 72);
+  return b + fixed + fixed / 4 + (64ll << 20);   // (buffers grow by a quarter)
 }
 
 }  // namespace aran
