@@ -61,8 +61,7 @@ struct DBuf {
   size_t cap = 0;
   void reserve(size_t n) {
     if (n <= cap) return;
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
+    release();               // empty too if the allocation fails
     size_t c = n + n / 4 + 64;
     ACHECK(cudaMalloc(&ptr, c * sizeof(T)));
     cap = c;
