@@ -127,9 +127,9 @@ def stage_rooflines(stage_ms: dict, stats: dict, info: dict, n: int, p: int, fp3
 
 
 def m2l_kernel_name(precision: str, p: int, choice: str) -> str:
-    """The M2L kernel a solve runs: choice is ARAN_M2L_KERNEL ("lanes",
-    "sibling", "tc" or empty); a kernel that does not serve the order or the
-    precision hands over to the next in tc, lanes, sibling."""
+    """The M2L kernel a mixed solve runs: choice is ARAN_M2L_KERNEL ("lanes",
+    "sibling", "tc" or empty); a kernel that does not serve the order hands
+    over to the next in tc, lanes, sibling."""
     if precision == "mixed" and p in (6, 10, 14, 16) and choice != "sibling":
         return (f"k_m2l_sibling_lanes<{p}> (rotate M2L, FP32 lane pairs, all levels, one launch "
                 "or one and its parts' sum)")
@@ -139,6 +139,15 @@ def m2l_kernel_name(precision: str, p: int, choice: str) -> str:
         return (f"k_m2l_tc<{p}> (rotate M2L as dense TF32 hi/lo products on tcgen05, "
                 "all levels, one launch)")
     return f"k_m2l_lanes<{p}> (rotate M2L, FP32 lane pairs, all levels, one launch)"
+
+
+def roofline_kernel(precision: str, p: int, choice: str) -> str:
+    """The kernel that the roofline entry describes: FP64 translations have one
+    kernel whatever the choice, mixed ones as m2l_kernel_name says."""
+    if precision == "fp64":
+        return ("k_m2l_fp64 (rotate M2L as dot products dealt to the lanes, all levels, one launch "
+                "and its segments' sum)")
+    return m2l_kernel_name(precision, p, choice)
 
 
 def m2l_flops(p: int) -> int:
@@ -854,7 +863,7 @@ def run_gpu(args):
     real = 4 if args.precision == "mixed" else 8
     alg_bytes = info["nodes"] * (p * (p + 1) // 2 + (p + 1) * (p + 2) // 2) * 2 * real * 2
     # the M2L kernel the library ran
-    m2l_kernel = m2l_kernel_name(args.precision, p, os.environ.get("ARAN_M2L_KERNEL", ""))
+    m2l_kernel = roofline_kernel(args.precision, p, os.environ.get("ARAN_M2L_KERNEL", ""))
     traffic = args.m2l_traffic
     if (traffic is None and args.workload == "plummer4m" and p == 12
             and m2l_kernel.startswith("k_m2l_lanes")):
