@@ -125,6 +125,7 @@ struct DevTree {
   int n_parents = 0;
   int n_big = 0;
   int n_heavy = 0;                    // heavy near ranges (the chunked P2P pass)
+  int max_leaf = 0;                   // no leaf holds more particles
   int64_t n_far = 0;
   bool far_counted = false;           // far_off and n_far made (count_far_lists)
   bool far_built = false;             // far_src/far_dir written (build_far_lists)
@@ -228,7 +229,7 @@ struct AranGpuSolver3d {
   aran::DBuf<float> tc_tab;
   aran::DBuf<int8_t> tc_dvec;
   int tc_p = -1;
-  // sums of the segments (lane-parallel FP32) or parts (FP64) of an M2L pass
+  // sums of the segments of an M2L pass (FP64: before it of the P2M)
   aran::DBuf<float> m2l_part;
   aran::DBuf<double> m2l_part64;
   aran::DBuf<int> sys_off;

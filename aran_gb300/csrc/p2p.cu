@@ -20,6 +20,8 @@
 // the FP64 positions.
 #include <cub/cub.cuh>
 
+#include <algorithm>
+
 #include "internal.cuh"
 #include "f32x2.cuh"
 
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(128, 8) k_p2p64(
   const int nt = tbe.y - tbe.x;
   const int r0 = BIG ? 0 : near_off[L], r1 = BIG ? 1 : near_off[L + 1];
   const long long guard = __double_as_longlong(FIELD ? 1e-10 : 0.);
-  for (int tb = 0; tb < nt; tb += 128) {
+  for (int tb = blockIdx.y * 128; tb < nt; tb += 128 * gridDim.y) {
     const int rem = min(nt - tb, 128);
     const int s = 128 / rem;                  // threads per target
     const int ti = threadIdx.x / s, sub = threadIdx.x - ti * s;
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(128, 8) k_p2p64(
 // pairs: a leaf of n targets gets floor(T / n) threads per target, so the
 // lanes are busy whatever n is.  The pair loop has no branch: pairs closer
 // than h/8 (and the point itself) are left out, and a thread whose part held
-// one adds those pairs from the FP64 positions afterwards.  Up to RUN pairs are
+// one adds those pairs from the FP64 positions afterwards.  Up to 22 pairs are
 // summed plainly, the runs in Kahan sums (one run a tile, 128 pairs, was 6 to 10 %
 // faster on leaves of 40 points and more, with three times the rounding error
 // of a warp per leaf's runs of up to 32 sources; shorter runs where leaves, and with
@@ -255,7 +257,6 @@ __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
     const real4<float> *__restrict__ rel32, const float4 *__restrict__ phi,
     const float4 *__restrict__ plo, double *__restrict__ acc_pot, double *__restrict__ acc_fld) {
   constexpr int NV = FIELD ? 4 : 1;
-  constexpr int RUN = T == 64 ? 8 : 22;           // pairs summed plainly
   // pair p of the tile: (-x0, -x1, -y0, -y1) and (-z0, -z1, q0, q1)
   __shared__ ulonglong2 tA[T], tB[T];
   __shared__ int tj[2 * T];                       // their particles
@@ -274,9 +275,10 @@ __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
   const float4 tch = chi[L], tcl = clo[L];
   const float thr2 = FIELD ? fmaxf(tch.w, 1e-10f) : tch.w;
   const int r0 = BIG ? 0 : near_off[L], r1 = BIG ? 1 : near_off[L + 1];
-  for (int tb = 0; tb < nt; tb += T) {
+  for (int tb = blockIdx.y * T; tb < nt; tb += T * gridDim.y) {
     const int rem = min(nt - tb, T);
     const int S = T / rem;                        // threads per target
+    const int run = T == 64 && rem <= 24 ? 8 : 22;   // pairs summed plainly
     // target by target within a part, so that a warp reads few pairs at a time
     const int sub = threadIdx.x / rem, ti = threadIdx.x - sub * rem;
     const bool active = sub < S;
@@ -345,8 +347,8 @@ __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
         __syncthreads();
         if (active) {
           unsigned close = 0;   // 1 + pair of the last close pair, above it the one before
-          for (int p0 = sub; p0 < np; p0 += RUN * S) {
-            const int p1 = min(np, p0 + RUN * S);
+          for (int p0 = sub; p0 < np; p0 += run * S) {
+            const int p1 = min(np, p0 + run * S);
             uint64_t p2[NV];
 #pragma unroll
             for (int c = 0; c < NV; ++c) p2[c] = 0ull;
@@ -443,6 +445,14 @@ __global__ void __launch_bounds__(T, 1280 / T) k_p2p_tile(
   }
 }
 
+// A leaf above the capacity (depth limit, leaf predicate) goes to several blocks, T
+// targets at a time; not too many, as most leaves have none for them.  6,000
+// coincident points in one leaf at capacity 16: mixed 7.3 ms, 208 with one block of
+// 64 threads (104 with a warp per leaf and chunks of 128 threads), FP64 11 ms, 83.
+int leaf_tiles(const DevTree &t, int T) {
+  return std::min({ceil_div(t.max_leaf, T), 2048 / T, 1 + 100000 / t.nleaves});
+}
+
 template <bool FIELD>
 void launch_mixed(AranGpuSolver3d *s, cudaStream_t st) {
   DevTree &t = s->tree;
@@ -453,8 +463,9 @@ void launch_mixed(AranGpuSolver3d *s, cudaStream_t st) {
   // its company in a forest.)
   const bool small = s->cfg.maxbox <= 24;
   const int T = small ? 64 : 128;
+  const int tiles = leaf_tiles(t, T);
   auto run = [&](auto kern, int grid) {
-    kern<<<grid, T, 0, st>>>(
+    kern<<<dim3(grid, tiles), T, 0, st>>>(
         t.big_items.ptr, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, t.leaf_chi.ptr,
         t.leaf_clo.ptr, s->sx.ptr, s->sy.ptr, s->sz.ptr, s->rel32.ptr, s->abs_hi.ptr,
         s->abs_lo.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
@@ -468,7 +479,7 @@ void launch_mixed(AranGpuSolver3d *s, cudaStream_t st) {
 template <bool FIELD, bool BIG>
 void launch_fp64(AranGpuSolver3d *s, int grid, cudaStream_t st) {
   DevTree &t = s->tree;
-  k_p2p64<FIELD, BIG><<<grid, 128, 0, st>>>(
+  k_p2p64<FIELD, BIG><<<dim3(grid, leaf_tiles(t, 128)), 128, 0, st>>>(
       t.big_items.ptr, t.near_off.ptr, t.near_rng.ptr, t.leaf_be.ptr, s->sx.ptr, s->sy.ptr,
       s->sz.ptr, s->sq.ptr, s->acc_pot.ptr, s->acc_fld.ptr);
   ACHECK(cudaGetLastError());

@@ -412,6 +412,8 @@ __device__ __forceinline__ bool adjacent_ml(const int *ijk, const uint8_t *depth
 // totals that the host reads after the counting pass
 struct NearTotals {
   int chunks, heavy;
+  int over;             // particles of the largest leaf above the capacity (depth limit,
+                        // leaf predicate), 0 if there is none
 };
 
 // chunks of a range of c points in the chunked P2P pass, 0 if it is not heavy
@@ -435,8 +437,9 @@ __global__ void k_near_warp(int nbound, const int *__restrict__ nleaves_p,
                             const int *__restrict__ parent, const int *__restrict__ col,
                             const int *__restrict__ ncol, const int *__restrict__ lf_begin,
                             const int *__restrict__ lf_end, int *__restrict__ near_cnt,
-                            NearTotals *__restrict__ tot, const int *__restrict__ near_off,
-                            int *__restrict__ near_rng, int *__restrict__ big) {
+                            int maxbox, NearTotals *__restrict__ tot,
+                            const int *__restrict__ near_off, int *__restrict__ near_rng,
+                            int *__restrict__ big) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int L = (int)(g >> 5), lane = (int)(g & 31);
   if (L >= nbound) return;
@@ -445,6 +448,7 @@ __global__ void k_near_warp(int nbound, const int *__restrict__ nleaves_p,
     return;
   }
   int a = leaf_node[L];
+  if (!WRITE && lane == 0 && end[a] - begin[a] > maxbox) atomicMax(&tot->over, end[a] - begin[a]);
   int k = WRITE ? near_off[L] : 0;
   int chunks = 0, heavy = 0;
   bool own = true;
@@ -509,7 +513,7 @@ __global__ void k_near(int nbound, const int *__restrict__ nleaves_p,
                        const uint8_t *__restrict__ depth, int T, int *__restrict__ near_cnt,
                        const int *__restrict__ near_off, int *__restrict__ near_rng,
                        int *__restrict__ semi_cnt, const int *__restrict__ semi_off,
-                       int *__restrict__ semi_node, int *__restrict__ semi_leaf,
+                       int *__restrict__ semi_node, int *__restrict__ semi_leaf, int maxbox,
                        NearTotals *__restrict__ tot, int *__restrict__ big, int mode) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= nbound) return;
@@ -518,6 +522,7 @@ __global__ void k_near(int nbound, const int *__restrict__ nleaves_p,
     return;
   }
   int node = leaf_node[L];
+  if (!mode && end[node] - begin[node] > maxbox) atomicMax(&tot->over, end[node] - begin[node]);
   int k = 0, ks = 0;
   int w = mode ? near_off[L] : 0;
   int ws = mode ? semi_off[L] : 0;
@@ -1044,7 +1049,7 @@ void build_lists(AranGpuSolver3d *s) {
   const int T = s->cfg.semifar_threshold;
   t.near_off.reserve(nlb + 1);
   if (T > 0) t.semi_off.reserve(nlb + 1);
-  cntbuf.reserve(2 * ((size_t)nlb + 1) + 2);
+  cntbuf.reserve(2 * ((size_t)nlb + 1) + sizeof(NearTotals) / sizeof(int));
   int *semi_cnt = cntbuf.ptr + nlb + 1;
   NearTotals *tot = reinterpret_cast<NearTotals *>(semi_cnt + nlb + 1);
   ACHECK(cudaMemsetAsync(cntbuf.ptr + nlb, 0, sizeof(int), st));
@@ -1055,13 +1060,13 @@ void build_lists(AranGpuSolver3d *s) {
           nlb, nleaves_p, t.leaf_node.ptr, t.begin.ptr, t.end.ptr, t.child.ptr, t.parent.ptr,
           t.col.ptr, t.ncol.ptr, t.lf_begin.ptr, t.lf_end.ptr, t.ijk.ptr, t.depth.ptr, T,
           cntbuf.ptr, t.near_off.ptr, t.near_rng.ptr, semi_cnt, t.semi_off.ptr, t.semi_node.ptr,
-          t.semi_leaf.ptr, tot, t.big_rng.ptr, write);
+          t.semi_leaf.ptr, s->cfg.maxbox, tot, t.big_rng.ptr, write);
     } else {
       auto kern = write ? k_near_warp<true> : k_near_warp<false>;
       kern<<<ceil_div(32 * (int64_t)nlb, TB), TB, 0, st>>>(
           nlb, nleaves_p, t.leaf_node.ptr, t.begin.ptr, t.end.ptr, t.child.ptr, t.parent.ptr,
-          t.col.ptr, t.ncol.ptr, t.lf_begin.ptr, t.lf_end.ptr, cntbuf.ptr, tot, t.near_off.ptr,
-          t.near_rng.ptr, t.big_rng.ptr);
+          t.col.ptr, t.ncol.ptr, t.lf_begin.ptr, t.lf_end.ptr, cntbuf.ptr, s->cfg.maxbox, tot,
+          t.near_off.ptr, t.near_rng.ptr, t.big_rng.ptr);
     }
     ACHECK(cudaGetLastError());
     s->launches++;
@@ -1082,6 +1087,7 @@ void build_lists(AranGpuSolver3d *s) {
   const int nrng = hb[4], nsemi = hb[5];
   t.n_big = hb[8];
   t.n_heavy = hb[9];
+  t.max_leaf = std::max(s->cfg.maxbox, hb[10]);
   t.n_near_rng = nrng;
   t.n_semi = nsemi;
   t.near_rng.reserve(2 * (size_t)nrng + 2);
