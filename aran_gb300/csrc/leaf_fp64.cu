@@ -15,26 +15,30 @@ __device__ __forceinline__ double leaf_inv_scale(int depth, double scale_e) {
   return ldexp(1.0, depth) / scale_e;    // 1/h_d = 2^d / 2^E (exact power of two)
 }
 
-// P2M, a warp per run of leaves: those that start in the warp's span of kSpan
-// sorted particles, taken 32 particles at a time whatever leaves they lie in (a
+// P2M.  A leaf's particles are taken in segments of 32 from its first on, and a
+// leaf's sum is the sum of its segments in order (k_p2m64_sum), each added up
+// particle by particle: what else is solved, and with it the leaf's place among the
+// sorted particles, does not change its bits.  A warp takes the segments that start
+// in its kSpan places, 32 particles at a time whatever segments they lie in (a
 // warp per leaf keeps as many lanes busy as the leaf has points).  A lane makes
 // its particle's q S_l^m in m-major order (six operations a coefficient) into
 // shared memory; every 32 values the lanes turn to the values, a lane one of them,
-// and add it up particle by particle (one addition a value and particle; by
-// shuffles over the warp it was five on every lane).  A leaf's sum is that of
-// its segments of 32 particles, each added up from its first particle: what else
-// is solved, and with it the leaf's place in a span, does not change its bits.
-// 200k Plummer particles (18 a leaf), order 12: 0.51 ms, 1.44 with a warp per
-// leaf and shuffles (0.34 with the parts of a leaf added as they come, the whole
-// solve 38.1 ms either way); 10k 0.12 ms, 0.15 and 0.23 with spans of 64 and 128.
-constexpr int kSpan = 32;
+// and add it up (one addition a value and particle; by shuffles over the warp it was
+// five on every lane).  The first segment of a leaf goes to its multipole, the
+// others to a workspace, at the window of 32 places in which they start: no two start
+// in one.  With few segments (segs > 0) a warp takes one, segment u mod segs of leaf
+// u / segs: fewer rounds in turn, and few CTAs, which stay clear of the near
+// field's.  200k Plummer particles (18 a leaf), order 12: 0.48 ms, 1.44 with a warp per
+// leaf and shuffles (0.34 with parts of leaves added as they come; the solve 38.1
+// ms either way); 3k particles (order 12) 0.045 ms.
+constexpr int kSpan = 32, kFewSegs = 4096;
 
 __global__ void __launch_bounds__(32 * kWarps)
-    k_p2m64(int64_t n, int nleaves, const int *__restrict__ win_leaf,
+    k_p2m64(int64_t n, int nleaves, int segs, const int *__restrict__ win_leaf,
             const int2 *__restrict__ leaf_be, const int *__restrict__ leaf_node,
             const uint8_t *__restrict__ depth, const real4<double> *__restrict__ rel, int p,
             const double *__restrict__ rec_g, const double *__restrict__ p2mf_g, double scale_e,
-            double *__restrict__ mult) {
+            double *__restrict__ mult, double *__restrict__ more) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nm = tri(p);
   double *rec = reinterpret_cast<double *>(smem_raw);   // (c0, c1) by (l, m)
@@ -52,23 +56,43 @@ __global__ void __launch_bounds__(32 * kWarps)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   buf += w * (32 * 33 + 2 * nm);
   double *carry = buf + 32 * 33;           // sums of a segment that goes on
-  // first leaf that starts at or behind a place (a multiple of 32)
-  auto leaf_from = [&](int64_t at) -> int {
-    if (at >= n) return nleaves;
-    const int L = win_leaf[at >> 5];
-    return leaf_be[L].x < at ? L + 1 : L;
+  // first segment that starts at or behind a place: its leaf and its own place (the
+  // whole warp asks)
+  auto segment_from = [&](int64_t at, int &leaf) -> int {
+    leaf = nleaves;
+    if (at >= n) return (int)n;
+    const int L = win_leaf[at >> 5];     // of the place's window of 32
+    leaf = L + __popc(__ballot_sync(kFull, L + lane < nleaves &&
+                                               leaf_be[min(L + lane, nleaves - 1)].x < at));
+    if (leaf > L) {                      // the place may lie inside the leaf before
+      const int2 be = leaf_be[leaf - 1];
+      const int64_t next = be.x + ((at - be.x + 31) & ~(int64_t)31);
+      if (next < be.y) {
+        --leaf;
+        return (int)next;
+      }
+    }
+    return leaf < nleaves ? leaf_be[leaf].x : (int)n;
   };
-  const int64_t span = blockIdx.x * (int64_t)kWarps + w;
-  int L0 = leaf_from(kSpan * span);        // leaf of the round's first particle
-  const int L1 = leaf_from(kSpan * (span + 1));
-  if (L0 >= L1) return;
-  const int stop = leaf_be[L1 - 1].y;
-  bool goes_on = false;                    // L0 began in a round before
-  for (int base = leaf_be[L0].x; base < stop; base += 32) {
+  const int64_t u = blockIdx.x * (int64_t)kWarps + w;
+  int L0, base, stop;                      // L0: leaf of the round's first particle
+  if (segs > 0) {
+    L0 = (int)(u / segs);
+    if (L0 >= nleaves) return;
+    const int2 be = leaf_be[L0];
+    base = be.x + 32 * (int)(u - (int64_t)L0 * segs);
+    stop = min(base + 32, be.y);
+  } else {
+    int L1;
+    base = segment_from(kSpan * u, L0);
+    stop = segment_from(kSpan * (u + 1), L1);
+  }
+  bool goes_on = false;                    // its segment began in a round before
+  for (; base < stop; base += 32) {
     const int cnt = min(stop - base, 32);
     // bit i: particle base + i starts a leaf, a segment (never the first)
     unsigned bit = 0;
-    if (lane > 0 && L0 + lane < L1) {
+    if (lane > 0 && L0 + lane < nleaves) {
       const int at = leaf_be[L0 + lane].x - base;
       if (at < cnt) bit = 1u << at;
     }
@@ -109,9 +133,10 @@ __global__ void __launch_bounds__(32 * kWarps)
           const int2 be = leaf_be[l];
           const bool last = base + j == be.y;
           if (last || ((base + j - be.x) & 31) == 0) {   // a segment ends
-            double *out = mult + 2 * (size_t)nm * leaf_node[l] + c;
-            if (base + j - be.x > 32) sum = *out + sum;
-            *out = last ? f * sum : sum;
+            const int k0 = (base + j - 1 - be.x) & ~31;    // its place in the leaf
+            double *out = k0 == 0 ? mult + 2 * (size_t)nm * leaf_node[l]
+                                  : more + 2 * (size_t)nm * ((be.x + k0) >> 5);
+            out[c] = f * sum;
             sum = 0.;
             if (last) ++l;
           }
@@ -143,8 +168,28 @@ __global__ void __launch_bounds__(32 * kWarps)
       }
     }
     L0 += __popc(starts);
-    goes_on = leaf_be[L0].y != base + cnt;
-    if (!goes_on) ++L0;
+    const int2 be = leaf_be[L0];
+    goes_on = ((base + cnt - be.x) & 31) != 0 && be.y != base + cnt;
+    if (be.y == base + cnt) ++L0;
+  }
+}
+
+// the segments of leaves of more than 32 particles in order, 32 threads per leaf, 128
+// where there are many values
+__global__ void __launch_bounds__(128)
+    k_p2m64_sum(int nleaves, int per, const int2 *__restrict__ leaf_be,
+                const int *__restrict__ leaf_node, int nv, const double *__restrict__ more,
+                double *__restrict__ mult) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int L = (int)(g / per);
+  if (L >= nleaves) return;
+  const int2 be = leaf_be[L];
+  if (be.y - be.x <= 32) return;
+  double *out = mult + (size_t)nv * leaf_node[L];
+  for (int c = (int)(g - (int64_t)L * per); c < nv; c += per) {
+    double v = out[c];
+    for (int at = be.x + 32; at < be.y; at += 32) v += more[(size_t)nv * (at >> 5) + c];
+    out[c] = v;
   }
 }
 
@@ -265,11 +310,23 @@ void launch_p2m64(AranGpuSolver3d *s, cudaStream_t st) {
   const size_t sm = (size_t)3 * nm * sizeof(double) + ((nm + 1) & ~1) * sizeof(int) +
                     (size_t)kWarps * (32 * 33 + 2 * nm) * sizeof(double);
   smem_opt_in(k_p2m64, sm);
-  k_p2m64<<<ceil_div((t.n + kSpan - 1) / kSpan, kWarps), 32 * kWarps, sm, st>>>(
-      t.n, t.nleaves, t.win_leaf.ptr, t.leaf_be.ptr, t.leaf_node.ptr, t.depth.ptr, s->rel64.ptr, p,
-      tb.rec.ptr, tb.p2mf.ptr, s->scale_e, s->mult64.ptr);
+  s->m2l_part64.reserve(2 * (size_t)nm * ceil_div(t.n, 32));   // free until the M2L
+  // few segments: a warp each, in few CTAs, which stay clear of the near field's
+  const int per_leaf = ceil_div(t.max_leaf, 32);
+  const bool few = t.nleaves * (int64_t)per_leaf <= kFewSegs;
+  const int64_t warps = few ? t.nleaves * (int64_t)per_leaf : ceil_div(t.n, kSpan);
+  k_p2m64<<<ceil_div(warps, kWarps), 32 * kWarps, sm, st>>>(
+      t.n, t.nleaves, few ? per_leaf : 0, t.win_leaf.ptr, t.leaf_be.ptr, t.leaf_node.ptr, t.depth.ptr,
+      s->rel64.ptr, p, tb.rec.ptr, tb.p2mf.ptr, s->scale_e, s->mult64.ptr, s->m2l_part64.ptr);
   ACHECK(cudaGetLastError());
   s->launches++;
+  if (t.max_leaf > 32) {
+    const int per = nm > 64 ? 128 : 32;
+    k_p2m64_sum<<<ceil_div(t.nleaves * (int64_t)per, 128), 128, 0, st>>>(
+        t.nleaves, per, t.leaf_be.ptr, t.leaf_node.ptr, 2 * nm, s->m2l_part64.ptr, s->mult64.ptr);
+    ACHECK(cudaGetLastError());
+    s->launches++;
+  }
 }
 
 void launch_l2p64(AranGpuSolver3d *s, cudaStream_t st) {

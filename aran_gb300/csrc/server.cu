@@ -124,7 +124,10 @@ int64_t footprint_bytes(const AranGpuConfig3d *c, int64_t n) {
   b += nodes * (int64_t)(tri(p) + tri(p + 1)) * 2 * real;          // expansions
   b += nodes * (189 * 6 + 8) + nodes * 60 * 8;                     // far/near lists
   // (trees have half as many nodes or fewer, eight to a parent)
-  int64_t fixed = table_bytes(p, real) + m2l_sum_bytes(p, real, 16 + nodes / 16);
+  int64_t sums = m2l_sum_bytes(p, real, 16 + nodes / 16);
+  const int64_t segments = mixed ? 0 : (n / 32 + 1) * 16 * tri(p);   // the P2M's, same buffer
+  if (sums < segments) sums = segments;
+  int64_t fixed = table_bytes(p, real) + sums;
   if (mixed && p >= 16 && c->flavour != ARAN_FLAVOUR_KKYLIN)       // FP64 root levels
     fixed += table_bytes(p, 8) + m2l_sum_bytes(p, 8, 72);
   return b + fixed + fixed / 4 + (64ll << 20);   // (buffers grow by a quarter)
