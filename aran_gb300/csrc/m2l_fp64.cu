@@ -22,10 +22,10 @@
 //    of a parent) read the same table at about the same time.  Tables are
 //    streamed from L2 in the order the lanes use them: [round][step][lane].
 //
-// A target's sum is the sum of kF64Segs segments of the units (offsets or pairs):
-// a CTA takes one segment of a parent and leaves its sum in a workspace, the
-// segments are added in order.  So a system's bits do not depend on what else is
-// solved, as they did when passes with few parents alone were split.
+// A target's sum is the sum of fixed segments of the units (offsets or pairs), each
+// summed on its own and added in order, so a system's bits do not depend on what else
+// is solved.  In passes of few parents a CTA takes one segment of a parent and
+// leaves its sum in a workspace, in passes of many it takes them all.
 // Measured on GB300 against the sibling kernel in FP64: 200k Plummer particles
 // at order 12, the whole solve with the near field beside it on the same pipe,
 // 40.2 ms, 48.4 before (42.0 with two CTAs an SM); eight served requests, two of
@@ -33,6 +33,7 @@
 // leaf_fp64.cu).  60k Plummer particles, this kernel alone: 3.8 ms, the FP64 pipe
 // active 92 % of the cycles.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -42,7 +43,7 @@ namespace aran {
 namespace {
 
 constexpr int kF64Warps = 8;
-constexpr int kF64Segs = 16;
+constexpr int kF64Segs = 16;               // segments of the units
 
 // first unit of a segment
 __device__ __forceinline__ int seg_unit(int seg, int nunits) {
@@ -181,8 +182,9 @@ __host__ __device__ inline int m2l_fp64_warp(int p, int mode) {
   return m2l_fp64_a(p, mode) + (mode != kF64Single && 4 * nm > 2 * nl ? 4 * nm : 2 * nl);
 }
 
-// R rounds of 32 lanes over the tri(p+1) local coefficients
-template <int R>
+// R rounds of 32 lanes over the tri(p+1) local coefficients.  WHOLE: a CTA takes all
+// segments, adding them up in the locals; else segment blockIdx.y
+template <int R, bool WHOLE>
 __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
     k_m2l_fp64(int nparents, int nunits, int mode, const int *__restrict__ parents,
                const int *__restrict__ child, const int *__restrict__ begin,
@@ -193,7 +195,8 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
                const unsigned *__restrict__ units, const double *__restrict__ tabs,
                const double *__restrict__ dir, int dstride, int ph_off,
                const uint8_t *__restrict__ lm, double scale_e,
-               const cplx<double> *__restrict__ mult, cplx<double> *__restrict__ parts) {
+               const cplx<double> *__restrict__ mult, cplx<double> *__restrict__ loc,
+               cplx<double> *__restrict__ parts, uint8_t *__restrict__ marks) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int grid[216];
   const int nm = tri(p), nl = tri(p + 1);
@@ -235,12 +238,44 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
   cplx<double> acc[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) acc[r] = cmake(0., 0.);
-  const int seg = blockIdx.y, u1 = seg_unit(seg + 1, nunits);
-  for (int u = seg_unit(seg, nunits); u < u1; ++u) {
+  bool any = false;                        // the segment has a source
+  // a segment's sum: onto the local, zero before the pass (up to order 6 kept in
+  // registers: one round), or to its place in the workspace with a mark that it is
+  // there
+  const double ih = ldexp(1.0, depth[t]) / scale_e;
+  cplx<double> total = cmake(0., 0.);
+  auto finish = [&](int seg) {
+    const size_t at = ((size_t)seg * nparents + pb) * kF64Warps + w;
+    if (!WHOLE && lane == 0) marks[at] = any;
+    if (!any) return;
+    cplx<double> *out = WHOLE ? loc + (size_t)t * nl : parts + at * nl;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int k = lane + 32 * r;
+      if (k < nl) {
+        const int l = lm[2 * k], m = lm[2 * k + 1];
+        const bool sg = ((bz & (l + m)) ^ (bx & m)) & 1, cj = bx ^ by;
+        const cplx<double> v = cmake(flip(acc[r].re * ih, sg), flip(acc[r].im * ih, sg ^ cj));
+        if (WHOLE && R == 1) total = cadd(total, v);
+        else out[k] = WHOLE ? cadd(out[k], v) : v;
+        if (WHOLE) acc[r] = cmake(0., 0.);
+      }
+    }
+    any = false;
+  };
+  int seg = WHOLE ? 0 : blockIdx.y, u = seg_unit(seg, nunits);
+  int next = seg_unit(seg + 1, nunits);
+  for (;; ++u) {
+    if (u == next) {
+      finish(seg);
+      if (!WHOLE || ++seg == kF64Segs) break;
+      next = seg_unit(seg + 1, nunits);
+    }
     const unsigned code = units[u];
     const int a = code & 7, b = (code >> 3) & 7, c = (code >> 6) & 7;
     int s0 = source_of(a, b, c), s1 = (code & 512u) ? source_of(6 - a, 6 - b, 6 - c) : -1;
     if (s0 < 0 && s1 < 0) continue;
+    any = true;
     // the opposite source alone: its terms with (-1)^l, odd degrees negated;
     // a pair taken singly: one after the other
     const bool both = s0 >= 0 && s1 >= 0;
@@ -354,33 +389,27 @@ __global__ void __launch_bounds__(32 * kF64Warps, R <= 5 ? 3 : 2)
       __syncwarp();
     }
   }
-  const double ih = ldexp(1.0, depth[t]) / scale_e;
-  cplx<double> *out = parts + (((size_t)seg * nparents + pb) * kF64Warps + w) * nl;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int k = lane + 32 * r;
-    if (k < nl) {
-      const int l = lm[2 * k], m = lm[2 * k + 1];
-      const bool sg = ((bz & (l + m)) ^ (bx & m)) & 1, cj = bx ^ by;
-      out[k] = cmake(flip(acc[r].re * ih, sg), flip(acc[r].im * ih, sg ^ cj));
-    }
-  }
+  if (WHOLE && R == 1 && lane < nl) loc[(size_t)t * nl + lane] = total;
 }
 
-// the segments added in order, one warp per child
+// the segments added in order onto the locals (zero before the pass), one warp per
+// child
 __global__ void __launch_bounds__(32 * kF64Warps)
-    k_m2l_parts_sum(int nparents, const int *__restrict__ parents,
-                    const int *__restrict__ child, const int *__restrict__ begin,
-                    const int *__restrict__ end, int nl, const cplx<double> *__restrict__ parts,
+    k_m2l_parts_sum(int nparents, const int *__restrict__ parents, const int *__restrict__ child,
+                    const int *__restrict__ begin, const int *__restrict__ end, int nl,
+                    const cplx<double> *__restrict__ parts, const uint8_t *__restrict__ marks,
                     cplx<double> *__restrict__ loc) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int t = child[parents[blockIdx.x]] + w;
   if (end[t] <= begin[t]) return;
-  const size_t step = (size_t)nparents * kF64Warps * nl;
-  const cplx<double> *p = parts + ((size_t)blockIdx.x * kF64Warps + w) * nl;
+  const size_t step = (size_t)nparents * kF64Warps, at = (size_t)blockIdx.x * kF64Warps + w;
+  const bool there = lane < kF64Segs && marks[lane < kF64Segs ? lane * step + at : 0];
+  const unsigned segs = __ballot_sync(0xffffffffu, there);
+  if (segs == 0) return;
   for (int c = lane; c < nl; c += 32) {
-    cplx<double> v = cmake(0., 0.);
-    for (int k = 0; k < kF64Segs; ++k) v = cadd(v, p[k * step + c]);
+    cplx<double> v = loc[(size_t)t * nl + c];
+    for (unsigned m = segs; m; m &= m - 1)
+      v = cadd(v, parts[((__ffs(m) - 1) * step + at) * nl + c]);
     loc[(size_t)t * nl + c] = v;
   }
 }
@@ -425,9 +454,10 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
   OpTables<double> &tb = s->t64;
   const M2lFp64Tables &f = tb.m2l64;
   const int p = s->cfg.order, nm = tri(p), nl = tri(p + 1);
-  int dev_smem = 0, sm_smem = 0;
+  int dev_smem = 0, sm_smem = 0, nsm = 0;
   ACHECK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
   ACHECK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
+  ACHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
   // Pairs, made at once (16 warps an SM or more up to order 20); read twice where
   // that keeps 16 warps (orders 21 to 23): order 22, 60k Plummer particles, M2L 44
   // ms, 71 made at once, 50 singly; 2 to 3 % slower below.  Above, read twice by
@@ -449,34 +479,58 @@ void launch_m2l_fp64(AranGpuSolver3d *s, const int *parents, int count, cudaStre
     mode = kF64Single;
   }
   const size_t sm = bytes(nw, mode);
-  // As many parents at a time as the workspace holds.  (One CTA for all segments of a
-  // parent, adding them up as it goes, takes as long or longer: 1,574 parents of
-  // order 12, 200k Plummer particles, 16.3 ms against 14.3; 8,155 parents 77.9
-  // against 77.0.)
-  const size_t per = (size_t)kF64Segs * kF64Warps * nl;     // sums of a parent
-  const int most = (int)(kM2lFp64PartBytes / (int64_t)(per * sizeof(cplx<double>)));
-  const int step = ceil_div(count, ceil_div(count, most));
-  s->m2l_part64.reserve(2 * per * step);
+  // A CTA per segment where one per parent would leave the last wave of CTAs a large
+  // part of the pass: 176 parents of order 12 1.28 ms, 3.1 with a CTA for all
+  // segments, 1,574 14.3 and 16.1, 3,941 36.7 and 37.6; forests of small systems,
+  // whose parents have few sources for a CTA's set-up, the other way about from fewer
+  // on: 2,500 parents in 300 systems, order 16, 24.9 and 19.3 ms, 21,600 in
+  // 300 319 and 291, 2,880 in 40 42.6 either way, 335 in 40 3.5 either way.
+  const bool whole = count > 24 * nsm || (count > 8 * nsm && count < 32 * (int64_t)s->nsys);
+  const size_t per = (size_t)kF64Segs * kF64Warps;         // segments' sums of a parent
+  int step = count;
+  cplx<double> *parts = nullptr;
+  uint8_t *marks = nullptr;
+  if (!whole) {
+    // as many parents at a time as the workspace holds
+    const int most = (int)(kM2lFp64PartBytes / (int64_t)(per * nl * sizeof(cplx<double>)));
+    step = ceil_div(count, ceil_div(count, most));
+    s->m2l_part64.reserve(per * step * (2 * nl + 1));
+    parts = reinterpret_cast<cplx<double> *>(s->m2l_part64.ptr);
+    marks = reinterpret_cast<uint8_t *>(parts + per * step * nl);
+  }
   const cplx<double> *mult = reinterpret_cast<cplx<double> *>(s->mult64.ptr);
   cplx<double> *loc = reinterpret_cast<cplx<double> *>(s->loc64.ptr);
-  cplx<double> *parts = reinterpret_cast<cplx<double> *>(s->m2l_part64.ptr);
-  auto kern = nl <= 96 ? k_m2l_fp64<3>
-                       : (nl <= 160 ? k_m2l_fp64<5> : (nl <= 256 ? k_m2l_fp64<8> : k_m2l_fp64<16>));
-  smem_opt_in(kern, sm);
-  for (int first = 0; first < count; first += step) {
-    const int cnt = std::min(step, count - first);
-    kern<<<dim3(cnt * (kF64Warps / nw), kF64Segs), 32 * nw, sm, st>>>(
-        cnt, f.nunits, mode, parents + first, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
-        t.ncol.ptr, t.ijk.ptr, t.depth.ptr, p, f.sched,
-        reinterpret_cast<const F64Task *>(f.task.ptr), f.trip.ptr, f.units.ptr, f.tabs.ptr,
-        tb.dir_m2l.ptr, dir_offset(p, 0, 6), dir_offset(p, 0, 4), tb.lm.ptr, s->scale_e, mult,
-        parts);
-    ACHECK(cudaGetLastError());
-    k_m2l_parts_sum<<<cnt, 32 * kF64Warps, 0, st>>>(cnt, parents + first, t.child.ptr, t.begin.ptr,
-                                                    t.end.ptr, nl, parts, loc);
-    ACHECK(cudaGetLastError());
-    s->launches += 2;
-  }
+  auto run = [&](auto kern) {
+    smem_opt_in(kern, sm);
+    for (int first = 0; first < count; first += step) {
+      const int cnt = std::min(step, count - first);
+      kern<<<dim3(cnt * (kF64Warps / nw), whole ? 1 : kF64Segs), 32 * nw, sm, st>>>(
+          cnt, f.nunits, mode, parents + first, t.child.ptr, t.begin.ptr, t.end.ptr, t.col.ptr,
+          t.ncol.ptr, t.ijk.ptr, t.depth.ptr, p, f.sched,
+          reinterpret_cast<const F64Task *>(f.task.ptr), f.trip.ptr, f.units.ptr, f.tabs.ptr,
+          tb.dir_m2l.ptr, dir_offset(p, 0, 6), dir_offset(p, 0, 4), tb.lm.ptr, s->scale_e, mult,
+          loc, parts, marks);
+      ACHECK(cudaGetLastError());
+      s->launches++;
+      if (!whole) {
+        k_m2l_parts_sum<<<cnt, 32 * kF64Warps, 0, st>>>(cnt, parents + first, t.child.ptr,
+                                                        t.begin.ptr, t.end.ptr, nl, parts, marks,
+                                                        loc);
+        ACHECK(cudaGetLastError());
+        s->launches++;
+      }
+    }
+  };
+  auto pick = [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    if (whole) run(k_m2l_fp64<R, true>);
+    else run(k_m2l_fp64<R, false>);
+  };
+  if (nl <= 32) pick(std::integral_constant<int, 1>{});
+  else if (nl <= 96) pick(std::integral_constant<int, 3>{});
+  else if (nl <= 160) pick(std::integral_constant<int, 5>{});
+  else if (nl <= 256) pick(std::integral_constant<int, 8>{});
+  else pick(std::integral_constant<int, 16>{});
 }
 
 }  // namespace aran
