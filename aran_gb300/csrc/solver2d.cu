@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(128) k2_m2l(int nn, int p, const int *__restri
         if (i > p) break;
         const double *row = tab + i * SP;
         zd sum = cmake(0.0, 0.0);
-        for (int j = 1; j < p; ++j) {
+        for (int j = p - 1; j >= 1; --j) {      // small terms first, as in Horner's rule
           sum.re = fma(row[j], ms[j].re, sum.re);
           sum.im = fma(row[j], ms[j].im, sum.im);
         }
