@@ -359,14 +359,16 @@ __global__ void k2_leaf_ranges(int nn, int n, const int *__restrict__ begin, con
 }
 
 // near leaf-ordinal ranges of leaf L; mode 0 counts (zero for the ordinals from
-// the last leaf up to nbound), mode 1 writes
+// the last leaf up to nbound; over: particles of the largest leaf above the
+// capacity), mode 1 writes
 __global__ void k2_near(int nbound, const int *__restrict__ nleaves_p,
                         const int *__restrict__ leaf_node, const int *__restrict__ begin,
                         const int *__restrict__ end, const int *__restrict__ child,
                         const int *__restrict__ parent, const int *__restrict__ col,
                         const int *__restrict__ ncol, const int *__restrict__ lf_begin,
                         const int *__restrict__ lf_end, int *__restrict__ near_cnt,
-                        const int *__restrict__ near_off, int2 *__restrict__ near_rng, int mode) {
+                        const int *__restrict__ near_off, int2 *__restrict__ near_rng, int maxbox,
+                        int *__restrict__ over, int mode) {
   int L = blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= nbound) return;
   if (L >= *nleaves_p) {
@@ -374,6 +376,7 @@ __global__ void k2_near(int nbound, const int *__restrict__ nleaves_p,
     return;
   }
   int node = leaf_node[L];
+  if (!mode && end[node] - begin[node] > maxbox) atomicMax(over, end[node] - begin[node]);
   int k = 0;
   int w = mode ? near_off[L] : 0;
   for (int j = 0; j < ncol[node]; ++j) {
@@ -628,7 +631,7 @@ __global__ void __launch_bounds__(128) k2_p2p(int nleaves, const int *__restrict
   const int L = blockIdx.x;
   const int b = leaf_be[L], nt = leaf_be[L + 1] - b;
   const int r0 = near_off[L], r1 = near_off[L + 1];
-  for (int tb = 0; tb < nt; tb += 128) {
+  for (int tb = blockIdx.y * 128; tb < nt; tb += 128 * gridDim.y) {
     const int rem = min(nt - tb, 128);
     const int s = 128 / rem;                  // threads per target
     const int ti = threadIdx.x / s, sub = threadIdx.x - ti * s;
@@ -980,7 +983,7 @@ __global__ void __launch_bounds__(T, T == 32 ? 32 : 1280 / T) k2f_p2p(int nleave
   const float clx = (float)(cx - (double)chx), cly = (float)(cy - (double)chy);
   const double hh = node_size2(sysbox, sysn[node], depth[node]);
   const float thr2 = (float)(hh * hh / 64.0);
-  for (int tb = 0; tb < nt; tb += T) {
+  for (int tb = blockIdx.y * T; tb < nt; tb += T * gridDim.y) {
     const int rem = min(nt - tb, T);
     const int S = T / rem;                      // threads per target
     const int sub = threadIdx.x / rem, ti = threadIdx.x - sub * rem;
@@ -1184,7 +1187,8 @@ struct AranGpuSolver2d {
   aran::DBuf<double> sysbox;
   aran::DBuf<uint64_t> keys_in, keys_out;
   aran::DBuf<int> idx_in, perm, incl, flags;
-  aran::DBuf<int> err2;   // input checks of the key pass
+  aran::DBuf<int> err2;   // input checks of the key pass, largest leaf above the capacity
+  int max_leaf = 0;       // no leaf holds more particles
   aran::DBuf<int> internal;   // places and parents of the internal nodes
   int *h_small = nullptr;     // pinned host words for the readbacks
   aran::DBuf<uint8_t> cub_tmp;
@@ -1386,8 +1390,8 @@ void build_forest(AranGpuSolver2d *s, int nsys, const double *dxy, const double 
   s->keys_out.reserve(n);
   s->idx_in.reserve(n);
   s->perm.reserve(n);
-  s->err2.reserve(1);
-  ACHECK(cudaMemsetAsync(s->err2.ptr, 0, sizeof(int), st));
+  s->err2.reserve(2);
+  ACHECK(cudaMemsetAsync(s->err2.ptr, 0, 2 * sizeof(int), st));
   k2_keys<<<ceil_div(n, TB), TB, 0, st>>>(n, nsys, s->offs.ptr, s->sysbox.ptr, dxy, dq,
                                            s->keys_in.ptr, s->idx_in.ptr, s->err2.ptr);
   s->launches++;
@@ -1468,7 +1472,7 @@ void build_lists2(AranGpuSolver2d *s) {
     k2_near<<<ceil_div(nlb, TB), TB, 0, st>>>(
         nlb, nleaves_p, s->leaf_node.ptr, s->begin.ptr, s->end.ptr, s->child.ptr, s->parent.ptr,
         s->col.ptr, s->ncol.ptr, s->lf_begin.ptr, s->lf_end.ptr, s->flags.ptr, s->near_off.ptr,
-        s->near_rng.ptr, mode);
+        s->near_rng.ptr, s->cfg.maxbox, s->err2.ptr + 1, mode);
     ACHECK(cudaGetLastError());
     s->launches++;
   };
@@ -1479,10 +1483,12 @@ void build_lists2(AranGpuSolver2d *s) {
   ACHECK(cudaMemcpyAsync(hb, s->far_off.ptr + nn, sizeof(int), cudaMemcpyDeviceToHost, st));
   ACHECK(cudaMemcpyAsync(hb + 1, nleaves_p, sizeof(int), cudaMemcpyDeviceToHost, st));
   ACHECK(cudaMemcpyAsync(hb + 2, s->near_off.ptr + nlb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ACHECK(cudaMemcpyAsync(hb + 3, s->err2.ptr + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
   ACHECK(cudaStreamSynchronize(st));
   s->nfar = hb[0];
   s->nleaves = hb[1];
   s->nrng = hb[2];
+  s->max_leaf = std::max(s->cfg.maxbox, hb[3]);
   s->far_src.reserve(s->nfar + 1);
   k2_far<<<ceil_div(nn, TB), TB, 0, st>>>(nn, s->begin.ptr, s->end.ptr, s->child.ptr, s->parent.ptr,
                                            s->ij.ptr, s->col.ptr, s->ncol.ptr, nullptr, s->far_off.ptr,
@@ -1491,6 +1497,13 @@ void build_lists2(AranGpuSolver2d *s) {
   s->near_rng.reserve(s->nrng + 1);
   near(1);
   ACHECK(cudaEventRecord(s->ev[2 * Stage::LISTS + 1], st));
+}
+
+// blocks for a leaf: several for leaves above the capacity, as in 3D (leaf_tiles in
+// p2p.cu).  6,000 points within 1e-8, capacity 8: mixed 6 ms, 357 with one block of 32
+// threads (327 with a warp per leaf before), FP64 12 ms, 173
+int leaf_tiles2(const AranGpuSolver2d *s, int T) {
+  return std::min({ceil_div(s->max_leaf, T), 2048 / T, 1 + 100000 / s->nleaves});
 }
 
 void run_passes2_mixed(AranGpuSolver2d *s, double *dacc) {
@@ -1511,7 +1524,7 @@ void run_passes2_mixed(AranGpuSolver2d *s, double *dacc) {
   // occupancy of the batch: a system's bits do not depend on its company.)
   const int T = s->cfg.maxbox <= 64 ? 32 : 128;
   auto p2p = T == 32 ? k2f_p2p<32> : k2f_p2p<128>;
-  p2p<<<nl, T, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr,
+  p2p<<<dim3(nl, leaf_tiles2(s, T)), T, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr,
                                  s->leaf_node.ptr, s->nsys_.ptr, s->depth.ptr, s->sysbox.ptr,
                                  s->center.ptr, s->sx.ptr, s->sy.ptr, s->sq.ptr, s->hl.ptr,
                                  s->near_acc.ptr);
@@ -1582,7 +1595,7 @@ void run_passes2(AranGpuSolver2d *s, double *dacc) {
   ACHECK(cudaEventRecord(s->ev_lists, st));
   ACHECK(cudaStreamWaitEvent(s1, s->ev_lists, 0));
   ACHECK(cudaEventRecord(s->ev[2 * Stage::P2P], s1));
-  k2_p2p<<<nl, 128, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr, s->sx.ptr,
+  k2_p2p<<<dim3(nl, leaf_tiles2(s, 128)), 128, 0, s1>>>(nl, s->leaf_be.ptr, s->near_off.ptr, s->near_rng.ptr, s->sx.ptr,
                              s->sy.ptr, s->sq.ptr, s->near_acc.ptr);
   ACHECK(cudaGetLastError());
   s->launches++;

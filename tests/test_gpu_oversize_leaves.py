@@ -57,3 +57,36 @@ def test_time_at_small_capacities(aran):
                 t.append(s.timings()["p2p"])
         ms[maxbox] = min(t)
     assert ms[16] < 1.5 * ms[64], ms
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [9, 32, 33, 128, 129, 700, 4200])
+def test_2d_against_the_direct_sum(aran, oracle, n, precision):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-0.9, -0.1, (n + 1, 2))
+    x[n] = 0.8
+    q = rng.uniform(-1.0, 1.0, n + 1)
+    z = x[:, 0] + 1j * x[:, 1]
+    d = z[:, None] - z[None]
+    np.fill_diagonal(d, np.inf)
+    with aran.Solver2d(maxbox=8, order=8, precision=precision, max_depth=1) as s:
+        a = s.solve(x, q)
+    if precision == "mixed":   # a pair: offset and reciprocal, as in 3D
+        assert np.all(np.abs(a - (q / d).sum(1)) <= 2e-6 * np.abs(q / d).sum(1))
+    else:
+        ref = oracle.direct2d(x, q)
+        assert np.linalg.norm(a - ref) < 1e-12 * np.linalg.norm(ref)
+
+
+def test_2d_time_at_small_capacities(aran):
+    x = np.random.default_rng(2).uniform(-0.9, -0.1, (6000, 2))
+    q = np.ones(len(x))
+    ms = {}
+    for maxbox in (8, 200):
+        with aran.Solver2d(maxbox=maxbox, order=8, precision="mixed", max_depth=1) as s:
+            t = []
+            for _ in range(4):
+                s.solve(x, q)
+                t.append(s.timings()["p2p"])
+        ms[maxbox] = min(t)
+    assert ms[8] < 1.5 * ms[200], ms
