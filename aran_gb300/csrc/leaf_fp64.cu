@@ -19,7 +19,7 @@ __device__ __forceinline__ double leaf_inv_scale(int depth, double scale_e) {
 // leaf's sum is the sum of its segments in order (k_p2m64_sum), each added up
 // particle by particle: what else is solved, and with it the leaf's place among the
 // sorted particles, does not change its bits.  A warp takes the segments that start
-// in its kSpan places, 32 particles at a time whatever segments they lie in (a
+// in its span of places, 32 particles at a time whatever segments they lie in (a
 // warp per leaf keeps as many lanes busy as the leaf has points).  A lane makes
 // its particle's q S_l^m in m-major order (six operations a coefficient) into
 // shared memory; every 32 values the lanes turn to the values, a lane one of them,
@@ -28,13 +28,14 @@ __device__ __forceinline__ double leaf_inv_scale(int depth, double scale_e) {
 // others to a workspace, at the window of 32 places in which they start: no two start
 // in one.  With few segments (segs > 0) a warp takes one, segment u mod segs of leaf
 // u / segs: fewer rounds in turn, and few CTAs, which stay clear of the near
-// field's.  200k Plummer particles (18 a leaf), order 12: 0.48 ms, 1.44 with a warp per
-// leaf and shuffles (0.34 with parts of leaves added as they come; the solve 38.1
-// ms either way); 3k particles (order 12) 0.045 ms.
-constexpr int kSpan = 32, kFewSegs = 4096;
+// field's.  Order 12, Plummer particles: 200k (18 a leaf) 0.43 ms, 0.48 with spans of 32,
+// 1.44 with a warp per leaf and shuffles (0.34 with parts of leaves added as they come;
+// the solve 38.1 ms either way); 4M 7.1 and 8.2 ms; 3k 0.045 ms.
+constexpr int kFewSegs = 4096;
 
 __global__ void __launch_bounds__(32 * kWarps)
-    k_p2m64(int64_t n, int nleaves, int segs, const int *__restrict__ win_leaf,
+    k_p2m64(int64_t n, int nleaves, int segs, int span,
+            const int *__restrict__ win_leaf,
             const int2 *__restrict__ leaf_be, const int *__restrict__ leaf_node,
             const uint8_t *__restrict__ depth, const real4<double> *__restrict__ rel, int p,
             const double *__restrict__ rec_g, const double *__restrict__ p2mf_g, double scale_e,
@@ -84,8 +85,8 @@ __global__ void __launch_bounds__(32 * kWarps)
     stop = min(base + 32, be.y);
   } else {
     int L1;
-    base = segment_from(kSpan * u, L0);
-    stop = segment_from(kSpan * (u + 1), L1);
+    base = segment_from(span * u, L0);
+    stop = segment_from(span * (u + 1), L1);
   }
   bool goes_on = false;                    // its segment began in a round before
   for (; base < stop; base += 32) {
@@ -314,10 +315,11 @@ void launch_p2m64(AranGpuSolver3d *s, cudaStream_t st) {
   // few segments: a warp each, in few CTAs, which stay clear of the near field's
   const int per_leaf = ceil_div(t.max_leaf, 32);
   const bool few = t.nleaves * (int64_t)per_leaf <= kFewSegs;
-  const int64_t warps = few ? t.nleaves * (int64_t)per_leaf : ceil_div(t.n, kSpan);
+  const int span = t.n < 150000 ? 32 : 128;   // 100k particles 0.28 ms, 0.29 with 128
+  const int64_t warps = few ? t.nleaves * (int64_t)per_leaf : ceil_div(t.n, span);
   k_p2m64<<<ceil_div(warps, kWarps), 32 * kWarps, sm, st>>>(
-      t.n, t.nleaves, few ? per_leaf : 0, t.win_leaf.ptr, t.leaf_be.ptr, t.leaf_node.ptr, t.depth.ptr,
-      s->rel64.ptr, p, tb.rec.ptr, tb.p2mf.ptr, s->scale_e, s->mult64.ptr, s->m2l_part64.ptr);
+      t.n, t.nleaves, few ? per_leaf : 0, span, t.win_leaf.ptr, t.leaf_be.ptr, t.leaf_node.ptr,
+      t.depth.ptr, s->rel64.ptr, p, tb.rec.ptr, tb.p2mf.ptr, s->scale_e, s->mult64.ptr, s->m2l_part64.ptr);
   ACHECK(cudaGetLastError());
   s->launches++;
   if (t.max_leaf > 32) {
