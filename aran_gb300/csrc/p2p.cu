@@ -8,16 +8,16 @@
 // instead of the symmetric update).
 //
 // Work decomposition: a block per target leaf (k_p2p_tile in mixed precision,
-// k_p2p64 in FP64).  Near ranges of more than kBigRange
-// points (a coarse leaf next to a deep subtree, common in clustered sets) are
-// cut into leaf-aligned chunks processed by extra blocks that accumulate
+// k_p2p64 in FP64), several for a leaf above the capacity.  Near ranges of more than
+// kBigRange points (a coarse leaf next to a deep subtree, common in clustered
+// sets) are cut into leaf-aligned chunks processed by extra blocks that accumulate
 // atomically.
 //
-// Mixed precision: positions are FP32 relative to their leaf centre, the
-// centre difference comes from FP32 hi+lo centre pairs, per-source-leaf FP32
-// partial sums go into FP64 accumulators, and pairs closer than 1/8 of the
-// target leaf size (where FP32 cancellation would show) are recomputed from
-// the FP64 positions.
+// Mixed precision: a source's offset from the target leaf's centre comes from
+// FP32 hi + lo positions in the box, short runs of FP32 terms go into Kahan sums
+// and those into the FP64 accumulators, and pairs closer than 1/8 of the target
+// leaf size (where FP32 cancellation would show) are made from the FP64
+// positions.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -241,11 +241,11 @@ __global__ void __launch_bounds__(128, 8) k_p2p64(
 // two pairs; about two thirds of the instructions are the pair loop's.
 // Measured on GB300 against a warp per leaf with 1 to 32 lanes per target (in
 // powers of two), sources staged leaf by leaf and pairs taken singly: 300k
-// blobs (leaf 64) 0.45 ms, 1.08 before; 4M Plummer 3.9 ms, 5.2; 10k uniform
-// (leaf 20, potential) 0.02 ms, 0.09; heavy chunks of a 2M Plummer set 0.36
-// ms, 0.94.  T = 64, 96 and 256 took 0.68, 0.70 and 0.66 ms on the blobs
-// where 128 took 0.61; tiles of twice and four times the sources changed
-// nothing; 10 blocks an SM with 48 registers a thread beat 8, 6 and 12.
+// blobs (leaf 64) 0.48 ms, 1.08 before; 4M Plummer 3.7 ms, 5.2; 10k uniform
+// (leaf 20, potential) 0.02 ms, 0.09.  With one run a tile T = 64, 96 and 256 took
+// 0.68, 0.70 and 0.66 ms on the blobs where 128 took 0.61; tiles of twice and four
+// times the sources changed nothing; 10 blocks an SM with 48 registers a thread beat
+// 8, 6 and 12.
 constexpr int kP2pRanges = 32;   // near ranges taken together
 
 template <bool FIELD, bool BIG, int T>

@@ -108,8 +108,8 @@ int check_config(const AranGpuConfig3d *c) {
     return fail(ARAN_ERR_INVALID, "unknown precision");
   if (c->max_depth < 0 || c->max_depth > kKeyBits)
     return fail(ARAN_ERR_INVALID, "max_depth must be in [0, 21]");
-  // mixed-precision kkylin takes orders up to 16 (its recurrences' factors
-  // leave the FP32 range above)
+  // mixed-precision kkylin takes orders up to 16: the limit of the flavour's own
+  // recurrences in FP32, kept although the rotation kernels do not need it
   if (c->flavour == ARAN_FLAVOUR_KKYLIN && c->precision == ARAN_PRECISION_MIXED && c->order > 16)
     return fail(ARAN_ERR_INVALID, "mixed-precision kkylin takes orders up to 16");
   return ARAN_OK;

@@ -35,7 +35,8 @@ extern "C" {
 
 /* M2M/M2L/L2L flavours: aran_development3d_{m2l,m2l_kkylin,m2l_rotate}
  * (aran/arandevelopment3d.c:306-313,362-369,423-430).  NORMAL and
- * KKYLIN apply the same operators as ROTATE and run its kernels. */
+ * KKYLIN apply the same operators as ROTATE and run its kernels; mixed
+ * KKYLIN solves take orders up to 16 and have no FP64 root levels. */
 #define ARAN_FLAVOUR_NORMAL 0
 #define ARAN_FLAVOUR_KKYLIN 1
 #define ARAN_FLAVOUR_ROTATE 2
@@ -104,13 +105,13 @@ int aran_gpu_solver3d_solve_forest (AranGpuSolver3d *s, int nsys, const int64_t 
                                     double *pot, double *field, int mem);
 
 /* M2L kernel of the FP32 part of mixed solves (rotation flavours):
- * ARAN_M2L_AUTO: the lane-parallel kernel at orders 4, 8 and 12, else the
+ * ARAN_M2L_AUTO: the lane-parallel kernel at even orders 4 to 16, else the
  * sibling kernel with the library's table slots and parents per CTA;
  * ARAN_M2L_LANES / ARAN_M2L_SIBLING: that kernel (nst table slots in {1, 2,
  * 3} and g parents per CTA in {1, 2}; 0 and 0 = the library's choice);
  * ARAN_M2L_TENSOR: the tcgen05 kernel at orders 8 and 12 (TF32 products with
  * a hi/lo split, the accumulator drained into FP32 registers per offset;
- * about twice the FP32 kernels' rounding error, 5e-7 against 3e-7 relative
+ * about twice the FP32 kernels' rounding error, 5e-7 against 2e-7 relative
  * at order 12).  Where the chosen kernel does not
  * serve the order the next one in the order tensor, lanes, sibling does.
  * Without a call, $ARAN_M2L_KERNEL ("lanes", "sibling", "tc") picks. */
