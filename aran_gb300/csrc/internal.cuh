@@ -112,8 +112,6 @@ struct DevTree {
   DBuf<int> leaf_node;                // leaf ordinal -> node
   DBuf<int> win_leaf;                 // leaf of particle 32 w (windows of 32 particles)
   DBuf<int> near_off, near_rng;       // CSR over leaves of [lf_a, lf_b) ranges (2 ints)
-  DBuf<int> m2l_targets;              // nodes with non-empty far lists
-  int n_m2l_targets = 0;
   DBuf<int2> leaf_be;                 // particle [begin, end) per leaf ordinal
   DBuf<float4> leaf_chi, leaf_clo;    // FP32 leaf centre in the box, hi + lo; chi.w = close-pair r^2
   DBuf<int4> big_items;               // (leaf, lf_a, lf_b, 0): chunks of heavy near ranges

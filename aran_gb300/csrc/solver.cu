@@ -188,7 +188,6 @@ void aran_gpu_solver3d_destroy(AranGpuSolver3d *s) {
   t.lf_begin.release(); t.lf_end.release(); t.far_off.release(); t.far_src.release();
   t.far_dir.release(); t.leaf_node.release(); t.win_leaf.release(); t.near_off.release();
   t.near_rng.release();
-  t.m2l_targets.release();
   for (auto *tb : {&s->t64}) {
     tb->rec.release(); tb->p2mf.release(); tb->vt.release(); tb->vm.release(); tb->vl.release();
     tb->gz.release(); tb->gm.release(); tb->dir_m2l.release(); tb->dir_m2m.release();
